@@ -15,6 +15,7 @@
 #include "engine_impl.cuh"
 #include "one_e.cuh"
 #include "siblings.h"
+#include "_gen/boys_tables.cuh"
 
 static const char *kLetters = "spdfg";
 static char g_class_names[55][16];
@@ -29,23 +30,6 @@ static double md_v1_prim_flops(int la, int lb, int lc, int ld) {
 }
 static double md_v1_digest_flops(int la, int lb, int lc, int ld) {
   return 24.0 * nfun(la) * nfun(lb) * nfun(lc) * nfun(ld);
-}
-
-static double host_boys_row(int nmax, long double T, double *F) {
-  long double term = 1.0L / (2 * nmax + 1), sum = term;
-  for (int k = 1; k < 2000; k++) {
-    term *= 2.0L * T / (2 * nmax + 2 * k + 1);
-    sum += term;
-    if (term < sum * 1e-22L) break;
-  }
-  long double ex = expl(-T);
-  long double f = ex * sum;
-  F[nmax] = (double)f;
-  for (int m = nmax - 1; m >= 0; m--) {
-    f = (2.0L * T * f + ex) / (2 * m + 1);
-    F[m] = (double)f;
-  }
-  return 0;
 }
 
 // Primitive pairs of shell pair (a, b); prim_thresh = 0 keeps all of them, otherwise a
@@ -402,15 +386,14 @@ cqg_status cqg_create(cqg_ctx **out, int device) {
     delete ctx;
     return CQG_ERR_CUDA;
   }
-  // Boys table
-  std::vector<double> tab(BOYS_TABLE_SIZE);
-  for (int i = 0; i < BOYS_NT; ++i) host_boys_row(BOYS_NORD - 1, (long double)i / 10.0L, &tab[i * BOYS_NORD]);
-  for (int i = 0; i < BOYS_NT; ++i) tab[BOYS_NT * BOYS_NORD + i] = (double)expl(-(long double)i / 10.0L);
-  if (ctx->d_boys.reserve(tab.size()) != cudaSuccess ||
-      cudaMemcpy(ctx->d_boys.p, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) {
+  // the Boys tables are constants of the module: nothing to compute, allocate or upload
+  void *boys = nullptr, *rows = nullptr;
+  if (cudaGetSymbolAddress(&boys, kBoysTable) != cudaSuccess || cudaGetSymbolAddress(&rows, kBoysRows) != cudaSuccess) {
     delete ctx;
     return CQG_ERR_CUDA;
   }
+  ctx->boys = (const double *)boys;
+  ctx->boys_rows = (const double *)rows;
   for (int i = 0; i < 4 + 2 * CQG_NQC + 2; ++i) cudaEventCreate(&ctx->ev[i]);
   for (int k = 0; k < CQG_NQC; ++k) ctx->sibling_min[k] = default_sibling_min(k);
   ctx->events = true;
@@ -429,7 +412,7 @@ cqg_status cqg_destroy(cqg_ctx *ctx) {
   ctx->d_coef.release(); ctx->d_allpairs.release(); ctx->d_oe.release(); ctx->d_charges.release();
   ctx->d_shmol.release(); ctx->d_mshoff.release(); ctx->d_mnsh.release(); ctx->d_mnbf.release();
   ctx->d_molbk.release(); ctx->d_mxoff.release(); ctx->d_mMoff.release(); ctx->d_active.release();
-  ctx->d_prim.release(); ctx->d_boys.release();
+  ctx->d_prim.release();
   ctx->d_M.release(); ctx->d_Mmax.release(); ctx->d_Mpair.release(); ctx->d_flags.release();
   ctx->d_cnt.release(); ctx->d_off.release(); ctx->d_range.release(); ctx->d_scan_tmp.release();
   ctx->d_qhead.release();
@@ -1479,7 +1462,7 @@ cqg_status cqg_one_e(cqg_ctx *ctx, int ncharge, const double *Z, const double *R
   OneEMols om;
   memset(&om, 0, sizeof(om));
   k_one_e<<<(unsigned)((np + 63) / 64), 64, 0, st>>>(sh, ctx->d_allpairs.p, np, ncharge, ctx->d_charges.p,
-                                                     (const double3 *)(ctx->d_charges.p + ncharge), ctx->d_boys.p, dS,
+                                                     (const double3 *)(ctx->d_charges.p + ncharge), ctx->boys, dS,
                                                      dT, dV, ldd, om);
   CUCHK(cudaGetLastError());
   if (!on_device) {
@@ -1576,7 +1559,7 @@ cqg_status cqg_one_e_batch(cqg_ctx *ctx, const int *ncharge_per_mol, const doubl
   om.batch = 1;
   const long long np = ctx->nallpairs;
   k_one_e<<<(unsigned)((np + 63) / 64), 64, 0, st>>>(sh, ctx->d_allpairs.p, np, nc, ctx->d_charges.p,
-                                                     (const double3 *)(ctx->d_charges.p + nc), ctx->d_boys.p, S, T,
+                                                     (const double3 *)(ctx->d_charges.p + nc), ctx->boys, S, T,
                                                      V, 0, om);
   CUCHK(cudaGetLastError());
   return CQG_OK;
@@ -1884,7 +1867,7 @@ cqg_status cqg_one_e_noalloc(cqg_ctx *ctx, int ncharge, const double *Z, const d
   memset(&om, 0, sizeof(om));
   const long long np = ctx->nallpairs;
   k_one_e<<<(unsigned)((np + 63) / 64), 64, 0, st>>>(sh, ctx->d_allpairs.p, np, ncharge, tab,
-                                                     (const double3 *)(tab + ncharge), ctx->d_boys.p, S, T, V, ld,
+                                                     (const double3 *)(tab + ncharge), ctx->boys, S, T, V, ld,
                                                      om);
   CUCHK(cudaGetLastError());
   return CQG_OK;

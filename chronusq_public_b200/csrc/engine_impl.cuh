@@ -8,6 +8,7 @@
 #include <cub/device/device_scan.cuh>
 
 #include <algorithm>
+#include <atomic>
 #include <climits>
 #include <cmath>
 #include <cstdio>
@@ -169,8 +170,8 @@ __device__ __forceinline__ void mol_view(const DigestGroups &dg, int g, int m, c
 template <int LA, int LB>
 __global__ void __launch_bounds__(128) k_schwarz(Pairs P, Shells S, const double *__restrict__ boys_g,
                                                  int beg, int end, double *__restrict__ Qout) {
-  __shared__ __align__(16) double boys[BOYS_NT * BOYS_SROW];
-  stage_boys<2 * (LA + LB)>(boys_g, boys);
+  __shared__ __align__(16) double boys[BOYS_ROWS_SIZE];
+  load_boys<2 * (LA + LB)>(boys_g, boys);
   __syncthreads();
   int i = beg + blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= end) return;
@@ -861,8 +862,8 @@ __device__ __forceinline__ void eri_jk_list(const uint2 *__restrict__ ql, const 
                                             const Pairs &P, const Shells &S, const double *__restrict__ boys_g,
                                             const DigestGroups &dg, unsigned long long *__restrict__ qhead,
                                             int chunk) {
-  __shared__ __align__(16) double boys[BOYS_NT * BOYS_SROW];
-  stage_boys<LA + LB + LC + LD>(boys_g, boys);
+  __shared__ __align__(16) double boys[BOYS_ROWS_SIZE];
+  load_boys<LA + LB + LC + LD>(boys_g, boys);
   __syncthreads();
   const long long beg = range[2 * blk], end = range[2 * blk + 1];
   const int lane = threadIdx.x & 31;
@@ -1010,8 +1011,8 @@ template <int LA, int LB, int LC, int LD, typename T, int NT>
 __global__ void __launch_bounds__(NT) k_eri_gc(const uint2 *__restrict__ ql, const long long *__restrict__ range,
                                                 int blk, Pairs P, Shells S, const double *__restrict__ boys_g,
                                                 DigestGroups dg, unsigned long long *__restrict__ qhead, int chunk) {
-  __shared__ __align__(16) double boys[BOYS_NT * BOYS_SROW];
-  stage_boys<LA + LB + LC + LD>(boys_g, boys);
+  __shared__ __align__(16) double boys[BOYS_ROWS_SIZE];
+  load_boys<LA + LB + LC + LD>(boys_g, boys);
   __syncthreads();
   const long long beg = range[2 * blk], end = range[2 * blk + 1];
   const int lane = threadIdx.x & 31;
@@ -1668,7 +1669,8 @@ struct cqg_ctx {
   DevBuf<unsigned long long> d_blkacc;
   int launches = 0;
   DevBuf<PrimPair> d_prim;
-  DevBuf<double> d_boys;
+  const double *boys = nullptr;        // kBoysTable (boys_eval) and kBoysRows (load_boys) on the context's
+  const double *boys_rows = nullptr;   // device: module constants, valid as long as its CUDA context
   long long prim_pairs_total = 0;
   std::vector<int> pair_np_host;
   // per-call scratch
@@ -1752,7 +1754,7 @@ static cudaError_t launch_warp(cqg_ctx *ctx, int blk, long long n, long long sbe
   const int qpw = (!SCHWARZ && ctx->shape_qpw[blk] > 0) ? ctx->shape_qpw[blk] : 1;
   k_eri_jk_warp<LA, LB, LC, LD, SCHWARZ, T><<<blocks, 32 * wpb, smem, st>>>(ctx->d_qlist.p, ctx->d_range.p, blk, sbeg,
                                                                        send, make_pairs(ctx), make_shells(ctx),
-                                                                       ctx->d_boys.p, dg, Q, ctx->d_qhead.p, qpw);
+                                                                       ctx->boys, dg, Q, ctx->d_qhead.p, qpw);
   return cudaGetLastError();
 }
 
@@ -1765,7 +1767,7 @@ static cudaError_t launch_schwarz(cqg_ctx *ctx, Pairs P, Shells S, int beg, int 
     memset(&dg, 0, sizeof(dg));
     return launch_warp<LA, LB, LA, LB, true, double>(ctx, 0, n, beg, end, 0, dg, Q);
   } else {
-    k_schwarz<LA, LB><<<(n + 127) / 128, 128>>>(P, S, ctx->d_boys.p, beg, end, Q);
+    k_schwarz<LA, LB><<<(n + 127) / 128, 128>>>(P, S, ctx->boys_rows, beg, end, Q);
     return cudaGetLastError();
   }
 }
@@ -1820,6 +1822,22 @@ static inline Mols make_mols(cqg_ctx *ctx) {
   return M;
 }
 
+// CTAs of `kernel` (128 threads, static shared memory) resident on one SM: the default grid of
+// the class kernels.  A persistent CTA beyond the resident ones starts only when a first one
+// has drained the queue: it copies its Boys rows and finds no work.  (With the copy
+// of load_boys: 8.59 -> 7.35 ms per (H2O)_11 cc-pVDZ build against twelve CTAs per SM.)  The count belongs to the kernel and the device
+// and is asked for once.
+template <typename K>
+static int resident_ctas(K kernel, int threads, int device, std::atomic<int> (&known)[64]) {
+  const int slot = (device >= 0 && device < 64) ? device : 0;
+  int n = known[slot].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, 0) != cudaSuccess || n < 1) n = 1;
+    known[slot].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
 typedef cudaError_t (*eri_launcher)(cqg_ctx *, int blk, long long n, cudaStream_t st, const DigestGroups &dg);
 
 // One launch of the sibling-group kernel of class (LA LB|LC LD) over list blk: CTAs of 64
@@ -1834,11 +1852,11 @@ static cudaError_t launch_gc(cqg_ctx *ctx, int blk, long long n, cudaStream_t st
   const int chunk = 32 * (ctx->shape_qpw[blk] > 0 ? ctx->shape_qpw[blk] : 1);
   if (nt == 64)
     k_eri_gc<LA, LB, LC, LD, T, 64><<<(unsigned)nb, 64, 0, st>>>(ctx->d_qlist.p, ctx->d_range.p, blk,
-                                                                make_pairs(ctx), make_shells(ctx), ctx->d_boys.p,
+                                                                make_pairs(ctx), make_shells(ctx), ctx->boys_rows,
                                                                 dg, ctx->d_qhead.p, chunk);
   else
     k_eri_gc<LA, LB, LC, LD, T, kEriThreads><<<(unsigned)nb, kEriThreads, 0, st>>>(
-        ctx->d_qlist.p, ctx->d_range.p, blk, make_pairs(ctx), make_shells(ctx), ctx->d_boys.p, dg, ctx->d_qhead.p,
+        ctx->d_qlist.p, ctx->d_range.p, blk, make_pairs(ctx), make_shells(ctx), ctx->boys_rows, dg, ctx->d_qhead.p,
         chunk);
   return cudaGetLastError();
 }
@@ -1858,19 +1876,18 @@ static cudaError_t launch_eri(cqg_ctx *ctx, int blk, long long n, cudaStream_t s
     if constexpr (is_variant_class(LA, LB, LC, LD)) {
       if (ctx->shape_var[blk] == 1) return launch_warp<LA, LB, LC, LD, false, T>(ctx, blk, n, 0, 0, st, dg, nullptr);
     }
-    const int cta = ctx->shape_cta[blk] > 0 ? ctx->shape_cta[blk] : 12;
-    const long long cap = (long long)ctx->nsm * cta;
-    long long nb = n > 0 ? std::min<long long>((n + kEriThreads - 1) / kEriThreads, cap) : cap;
-    const int chunk = 32 * (ctx->shape_qpw[blk] > 0 ? ctx->shape_qpw[blk] : 1);
     constexpr int mb = EriMinBlocks<LA, LB, LC, LD>::v;
-    if constexpr (mb > 0)
-      k_eri_jk_mb<LA, LB, LC, LD, T, mb><<<(unsigned)nb, kEriThreads, 0, st>>>(
-          ctx->d_qlist.p, ctx->d_range.p, blk, make_pairs(ctx), make_shells(ctx), ctx->d_boys.p, dg, ctx->d_qhead.p,
-          chunk);
-    else
-      k_eri_jk<LA, LB, LC, LD, T><<<(unsigned)nb, kEriThreads, 0, st>>>(ctx->d_qlist.p, ctx->d_range.p, blk,
-                                                                     make_pairs(ctx), make_shells(ctx),
-                                                                     ctx->d_boys.p, dg, ctx->d_qhead.p, chunk);
+    auto kernel = [] {
+      if constexpr (mb > 0) return &k_eri_jk_mb<LA, LB, LC, LD, T, mb>;
+      else return &k_eri_jk<LA, LB, LC, LD, T>;
+    }();
+    static std::atomic<int> known[64];
+    const int cta = ctx->shape_cta[blk] > 0 ? ctx->shape_cta[blk] : resident_ctas(kernel, kEriThreads, ctx->device, known);
+    const long long cap = (long long)ctx->nsm * cta;
+    const long long nb = n > 0 ? std::min<long long>((n + kEriThreads - 1) / kEriThreads, cap) : cap;
+    const int chunk = 32 * (ctx->shape_qpw[blk] > 0 ? ctx->shape_qpw[blk] : 1);
+    kernel<<<(unsigned)nb, kEriThreads, 0, st>>>(ctx->d_qlist.p, ctx->d_range.p, blk, make_pairs(ctx), make_shells(ctx),
+                                                 ctx->boys_rows, dg, ctx->d_qhead.p, chunk);
     return cudaGetLastError();
   }
 }

@@ -85,7 +85,7 @@ template <int L>
 __device__ __forceinline__ void restage(int &staged, const double *boys_g, double *boys) {
   if (staged == L) return;   // block-uniform: every thread tracks the same sequence of claims
   __syncthreads();
-  stage_boys<L>(boys_g, boys);
+  load_boys<L>(boys_g, boys);
   __syncthreads();
   staged = L;
 }
@@ -94,7 +94,7 @@ template <int TIER>
 __global__ void __launch_bounds__(kEriThreads, TIER == 1 ? 4 : 2)
     k_eri_fused(const uint2 *__restrict__ ql, const long long *__restrict__ range, Pairs P, Shells S,
                 const double *__restrict__ boys_g, DigestGroups dg, unsigned long long *__restrict__ head) {
-  __shared__ __align__(16) double boys[BOYS_NT * BOYS_SROW];
+  __shared__ __align__(16) double boys[BOYS_ROWS_SIZE];
   __shared__ long long s_beg[kMaxSlots], s_end[kMaxSlots], s_start[kMaxSlots + 1];
   __shared__ unsigned long long s_claim;
   constexpr int NC = TIER == 1 ? kNT1 : kNT2;
@@ -171,9 +171,9 @@ cudaError_t cqg_launch_fused(cqg_ctx *ctx, int tier, cudaStream_t st, const Dige
   const unsigned blocks = (unsigned)(ctx->nsm * per_sm);
   if (tier == 1)
     k_eri_fused<1><<<blocks, kEriThreads, 0, st>>>(ctx->d_qlist.p, ctx->d_range.p, make_pairs(ctx), make_shells(ctx),
-                                                   ctx->d_boys.p, dg, ctx->d_qhead.p + CQG_NLIST);
+                                                   ctx->boys_rows, dg, ctx->d_qhead.p + CQG_NLIST);
   else
     k_eri_fused<2><<<blocks, kEriThreads, 0, st>>>(ctx->d_qlist.p, ctx->d_range.p, make_pairs(ctx), make_shells(ctx),
-                                                   ctx->d_boys.p, dg, ctx->d_qhead.p + CQG_NLIST);
+                                                   ctx->boys_rows, dg, ctx->d_qhead.p + CQG_NLIST);
   return cudaGetLastError();
 }

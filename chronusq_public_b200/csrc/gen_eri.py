@@ -542,6 +542,47 @@ def members_header(specs):
     return "\n".join(parts) + "\n"
 
 
+# The Boys function's table (eri_common.cuh): BOYS_NT points T_i = 0.1 i, orders 0..BOYS_NORD-1.
+BOYS_NT, BOYS_NORD, BOYS_NTAYLOR, BOYS_MAXL = 361, 32, 8, 12
+
+
+def boys_header():
+    """Header text with the Boys tables as constants of the module: kBoysTable (F_n(0.1 i),
+    then exp(-0.1 i)) and kBoysRows (per L = 0..BOYS_MAXL the rows of load_boys).  The highest
+    order comes from its ascending series in extended precision, the lower ones by downward
+    recursion F_m = (2 T F_{m+1} + e^-T) / (2 m + 1)."""
+    ld = np.longdouble
+    T = np.arange(BOYS_NT, dtype=ld) / ld(10)
+    nmax = BOYS_NORD - 1
+    ex = np.exp(-T)
+    term = np.full(BOYS_NT, ld(1) / ld(2 * nmax + 1))
+    tot = term.copy()
+    for k in range(1, 400):
+        term = term * (ld(2) * T / ld(2 * nmax + 2 * k + 1))
+        tot += term
+    F = [None] * BOYS_NORD
+    F[nmax] = ex * tot
+    for m in range(nmax - 1, -1, -1):
+        F[m] = (ld(2) * T * F[m + 1] + ex) / ld(2 * m + 1)
+    F = np.stack(F, 1)                      # [i][n]
+    table = np.concatenate([F.reshape(-1), ex]).astype(np.float64)
+    inv_fact = [ld(1)]
+    for k in range(1, BOYS_NTAYLOR + 1):
+        inv_fact.append(inv_fact[-1] / ld(k))
+    rows = np.concatenate([
+        np.concatenate([F[:, L:L + BOYS_NTAYLOR + 1] * np.array(inv_fact), ex[:, None]], 1).reshape(-1)
+        for L in range(BOYS_MAXL + 1)]).astype(np.float64)
+
+    def array(name, v):
+        body = ",\n".join(", ".join(repr(float(x)) for x in v[k:k + 8]) for k in range(0, len(v), 8))
+        return "__device__ const __align__(16) double %s[%d] = {\n%s};" % (name, len(v), body)
+    return "\n".join([
+        "// GENERATED by gen_eri.py (Boys tables) -- do not edit.", "#pragma once",
+        "static_assert(BOYS_NT == %d && BOYS_NORD == %d && BOYS_NTAYLOR == %d && BOYS_MAXL == %d, \"table layout\");"
+        % (BOYS_NT, BOYS_NORD, BOYS_NTAYLOR, BOYS_MAXL),
+        array("kBoysTable", table), array("kBoysRows", rows), ""])
+
+
 def main(path, maxl=2):
     parts = ["// GENERATED by gen_eri.py -- do not edit.",
              "#pragma once",
@@ -576,6 +617,8 @@ def main(path, maxl=2):
         f.write("\n".join(parts))
     with open(os.path.join(os.path.dirname(os.path.abspath(path)), "eri_gc_classes.cuh"), "w") as f:
         f.write(members_header([q for q in GROUP_SPECS if max(q[:4]) <= maxl]))
+    with open(os.path.join(os.path.dirname(os.path.abspath(path)), "boys_tables.cuh"), "w") as f:
+        f.write(boys_header())
 
 
 if __name__ == "__main__":
