@@ -39,8 +39,10 @@ def test_rows_are_taylor_coefficients(tables, L):
     T = 0.1 * np.arange(g.BOYS_NT)
     fact = np.cumprod([1.0] + [float(k) for k in range(1, nt + 1)])
     assert np.allclose(row[:, :nt + 1] * fact, F[:, L:L + nt + 1], rtol=1e-15, atol=0)
-    assert np.allclose(row[:, nt + 1], np.exp(-T), rtol=1e-15, atol=0)
-    assert np.allclose(table[g.BOYS_NT * g.BOYS_NORD:], np.exp(-T), rtol=1e-15, atol=0)
+    # T = i / 10 exactly: the double nearest 3.6 is off by enough to show in e^-T
+    ex = np.exp(-np.arange(g.BOYS_NT, dtype=np.longdouble) / 10).astype(np.float64)
+    assert np.allclose(row[:, nt + 1], ex, rtol=1e-15, atol=0)
+    assert np.allclose(table[g.BOYS_NT * g.BOYS_NORD:], ex, rtol=1e-15, atol=0)
     # scipy's incomplete gamma function is good to a few 1e-14 relative; F_n(0) = 1 / (2 n + 1)
     for k in (0, nt):
         assert F[0, L + k] == pytest.approx(1.0 / (2 * (L + k) + 1), rel=1e-15)
