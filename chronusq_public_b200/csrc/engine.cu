@@ -13,6 +13,9 @@
 //   4. k_finalize    : AX += 0.5 (Gh + Gh^T)   (the 0.5*scale reduction of contract.h:189-193;
 //                      the scales are folded into the digest).
 #include "engine_impl.cuh"
+
+#include <mutex>
+
 #include "one_e.cuh"
 #include "siblings.h"
 #include "_gen/boys_tables.cuh"
@@ -232,6 +235,64 @@ static cqg_status upload_groups(cqg_ctx *ctx, const std::vector<int> &fam, doubl
   return CQG_OK;
 }
 
+// Side streams are leased to a context for its lifetime.  Making a set takes about 0.5 ms,
+// more than a small molecule's Fock build, so a destroyed context's set is kept for the next
+// context of its device: at most kSideSpare sets per process, the rest are destroyed.
+constexpr size_t kSideSpare = 8;
+static std::mutex g_side_mutex;
+static std::vector<SideStreams *> g_side_spare;
+
+static void destroy_side_streams(SideStreams *s) {
+  if (s->fork) cudaEventDestroy(s->fork);
+  for (int i = 0; i < kSideStreams; ++i) {
+    if (s->done[i]) cudaEventDestroy(s->done[i]);
+    if (s->st[i]) cudaStreamDestroy(s->st[i]);
+  }
+  delete s;
+}
+
+// Leases a set for the context's device (current); false when none can be made (the launches
+// then all go to the caller's stream).
+static bool lease_side_streams(cqg_ctx *ctx) {
+  if (ctx->side) return true;
+  {
+    std::lock_guard<std::mutex> lock(g_side_mutex);
+    for (size_t i = 0; i < g_side_spare.size(); ++i)
+      if (g_side_spare[i]->device == ctx->device) {
+        ctx->side = g_side_spare[i];
+        g_side_spare.erase(g_side_spare.begin() + i);
+        return true;
+      }
+  }
+  SideStreams *s = new SideStreams();
+  s->device = ctx->device;
+  bool ok = cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming) == cudaSuccess;
+  for (int i = 0; ok && i < kSideStreams; ++i)
+    ok = cudaStreamCreateWithFlags(&s->st[i], cudaStreamNonBlocking) == cudaSuccess &&
+         cudaEventCreateWithFlags(&s->done[i], cudaEventDisableTiming) == cudaSuccess;
+  if (!ok) {
+    cudaGetLastError();
+    destroy_side_streams(s);
+    return false;
+  }
+  ctx->side = s;
+  return true;
+}
+
+// The context's buffers are released first (a device-wide wait), so no work of its is left.
+static void return_side_streams(cqg_ctx *ctx) {
+  if (!ctx->side) return;
+  {
+    std::lock_guard<std::mutex> lock(g_side_mutex);
+    if (g_side_spare.size() < kSideSpare) {
+      g_side_spare.push_back(ctx->side);
+      ctx->side = nullptr;
+    }
+  }
+  if (ctx->side) destroy_side_streams(ctx->side);
+  ctx->side = nullptr;
+}
+
 // The active block table: bra-group tasks for the sibling classes, or pair tasks for all.
 static void select_block_table(cqg_ctx *ctx) {
   ctx->bt = ctx->siblings ? ctx->bt_group : ctx->bt_pair;
@@ -395,7 +456,10 @@ cqg_status cqg_create(cqg_ctx **out, int device) {
   ctx->boys = (const double *)boys;
   ctx->boys_rows = (const double *)rows;
   for (int i = 0; i < 4 + 2 * CQG_NQC + 2; ++i) cudaEventCreate(&ctx->ev[i]);
-  for (int k = 0; k < CQG_NQC; ++k) ctx->sibling_min[k] = default_sibling_min(k);
+  for (int k = 0; k < CQG_NQC; ++k) {
+    ctx->sibling_min[k] = default_sibling_min(k);
+    ctx->class_order[k] = k;
+  }
   ctx->events = true;
   cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, device);
   *out = ctx;
@@ -420,6 +484,7 @@ cqg_status cqg_destroy(cqg_ctx *ctx) {
   ctx->d_molgbk.release(); ctx->d_gsz.release(); ctx->d_gpoff.release(); ctx->d_gnp.release(); ctx->d_gwoff.release();
   ctx->d_glead.release(); ctx->d_pair_Qc.release(); ctx->d_gQ.release(); ctx->d_gw.release(); ctx->d_gprim.release();
   ctx->d_qmask.release(); ctx->d_masks.release(); ctx->d_mhead.release(); ctx->d_mslot.release();
+  return_side_streams(ctx);
   if (ctx->events)
     for (int i = 0; i < 4 + 2 * CQG_NQC + 2; ++i) cudaEventDestroy(ctx->ev[i]);
   delete ctx;
@@ -922,6 +987,43 @@ static cqg_status autotune_shapes(cqg_ctx *ctx, const long long *crange, cudaStr
   return CQG_OK;
 }
 
+// The class launches of one contraction, dealt in turn to the caller's stream and the side
+// streams: fork() makes the side streams wait for what the caller's stream holds so far,
+// next() gives the stream of the next launch, join() makes the caller's stream wait for the
+// side streams.  Everything a launch reads was written on the caller's stream before the
+// fork, and later work on that stream comes after the join, so the buffers' lifetimes are
+// those of a single-stream call; under capture the fork and join become graph edges.
+// With one launch, or per-class timing on, the caller's stream takes them all.
+struct ClassStreams {
+  cqg_ctx *ctx;
+  cudaStream_t st;
+  int n;          // side streams in use
+  int at = 0;
+  ClassStreams(cqg_ctx *c, cudaStream_t s, int launches, bool may_lease) : ctx(c), st(s), n(0) {
+    if (launches > 1 && !c->timing && (c->side || (may_lease && lease_side_streams(c))))
+      n = std::min(launches - 1, kSideStreams);
+  }
+  cudaError_t fork() {
+    if (n == 0) return cudaSuccess;
+    cudaError_t e = cudaEventRecord(ctx->side->fork, st);
+    for (int i = 0; i < n && e == cudaSuccess; ++i) e = cudaStreamWaitEvent(ctx->side->st[i], ctx->side->fork, 0);
+    return e;
+  }
+  cudaStream_t next() {
+    const int i = at;
+    at = at == n ? 0 : at + 1;
+    return i == 0 ? st : ctx->side->st[i - 1];
+  }
+  cudaError_t join() {
+    cudaError_t e = cudaSuccess;
+    for (int i = 0; i < n && e == cudaSuccess; ++i) {
+      e = cudaEventRecord(ctx->side->done[i], ctx->side->st[i]);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(st, ctx->side->done[i], 0);
+    }
+    return e;
+  }
+};
+
 // Sync-free contraction for CUDA-graph capture: the quartet list has a fixed capacity,
 // every class kernel reads its range from device memory and runs a persistent grid, and
 // nothing is read back.  Overflow of the capacity and invalid inputs are reported through
@@ -993,18 +1095,30 @@ static cqg_status contract_graph(cqg_ctx *ctx, int ngroups, const double *const 
       return CQG_ERR_CUDA;
     }
   }
-  for (int vb = 0; vb < CQG_NLIST; ++vb) {
-    const int k = vb % CQG_NQC, part = vb / CQG_NQC;
-    if (!ctx->class_possible[k] || class_fused(ctx->fused_tier, vb) || !list_launcher(vb)) continue;
-    if ((part & 1) && ctx->policy != CQG_PREC_MIXED) continue;   // FP32 lists are empty
-    if (part >= 2 && !ctx->bt.grouped[k]) continue;               // no sibling entries
-    cudaError_t e = list_launcher(vb)(ctx, vb, -1, st, dg);
+  std::vector<int> lists;
+  for (int o = 0; o < CQG_NQC; ++o) {
+    const int k = ctx->class_order[o];
+    for (int part = 0; part < kListParts; ++part) {
+      const int vb = part * CQG_NQC + k;
+      if (!ctx->class_possible[k] || class_fused(ctx->fused_tier, vb) || !list_launcher(vb)) continue;
+      if ((part & 1) && ctx->policy != CQG_PREC_MIXED) continue;   // FP32 lists are empty
+      if (part >= 2 && !ctx->bt.grouped[k]) continue;               // no sibling entries
+      lists.push_back(vb);
+    }
+  }
+  // the side streams are leased by now (cqg_set_graph_mode); a capture makes none
+  ClassStreams cs(ctx, st, (int)lists.size(), false);
+  CUCHK(cs.fork());
+  for (int vb : lists) {
+    cudaError_t e = list_launcher(vb)(ctx, vb, -1, cs.next(), dg);
     ++launches;
     if (e != cudaSuccess) {
-      ctx->err = std::string("eri kernel ") + cqg_class_name(k) + ": " + cudaGetErrorString(e);
+      ctx->err = std::string("eri kernel ") + cqg_class_name(vb % CQG_NQC) + ": " + cudaGetErrorString(e);
+      cs.join();
       return CQG_ERR_CUDA;
     }
   }
+  CUCHK(cs.join());
   for (int g = 0; g < ngroups; ++g) {
     dim3 grid((ctx->max_nbf + 31) / 32, (ctx->max_nbf + 31) / 32, ctx->nmol), blk(32, 8);
     k_finalize<<<grid, blk, 0, st>>>(dg.G[g], mols, AXg[g], ldax);
@@ -1153,7 +1267,7 @@ static cqg_status contract_device(cqg_ctx *ctx, int ngroups, const double *const
   memset(ctx->stats.class_ms, 0, sizeof(ctx->stats.class_ms));
   ctx->stats.ms_fused = 0.0;
   ctx->stats.fused_tier = ctx->fused_tier;
-  double mflops = 0, mflops32 = 0;
+  double mflops = 0, mflops32 = 0, class_work[CQG_NQC];
   long long nprimq = 0, nq32 = 0, nquart = 0;
   for (int k = 0; k < CQG_NQC; ++k) {
     // contracted quartets (a sibling-group entry of the list holds several)
@@ -1169,8 +1283,13 @@ static cqg_status contract_device(cqg_ctx *ctx, int ngroups, const double *const
     const double fp = md_v1_prim_flops(la, lb, lc, ld), fd = md_v1_digest_flops(la, lb, lc, ld);
     mflops += (double)hacc[kBlkAcc * b] * fp + (double)n64 * fd;
     mflops32 += (double)hacc[kBlkAcc * b + 2] * fp + (double)n32 * fd;
-    nprimq += (long long)(hacc[kBlkAcc * b + 1] + hacc[kBlkAcc * b + 3]);
+    const unsigned long long nprim = hacc[kBlkAcc * b + 1] + hacc[kBlkAcc * b + 3];
+    nprimq += (long long)nprim;
+    class_work[k] = (double)nprim * fp + (double)(n64 + n32) * fd;
   }
+  // most work first: the long launches start early and the short ones fill their tails
+  std::stable_sort(ctx->class_order, ctx->class_order + CQG_NQC,
+                   [&](int x, int y) { return class_work[x] > class_work[y]; });
   bool first_chunk = true;
   bool timed[CQG_NQC] = {false};
   for (size_t ch = 0; ch + 1 < chunk_vt.size(); ++ch) {
@@ -1226,7 +1345,13 @@ static cqg_status contract_device(cqg_ctx *ctx, int ngroups, const double *const
       if (ctx->timing) CUCHK(cudaEventRecord(ctx->ev[5 + 2 * CQG_NQC], st));
       ctx->launches += 1;
     }
-    for (int k = 0; k < CQG_NQC; ++k) {   // the class's lists: pair entries FP64, FP32, sibling entries FP64, FP32
+    int nlists = 0;
+    for (int vb = 0; vb < CQG_NLIST; ++vb)
+      if (crange[2 * vb + 1] > crange[2 * vb] && !class_fused(ctx->fused_tier, vb)) ++nlists;
+    ClassStreams cs(ctx, st, nlists, true);
+    CUCHK(cs.fork());
+    for (int o = 0; o < CQG_NQC; ++o) {   // the class's lists: pair entries FP64, FP32, sibling entries FP64, FP32
+      const int k = ctx->class_order[o];
       bool any_list = false;
       for (int part = 0; part < kListParts; ++part) {
         const int vb = part * CQG_NQC + k;
@@ -1240,12 +1365,14 @@ static cqg_status contract_device(cqg_ctx *ctx, int ngroups, const double *const
         if (n <= 0 || class_fused(ctx->fused_tier, vb)) continue;
         if (!list_launcher(vb)) {
           ctx->err = std::string("sibling entries for a class without the sibling form: ") + cqg_class_name(k);
+          cs.join();
           return CQG_ERR_STATE;
         }
         ctx->launches += 1;
-        cudaError_t e = list_launcher(vb)(ctx, vb, n, st, dg);
+        cudaError_t e = list_launcher(vb)(ctx, vb, n, cs.next(), dg);
         if (e != cudaSuccess) {
           ctx->err = std::string("eri kernel ") + cqg_class_name(k) + ": " + cudaGetErrorString(e);
+          cs.join();
           return CQG_ERR_CUDA;
         }
       }
@@ -1254,6 +1381,7 @@ static cqg_status contract_device(cqg_ctx *ctx, int ngroups, const double *const
         timed[k] = true;
       }
     }
+    CUCHK(cs.join());
     if (ctx->timing) {   // per-class device time (all lists of the class), summed over chunks
       CUCHK(cudaStreamSynchronize(st));
       for (int k = 0; k < CQG_NQC; ++k) {
@@ -1624,6 +1752,7 @@ cqg_status cqg_set_graph_mode(cqg_ctx *ctx, long long capacity, int max_groups) 
       ctx->graph_capacity = 0;
       return CQG_ERR_OOM;
     }
+    lease_side_streams(ctx);   // ahead of any capture
   }
   return CQG_OK;
 }

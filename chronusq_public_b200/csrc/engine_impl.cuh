@@ -1611,6 +1611,18 @@ struct DevBuf {
   }
 };
 
+// Side streams of the class launches besides the caller's.  One build is 21 launches in
+// double zeta, 55 in triple zeta; in series each waits for the last warp of the one before.
+// With seven side streams the tails overlap: one water in 6-31G(d) 1.53 -> 0.39 ms, O2 UHF
+// cc-pVDZ 3.09 -> 1.12 ms, (H2O)_11 cc-pVDZ 7.3 -> 4.9 ms, (H2O)_5 cc-pVTZ 25.8 -> 21.7 ms;
+// (H2O)_32, whose lists fill the GPU by themselves, within 1 %.
+constexpr int kSideStreams = 7;
+struct SideStreams {
+  int device = 0;
+  cudaStream_t st[kSideStreams] = {};
+  cudaEvent_t done[kSideStreams] = {}, fork = nullptr;
+};
+
 struct cqg_ctx {
   int device = 0;
   std::string err;
@@ -1702,6 +1714,10 @@ struct cqg_ctx {
   DevBuf<unsigned long long> d_mhead;
   DevBuf<long long> d_mslot;
   long long mask_steps_used = 0;      // steps the last count pass asked for
+  SideStreams *side = nullptr;   // leased on first use (ClassStreams in engine.cu)
+  // classes, most work first, as the last uncaptured contraction counted it (a captured one
+  // launches in this order)
+  int class_order[CQG_NQC];
   cudaEvent_t ev[4 + 2 * CQG_NQC + 2];
   bool events = false;
   cqg_stats stats;
