@@ -88,7 +88,10 @@ static cqg_status upload_pairs(cqg_ctx *ctx, double prim_thresh) {
     npr[i] = (int)prim.size() - poff[i];
   }
   ctx->prim_pairs_total = (long long)prim.size();
-  ctx->pair_np_host = npr;
+  for (int c = 0; c < CQG_NPC; ++c) {
+    ctx->pc_np_max[c] = 0;
+    for (int i = ctx->pc_beg[c]; i < ctx->pc_beg[c + 1]; ++i) ctx->pc_np_max[c] = std::max(ctx->pc_np_max[c], npr[i]);
+  }
   if (ctx->d_pair_sh.reserve(np) || ctx->d_pair_Q.reserve(np) || ctx->d_pair_poff.reserve(np) ||
       ctx->d_pair_np.reserve(np) || ctx->d_pair_kk.reserve(np) || ctx->d_prim.reserve(prim.size())) {
     ctx->err = "device allocation for pair data failed";

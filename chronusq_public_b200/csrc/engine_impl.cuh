@@ -838,9 +838,9 @@ __device__ __forceinline__ void digest(const double *v, double deg, int a0, int 
 }
 
 template <int LA, int LB, int LC, int LD, typename T>
-__device__ __forceinline__ void eri_jk_one(const uint2 *__restrict__ ql, long long i, long long wfirst, long long end,
-                                           const Pairs &P, const Shells &S, const double *boys,
-                                           const DigestGroups &dg);
+__device__ __forceinline__ int eri_jk_one(const uint2 *__restrict__ ql, long long i, long long wfirst, long long end,
+                                          const Pairs &P, const Shells &S, const double *boys,
+                                          const DigestGroups &dg, int ls);
 
 // Per-thread class kernel: persistent grid over the class's quartet range; the Boys rows
 // of this class are staged in shared memory once per block.  T is the arithmetic type of
@@ -857,33 +857,61 @@ constexpr int kEriThreads = CQG_ERI_THREADS;
 // quartets (a multiple of 32), each claimed by one warp with an atomic add on the list's
 // head counter qhead[blk] (zeroed before the launch), so warps that drew cheap quartets
 // take more chunks instead of idling at the tail of a static split.
+//
+// A quartet's primitive quartets are a serial chain of its lane (64 x 64 of them for four
+// 1s or 2s shells of oxygen: 0.25 ms), which bounds the launches that do not fill the GPU.
+// So 2^ls lanes share a quartet:
+//  - as many as a list shorter than a quarter of the GPU's lanes leaves for each (the other
+//    classes' launches run beside it), and
+//  - while the warp draws heavy bras, as many as bring a lane's share of bra x heaviest ket
+//    to kLaneWork primitive quartets per quartet the list has for each lane: a longer chain
+//    than that ends before the list does.  The bra is that of the list's first quartet, then
+//    that of the warp's last chunk (lists are sorted heaviest bra first).
+// Sharing has a price, fewer quartets per digest, so longer lists do without.  Measured:
+// one water in 6-31G(d) 390 -> 259 us, O2 UHF cc-pVDZ 1120 -> 282 us, (H2O)_5 6-31G(d) 733 ->
+// 626 us; with every list that leaves a lane idle shared, (H2O)_5 took 819 us.
+struct LaneShare {
+  int lanes;    // lanes the class can have resident on the GPU
+  int nk_max;   // primitive pairs of the class's heaviest ket
+};
+constexpr int kLaneWork = 256;
 template <int LA, int LB, int LC, int LD, typename T>
 __device__ __forceinline__ void eri_jk_list(const uint2 *__restrict__ ql, const long long *__restrict__ range, int blk,
                                             const Pairs &P, const Shells &S, const double *__restrict__ boys_g,
                                             const DigestGroups &dg, unsigned long long *__restrict__ qhead,
-                                            int chunk) {
+                                            int chunk, LaneShare share) {
   __shared__ __align__(16) double boys[BOYS_ROWS_SIZE];
   load_boys<LA + LB + LC + LD>(boys_g, boys);
   __syncthreads();
   const long long beg = range[2 * blk], end = range[2 * blk + 1];
+  if (beg >= end) return;
   const int lane = threadIdx.x & 31;
+  int ls0 = 0;
+  while (ls0 < 5 && ((end - beg) << (ls0 + 3)) <= share.lanes) ++ls0;
+  const int target = (int)min((long long)INT_MAX, kLaneWork * max(1ll, (end - beg) / share.lanes));
+  int nb = P.np[ql[beg].x];
   for (;;) {
+    int ls = ls0;
+    while (ls < 5 && ((nb * share.nk_max) >> ls) > target) ++ls;
+    const int step = 32 >> ls, take = ls ? step : chunk;
     unsigned long long c0 = 0;
-    if (lane == 0) c0 = atomicAdd(qhead + blk, (unsigned long long)chunk);
+    if (lane == 0) c0 = atomicAdd(qhead + blk, (unsigned long long)take);
     c0 = __shfl_sync(0xffffffffu, c0, 0);
     const long long cfirst = beg + (long long)c0;
     if (cfirst >= end) return;   // the whole list is claimed
-    const long long cend = min(cfirst + (long long)chunk, end);
-    for (long long wfirst = cfirst; wfirst < cend; wfirst += 32)
-      eri_jk_one<LA, LB, LC, LD, T>(ql, wfirst + lane, wfirst, cend, P, S, boys, dg);
+    const long long cend = min(cfirst + (long long)take, end);
+    for (long long wfirst = cfirst; wfirst < cend; wfirst += step)
+      nb = eri_jk_one<LA, LB, LC, LD, T>(ql, wfirst + (lane >> ls), wfirst, cend, P, S, boys, dg, ls);
+    nb = __shfl_sync(0xffffffffu, nb, 0);
   }
 }
 
 template <int LA, int LB, int LC, int LD, typename T>
 __global__ void __launch_bounds__(kEriThreads) k_eri_jk(const uint2 *__restrict__ ql, const long long *__restrict__ range,
                                                 int blk, Pairs P, Shells S, const double *__restrict__ boys_g,
-                                                DigestGroups dg, unsigned long long *__restrict__ qhead, int chunk) {
-  eri_jk_list<LA, LB, LC, LD, T>(ql, range, blk, P, S, boys_g, dg, qhead, chunk);
+                                                DigestGroups dg, unsigned long long *__restrict__ qhead, int chunk,
+                                                LaneShare share) {
+  eri_jk_list<LA, LB, LC, LD, T>(ql, range, blk, P, S, boys_g, dg, qhead, chunk, share);
 }
 
 // Classes whose kernel is compiled for MB resident CTAs per SM (launch bounds with a
@@ -907,31 +935,51 @@ template <>
 struct EriMinBlocks<2, 0, 1, 0> {
   static constexpr int v = 3;
 };
+template <>
+struct EriMinBlocks<2, 1, 0, 0> {   // 168 registers, as without the lane sharing of eri_jk_plain (else 242)
+  static constexpr int v = 3;
+};
 
 template <int LA, int LB, int LC, int LD, typename T, int MB>
 __global__ void __launch_bounds__(kEriThreads, MB) k_eri_jk_mb(const uint2 *__restrict__ ql,
                                                        const long long *__restrict__ range, int blk, Pairs P,
                                                        Shells S, const double *__restrict__ boys_g, DigestGroups dg,
-                                                       unsigned long long *__restrict__ qhead, int chunk) {
-  eri_jk_list<LA, LB, LC, LD, T>(ql, range, blk, P, S, boys_g, dg, qhead, chunk);
+                                                       unsigned long long *__restrict__ qhead, int chunk,
+                                                       LaneShare share) {
+  eri_jk_list<LA, LB, LC, LD, T>(ql, range, blk, P, S, boys_g, dg, qhead, chunk, share);
 }
 
-// One list entry (pair quartet) per lane with the class's per-thread code and its digest.
+// One list entry (pair quartet) per 2^ls lanes with the class's per-thread code and its
+// digest.  With ls > 0 the lanes of a quartet take equal parts of its bra and, past the bra's
+// primitive pairs, of its ket, and their integrals are summed before the first of them
+// digests.  Returns the primitive pairs of the lane's bra.
 template <int LA, int LB, int LC, int LD, typename T>
-__device__ __forceinline__ void eri_jk_plain(const uint2 e, const bool valid, const Pairs &P, const Shells &S,
-                                             const double *boys, const DigestGroups &dg) {
+__device__ __forceinline__ int eri_jk_plain(const uint2 e, const bool valid, const Pairs &P, const Shells &S,
+                                            const double *boys, const DigestGroups &dg, int ls) {
   constexpr int NA = nfun_c(LA), NB = nfun_c(LB), NC = nfun_c(LC), ND = nfun_c(LD);
   const int2 ab = P.sh[e.x], cd = P.sh[e.y];
+  const int nb = P.np[e.x], nk = P.np[e.y];
   double v[NA * NB * NC * ND];
   if (valid) {
     const double3 A = S.center[ab.x], B = S.center[ab.y], C = S.center[cd.x], D = S.center[cd.y];
+    const PrimPair *bp = P.prim + P.poff[e.x], *kp = P.prim + P.poff[e.y];
+    int nb1 = nb, nk1 = nk;
+    if (ls) {
+      const int s = threadIdx.x & ((1 << ls) - 1);
+      int lb = 0;   // bra parts 2^lb <= nb, ket parts 2^(ls - lb)
+      while (lb < ls && (2 << lb) <= nb) ++lb;
+      const int lk = ls - lb, sb = s >> lk, sk = s & ((1 << lk) - 1);
+      const int b0 = (nb * sb) >> lb, k0 = (nk * sk) >> lk;
+      nb1 = ((nb * (sb + 1)) >> lb) - b0;
+      nk1 = ((nk * (sk + 1)) >> lk) - k0;
+      bp += b0;
+      kp += k0;
+    }
     if constexpr (sizeof(T) == sizeof(double)) {
-      EriClass<LA, LB, LC, LD>::template run<double>(P.prim + P.poff[e.x], P.np[e.x], P.prim + P.poff[e.y],
-                                                     P.np[e.y], A, B, C, D, boys, v);
+      EriClass<LA, LB, LC, LD>::template run<double>(bp, nb1, kp, nk1, A, B, C, D, boys, v);
     } else {
       T vt[NA * NB * NC * ND];
-      EriClass<LA, LB, LC, LD>::template run<T>(P.prim + P.poff[e.x], P.np[e.x], P.prim + P.poff[e.y], P.np[e.y],
-                                                A, B, C, D, boys, vt);
+      EriClass<LA, LB, LC, LD>::template run<T>(bp, nb1, kp, nk1, A, B, C, D, boys, vt);
 #pragma unroll
       for (int k = 0; k < NA * NB * NC * ND; ++k) v[k] = (double)vt[k];
     }
@@ -939,10 +987,16 @@ __device__ __forceinline__ void eri_jk_plain(const uint2 e, const bool valid, co
 #pragma unroll
     for (int k = 0; k < NA * NB * NC * ND; ++k) v[k] = 0.0;
   }
+  for (int o = (1 << ls) >> 1; o > 0; o >>= 1) {
+#pragma unroll
+    for (int k = 0; k < NA * NB * NC * ND; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+  }
   const unsigned bra0 = __shfl_sync(0xffffffffu, e.x, 0);
   const bool uniform = __all_sync(0xffffffffu, e.x == bra0);
   const double deg = (ab.x == ab.y ? 1.0 : 2.0) * (cd.x == cd.y ? 1.0 : 2.0) * (e.x == e.y ? 1.0 : 2.0);
-  digest<NA, NB, NC, ND>(v, deg, S.bf[ab.x], S.bf[ab.y], S.bf[cd.x], S.bf[cd.y], dg, valid, uniform, S.mol[ab.x]);
+  digest<NA, NB, NC, ND>(v, deg, S.bf[ab.x], S.bf[ab.y], S.bf[cd.x], S.bf[cd.y], dg,
+                         valid && (threadIdx.x & ((1 << ls) - 1)) == 0, uniform, S.mol[ab.x]);
+  return nb;
 }
 
 // One sibling-group entry per lane: the generated sibling form evaluates the MB x MK member
@@ -996,12 +1050,12 @@ __device__ __forceinline__ void eri_jk_group(const uint2 e, const bool valid, co
 }
 
 template <int LA, int LB, int LC, int LD, typename T>
-__device__ __forceinline__ void eri_jk_one(const uint2 *__restrict__ ql, long long i, long long wfirst, long long end,
-                                           const Pairs &P, const Shells &S, const double *boys,
-                                           const DigestGroups &dg) {
+__device__ __forceinline__ int eri_jk_one(const uint2 *__restrict__ ql, long long i, long long wfirst, long long end,
+                                          const Pairs &P, const Shells &S, const double *boys,
+                                          const DigestGroups &dg, int ls) {
   const bool valid = i < end;
   const uint2 e = ql[valid ? i : wfirst];
-  eri_jk_plain<LA, LB, LC, LD, T>(e, valid, P, S, boys, dg);
+  return eri_jk_plain<LA, LB, LC, LD, T>(e, valid, P, S, boys, dg, ls);
 }
 
 // Sibling-group list of class (LA LB|LC LD): the work queue and persistent grid of
@@ -1684,7 +1738,7 @@ struct cqg_ctx {
   const double *boys = nullptr;        // kBoysTable (boys_eval) and kBoysRows (load_boys) on the context's
   const double *boys_rows = nullptr;   // device: module constants, valid as long as its CUDA context
   long long prim_pairs_total = 0;
-  std::vector<int> pair_np_host;
+  int pc_np_max[CQG_NPC] = {0};   // most primitive pairs of a pair, per class
   // per-call scratch
   DevBuf<double> d_M, d_Mmax, d_Mpair;
   DevBuf<int> d_flags;
@@ -1898,12 +1952,15 @@ static cudaError_t launch_eri(cqg_ctx *ctx, int blk, long long n, cudaStream_t s
       else return &k_eri_jk<LA, LB, LC, LD, T>;
     }();
     static std::atomic<int> known[64];
-    const int cta = ctx->shape_cta[blk] > 0 ? ctx->shape_cta[blk] : resident_ctas(kernel, kEriThreads, ctx->device, known);
+    const int resident = resident_ctas(kernel, kEriThreads, ctx->device, known);
+    const LaneShare share = {ctx->nsm * resident * kEriThreads, ctx->pc_np_max[pair_class_c(LC, LD)]};
+    const int cta = ctx->shape_cta[blk] > 0 ? ctx->shape_cta[blk] : resident;
     const long long cap = (long long)ctx->nsm * cta;
-    const long long nb = n > 0 ? std::min<long long>((n + kEriThreads - 1) / kEriThreads, cap) : cap;
+    // up to 32 lanes per quartet (eri_jk_list)
+    const long long nb = n > 0 ? std::min<long long>((32 * n + kEriThreads - 1) / kEriThreads, cap) : cap;
     const int chunk = 32 * (ctx->shape_qpw[blk] > 0 ? ctx->shape_qpw[blk] : 1);
     kernel<<<(unsigned)nb, kEriThreads, 0, st>>>(ctx->d_qlist.p, ctx->d_range.p, blk, make_pairs(ctx), make_shells(ctx),
-                                                 ctx->boys_rows, dg, ctx->d_qhead.p, chunk);
+                                                 ctx->boys_rows, dg, ctx->d_qhead.p, chunk, share);
     return cudaGetLastError();
   }
 }

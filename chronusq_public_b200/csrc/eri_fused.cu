@@ -78,7 +78,7 @@ __device__ __forceinline__ void fused_chunk(const uint2 *__restrict__ ql, long l
                                             const DigestGroups &dg) {
   const int lane = threadIdx.x & 31;
   for (long long wfirst = cfirst + (threadIdx.x & ~31); wfirst < cend; wfirst += blockDim.x)
-    eri_jk_one<LA, LB, LC, LD, T>(ql, wfirst + lane, wfirst, cend, P, S, boys, dg);
+    eri_jk_one<LA, LB, LC, LD, T>(ql, wfirst + lane, wfirst, cend, P, S, boys, dg, 0);
 }
 
 template <int L>
