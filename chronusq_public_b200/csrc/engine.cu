@@ -296,6 +296,20 @@ static void return_side_streams(cqg_ctx *ctx) {
   ctx->side = nullptr;
 }
 
+// The class launches of the one-electron kernels over the context's pairs (sorted by class),
+// dealt to the side streams when the context holds or may lease them.
+static OneEShells make_one_e_shells(const cqg_ctx *ctx) {
+  OneEShells sh;
+  sh.L = ctx->d_shL.p;
+  sh.nprim = ctx->d_shnp.p;
+  sh.poff = ctx->d_shpoff.p;
+  sh.bf = ctx->d_bf.p;
+  sh.alpha = ctx->d_alpha.p;
+  sh.coef = ctx->d_coef.p;
+  sh.center = ctx->d_center.p;
+  return sh;
+}
+
 // The active block table: bra-group tasks for the sibling classes, or pair tasks for all.
 static void select_block_table(cqg_ctx *ctx) {
   ctx->bt = ctx->siblings ? ctx->bt_group : ctx->bt_pair;
@@ -399,6 +413,99 @@ static const eri_launcher *const kEriLaunch = kEriTables.t;      // FP64 class l
 static const eri_launcher *const kEriLaunch32 = kEriTables.t + CQG_NQC;
 static inline eri_launcher list_launcher(int vb) { return kEriTables.t[vb]; }
 
+// The class launches of one contraction, dealt in turn to the caller's stream and the side
+// streams: fork() makes the side streams wait for what the caller's stream holds so far,
+// next() gives the stream of the next launch, join() makes the caller's stream wait for the
+// side streams.  Everything a launch reads was written on the caller's stream before the
+// fork, and later work on that stream comes after the join, so the buffers' lifetimes are
+// those of a single-stream call; under capture the fork and join become graph edges.
+// With one launch, or per-class timing on, the caller's stream takes them all.
+struct ClassStreams {
+  cqg_ctx *ctx;
+  cudaStream_t st;
+  int n;          // side streams in use
+  int at = 0;
+  ClassStreams(cqg_ctx *c, cudaStream_t s, int launches, bool may_lease) : ctx(c), st(s), n(0) {
+    if (launches > 1 && !c->timing && (c->side || (may_lease && lease_side_streams(c))))
+      n = std::min(launches - 1, kSideStreams);
+  }
+  cudaError_t fork() {
+    if (n == 0) return cudaSuccess;
+    cudaError_t e = cudaEventRecord(ctx->side->fork, st);
+    for (int i = 0; i < n && e == cudaSuccess; ++i) e = cudaStreamWaitEvent(ctx->side->st[i], ctx->side->fork, 0);
+    return e;
+  }
+  cudaStream_t next() {
+    const int i = at;
+    at = at == n ? 0 : at + 1;
+    return i == 0 ? st : ctx->side->st[i - 1];
+  }
+  cudaError_t join() {
+    cudaError_t e = cudaSuccess;
+    for (int i = 0; i < n && e == cudaSuccess; ++i) {
+      e = cudaEventRecord(ctx->side->done[i], ctx->side->st[i]);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(st, ctx->side->done[i], 0);
+    }
+    return e;
+  }
+};
+
+// One launch of `kernel` per pair class (LA LB) of the context, most work first (the low
+// angular momenta have the long contractions and most pairs), each a resident grid.
+template <typename Launch>
+static cudaError_t each_pair_class(cqg_ctx *ctx, cudaStream_t st, bool may_lease, Launch launch) {
+  int n = 0;
+  for (int c = 0; c < CQG_NPC; ++c) n += ctx->pc_beg[c + 1] > ctx->pc_beg[c];
+  ClassStreams cs(ctx, st, n, may_lease);
+  cudaError_t e = cs.fork();
+  for (int c = 0; c < CQG_NPC && e == cudaSuccess; ++c) {
+    const long long np = ctx->pc_beg[c + 1] - ctx->pc_beg[c];
+    if (np > 0) e = launch(c, ctx->d_pair_sh.p + ctx->pc_beg[c], np, cs.next());
+  }
+  const cudaError_t j = cs.join();
+  return e != cudaSuccess ? e : j;
+}
+
+template <int LA, int LB>
+static cudaError_t launch_one_e(cqg_ctx *ctx, const int2 *pairs, long long np, cudaStream_t st, int ncharge,
+                                const double *zr, double *S, double *T, double *V, int ld, const OneEMols &om) {
+  static std::atomic<int> known[64];
+  const int resident = resident_ctas(&k_one_e_class<LA, LB>, 32 * OE_WARPS, ctx->device, known);
+  const long long nb = std::min<long long>((np + OE_WARPS - 1) / OE_WARPS, (long long)ctx->nsm * resident);
+  k_one_e_class<LA, LB><<<(unsigned)nb, 32 * OE_WARPS, 0, st>>>(make_one_e_shells(ctx), pairs, np, ncharge, zr,
+                                                                (const double3 *)(zr + ncharge), ctx->boys_rows, S, T,
+                                                                V, ld, om);
+  return cudaGetLastError();
+}
+template <int LA, int LB>
+static cudaError_t launch_dipole(cqg_ctx *ctx, const int2 *pairs, long long np, cudaStream_t st, double3 O, double *D,
+                                 int ld) {
+  const long long nb = std::min<long long>((np + OE_WARPS - 1) / OE_WARPS, 16ll * ctx->nsm);
+  k_dipole_class<LA, LB><<<(unsigned)nb, 32 * OE_WARPS, 0, st>>>(make_one_e_shells(ctx), pairs, np, O, D, ld,
+                                                                 ctx->nbf);
+  return cudaGetLastError();
+}
+#define CQG_PAIR_CLASS_SWITCH(c, F, ...)      \
+  switch (c) {                                \
+    case 0: return F<0, 0>(__VA_ARGS__);      \
+    case 1: return F<1, 0>(__VA_ARGS__);      \
+    case 2: return F<1, 1>(__VA_ARGS__);      \
+    case 3: return F<2, 0>(__VA_ARGS__);      \
+    case 4: return F<2, 1>(__VA_ARGS__);      \
+    case 5: return F<2, 2>(__VA_ARGS__);      \
+    case 6: return F<3, 0>(__VA_ARGS__);      \
+    case 7: return F<3, 1>(__VA_ARGS__);      \
+    case 8: return F<3, 2>(__VA_ARGS__);      \
+    default: return F<3, 3>(__VA_ARGS__);     \
+  }
+// S, T, V of every pair; zr holds the charges, then their positions (3 each)
+static cudaError_t run_one_e(cqg_ctx *ctx, cudaStream_t st, bool may_lease, int ncharge, const double *zr, double *S,
+                             double *T, double *V, int ld, const OneEMols &om) {
+  return each_pair_class(ctx, st, may_lease, [&](int c, const int2 *pairs, long long np, cudaStream_t s) -> cudaError_t {
+    CQG_PAIR_CLASS_SWITCH(c, launch_one_e, ctx, pairs, np, s, ncharge, zr, S, T, V, ld, om)
+  });
+}
+
 extern "C" {
 
 const char *cqg_version(void) { return "cqgpu 0.1 (sm_100a, MD FP64)"; }
@@ -476,7 +583,7 @@ cqg_status cqg_destroy(cqg_ctx *ctx) {
   ctx->d_pair_sh.release(); ctx->d_pair_Q.release(); ctx->d_pair_poff.release(); ctx->d_pair_np.release();
   ctx->d_pair_kk.release(); ctx->d_blkacc.release();
   ctx->d_shL.release(); ctx->d_shnp.release(); ctx->d_shpoff.release(); ctx->d_alpha.release();
-  ctx->d_coef.release(); ctx->d_allpairs.release(); ctx->d_oe.release(); ctx->d_charges.release();
+  ctx->d_coef.release(); ctx->d_oe.release(); ctx->d_charges.release();
   ctx->d_shmol.release(); ctx->d_mshoff.release(); ctx->d_mnsh.release(); ctx->d_mnbf.release();
   ctx->d_molbk.release(); ctx->d_mxoff.release(); ctx->d_mMoff.release(); ctx->d_active.release();
   ctx->d_prim.release();
@@ -624,22 +731,16 @@ cqg_status cqg_set_basis_batch(cqg_ctx *ctx, int nmol, const int *nshell_per_mol
   CUCHK(cudaMemcpy(ctx->d_mMoff.p, ctx->m_Moff.data(), nmol * sizeof(long long), cudaMemcpyHostToDevice));
   ctx->h_active.assign(nmol, 1);
   CUCHK(cudaMemcpy(ctx->d_active.p, ctx->h_active.data(), nmol, cudaMemcpyHostToDevice));
-  // raw shells (one-electron integrals) and the list of all pairs a >= b within each molecule
+  // raw shells (one-electron integrals)
   {
-    std::vector<int2> allp;
-    for (int m = 0; m < nmol; ++m)
-      for (int a = ctx->m_shoff[m]; a < ctx->m_shoff[m] + ctx->m_nsh[m]; ++a)
-        for (int b = ctx->m_shoff[m]; b <= a; ++b) allp.push_back(make_int2(a, b));
-    ctx->nallpairs = (long long)allp.size();
     if (ctx->d_shL.reserve(nshell) || ctx->d_shnp.reserve(nshell) || ctx->d_shpoff.reserve(nshell) ||
-        ctx->d_alpha.reserve(tot) || ctx->d_coef.reserve(tot) || ctx->d_allpairs.reserve(allp.size()))
+        ctx->d_alpha.reserve(tot) || ctx->d_coef.reserve(tot))
       return CQG_ERR_OOM;
     CUCHK(cudaMemcpy(ctx->d_shL.p, L, nshell * sizeof(int), cudaMemcpyHostToDevice));
     CUCHK(cudaMemcpy(ctx->d_shnp.p, nprim, nshell * sizeof(int), cudaMemcpyHostToDevice));
     CUCHK(cudaMemcpy(ctx->d_shpoff.p, ctx->hpoff.data(), nshell * sizeof(int), cudaMemcpyHostToDevice));
     CUCHK(cudaMemcpy(ctx->d_alpha.p, alpha, tot * sizeof(double), cudaMemcpyHostToDevice));
     CUCHK(cudaMemcpy(ctx->d_coef.p, coef, tot * sizeof(double), cudaMemcpyHostToDevice));
-    CUCHK(cudaMemcpy(ctx->d_allpairs.p, allp.data(), allp.size() * sizeof(int2), cudaMemcpyHostToDevice));
   }
   // pairs within each molecule, by class, internal orientation L_a >= L_b (a >= b when equal L)
   std::vector<std::vector<int2>> bycls(CQG_NPC);
@@ -989,43 +1090,6 @@ static cqg_status autotune_shapes(cqg_ctx *ctx, const long long *crange, cudaStr
   cudaEventDestroy(e1);
   return CQG_OK;
 }
-
-// The class launches of one contraction, dealt in turn to the caller's stream and the side
-// streams: fork() makes the side streams wait for what the caller's stream holds so far,
-// next() gives the stream of the next launch, join() makes the caller's stream wait for the
-// side streams.  Everything a launch reads was written on the caller's stream before the
-// fork, and later work on that stream comes after the join, so the buffers' lifetimes are
-// those of a single-stream call; under capture the fork and join become graph edges.
-// With one launch, or per-class timing on, the caller's stream takes them all.
-struct ClassStreams {
-  cqg_ctx *ctx;
-  cudaStream_t st;
-  int n;          // side streams in use
-  int at = 0;
-  ClassStreams(cqg_ctx *c, cudaStream_t s, int launches, bool may_lease) : ctx(c), st(s), n(0) {
-    if (launches > 1 && !c->timing && (c->side || (may_lease && lease_side_streams(c))))
-      n = std::min(launches - 1, kSideStreams);
-  }
-  cudaError_t fork() {
-    if (n == 0) return cudaSuccess;
-    cudaError_t e = cudaEventRecord(ctx->side->fork, st);
-    for (int i = 0; i < n && e == cudaSuccess; ++i) e = cudaStreamWaitEvent(ctx->side->st[i], ctx->side->fork, 0);
-    return e;
-  }
-  cudaStream_t next() {
-    const int i = at;
-    at = at == n ? 0 : at + 1;
-    return i == 0 ? st : ctx->side->st[i - 1];
-  }
-  cudaError_t join() {
-    cudaError_t e = cudaSuccess;
-    for (int i = 0; i < n && e == cudaSuccess; ++i) {
-      e = cudaEventRecord(ctx->side->done[i], ctx->side->st[i]);
-      if (e == cudaSuccess) e = cudaStreamWaitEvent(st, ctx->side->done[i], 0);
-    }
-    return e;
-  }
-};
 
 // Sync-free contraction for CUDA-graph capture: the quartet list has a fixed capacity,
 // every class kernel reads its range from device memory and runs a persistent grid, and
@@ -1577,25 +1641,13 @@ cqg_status cqg_one_e(cqg_ctx *ctx, int ncharge, const double *Z, const double *R
     dV = dT + (size_t)n * n;
     ldd = n;
   }
-  OneEShells sh;
-  sh.L = ctx->d_shL.p;
-  sh.nprim = ctx->d_shnp.p;
-  sh.poff = ctx->d_shpoff.p;
-  sh.bf = ctx->d_bf.p;
-  sh.alpha = ctx->d_alpha.p;
-  sh.coef = ctx->d_coef.p;
-  sh.center = ctx->d_center.p;
   if (ctx->nmol != 1) {
     ctx->err = "cqg_one_e is for single-molecule contexts; use cqg_one_e_batch";
     return CQG_ERR_STATE;
   }
-  const long long np = ctx->nallpairs;
   OneEMols om;
   memset(&om, 0, sizeof(om));
-  k_one_e<<<(unsigned)((np + 63) / 64), 64, 0, st>>>(sh, ctx->d_allpairs.p, np, ncharge, ctx->d_charges.p,
-                                                     (const double3 *)(ctx->d_charges.p + ncharge), ctx->boys, dS,
-                                                     dT, dV, ldd, om);
-  CUCHK(cudaGetLastError());
+  CUCHK(run_one_e(ctx, st, true, ncharge, ctx->d_charges.p, dS, dT, dV, ldd, om));
   if (!on_device) {
     double *outs[3] = {S, T, V};
     const double *ins[3] = {dS, dT, dV};
@@ -1631,18 +1683,10 @@ cqg_status cqg_dipole(cqg_ctx *ctx, const double *origin, double *D, int ld, int
     dD = ctx->d_oe.p;
     ldd = n;
   }
-  OneEShells sh;
-  sh.L = ctx->d_shL.p;
-  sh.nprim = ctx->d_shnp.p;
-  sh.poff = ctx->d_shpoff.p;
-  sh.bf = ctx->d_bf.p;
-  sh.alpha = ctx->d_alpha.p;
-  sh.coef = ctx->d_coef.p;
-  sh.center = ctx->d_center.p;
-  const long long np = ctx->nallpairs;
-  k_dipole<<<(unsigned)((np + 63) / 64), 64, 0, st>>>(sh, ctx->d_allpairs.p, np,
-                                                      make_double3(origin[0], origin[1], origin[2]), dD, ldd, n);
-  CUCHK(cudaGetLastError());
+  const double3 O = make_double3(origin[0], origin[1], origin[2]);
+  CUCHK(each_pair_class(ctx, st, true, [&](int c, const int2 *pairs, long long np, cudaStream_t s) -> cudaError_t {
+    CQG_PAIR_CLASS_SWITCH(c, launch_dipole, ctx, pairs, np, s, O, dD, ldd)
+  }));
   if (!on_device) {
     for (int k = 0; k < 3; ++k)
       CUCHK(cudaMemcpy2DAsync(D + (size_t)k * ld * n, ld * sizeof(double), dD + (size_t)k * n * n,
@@ -1674,25 +1718,13 @@ cqg_status cqg_one_e_batch(cqg_ctx *ctx, const int *ncharge_per_mol, const doubl
   CUCHK(cudaMemcpyAsync(ctx->d_charges.p, zr.data(), 4 * (size_t)std::max(nc, 1) * sizeof(double),
                         cudaMemcpyHostToDevice, st));
   CUCHK(cudaMemcpyAsync(dcoff, coff.data(), (nmol + 1) * sizeof(int), cudaMemcpyHostToDevice, st));
-  OneEShells sh;
-  sh.L = ctx->d_shL.p;
-  sh.nprim = ctx->d_shnp.p;
-  sh.poff = ctx->d_shpoff.p;
-  sh.bf = ctx->d_bf.p;
-  sh.alpha = ctx->d_alpha.p;
-  sh.coef = ctx->d_coef.p;
-  sh.center = ctx->d_center.p;
   OneEMols om;
   om.shmol = ctx->d_shmol.p;
   om.xoff = ctx->d_mxoff.p;
   om.nbf = ctx->d_mnbf.p;
   om.coff = dcoff;
   om.batch = 1;
-  const long long np = ctx->nallpairs;
-  k_one_e<<<(unsigned)((np + 63) / 64), 64, 0, st>>>(sh, ctx->d_allpairs.p, np, nc, ctx->d_charges.p,
-                                                     (const double3 *)(ctx->d_charges.p + nc), ctx->boys, S, T,
-                                                     V, 0, om);
-  CUCHK(cudaGetLastError());
+  CUCHK(run_one_e(ctx, st, true, nc, ctx->d_charges.p, S, T, V, 0, om));
   return CQG_OK;
 }
 
@@ -1987,21 +2019,9 @@ cqg_status cqg_one_e_noalloc(cqg_ctx *ctx, int ncharge, const double *Z, const d
     CUCHK(cudaMemcpyAsync(tab, Z, (size_t)ncharge * sizeof(double), cudaMemcpyDefault, st));
     CUCHK(cudaMemcpyAsync(tab + ncharge, R, 3 * (size_t)ncharge * sizeof(double), cudaMemcpyDefault, st));
   }
-  OneEShells sh;
-  sh.L = ctx->d_shL.p;
-  sh.nprim = ctx->d_shnp.p;
-  sh.poff = ctx->d_shpoff.p;
-  sh.bf = ctx->d_bf.p;
-  sh.alpha = ctx->d_alpha.p;
-  sh.coef = ctx->d_coef.p;
-  sh.center = ctx->d_center.p;
   OneEMols om;
   memset(&om, 0, sizeof(om));
-  const long long np = ctx->nallpairs;
-  k_one_e<<<(unsigned)((np + 63) / 64), 64, 0, st>>>(sh, ctx->d_allpairs.p, np, ncharge, tab,
-                                                     (const double3 *)(tab + ncharge), ctx->boys, S, T, V, ld,
-                                                     om);
-  CUCHK(cudaGetLastError());
+  CUCHK(run_one_e(ctx, st, false, ncharge, tab, S, T, V, ld, om));   // leases (and so makes) no streams
   return CQG_OK;
 }
 

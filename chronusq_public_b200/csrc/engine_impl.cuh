@@ -1705,7 +1705,7 @@ struct cqg_ctx {
   bool class_possible[CQG_NQC] = {false};
   // molecules of the context (a batch when nmol > 1)
   int nmol = 0, max_nsh = 0, max_nbf = 0;
-  long long packed = 0, Mtotal = 0, nallpairs = 0;
+  long long packed = 0, Mtotal = 0;
   std::vector<int> hshmol, m_shoff, m_nsh, m_nbf;
   std::vector<long long> m_xoff, m_Moff;
   std::vector<unsigned char> h_active;
@@ -1729,7 +1729,6 @@ struct cqg_ctx {
   DevBuf<int> d_pair_poff, d_pair_np, d_pair_kk;
   DevBuf<int> d_shL, d_shnp, d_shpoff;
   DevBuf<double> d_alpha, d_coef;
-  DevBuf<int2> d_allpairs;
   DevBuf<double> d_oe;       // host-mode staging of S, T, V
   DevBuf<double> d_charges;  // Z then R (3 per charge)
   DevBuf<unsigned long long> d_blkacc;
