@@ -88,6 +88,8 @@ static cqg_status upload_pairs(cqg_ctx *ctx, double prim_thresh) {
     npr[i] = (int)prim.size() - poff[i];
   }
   ctx->prim_pairs_total = (long long)prim.size();
+  for (int c = 0; c <= CQG_NPC; ++c)
+    ctx->pc_prim[c] = ctx->pc_beg[c] < (int)np ? poff[ctx->pc_beg[c]] : (int)prim.size();
   for (int c = 0; c < CQG_NPC; ++c) {
     ctx->pc_np_max[c] = 0;
     for (int i = ctx->pc_beg[c]; i < ctx->pc_beg[c + 1]; ++i) ctx->pc_np_max[c] = std::max(ctx->pc_np_max[c], npr[i]);
@@ -104,6 +106,39 @@ static cqg_status upload_pairs(cqg_ctx *ctx, double prim_thresh) {
   CUCHK(cudaMemcpy(ctx->d_pair_kk.p, kk.data(), np * sizeof(int), cudaMemcpyHostToDevice));
   if (!prim.empty())
     CUCHK(cudaMemcpy(ctx->d_prim.p, prim.data(), prim.size() * sizeof(PrimPair), cudaMemcpyHostToDevice));
+  return CQG_OK;
+}
+
+// Expansion tables of the current primitive pairs, for the tensor-core classes.  They need a
+// d or f shell: without one no class uses them and none are built.
+static cqg_status build_expansions(cqg_ctx *ctx) {
+  if (ctx->maxl < 2) return CQG_OK;
+  static const int size[CQG_NPC] = {
+      warpmd::ExpansionDims<0, 0>::SIZE, warpmd::ExpansionDims<1, 0>::SIZE, warpmd::ExpansionDims<1, 1>::SIZE,
+      warpmd::ExpansionDims<2, 0>::SIZE, warpmd::ExpansionDims<2, 1>::SIZE, warpmd::ExpansionDims<2, 2>::SIZE,
+      warpmd::ExpansionDims<3, 0>::SIZE, warpmd::ExpansionDims<3, 1>::SIZE, warpmd::ExpansionDims<3, 2>::SIZE,
+      warpmd::ExpansionDims<3, 3>::SIZE};
+  size_t total = 0;
+  for (int c = 0; c < CQG_NPC; ++c) {
+    ctx->exp_off[c] = total;
+    total += (size_t)(ctx->pc_prim[c + 1] - ctx->pc_prim[c]) * size[c];
+    ctx->exp_prim0[c] = ctx->pc_prim[c];
+  }
+  if (ctx->d_exp.reserve(std::max<size_t>(total, 1)) != cudaSuccess) {
+    ctx->err = "device allocation for the expansion tables failed";
+    return CQG_ERR_OOM;
+  }
+  CUCHK((launch_expansions<0, 0>(ctx)));
+  CUCHK((launch_expansions<1, 0>(ctx)));
+  CUCHK((launch_expansions<1, 1>(ctx)));
+  CUCHK((launch_expansions<2, 0>(ctx)));
+  CUCHK((launch_expansions<2, 1>(ctx)));
+  CUCHK((launch_expansions<2, 2>(ctx)));
+  CUCHK((launch_expansions<3, 0>(ctx)));
+  CUCHK((launch_expansions<3, 1>(ctx)));
+  CUCHK((launch_expansions<3, 2>(ctx)));
+  CUCHK((launch_expansions<3, 3>(ctx)));
+  CUCHK(cudaDeviceSynchronize());   // written on the legacy stream, read on the callers' streams
   return CQG_OK;
 }
 
@@ -569,6 +604,9 @@ cqg_status cqg_create(cqg_ctx **out, int device) {
   for (int k = 0; k < CQG_NQC; ++k) {
     ctx->sibling_min[k] = default_sibling_min(k);
     ctx->class_order[k] = k;
+    int i, j;
+    qclass_split(k, i, j);
+    ctx->shape_var[k] = is_tensor_first(kPairClass[i][0], kPairClass[i][1], kPairClass[j][0], kPairClass[j][1]);
   }
   ctx->events = true;
   cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, device);
@@ -586,7 +624,7 @@ cqg_status cqg_destroy(cqg_ctx *ctx) {
   ctx->d_coef.release(); ctx->d_oe.release(); ctx->d_charges.release();
   ctx->d_shmol.release(); ctx->d_mshoff.release(); ctx->d_mnsh.release(); ctx->d_mnbf.release();
   ctx->d_molbk.release(); ctx->d_mxoff.release(); ctx->d_mMoff.release(); ctx->d_active.release();
-  ctx->d_prim.release();
+  ctx->d_prim.release(); ctx->d_exp.release();
   ctx->d_M.release(); ctx->d_Mmax.release(); ctx->d_Mpair.release(); ctx->d_flags.release();
   ctx->d_cnt.release(); ctx->d_off.release(); ctx->d_range.release(); ctx->d_scan_tmp.release();
   ctx->d_qhead.release();
@@ -911,6 +949,8 @@ cqg_status cqg_set_basis_batch(cqg_ctx *ctx, int nmol, const int *nshell_per_mol
   st = upload_pairs(ctx, 1e-24);
   if (st != CQG_OK) return st;
   st = upload_groups(ctx, fam, 1e-24);
+  if (st != CQG_OK) return st;
+  st = build_expansions(ctx);
   if (st != CQG_OK) return st;
   {
     cqg_status bst = build_block_tables(ctx);

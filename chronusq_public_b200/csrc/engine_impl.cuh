@@ -1088,68 +1088,98 @@ __global__ void __launch_bounds__(NT) k_eri_gc(const uint2 *__restrict__ ql, con
 }
 
 // ------------------------------------------------------------- warp-mode classes ---
-// SCHWARZ = false: quartets from the list, J/K digest.  SCHWARZ = true: "quartet" i is
-// pair i with itself, and the kernel writes Q(i) = sqrt(max |(ab|ab)| diagonal).
-// One FP64 tensor-core step D += A B on an 8x8x4 tile (mma.sync m8n8k4 .f64).  Fragments:
-// a = A[g][t], b = B[t][g], d[i] = D[g][2t+i] with g = lane / 4, t = lane % 4.
-__device__ __forceinline__ void dmma_884(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
-
-// Whether a warp class runs its two Hermite contractions on the FP64 tensor cores:
-//   W[h][cd] += sum_k R[h + k] KC[k][cd]     (per primitive quartet; KC = signed ket E products)
-//   C[ab][cd] += sum_h EB[ab][h] W[h][cd]    (per bra primitive pair)
-// W's 8x8 tiles are held in registers across the ket loop, so classes with more than 25
-// tiles keep the shared-memory loops.  FP32 lists use the same FP64 tiles: their R and E
-// values are FP32 and the products are accumulated in FP64.
-template <int LA, int LB, int LC, int LD, bool SCHWARZ, typename T>
-struct WarpMma {
-  static constexpr int HP = warpmd::nherm(LA + LB), HQ = warpmd::nherm(LC + LD);
-  static constexpr int NCCD = warpmd::ncart(LC) * warpmd::ncart(LD), NCAB = warpmd::ncart(LA) * warpmd::ncart(LB);
-  static constexpr int MT = (HP + 7) / 8, NT = (NCCD + 7) / 8, KT = (HQ + 3) / 4;
-  static constexpr int MTC = (NCAB + 7) / 8, KTH = (HP + 3) / 4;
-  static constexpr bool on = !SCHWARZ && MT * NT <= 25;
-  // larger classes accumulate W in shared memory, NTB column tiles at a time
-  static constexpr bool onS = !SCHWARZ && !on;
-  static constexpr int NTB = MT >= 25 ? 1 : 25 / MT;
-  static constexpr bool any = on || onS;
-};
-
-template <int LA, int LB, int LC, int LD, bool SCHWARZ, typename T>
-__global__ void __launch_bounds__(128) k_eri_jk_warp(const uint2 *__restrict__ ql, const long long *__restrict__ range,
-                                                     int blk, long long sbeg, long long send, Pairs P, Shells S,
-                                                     const double *__restrict__ boys, DigestGroups dg,
-                                                     double *__restrict__ Qout, unsigned long long *__restrict__ qhead,
-                                                     int qpw) {
-  using WD = warpmd::WarpDims<LA, LB, LC, LD>;
-  constexpr int L = WD::L, NCCD = WD::NCCD;
-  constexpr int NBUF = (WD::NW > WD::NC) ? WD::NW : WD::NC;
-  extern __shared__ double smem[];
-  // decode tables: Hermite (t,u,v) of index h, and Cartesian exponents of bra / ket pairs,
-  // packed 4 bits per exponent
-  __shared__ int s_h[WD::HL];
-  __shared__ int s_cab[WD::NCAB];
-  __shared__ int s_ccd[NCCD];
-  using MM = WarpMma<LA, LB, LC, LD, SCHWARZ, T>;
-  // s_sum[h * HQ + k]: index of the Hermite triple h + k (bra h, ket k) in R
-  __shared__ short s_sum[MM::any ? MM::HP * MM::HQ : 1];
-  if constexpr (MM::any) {
-    for (int k = threadIdx.x; k < MM::HP * MM::HQ; k += blockDim.x) {
-      int t1, u1, v1, t2, u2, v2;
-      warpmd::herm_of(k / MM::HQ, t1, u1, v1);
-      warpmd::herm_of(k % MM::HQ, t2, u2, v2);
-      s_sum[k] = (short)warpmd::hidx(t1 + t2, u1 + u2, v1 + v2);
+// J/K digest of one quartet by a warp: V [a][b][c][d] in shared memory, lanes spread over the
+// elements of Gh (the same updates as digest()).  Xs: shared memory for the density blocks.
+template <int LA, int LB, int LC, int LD>
+__device__ __forceinline__ void digest_warp(const double *V, double *Xs, const DigestGroups &dg, int a0, int b0, int c0,
+                                            int d0, int mol, double deg, int lane) {
+  constexpr int NA = nfun_c(LA), NB = nfun_c(LB), NC = nfun_c(LC), ND = nfun_c(LD);
+  // staged blocks: X(d,c) [NC*ND], X(b,a) [NA*NB], X(b,d), X(a,c), X(b,c), X(a,d)
+  double *xdc = Xs, *xba = xdc + NC * ND, *xbd = xba + NA * NB, *xac = xbd + NB * ND;
+  double *xbc = xac + NA * NC, *xad = xbc + NB * NC;
+  for (int g = 0; g < dg.ng; ++g) {
+    const double *Xv;
+    double *G;
+    size_t ld, n;
+    mol_view(dg, g, mol, Xv, G, ld, n);
+    const double *__restrict__ Xm = Xv;
+    const double sJ = dg.sJ[g] * deg, sK = 0.5 * dg.sK[g] * deg;
+    __syncwarp();
+    for (int k = lane; k < NC * ND; k += 32) xdc[k] = __ldg(Xm + (d0 + k % ND) + (c0 + k / ND) * ld);
+    for (int k = lane; k < NA * NB; k += 32) xba[k] = __ldg(Xm + (b0 + k % NB) + (a0 + k / NB) * ld);
+    for (int k = lane; k < NB * ND; k += 32) xbd[k] = __ldg(Xm + (b0 + k / ND) + (d0 + k % ND) * ld);
+    for (int k = lane; k < NA * NC; k += 32) xac[k] = __ldg(Xm + (a0 + k / NC) + (c0 + k % NC) * ld);
+    for (int k = lane; k < NB * NC; k += 32) xbc[k] = __ldg(Xm + (b0 + k / NC) + (c0 + k % NC) * ld);
+    for (int k = lane; k < NA * ND; k += 32) xad[k] = __ldg(Xm + (a0 + k / ND) + (d0 + k % ND) * ld);
+    __syncwarp();
+    // every update is written with the index that varies fastest across lanes as the
+    // row (k_finalize symmetrises Gh), so a warp's atomics fall on consecutive addresses
+    if (dg.sJ[g] != 0.0) {
+      for (int k = lane; k < NA * NB; k += 32) {
+        const int a = k / NB, b = k % NB;
+        double s = 0.0;
+        for (int cd = 0; cd < NC * ND; ++cd) s += xdc[cd] * V[k * NC * ND + cd];
+        atomicAdd(G + (b0 + b) + (a0 + a) * n, sJ * s);
+      }
+      for (int k = lane; k < NC * ND; k += 32) {
+        const int c = k / ND, d = k % ND;
+        double s = 0.0;
+        for (int ab2 = 0; ab2 < NA * NB; ++ab2) s += xba[ab2] * V[ab2 * NC * ND + k];
+        atomicAdd(G + (d0 + d) + (c0 + c) * n, sJ * s);
+      }
+    }
+    if (dg.sK[g] != 0.0) {
+      for (int k = lane; k < NA * NC; k += 32) {   // G(a,c) += X(b,d) v
+        const int a = k / NC, c = k % NC;
+        double s = 0.0;
+        for (int b = 0; b < NB; ++b)
+          for (int d = 0; d < ND; ++d) s += xbd[b * ND + d] * V[((a * NB + b) * NC + c) * ND + d];
+        atomicAdd(G + (c0 + c) + (a0 + a) * n, sK * s);
+      }
+      for (int k = lane; k < NB * ND; k += 32) {   // G(b,d) += X(a,c) v
+        const int b = k / ND, d = k % ND;
+        double s = 0.0;
+        for (int a = 0; a < NA; ++a)
+          for (int c = 0; c < NC; ++c) s += xac[a * NC + c] * V[((a * NB + b) * NC + c) * ND + d];
+        atomicAdd(G + (d0 + d) + (b0 + b) * n, sK * s);
+      }
+      for (int k = lane; k < NA * ND; k += 32) {   // G(a,d) += X(b,c) v
+        const int a = k / ND, d = k % ND;
+        double s = 0.0;
+        for (int b = 0; b < NB; ++b)
+          for (int c = 0; c < NC; ++c) s += xbc[b * NC + c] * V[((a * NB + b) * NC + c) * ND + d];
+        atomicAdd(G + (d0 + d) + (a0 + a) * n, sK * s);
+      }
+      for (int k = lane; k < NB * NC; k += 32) {   // G(b,c) += X(a,d) v
+        const int b = k / NC, c = k % NC;
+        double s = 0.0;
+        for (int a = 0; a < NA; ++a)
+          for (int d = 0; d < ND; ++d) s += xad[a * ND + d] * V[((a * NB + b) * NC + c) * ND + d];
+        atomicAdd(G + (c0 + c) + (b0 + b) * n, sK * s);
+      }
     }
   }
+}
+
+// Schwarz bounds of the pair classes whose (ab|ab) is a warp class: Q(i) = sqrt(max |(ab|ab)|)
+// for pairs [beg, end), a warp per pair (set-up only).
+template <int LA, int LB>
+__global__ void __launch_bounds__(128) k_schwarz_warp(Pairs P, Shells S, const double *__restrict__ boys, int beg,
+                                                      int end, double *__restrict__ Qout) {
+  using WD = warpmd::WarpDims<LA, LB>;
+  constexpr int L = WD::L;
+  extern __shared__ double smem[];
+  // decode tables: Hermite (t,u,v) of index h and Cartesian exponents of the pair, packed 4
+  // bits per exponent
+  __shared__ int s_h[WD::HP];
+  __shared__ int s_cab[WD::NCAB];
   // s_rec[h], h >= 1: the downward recursion R^n_h = P_d R^{n+1}_a + m R^{n+1}_b of Hermite
   // triple h, packed as a | b << 10 | d << 20 | m << 22 (d = 0, 1, 2 for x, y, z)
   __shared__ int s_rec[WD::HL];
   for (int k = threadIdx.x; k < WD::HL; k += blockDim.x) {
     int t, u, v;
     warpmd::herm_of(k, t, u, v);
-    s_h[k] = t | (u << 4) | (v << 8);
+    if (k < WD::HP) s_h[k] = t | (u << 4) | (v << 8);
     int a = 0, b = 0, d = 0, m = 0;
     if (t > 0) {
       a = warpmd::hidx(t - 1, u, v);
@@ -1171,422 +1201,136 @@ __global__ void __launch_bounds__(128) k_eri_jk_warp(const uint2 *__restrict__ q
     warpmd::cart_of(LB, k % warpmd::ncart(LB), x1, y1, z1);
     s_cab[k] = x0 | (y0 << 4) | (z0 << 8) | (x1 << 12) | (y1 << 16) | (z1 << 20);
   }
-  for (int k = threadIdx.x; k < NCCD; k += blockDim.x) {
-    int x0, y0, z0, x1, y1, z1;
-    warpmd::cart_of(LC, k / warpmd::ncart(LD), x0, y0, z0);
-    warpmd::cart_of(LD, k % warpmd::ncart(LD), x1, y1, z1);
-    s_ccd[k] = x0 | (y0 << 4) | (z0 << 8) | (x1 << 12) | (y1 << 16) | (z1 << 20);
-  }
   __syncthreads();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  // per warp: staged density blocks (double) then the T work arrays
-  constexpr size_t WARP_BYTES = sizeof(double) * WD::NXS + sizeof(T) * (3 * WD::NEB + 3 * WD::NEK + 2 * WD::HL + 2 * NBUF);
-  constexpr size_t WARP_STRIDE = (WARP_BYTES + 15) / 16 * 16;
-  double *Xs = reinterpret_cast<double *>(reinterpret_cast<char *>(smem) + wid * WARP_STRIDE);
-  T *Eb = reinterpret_cast<T *>(Xs + WD::NXS);
-  T *Ek = Eb + 3 * WD::NEB;
-  T *Ra = Ek + 3 * WD::NEK;
-  T *Rb = Ra + WD::HL;
-  T *W = Rb + WD::HL;
-  T *Cc = W + NBUF;
-  long long beg, end;
-  if (SCHWARZ) {
-    beg = sbeg;
-    end = send;
-  } else {
-    beg = range[2 * blk];
-    end = range[2 * blk + 1];
-  }
-  // list mode: each warp claims `qpw` quartets at a time from the work queue (head counter
-  // qhead[blk]); Schwarz mode: a static split of the pairs over the warps
-  const long long stride = (long long)gridDim.x * (blockDim.x >> 5);
-  long long q = SCHWARZ ? beg + (long long)blockIdx.x * (blockDim.x >> 5) + wid : end;
-  long long qend = end;
-  for (;;) {
-    if (SCHWARZ) {
-      if (q >= end) break;
-    } else if (q >= qend) {
-      unsigned long long c0 = 0;
-      if (lane == 0) c0 = atomicAdd(qhead + blk, (unsigned long long)qpw);
-      c0 = __shfl_sync(0xffffffffu, c0, 0);
-      q = beg + (long long)c0;
-      if (q >= end) break;
-      qend = min(q + (long long)qpw, end);
-    }
-    uint2 e;
-    if (SCHWARZ) e = make_uint2((unsigned)q, (unsigned)q);
-    else e = ql[q];
-    const int2 ab = P.sh[e.x], cdp = P.sh[e.y];
-    const double3 A = S.center[ab.x], B = S.center[ab.y], C = S.center[cdp.x], D = S.center[cdp.y];
-    const PrimPair *pbp = P.prim + P.poff[e.x];
-    const PrimPair *pkp = P.prim + P.poff[e.y];
-    const int nb = P.np[e.x], nk = P.np[e.y];
-    __syncwarp();
-    for (int k = lane; k < WD::NC; k += 32) Cc[k] = T(0);
-    for (int ib = 0; ib < nb; ++ib) {
-      const PrimPair bp = pbp[ib];
-      __syncwarp();
+  double *Eb = smem + (size_t)wid * WD::SMEM, *Ek = Eb + 3 * WD::NE, *Ra = Ek + 3 * WD::NE, *Rb = Ra + WD::HL;
+  double *W = Rb + WD::HL, *Cc = W + WD::NBUF;
+  for (int i = beg + blockIdx.x * (blockDim.x >> 5) + wid; i < end; i += gridDim.x * (blockDim.x >> 5)) {
+    const int2 ab = P.sh[i];
+    const double3 A = S.center[ab.x], B = S.center[ab.y];
+    const PrimPair *pp = P.prim + P.poff[i];
+    const int np = P.np[i];
+    // E coefficients of a primitive pair, one direction per lane
+    auto expand = [&](double *E, const PrimPair &p) {
       if (lane < 3) {
-        const double Pc = lane == 0 ? bp.Px : (lane == 1 ? bp.Py : bp.Pz);
+        const double Pc = lane == 0 ? p.Px : (lane == 1 ? p.Py : p.Pz);
         const double Ac = lane == 0 ? A.x : (lane == 1 ? A.y : A.z);
         const double Bc = lane == 0 ? B.x : (lane == 1 ? B.y : B.z);
-        warpmd::build_E1<LA, LB, T>(Eb + lane * WD::NEB, T(Pc - Ac), T(Pc - Bc), T(0.5 * bp.ip));
+        warpmd::build_E1<LA, LB, double>(E + lane * WD::NE, Pc - Ac, Pc - Bc, 0.5 * p.ip);
       }
-      double wacc[MM::on ? MM::MT : 1][MM::on ? MM::NT : 1][2];
-      if constexpr (MM::on) {
-#pragma unroll
-        for (int mt = 0; mt < MM::MT; ++mt)
-#pragma unroll
-          for (int nt = 0; nt < MM::NT; ++nt) wacc[mt][nt][0] = wacc[mt][nt][1] = 0.0;
-      } else {
-        for (int k = lane; k < WD::NW; k += 32) W[k] = T(0);
-      }
-      for (int ik = 0; ik < nk; ++ik) {
-        const PrimPair kp = pkp[ik];
+    };
+    __syncwarp();
+    for (int k = lane; k < WD::NC; k += 32) Cc[k] = 0.0;
+    for (int ib = 0; ib < np; ++ib) {
+      const PrimPair bp = pp[ib];
+      __syncwarp();
+      expand(Eb, bp);
+      for (int k = lane; k < WD::NW; k += 32) W[k] = 0.0;
+      for (int ik = 0; ik < np; ++ik) {
+        const PrimPair kp = pp[ik];
         __syncwarp();
-        if (lane < 3) {
-          const double Pc = lane == 0 ? kp.Px : (lane == 1 ? kp.Py : kp.Pz);
-          const double Cc3 = lane == 0 ? C.x : (lane == 1 ? C.y : C.z);
-          const double Dc = lane == 0 ? D.x : (lane == 1 ? D.y : D.z);
-          warpmd::build_E1<LC, LD, T>(Ek + lane * WD::NEK, T(Pc - Cc3), T(Pc - Dc), T(0.5 * kp.ip));
-        }
+        expand(Ek, kp);
         const double pq = bp.p + kp.p;
         const double rpq = rsqrt(pq);
         const double rho = bp.p * kp.p * (rpq * rpq);
         const double X = bp.Px - kp.Px, Y = bp.Py - kp.Py, Z = bp.Pz - kp.Pz;
         double F[L + 1];
         boys_eval<L>(rho * (X * X + Y * Y + Z * Z), boys, F);
-        double fac[L + 1];
-        {
-          double f = bp.Kp * kp.Kp * rpq;
-          const double m2r = -2.0 * rho;
+        double f = bp.Kp * kp.Kp * rpq;
 #pragma unroll
-          for (int n = 0; n <= L; ++n) {
-            fac[n] = f * F[n];
-            f *= m2r;
-          }
+        for (int n = 0; n <= L; ++n) {
+          F[n] *= f;
+          f *= -2.0 * rho;
         }
         // R^{(n)}_{tuv}, n = L .. 0, ping-pong between Ra and Rb; level L in Ra when L even
-        T *prev = (L % 2 == 0) ? Rb : Ra;
-        T *cur = (L % 2 == 0) ? Ra : Rb;
-        const T Xt = T(X), Yt = T(Y), Zt = T(Z);
-        // level L: one entry
-        if (lane == 0) cur[0] = T(fac[L]);
+        double *prev = (L % 2 == 0) ? Rb : Ra;
+        double *cur = (L % 2 == 0) ? Ra : Rb;
+        if (lane == 0) cur[0] = F[L];
 #pragma unroll
         for (int n = L - 1; n >= 0; --n) {
-          T *t_ = prev;
+          double *t_ = prev;
           prev = cur;
           cur = t_;
           __syncwarp();
           const int cnt = warpmd::nherm(L - n);
           for (int h = lane; h < cnt; h += 32) {
-            T val;
-            if (h == 0) {
-              val = T(fac[n]);
-            } else {
+            double val = F[n];
+            if (h > 0) {
               const int r = s_rec[h];
               const int dr = (r >> 20) & 3;
-              const T pd = dr == 0 ? Xt : (dr == 1 ? Yt : Zt);
-              val = pd * prev[r & 1023] + T(r >> 22) * prev[(r >> 10) & 1023];
+              const double pd = dr == 0 ? X : (dr == 1 ? Y : Z);
+              val = pd * prev[r & 1023] + (double)(r >> 22) * prev[(r >> 10) & 1023];
             }
             cur[h] = val;
           }
         }
         __syncwarp();
-        const T *R = cur;  // level 0
-        if constexpr (MM::on) {
-          // A[h][k] = R[h + k] gathered from shared memory, B[k][cd] = signed ket E product
-          const int g = lane >> 2, tq = lane & 3;
-          constexpr int NTQ = WD::Q + 1;
-#pragma unroll
-          for (int kt = 0; kt < MM::KT; ++kt) {
-            const int k = kt * 4 + tq;
-            double a[MM::MT];
-#pragma unroll
-            for (int mt = 0; mt < MM::MT; ++mt) {
-              const int h = mt * 8 + g;
-              a[mt] = (h < MM::HP && k < MM::HQ) ? (double)R[s_sum[h * MM::HQ + k]] : 0.0;
-            }
-            const int kc = k < MM::HQ ? s_h[k] : 0;
-            const int kx = kc & 15, ky = (kc >> 4) & 15, kz = kc >> 8;
-#pragma unroll
-            for (int nt = 0; nt < MM::NT; ++nt) {
-              const int c = nt * 8 + g;
-              double b = 0.0;
-              if (k < MM::HQ && c < NCCD) {
-                const int cc = s_ccd[c];
-                const int cx = cc & 15, cy = (cc >> 4) & 15, cz = (cc >> 8) & 15;
-                const int dx = (cc >> 12) & 15, dy = (cc >> 16) & 15, dz = cc >> 20;
-                if (kx <= cx + dx && ky <= cy + dy && kz <= cz + dz) {
-                  b = (double)Ek[(cx * (LD + 1) + dx) * NTQ + kx] *
-                      (double)Ek[WD::NEK + (cy * (LD + 1) + dy) * NTQ + ky] *
-                      (double)Ek[2 * WD::NEK + (cz * (LD + 1) + dz) * NTQ + kz];
-                  if ((kx + ky + kz) & 1) b = -b;
-                }
-              }
-#pragma unroll
-              for (int mt = 0; mt < MM::MT; ++mt) dmma_884(wacc[mt][nt], a[mt], b);
-            }
-          }
-        } else if constexpr (MM::onS) {
-          // the same product, with W read from and written back to shared memory for each
-          // block of NTB column tiles (every element is owned by one lane throughout)
-          const int g = lane >> 2, tq = lane & 3;
-          constexpr int NTQ = WD::Q + 1;
-          for (int n0 = 0; n0 < MM::NT; n0 += MM::NTB) {
-            double wb[MM::MT][MM::NTB][2];
-#pragma unroll
-            for (int mt = 0; mt < MM::MT; ++mt)
-#pragma unroll
-              for (int j = 0; j < MM::NTB; ++j)
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                  const int h = mt * 8 + g, c = (n0 + j) * 8 + tq * 2 + i;
-                  wb[mt][j][i] = (n0 + j < MM::NT && h < MM::HP && c < NCCD) ? (double)W[h * NCCD + c] : 0.0;
-                }
-#pragma unroll 1
-            for (int kt = 0; kt < MM::KT; ++kt) {
-              const int k = kt * 4 + tq;
-              double a[MM::MT];
-#pragma unroll
-              for (int mt = 0; mt < MM::MT; ++mt) {
-                const int h = mt * 8 + g;
-                a[mt] = (h < MM::HP && k < MM::HQ) ? (double)R[s_sum[h * MM::HQ + k]] : 0.0;
-              }
-              const int kc = k < MM::HQ ? s_h[k] : 0;
-              const int kx = kc & 15, ky = (kc >> 4) & 15, kz = kc >> 8;
-#pragma unroll
-              for (int j = 0; j < MM::NTB; ++j) {
-                const int c = (n0 + j) * 8 + g;
-                double b = 0.0;
-                if (k < MM::HQ && n0 + j < MM::NT && c < NCCD) {
-                  const int cc = s_ccd[c];
-                  const int cx = cc & 15, cy = (cc >> 4) & 15, cz = (cc >> 8) & 15;
-                  const int dx = (cc >> 12) & 15, dy = (cc >> 16) & 15, dz = cc >> 20;
-                  if (kx <= cx + dx && ky <= cy + dy && kz <= cz + dz) {
-                    b = (double)Ek[(cx * (LD + 1) + dx) * NTQ + kx] *
-                        (double)Ek[WD::NEK + (cy * (LD + 1) + dy) * NTQ + ky] *
-                        (double)Ek[2 * WD::NEK + (cz * (LD + 1) + dz) * NTQ + kz];
-                    if ((kx + ky + kz) & 1) b = -b;
-                  }
-                }
-#pragma unroll
-                for (int mt = 0; mt < MM::MT; ++mt) dmma_884(wb[mt][j], a[mt], b);
-              }
-            }
-#pragma unroll
-            for (int mt = 0; mt < MM::MT; ++mt)
-#pragma unroll
-              for (int j = 0; j < MM::NTB; ++j)
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                  const int h = mt * 8 + g, c = (n0 + j) * 8 + tq * 2 + i;
-                  if (n0 + j < MM::NT && h < MM::HP && c < NCCD) W[h * NCCD + c] = (T)wb[mt][j][i];
-                }
-          }
-        } else
+        const double *R = cur;  // level 0
         // W[tuv][cd] += sum (-1)^(tau+nu+phi) E^cd R
         for (int e2 = lane; e2 < WD::NW; e2 += 32) {
-          const int h = e2 / NCCD, c = e2 % NCCD;
-          const int hc = s_h[h], cc = s_ccd[c];
+          const int hc = s_h[e2 / WD::NCAB], cc = s_cab[e2 % WD::NCAB];
           const int t = hc & 15, u = (hc >> 4) & 15, v = hc >> 8;
           const int cx = cc & 15, cy = (cc >> 4) & 15, cz = (cc >> 8) & 15;
           const int dx = (cc >> 12) & 15, dy = (cc >> 16) & 15, dz = cc >> 20;
-          constexpr int NT = WD::Q + 1;
-          const T *ex = Ek + (cx * (LD + 1) + dx) * NT;
-          const T *ey = Ek + WD::NEK + (cy * (LD + 1) + dy) * NT;
-          const T *ez = Ek + 2 * WD::NEK + (cz * (LD + 1) + dz) * NT;
-          T s = T(0);
+          constexpr int NT = LA + LB + 1;
+          const double *ex = Ek + (cx * (LB + 1) + dx) * NT;
+          const double *ey = Ek + WD::NE + (cy * (LB + 1) + dy) * NT;
+          const double *ez = Ek + 2 * WD::NE + (cz * (LB + 1) + dz) * NT;
+          double s = 0.0;
           for (int a1 = 0; a1 <= cx + dx; ++a1)
             for (int a2 = 0; a2 <= cy + dy; ++a2) {
-              const T exy = ((a1 + a2) & 1 ? T(-1) : T(1)) * ex[a1] * ey[a2];
-              for (int a3 = 0; a3 <= cz + dz; ++a3) {
-                const T c3 = (a3 & 1) ? -ez[a3] : ez[a3];
-                s += exy * c3 * R[warpmd::hidx(t + a1, u + a2, v + a3)];
-              }
+              const double exy = ((a1 + a2) & 1 ? -1.0 : 1.0) * ex[a1] * ey[a2];
+              for (int a3 = 0; a3 <= cz + dz; ++a3)
+                s += exy * ((a3 & 1) ? -ez[a3] : ez[a3]) * R[warpmd::hidx(t + a1, u + a2, v + a3)];
             }
           W[e2] += s;
         }
       }
       __syncwarp();
-      if constexpr (MM::any) {
-        const int g = lane >> 2, tq = lane & 3;
-        constexpr int NTP = WD::P + 1;
-        // W tiles to shared memory, then C[ab][cd] += EB[ab][h] W[h][cd] on the tensor cores
-        if constexpr (MM::on) {
-#pragma unroll
-          for (int mt = 0; mt < MM::MT; ++mt)
-#pragma unroll
-            for (int nt = 0; nt < MM::NT; ++nt)
-#pragma unroll
-              for (int i = 0; i < 2; ++i) {
-                const int h = mt * 8 + g, c = nt * 8 + tq * 2 + i;
-                if (h < MM::HP && c < NCCD) W[h * NCCD + c] = wacc[mt][nt][i];
-              }
-        }
-        __syncwarp();
-        for (int mtc = 0; mtc < MM::MTC; ++mtc) {
-          const int abi = mtc * 8 + g;
-          const int cab = abi < MM::NCAB ? s_cab[abi] : 0;
-          const int ax = cab & 15, ay = (cab >> 4) & 15, az = (cab >> 8) & 15;
-          const int bx = (cab >> 12) & 15, by = (cab >> 16) & 15, bz = cab >> 20;
-          for (int nt = 0; nt < MM::NT; ++nt) {
-            double cf[2];
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-              const int c = nt * 8 + tq * 2 + i;
-              cf[i] = (abi < MM::NCAB && c < NCCD) ? (double)Cc[abi * NCCD + c] : 0.0;
-            }
-#pragma unroll
-            for (int kt = 0; kt < MM::KTH; ++kt) {
-              const int h = kt * 4 + tq;
-              double a = 0.0;
-              if (abi < MM::NCAB && h < MM::HP) {
-                const int hc = s_h[h];
-                const int t = hc & 15, u = (hc >> 4) & 15, v = hc >> 8;
-                if (t <= ax + bx && u <= ay + by && v <= az + bz)
-                  a = (double)Eb[(ax * (LB + 1) + bx) * NTP + t] *
-                      (double)Eb[WD::NEB + (ay * (LB + 1) + by) * NTP + u] *
-                      (double)Eb[2 * WD::NEB + (az * (LB + 1) + bz) * NTP + v];
-              }
-              const int hb = kt * 4 + tq, cb = nt * 8 + g;
-              const double b = (hb < MM::HP && cb < NCCD) ? (double)W[hb * NCCD + cb] : 0.0;
-              dmma_884(cf, a, b);
-            }
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-              const int c = nt * 8 + tq * 2 + i;
-              if (abi < MM::NCAB && c < NCCD) Cc[abi * NCCD + c] = (T)cf[i];
-            }
-          }
-        }
-      } else
       // C[ab][cd] += sum_tuv E^ab_tuv W[tuv][cd]
       for (int e2 = lane; e2 < WD::NC; e2 += 32) {
-        const int abi = e2 / NCCD, c = e2 % NCCD;
-        const int cc = s_cab[abi];
+        const int cc = s_cab[e2 / WD::NCAB], c = e2 % WD::NCAB;
         const int ax = cc & 15, ay = (cc >> 4) & 15, az = (cc >> 8) & 15;
         const int bx = (cc >> 12) & 15, by = (cc >> 16) & 15, bz = cc >> 20;
-        constexpr int NT = WD::P + 1;
-        const T *ex = Eb + (ax * (LB + 1) + bx) * NT;
-        const T *ey = Eb + WD::NEB + (ay * (LB + 1) + by) * NT;
-        const T *ez = Eb + 2 * WD::NEB + (az * (LB + 1) + bz) * NT;
-        T s = T(0);
+        constexpr int NT = LA + LB + 1;
+        const double *ex = Eb + (ax * (LB + 1) + bx) * NT;
+        const double *ey = Eb + WD::NE + (ay * (LB + 1) + by) * NT;
+        const double *ez = Eb + 2 * WD::NE + (az * (LB + 1) + bz) * NT;
+        double s = 0.0;
         for (int a1 = 0; a1 <= ax + bx; ++a1)
           for (int a2 = 0; a2 <= ay + by; ++a2) {
-            const T exy = ex[a1] * ey[a2];
-            for (int a3 = 0; a3 <= az + bz; ++a3) s += exy * ez[a3] * W[warpmd::hidx(a1, a2, a3) * NCCD + c];
+            const double exy = ex[a1] * ey[a2];
+            for (int a3 = 0; a3 <= az + bz; ++a3) s += exy * ez[a3] * W[warpmd::hidx(a1, a2, a3) * WD::NCAB + c];
           }
         Cc[e2] += s;
       }
     }
     __syncwarp();
     // Cartesian -> spherical on pure axes (L > 1), ping-pong Cc <-> W
-    T *src = Cc, *dst = W;
+    double *src = Cc, *dst = W;
     {
-      int d[4] = {warpmd::ncart(LA), warpmd::ncart(LB), warpmd::ncart(LC), warpmd::ncart(LD)};
-      const int ls[4] = {LA, LB, LC, LD};
+      int d[4] = {warpmd::ncart(LA), warpmd::ncart(LB), warpmd::ncart(LA), warpmd::ncart(LB)};
+      const int ls[4] = {LA, LB, LA, LB};
 #pragma unroll
       for (int ax = 0; ax < 4; ++ax) {
         if (ls[ax] < 2) continue;
-        const double *Ct = ls[ax] == 2 ? kSph2 : kSph3;
-        warpmd::sph_axis<T>(src, dst, d, ax, ls[ax], Ct, lane);
+        warpmd::sph_axis<double>(src, dst, d, ax, ls[ax], ls[ax] == 2 ? kSph2 : kSph3, lane);
         d[ax] = 2 * ls[ax] + 1;
-        T *t_ = src;
+        double *t_ = src;
         src = dst;
         dst = t_;
         __syncwarp();
       }
     }
-    const T *V = src;   // [a][b][c][d] in the reference basis
-    constexpr int NA = WD::NSA, NB = WD::NSB, NC = WD::NSC, ND = WD::NSD;
-    if (SCHWARZ) {
-      double mx = 0.0;
-      for (int k = lane; k < NA * NB; k += 32) mx = fmax(mx, fabs((double)V[k * (NA * NB) + k]));
-      for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      if (lane == 0) Qout[q] = sqrt(mx);
-      q += stride;
-      continue;
-    }
-    const double deg = (ab.x == ab.y ? 1.0 : 2.0) * (cdp.x == cdp.y ? 1.0 : 2.0) * (e.x == e.y ? 1.0 : 2.0);
-    const int a0 = S.bf[ab.x], b0 = S.bf[ab.y], c0 = S.bf[cdp.x], d0 = S.bf[cdp.y];
-    const int mol = S.mol[ab.x];
-    // staged blocks: X(d,c) [NC*ND], X(b,a) [NA*NB], X(b,d), X(a,c), X(b,c), X(a,d)
-    double *xdc = Xs, *xba = xdc + NC * ND, *xbd = xba + NA * NB, *xac = xbd + NB * ND;
-    double *xbc = xac + NA * NC, *xad = xbc + NB * NC;
-    for (int g = 0; g < dg.ng; ++g) {
-      const double *Xv;
-      double *G;
-      size_t ld, n;
-      mol_view(dg, g, mol, Xv, G, ld, n);
-      const double *__restrict__ Xm = Xv;
-      const double sJ = dg.sJ[g] * deg, sK = 0.5 * dg.sK[g] * deg;
-      __syncwarp();
-      for (int k = lane; k < NC * ND; k += 32) xdc[k] = __ldg(Xm + (d0 + k % ND) + (c0 + k / ND) * ld);
-      for (int k = lane; k < NA * NB; k += 32) xba[k] = __ldg(Xm + (b0 + k % NB) + (a0 + k / NB) * ld);
-      for (int k = lane; k < NB * ND; k += 32) xbd[k] = __ldg(Xm + (b0 + k / ND) + (d0 + k % ND) * ld);
-      for (int k = lane; k < NA * NC; k += 32) xac[k] = __ldg(Xm + (a0 + k / NC) + (c0 + k % NC) * ld);
-      for (int k = lane; k < NB * NC; k += 32) xbc[k] = __ldg(Xm + (b0 + k / NC) + (c0 + k % NC) * ld);
-      for (int k = lane; k < NA * ND; k += 32) xad[k] = __ldg(Xm + (a0 + k / ND) + (d0 + k % ND) * ld);
-      __syncwarp();
-      // every update is written with the index that varies fastest across lanes as the
-      // row (k_finalize symmetrises Gh), so a warp's atomics fall on consecutive addresses
-      if (dg.sJ[g] != 0.0) {
-        for (int k = lane; k < NA * NB; k += 32) {
-          const int a = k / NB, b = k % NB;
-          double s = 0.0;
-          for (int cd = 0; cd < NC * ND; ++cd) s += xdc[cd] * V[k * NC * ND + cd];
-          atomicAdd(G + (b0 + b) + (a0 + a) * n, sJ * s);
-        }
-        for (int k = lane; k < NC * ND; k += 32) {
-          const int c = k / ND, d = k % ND;
-          double s = 0.0;
-          for (int ab2 = 0; ab2 < NA * NB; ++ab2) s += xba[ab2] * V[ab2 * NC * ND + k];
-          atomicAdd(G + (d0 + d) + (c0 + c) * n, sJ * s);
-        }
-      }
-      if (dg.sK[g] != 0.0) {
-        for (int k = lane; k < NA * NC; k += 32) {   // G(a,c) += X(b,d) v
-          const int a = k / NC, c = k % NC;
-          double s = 0.0;
-          for (int b = 0; b < NB; ++b)
-            for (int d = 0; d < ND; ++d) s += xbd[b * ND + d] * V[((a * NB + b) * NC + c) * ND + d];
-          atomicAdd(G + (c0 + c) + (a0 + a) * n, sK * s);
-        }
-        for (int k = lane; k < NB * ND; k += 32) {   // G(b,d) += X(a,c) v
-          const int b = k / ND, d = k % ND;
-          double s = 0.0;
-          for (int a = 0; a < NA; ++a)
-            for (int c = 0; c < NC; ++c) s += xac[a * NC + c] * V[((a * NB + b) * NC + c) * ND + d];
-          atomicAdd(G + (d0 + d) + (b0 + b) * n, sK * s);
-        }
-        for (int k = lane; k < NA * ND; k += 32) {   // G(a,d) += X(b,c) v
-          const int a = k / ND, d = k % ND;
-          double s = 0.0;
-          for (int b = 0; b < NB; ++b)
-            for (int c = 0; c < NC; ++c) s += xbc[b * NC + c] * V[((a * NB + b) * NC + c) * ND + d];
-          atomicAdd(G + (d0 + d) + (a0 + a) * n, sK * s);
-        }
-        for (int k = lane; k < NB * NC; k += 32) {   // G(b,c) += X(a,d) v
-          const int b = k / NC, c = k % NC;
-          double s = 0.0;
-          for (int a = 0; a < NA; ++a)
-            for (int d = 0; d < ND; ++d) s += xad[a * ND + d] * V[((a * NB + b) * NC + c) * ND + d];
-          atomicAdd(G + (c0 + c) + (b0 + b) * n, sK * s);
-        }
-      }
-    }
-    ++q;
+    constexpr int NAB = warpmd::nfun(LA) * warpmd::nfun(LB);
+    double mx = 0.0;
+    for (int k = lane; k < NAB; k += 32) mx = fmax(mx, fabs(src[k * NAB + k]));
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if (lane == 0) Qout[i] = sqrt(mx);
   }
 }
 
-template <int LA, int LB, int LC, int LD, typename T>
-static size_t warp_smem_bytes() {
-  using WD = warpmd::WarpDims<LA, LB, LC, LD>;
-  constexpr int NBUF = (WD::NW > WD::NC) ? WD::NW : WD::NC;
-  constexpr size_t WARP_BYTES = sizeof(double) * WD::NXS + sizeof(T) * (3 * WD::NEB + 3 * WD::NEK + 2 * WD::HL + 2 * NBUF);
-  return 4 * ((WARP_BYTES + 15) / 16 * 16);
-}
+#include "eri_tc.cuh"
 
 // AX += 0.5 (Gh + Gh^T), molecule blockIdx.z of the context
 static __global__ void k_finalize(const double *__restrict__ Gh0, Mols mols, double *__restrict__ AX0, int ldax) {
@@ -1737,6 +1481,12 @@ struct cqg_ctx {
   const double *boys = nullptr;        // kBoysTable (boys_eval) and kBoysRows (load_boys) on the context's
   const double *boys_rows = nullptr;   // device: module constants, valid as long as its CUDA context
   long long prim_pairs_total = 0;
+  // Hermite expansion tables (k_expansions) of each pair class's primitive pairs: offset in
+  // d_exp and index of the class's first primitive pair
+  DevBuf<double> d_exp;
+  size_t exp_off[CQG_NPC] = {0};
+  int exp_prim0[CQG_NPC] = {0};
+  int pc_prim[CQG_NPC + 1] = {0};   // first primitive pair of each pair class
   int pc_np_max[CQG_NPC] = {0};   // most primitive pairs of a pair, per class
   // per-call scratch
   DevBuf<double> d_M, d_Mmax, d_Mpair;
@@ -1799,31 +1549,47 @@ __host__ __device__ constexpr bool is_variant_class(int la, int lb, int lc, int 
           k == ((3 * 4 + 1) * 4 + 1) * 4 + 0 || k == ((3 * 4 + 2) * 4 + 0) * 4 + 0);    // (fp|ps), (fd|ss)
 }
 
-template <int LA, int LB, int LC, int LD, bool SCHWARZ, typename T>
-static cudaError_t launch_warp(cqg_ctx *ctx, int blk, long long n, long long sbeg, long long send, cudaStream_t st,
-                               const DigestGroups &dg, double *Q) {
+// Of those, the classes whose FP64 list starts on the tensor-core kernel: (H2O)_5 cc-pVTZ,
+// per-thread against tensor-core form, (fs|pp) 0.64 / 0.24 ms, (fs|ds) 0.30 / 0.27; the others
+// are faster per thread ((pp|pp) 1.79 / 3.07 ms on (H2O)_32 cc-pVDZ, (dp|ds) 1.59 / 1.96, (ds|pp)
+// 2.18 / 5.07), whose tiles would be mostly padding.
+__host__ __device__ constexpr bool is_tensor_first(int la, int lb, int lc, int ld) {
+  return la == 3 && lb == 0 && ((lc == 1 && ld == 1) || (lc == 2 && ld == 0));
+}
+
+// Dynamic shared memory above the default 48 KB, asked for once per kernel and device.
+template <typename K>
+static cudaError_t allow_smem(K kernel, size_t bytes, int device, std::atomic<bool> (&done)[64]) {
+  const int slot = (device >= 0 && device < 64) ? device : 0;
+  if (done[slot].load(std::memory_order_relaxed)) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess) done[slot].store(true, std::memory_order_relaxed);
+  return e;
+}
+
+// The tensor-core kernel over list blk.  Warps per CTA: as many as 200 KB of shared memory
+// hold, at most four; CTAs per SM: what fits, so that each persistent CTA is resident.
+template <int LA, int LB, int LC, int LD>
+static cudaError_t launch_tc(cqg_ctx *ctx, int blk, long long n, cudaStream_t st, const DigestGroups &dg) {
   if (n == 0) return cudaSuccess;   // n < 0: count unknown on the host (graph mode)
-  // the attribute belongs to the kernel on each device: set it once per device
-  static bool attr_set[64] = {};
-  const size_t per_warp = warp_smem_bytes<LA, LB, LC, LD, T>() / 4;
-  const int wpb_max = (int)std::max<size_t>(1, std::min<size_t>(4, (200u * 1024u) / per_warp));
-  const int dev_slot = (ctx->device >= 0 && ctx->device < 64) ? ctx->device : 0;
-  if (!attr_set[dev_slot]) {
-    cudaError_t e = cudaFuncSetAttribute(k_eri_jk_warp<LA, LB, LC, LD, SCHWARZ, T>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(per_warp * wpb_max));
-    if (e != cudaSuccess) return e;
-    attr_set[dev_slot] = true;
-  }
-  int wpb = wpb_max, cta = 16;
-  if (!SCHWARZ && ctx->shape_wpb[blk] > 0) wpb = std::min(wpb_max, ctx->shape_wpb[blk]);
-  if (!SCHWARZ && ctx->shape_cta[blk] > 0) cta = ctx->shape_cta[blk];
-  const size_t smem = per_warp * wpb;
+  using D = warpmd::TcDims<LA, LB, LC, LD>;
+  static std::atomic<bool> allowed[64];
+  constexpr size_t per_warp = sizeof(double) * D::WARP_DOUBLES;
+  constexpr int wpb_max = (int)(200u * 1024u / per_warp) < 1 ? 1 : (int)(200u * 1024u / per_warp) > 4 ? 4 : (int)(200u * 1024u / per_warp);
+  cudaError_t e = allow_smem(&k_eri_tc<LA, LB, LC, LD>, per_warp * wpb_max, ctx->device, allowed);
+  if (e != cudaSuccess) return e;
+  const int wpb = ctx->shape_wpb[blk] > 0 ? std::min(wpb_max, ctx->shape_wpb[blk]) : wpb_max;
+  const int cta = ctx->shape_cta[blk] > 0 ? ctx->shape_cta[blk]
+                                          : std::max(1, (int)(220u * 1024u / (per_warp * wpb + 1024)));
   const long long cap = (long long)ctx->nsm * cta;
   const int blocks = (int)(n > 0 ? std::min<long long>((n + wpb - 1) / wpb, cap) : cap);
-  const int qpw = (!SCHWARZ && ctx->shape_qpw[blk] > 0) ? ctx->shape_qpw[blk] : 1;
-  k_eri_jk_warp<LA, LB, LC, LD, SCHWARZ, T><<<blocks, 32 * wpb, smem, st>>>(ctx->d_qlist.p, ctx->d_range.p, blk, sbeg,
-                                                                       send, make_pairs(ctx), make_shells(ctx),
-                                                                       ctx->boys, dg, Q, ctx->d_qhead.p, qpw);
+  const int bc = pair_class_c(LA, LB), kc = pair_class_c(LC, LD);
+  const Expansions X = {ctx->d_exp.p + ctx->exp_off[bc], ctx->d_exp.p + ctx->exp_off[kc], ctx->exp_prim0[bc],
+                        ctx->exp_prim0[kc]};
+  const int take = std::min(32, ctx->shape_qpw[blk]);
+  k_eri_tc<LA, LB, LC, LD><<<blocks, 32 * wpb, per_warp * wpb, st>>>(ctx->d_qlist.p, ctx->d_range.p, blk,
+                                                                    make_pairs(ctx), make_shells(ctx), X,
+                                                                    ctx->boys_rows, dg, ctx->d_qhead.p, take);
   return cudaGetLastError();
 }
 
@@ -1832,13 +1598,29 @@ static cudaError_t launch_schwarz(cqg_ctx *ctx, Pairs P, Shells S, int beg, int 
   int n = end - beg;
   if (n <= 0) return cudaSuccess;
   if constexpr (is_warp_class(LA, LB, LA, LB)) {
-    DigestGroups dg;
-    memset(&dg, 0, sizeof(dg));
-    return launch_warp<LA, LB, LA, LB, true, double>(ctx, 0, n, beg, end, 0, dg, Q);
+    static std::atomic<bool> allowed[64];
+    constexpr size_t per_warp = sizeof(double) * warpmd::WarpDims<LA, LB>::SMEM;
+    constexpr int wpb = per_warp * 4 <= 200u * 1024u ? 4 : per_warp * 2 <= 200u * 1024u ? 2 : 1;
+    cudaError_t e = allow_smem(&k_schwarz_warp<LA, LB>, per_warp * wpb, ctx->device, allowed);
+    if (e != cudaSuccess) return e;
+    k_schwarz_warp<LA, LB><<<std::min((n + wpb - 1) / wpb, ctx->nsm * 16), 32 * wpb, per_warp * wpb>>>(
+        P, S, ctx->boys, beg, end, Q);
+    return cudaGetLastError();
   } else {
     k_schwarz<LA, LB><<<(n + 127) / 128, 128>>>(P, S, ctx->boys_rows, beg, end, Q);
     return cudaGetLastError();
   }
+}
+
+// Expansion tables of pair class (LA LB)
+template <int LA, int LB>
+static cudaError_t launch_expansions(cqg_ctx *ctx) {
+  constexpr int c = pair_class_c(LA, LB);
+  const int beg = ctx->pc_beg[c], n = ctx->pc_beg[c + 1] - beg;
+  if (n <= 0) return cudaSuccess;
+  k_expansions<LA, LB><<<std::min((n + 3) / 4, ctx->nsm * 16), 128>>>(
+      make_pairs(ctx), make_shells(ctx), beg, beg + n, ctx->exp_prim0[c], ctx->d_exp.p + ctx->exp_off[c]);
+  return cudaGetLastError();
 }
 
 static inline MaskCache make_mask_cache(cqg_ctx *ctx) {
@@ -1940,10 +1722,10 @@ template <int LA, int LB, int LC, int LD, typename T>
 static cudaError_t launch_eri(cqg_ctx *ctx, int blk, long long n, cudaStream_t st, const DigestGroups &dg) {
   if (n == 0) return cudaSuccess;   // n < 0: count unknown on the host (graph mode)
   if constexpr (is_warp_class(LA, LB, LC, LD)) {
-    return launch_warp<LA, LB, LC, LD, false, T>(ctx, blk, n, 0, 0, st, dg, nullptr);
+    return launch_tc<LA, LB, LC, LD>(ctx, blk, n, st, dg);
   } else {
     if constexpr (is_variant_class(LA, LB, LC, LD)) {
-      if (ctx->shape_var[blk] == 1) return launch_warp<LA, LB, LC, LD, false, T>(ctx, blk, n, 0, 0, st, dg, nullptr);
+      if (ctx->shape_var[blk] == 1) return launch_tc<LA, LB, LC, LD>(ctx, blk, n, st, dg);
     }
     constexpr int mb = EriMinBlocks<LA, LB, LC, LD>::v;
     auto kernel = [] {

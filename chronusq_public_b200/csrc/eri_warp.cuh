@@ -1,15 +1,6 @@
-// Warp-cooperative McMurchie-Davidson ERI + J/K digest for the high angular momentum
-// classes, whose per-quartet intermediates do not fit in one thread's registers.
-//
-// One warp evaluates one shell quartet at a time.  The 32 lanes share, in shared memory:
-//   Eb, Ek : 1D Hermite expansion coefficients E^{ij}_t of the bra / ket primitive pair
-//   R      : R_{tuv} for t+u+v <= L (built level by level, n = L .. 0)
-//   W      : W[tuv][cd] = sum_{tau nu phi} (-1)^{tau+nu+phi} E^{cd}_{tau nu phi} R_{t+tau,..}
-//            accumulated over ket primitive pairs (tuv over the bra Hermite set)
-//   C      : C[ab][cd] = sum_{tuv} E^{ab}_{tuv} W[tuv][cd], accumulated over bra primitives
-// then transform C to real solid harmonics for pure shells and digest into J and K with
-// the lanes spread over the output elements.  Same mathematics as the generated
-// per-thread functions (Helgaker, Jorgensen & Olsen ch. 9.9); only the work split differs.
+// Index helpers and the 1D Hermite expansion shared by the kernels that put a warp on a
+// quartet or pair: the tensor-core class kernels (eri_tc.cuh) and the Schwarz bounds of the
+// high pair classes (k_schwarz_warp in engine_impl.cuh).
 #pragma once
 #include "eri_common.cuh"
 
@@ -39,12 +30,6 @@ __device__ __forceinline__ void herm_of(int h, int &t, int &u, int &v) {
   while (nherm(n) <= h) ++n;
   cart_of(n, h - nherm(n - 1), t, u, v);
 }
-
-// Solid-harmonic coefficient tables (rows m=-l..l over CCA Cartesians), set by the host.
-struct SphTables {
-  double c2[5 * 6];
-  double c3[7 * 10];
-};
 
 template <int LA, int LB>
 struct PairDims {
@@ -86,11 +71,6 @@ __device__ __forceinline__ void build_E1(T *E, T PA, T PB, T o2p) {
     }
 }
 
-template <int L>
-__device__ __forceinline__ const double *sph_rows(const SphTables &st) {
-  return L == 2 ? st.c2 : st.c3;
-}
-
 // Transform axis `ax` of a 4-index block from Cartesian to spherical (pure shells).
 // in: dims d[0..3] (row-major), out: same with d[ax] -> 2l+1.  Lanes over output.
 template <typename T>
@@ -117,20 +97,16 @@ __device__ __forceinline__ void sph_axis(const T *in, T *out, const int *d, int 
   }
 }
 
-template <int LA, int LB, int LC, int LD>
+// Shared memory of a warp in k_schwarz_warp, (ab|ab) of one pair class.
+template <int LA, int LB>
 struct WarpDims {
-  static constexpr int L = LA + LB + LC + LD;
-  static constexpr int P = LA + LB, Q = LC + LD;
-  static constexpr int HP = nherm(P), HL = nherm(L);
-  static constexpr int NCAB = ncart(LA) * ncart(LB), NCCD = ncart(LC) * ncart(LD);
-  static constexpr int NEB = (LA + 1) * (LB + 1) * (P + 1), NEK = (LC + 1) * (LD + 1) * (Q + 1);
-  static constexpr int NW = HP * NCCD;
-  static constexpr int NC = NCAB * NCCD;
-  // shared doubles per warp: Eb[3], Ek[3], R (2 levels), W, C
-  static constexpr int SMEM = 3 * NEB + 3 * NEK + 2 * HL + NW + NC;
-  static constexpr int NSA = nfun(LA), NSB = nfun(LB), NSC = nfun(LC), NSD = nfun(LD);
-  // staged density blocks of the digest: (d,c), (b,a), (b,d), (a,c), (b,c), (a,d)
-  static constexpr int NXS = NSC * NSD + NSA * NSB + NSB * NSD + NSA * NSC + NSB * NSC + NSA * NSD;
+  static constexpr int L = 2 * (LA + LB);
+  static constexpr int HP = nherm(LA + LB), HL = nherm(L);
+  static constexpr int NCAB = ncart(LA) * ncart(LB);
+  static constexpr int NE = PairDims<LA, LB>::NE;
+  static constexpr int NW = HP * NCAB, NC = NCAB * NCAB, NBUF = NW > NC ? NW : NC;
+  // doubles per warp: E of bra and ket (3 directions), R (2 levels), W, C
+  static constexpr int SMEM = 6 * NE + 2 * HL + 2 * NBUF;
 };
 
 }  // namespace warpmd
