@@ -14,11 +14,87 @@
 //                      the scales are folded into the digest).
 #include "engine_impl.cuh"
 
+#include <map>
 #include <mutex>
 
 #include "one_e.cuh"
 #include "siblings.h"
 #include "_gen/boys_tables.cuh"
+
+// ---- device memory pool ----
+// Setting up a basis takes about forty buffers, and cudaMalloc and cudaFree were most of its
+// time (each free waits for the device; together 4 to 20 ms for ten waters).  Freed blocks are
+// kept for the next request of their size class: powers of two up to 1 MiB, eighths of one
+// above.  (With the primitive pairs formed on the device as well, setting up (H2O)_10 cc-pVDZ
+// takes 2.1 ms instead of 13.4.)  Blocks above kPoolLargest are not kept, and at most kPoolKeep bytes are per process
+// and device; a request that the device cannot meet gives the kept blocks back first.
+namespace {
+constexpr size_t kPoolLargest = 64u << 20, kPoolKeep = 256u << 20;
+struct DevicePool {
+  std::mutex mutex;
+  std::multimap<size_t, void *> blocks;
+  size_t kept = 0;
+};
+DevicePool &device_pool(int device) {
+  static DevicePool pools[64];
+  return pools[(device >= 0 && device < 64) ? device : 0];
+}
+size_t pool_size(size_t bytes) {
+  size_t p = 512;
+  while (p < bytes) p <<= 1;
+  if (p <= (1u << 20)) return p;
+  const size_t step = p / 16;   // an eighth of the power of two below
+  return (bytes + step - 1) / step * step;
+}
+}  // namespace
+
+cudaError_t cqg_pool_alloc(void **p, size_t *bytes, int *device) {
+  cudaError_t e = cudaGetDevice(device);
+  if (e != cudaSuccess) return e;
+  const size_t size = *bytes > kPoolLargest ? *bytes : pool_size(*bytes);
+  DevicePool &pool = device_pool(*device);
+  if (*device < 64 && size <= kPoolLargest) {
+    std::lock_guard<std::mutex> lock(pool.mutex);
+    auto it = pool.blocks.find(size);
+    if (it != pool.blocks.end()) {
+      *p = it->second;
+      *bytes = size;
+      pool.kept -= size;
+      pool.blocks.erase(it);
+      return cudaSuccess;
+    }
+  }
+  e = cudaMalloc(p, size);
+  if (e == cudaErrorMemoryAllocation) {   // give the kept blocks back and try once more
+    cudaGetLastError();
+    {
+      std::lock_guard<std::mutex> lock(pool.mutex);
+      for (auto &b : pool.blocks) cudaFree(b.second);
+      pool.blocks.clear();
+      pool.kept = 0;
+    }
+    e = cudaMalloc(p, size);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return e;
+  }
+  *bytes = size;
+  return cudaSuccess;
+}
+
+void cqg_pool_free(void *p, size_t bytes, int device) {
+  if (device < 64 && bytes <= kPoolLargest) {
+    DevicePool &pool = device_pool(device);
+    std::lock_guard<std::mutex> lock(pool.mutex);
+    if (pool.kept + bytes <= kPoolKeep) {
+      pool.blocks.emplace(bytes, p);
+      pool.kept += bytes;
+      return;
+    }
+  }
+  cudaFree(p);
+}
 
 static const char *kLetters = "spdfg";
 static char g_class_names[55][16];
@@ -35,35 +111,96 @@ static double md_v1_digest_flops(int la, int lb, int lc, int ld) {
   return 24.0 * nfun(la) * nfun(lb) * nfun(lc) * nfun(ld);
 }
 
-// Primitive pairs of shell pair (a, b); prim_thresh = 0 keeps all of them, otherwise a
-// pair whose s-type bound sqrt((ij|ij)) (with a (1+|AB|)^(la+lb) allowance) is below
-// prim_thresh is dropped.
-static void pair_prims(const cqg_ctx *ctx, int a, int b, double prim_thresh, std::vector<PrimPair> &out) {
-  const double pi = 3.14159265358979323846;
-  const double s2pi52 = std::sqrt(2.0 * std::pow(pi, 2.5));
-  const double *A = &ctx->hcent[3 * a], *B = &ctx->hcent[3 * b];
-  double AB2 = 0;
-  for (int x = 0; x < 3; ++x) AB2 += (A[x] - B[x]) * (A[x] - B[x]);
-  const double ABn = std::sqrt(AB2);
-  for (int ia = 0; ia < ctx->hnprim[a]; ++ia)
-    for (int ib = 0; ib < ctx->hnprim[b]; ++ib) {
-      double al = ctx->halpha[ctx->hpoff[a] + ia], be = ctx->halpha[ctx->hpoff[b] + ib];
-      double ca = ctx->hcoef[ctx->hpoff[a] + ia], cb = ctx->hcoef[ctx->hpoff[b] + ib];
-      double p = al + be;
-      double K = ca * cb * std::exp(-al * be / p * AB2);
-      if (prim_thresh > 0) {
-        double bound = std::fabs(K) * s2pi52 / (p * std::pow(2.0 * p, 0.25)) * std::pow(1.0 + ABn, ctx->hL[a] + ctx->hL[b]);
-        if (bound < prim_thresh) continue;
-      }
+// the context's shells as the one-electron and primitive-pair kernels take them
+static OneEShells make_one_e_shells(const cqg_ctx *ctx) {
+  OneEShells sh;
+  sh.L = ctx->d_shL.p;
+  sh.nprim = ctx->d_shnp.p;
+  sh.poff = ctx->d_shpoff.p;
+  sh.bf = ctx->d_bf.p;
+  sh.alpha = ctx->d_alpha.p;
+  sh.coef = ctx->d_coef.p;
+  sh.center = ctx->d_center.p;
+  return sh;
+}
+
+// ---- primitive pairs ----
+constexpr double kPrimThresh = 1e-24;   // primitive pairs below this bound are dropped
+// sqrt(2 pi^(5/2))
+constexpr double kS2Pi52 = 5.914967172795613;
+
+// Primitive pair (ia, ib) of a shell pair at distance^2 AB2 without its contraction
+// coefficients; returns the factor f of its screening bound |c_a c_b K| f, the s-type
+// sqrt((ij|ij)) with a (1+|AB|)^(la+lb) allowance (grow).
+__host__ __device__ inline double prim_pair(double al, double be, const double3 &A, const double3 &B, double AB2,
+                                            double grow, PrimPair &pp, double &K) {
+  const double p = al + be;
+  K = exp(-al * be / p * AB2);
+  pp.p = p;
+  pp.ip = 1.0 / p;
+  pp.Kp = kS2Pi52 * K / p;
+  pp.Px = (al * A.x + be * B.x) / p;
+  pp.Py = (al * A.y + be * B.y) / p;
+  pp.Pz = (al * A.z + be * B.z) / p;
+  return kS2Pi52 / (p * sqrt(sqrt(2.0 * p))) * grow;
+}
+__host__ __device__ inline double prim_grow(double AB2, int l) {
+  const double x = 1.0 + sqrt(AB2);
+  double g = 1.0;
+  for (int k = 0; k < l; ++k) g *= x;
+  return g;
+}
+
+// Sibling groups before the sort: group g's members are the shell pairs sh[start[g] ..
+// start[g + 1]), each in the leader's shell order.  count[g] = primitive pairs that some
+// member keeps.  A thread per group: an exp and a few multiplications per primitive pair.
+static __global__ void k_count_prims(OneEShells S, const int *__restrict__ start, const int2 *__restrict__ sh,
+                                     int ngroups, double thresh, int *__restrict__ count) {
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= ngroups) return;
+  const int m0 = start[g], m1 = start[g + 1], a = sh[m0].x, b = sh[m0].y;
+  const double3 A = S.center[a], B = S.center[b];
+  const double AB2 = (A.x - B.x) * (A.x - B.x) + (A.y - B.y) * (A.y - B.y) + (A.z - B.z) * (A.z - B.z);
+  const double grow = prim_grow(AB2, S.L[a] + S.L[b]);
+  int n = 0;
+  for (int ia = 0; ia < S.nprim[a]; ++ia)
+    for (int ib = 0; ib < S.nprim[b]; ++ib) {
       PrimPair pp;
-      pp.p = p;
-      pp.ip = 1.0 / p;
-      pp.Kp = s2pi52 * K / p;
-      pp.Px = (al * A[0] + be * B[0]) / p;
-      pp.Py = (al * A[1] + be * B[1]) / p;
-      pp.Pz = (al * A[2] + be * B[2]) / p;
-      out.push_back(pp);
+      double K;
+      const double f = prim_pair(S.alpha[S.poff[a] + ia], S.alpha[S.poff[b] + ib], A, B, AB2, grow, pp, K);
+      bool keep = false;
+      for (int m = m0; m < m1 && !keep; ++m)
+        keep = fabs(S.coef[S.poff[sh[m].x] + ia] * S.coef[S.poff[sh[m].y] + ib] * K) * f >= thresh;
+      n += keep;
     }
+  count[g] = n;
+}
+
+// Primitive pairs of shell pairs [0, n), a thread per pair: their number (out == null), or
+// the pairs themselves from out + poff[i].  thresh = 0 keeps all.
+static __global__ void k_prims(OneEShells S, const int2 *__restrict__ sh, int n, double thresh, int *__restrict__ np,
+                               const int *__restrict__ poff, PrimPair *__restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int a = sh[i].x, b = sh[i].y;
+  const double3 A = S.center[a], B = S.center[b];
+  const double AB2 = (A.x - B.x) * (A.x - B.x) + (A.y - B.y) * (A.y - B.y) + (A.z - B.z) * (A.z - B.z);
+  const double grow = prim_grow(AB2, S.L[a] + S.L[b]);
+  int k = 0;
+  for (int ia = 0; ia < S.nprim[a]; ++ia)
+    for (int ib = 0; ib < S.nprim[b]; ++ib) {
+      PrimPair pp;
+      double K;
+      const double f = prim_pair(S.alpha[S.poff[a] + ia], S.alpha[S.poff[b] + ib], A, B, AB2, grow, pp, K);
+      const double c = S.coef[S.poff[a] + ia] * S.coef[S.poff[b] + ib];
+      if (thresh > 0.0 && fabs(c * K) * f < thresh) continue;
+      if (out) {
+        pp.Kp *= c;
+        out[poff[i] + k] = pp;
+      }
+      ++k;
+    }
+  if (!out) np[i] = k;
 }
 
 // primitive-count bucket of a shell pair: warps of the ERI kernels see kets of one bucket
@@ -74,38 +211,35 @@ static inline int prim_bucket(int np) {
   return CQG_NBUCKET - 1;
 }
 
-// build primitive-pair data for the current pair ordering and upload all pair arrays
-static cqg_status upload_pairs(cqg_ctx *ctx, double prim_thresh) {
-  size_t np = ctx->pair_sh.size();
-  std::vector<int> poff(np), npr(np), kk(np);
-  std::vector<PrimPair> prim;
-  prim.reserve(np * 4);
+// Primitive pairs of the current pair order, npr[i] of pair i (those that reach `thresh`;
+// 0: all), and the pair arrays, to the device.
+static cqg_status upload_pairs(cqg_ctx *ctx, double thresh, const std::vector<int> &npr) {
+  const size_t np = ctx->pair_sh.size();
+  std::vector<int> poff(np), kk(np);
+  int total = 0;
   for (size_t i = 0; i < np; ++i) {
-    int a = ctx->pair_sh[i].x, b = ctx->pair_sh[i].y;
-    poff[i] = (int)prim.size();
-    kk[i] = ctx->hnprim[a] * ctx->hnprim[b];
-    pair_prims(ctx, a, b, prim_thresh, prim);
-    npr[i] = (int)prim.size() - poff[i];
+    poff[i] = total;
+    kk[i] = ctx->hnprim[ctx->pair_sh[i].x] * ctx->hnprim[ctx->pair_sh[i].y];
+    total += npr[i];
   }
-  ctx->prim_pairs_total = (long long)prim.size();
-  for (int c = 0; c <= CQG_NPC; ++c)
-    ctx->pc_prim[c] = ctx->pc_beg[c] < (int)np ? poff[ctx->pc_beg[c]] : (int)prim.size();
+  for (int c = 0; c <= CQG_NPC; ++c) ctx->pc_prim[c] = ctx->pc_beg[c] < (int)np ? poff[ctx->pc_beg[c]] : total;
   for (int c = 0; c < CQG_NPC; ++c) {
     ctx->pc_np_max[c] = 0;
     for (int i = ctx->pc_beg[c]; i < ctx->pc_beg[c + 1]; ++i) ctx->pc_np_max[c] = std::max(ctx->pc_np_max[c], npr[i]);
   }
   if (ctx->d_pair_sh.reserve(np) || ctx->d_pair_Q.reserve(np) || ctx->d_pair_poff.reserve(np) ||
-      ctx->d_pair_np.reserve(np) || ctx->d_pair_kk.reserve(np) || ctx->d_prim.reserve(prim.size())) {
+      ctx->d_pair_np.reserve(np) || ctx->d_pair_kk.reserve(np) || ctx->d_prim.reserve(std::max(total, 1))) {
     ctx->err = "device allocation for pair data failed";
     return CQG_ERR_OOM;
   }
-  CUCHK(cudaMemcpy(ctx->d_pair_sh.p, ctx->pair_sh.data(), np * sizeof(int2), cudaMemcpyHostToDevice));
-  CUCHK(cudaMemcpy(ctx->d_pair_Q.p, ctx->pair_Q.data(), np * sizeof(double), cudaMemcpyHostToDevice));
-  CUCHK(cudaMemcpy(ctx->d_pair_poff.p, poff.data(), np * sizeof(int), cudaMemcpyHostToDevice));
-  CUCHK(cudaMemcpy(ctx->d_pair_np.p, npr.data(), np * sizeof(int), cudaMemcpyHostToDevice));
-  CUCHK(cudaMemcpy(ctx->d_pair_kk.p, kk.data(), np * sizeof(int), cudaMemcpyHostToDevice));
-  if (!prim.empty())
-    CUCHK(cudaMemcpy(ctx->d_prim.p, prim.data(), prim.size() * sizeof(PrimPair), cudaMemcpyHostToDevice));
+  CUCHK(cudaMemcpyAsync(ctx->d_pair_sh.p, ctx->pair_sh.data(), np * sizeof(int2), cudaMemcpyHostToDevice, 0));
+  CUCHK(cudaMemcpyAsync(ctx->d_pair_Q.p, ctx->pair_Q.data(), np * sizeof(double), cudaMemcpyHostToDevice, 0));
+  CUCHK(cudaMemcpyAsync(ctx->d_pair_poff.p, poff.data(), np * sizeof(int), cudaMemcpyHostToDevice, 0));
+  CUCHK(cudaMemcpyAsync(ctx->d_pair_np.p, npr.data(), np * sizeof(int), cudaMemcpyHostToDevice, 0));
+  CUCHK(cudaMemcpyAsync(ctx->d_pair_kk.p, kk.data(), np * sizeof(int), cudaMemcpyHostToDevice, 0));
+  k_prims<<<(unsigned)((np + 127) / 128), 128>>>(make_one_e_shells(ctx), ctx->d_pair_sh.p, (int)np, thresh, nullptr,
+                                                  ctx->d_pair_poff.p, ctx->d_prim.p);
+  CUCHK(cudaGetLastError());
   return CQG_OK;
 }
 
@@ -138,53 +272,39 @@ static cqg_status build_expansions(cqg_ctx *ctx) {
   CUCHK((launch_expansions<3, 1>(ctx)));
   CUCHK((launch_expansions<3, 2>(ctx)));
   CUCHK((launch_expansions<3, 3>(ctx)));
-  CUCHK(cudaDeviceSynchronize());   // written on the legacy stream, read on the callers' streams
   return CQG_OK;
 }
 
 // Unit-coefficient primitive pairs of a sibling group and its members' coefficient
 // products.  members[0] leads the group; the primitive pair (ia, ib) couples primitive ia of
 // the leader's first shell with primitive ib of its second (the members share the
-// exponents).  A primitive pair is kept when any member's bound |c_a c_b K| of pair_prims
-// reaches prim_thresh (the union of the members' screened primitive pairs).  w gets `rows`
-// rows, one value per kept primitive pair: row k = member k's products c_a(ia) c_b(ib), zero
-// for the rows past the last member.
-static void group_prims(const cqg_ctx *ctx, const int *members, int m, int rows, double prim_thresh,
-                        const std::vector<int> &fam, std::vector<PrimPair> &out, std::vector<double> &w) {
-  const double pi = 3.14159265358979323846;
-  const double s2pi52 = std::sqrt(2.0 * std::pow(pi, 2.5));
+// exponents).  A primitive pair is kept when any member keeps it (k_count_prims' rule).  w
+// gets `rows` rows, one value per kept primitive pair: row k = member k's products
+// c_a(ia) c_b(ib), zero for the rows past the last member.
+static void group_prims(const cqg_ctx *ctx, const int *members, int m, int rows, double thresh,
+                        std::vector<PrimPair> &out, std::vector<double> &w) {
   const int a = ctx->pair_sh[members[0]].x, b = ctx->pair_sh[members[0]].y;
-  const double *A = &ctx->hcent[3 * a], *B = &ctx->hcent[3 * b];
-  double AB2 = 0;
-  for (int x = 0; x < 3; ++x) AB2 += (A[x] - B[x]) * (A[x] - B[x]);
-  const double ABn = std::sqrt(AB2);
+  const double *a3 = &ctx->hcent[3 * a], *b3 = &ctx->hcent[3 * b];
+  const double3 A = make_double3(a3[0], a3[1], a3[2]), B = make_double3(b3[0], b3[1], b3[2]);
+  const double AB2 = (A.x - B.x) * (A.x - B.x) + (A.y - B.y) * (A.y - B.y) + (A.z - B.z) * (A.z - B.z);
+  const double grow = prim_grow(AB2, ctx->hL[a] + ctx->hL[b]);
   // coefficient arrays of each member, in the leader's shell order
   std::vector<const double *> ca(m), cb(m);
   for (int k = 0; k < m; ++k) {
     const int x = ctx->pair_sh[members[k]].x, y = ctx->pair_sh[members[k]].y;
-    const bool same = cqg_sib::same_orientation(x, a, fam);
+    const bool same = cqg_sib::same_orientation(x, a, ctx->fam);
     ca[k] = &ctx->hcoef[ctx->hpoff[same ? x : y]];
     cb[k] = &ctx->hcoef[ctx->hpoff[same ? y : x]];
   }
   std::vector<std::vector<double>> wk(rows);
   for (int ia = 0; ia < ctx->hnprim[a]; ++ia)
     for (int ib = 0; ib < ctx->hnprim[b]; ++ib) {
-      const double al = ctx->halpha[ctx->hpoff[a] + ia], be = ctx->halpha[ctx->hpoff[b] + ib];
-      const double p = al + be;
-      const double K = std::exp(-al * be / p * AB2);
-      bool keep = prim_thresh <= 0;
-      if (!keep) {
-        const double f = s2pi52 / (p * std::pow(2.0 * p, 0.25)) * std::pow(1.0 + ABn, ctx->hL[a] + ctx->hL[b]);
-        for (int k = 0; k < m && !keep; ++k) keep = std::fabs(ca[k][ia] * cb[k][ib] * K) * f >= prim_thresh;
-      }
-      if (!keep) continue;
       PrimPair pp;
-      pp.p = p;
-      pp.ip = 1.0 / p;
-      pp.Kp = s2pi52 * K / p;
-      pp.Px = (al * A[0] + be * B[0]) / p;
-      pp.Py = (al * A[1] + be * B[1]) / p;
-      pp.Pz = (al * A[2] + be * B[2]) / p;
+      double K;
+      const double f = prim_pair(ctx->halpha[ctx->hpoff[a] + ia], ctx->halpha[ctx->hpoff[b] + ib], A, B, AB2, grow, pp, K);
+      bool keep = false;
+      for (int k = 0; k < m && !keep; ++k) keep = std::fabs(ca[k][ia] * cb[k][ib] * K) * f >= thresh;
+      if (!keep) continue;
       out.push_back(pp);
       for (int k = 0; k < rows; ++k) wk[k].push_back(k < m ? ca[k][ia] * cb[k][ib] : 0.0);
     }
@@ -228,8 +348,8 @@ static bool pair_class_in_groups(int c) {
 }
 
 // Group data of the current pair order (leaders: unit primitive pairs and member weights)
-// and the group index arrays, to the device.
-static cqg_status upload_groups(cqg_ctx *ctx, const std::vector<int> &fam, double prim_thresh) {
+// and the group index arrays, to the device; only contractions with siblings on read them.
+static cqg_status upload_groups(cqg_ctx *ctx, double prim_thresh) {
   const int np = (int)ctx->pair_sh.size();
   std::vector<int> gpoff(np, 0), gnp(np, 0), gwoff(np, 0);
   std::vector<PrimPair> prim;
@@ -245,19 +365,18 @@ static cqg_status upload_groups(cqg_ctx *ctx, const std::vector<int> &fam, doubl
       for (int k = 0; k < m; ++k) members[k] = i + k;
       gpoff[i] = (int)prim.size();
       gwoff[i] = (int)w.size();
-      group_prims(ctx, members.data(), m, rows, prim_thresh, fam, prim, w);
+      group_prims(ctx, members.data(), m, rows, prim_thresh, prim, w);
       gnp[i] = (int)prim.size() - gpoff[i];
     }
   }
   const size_t ng = ctx->glead.size();
-  if (ctx->d_pair_Qc.reserve(np) || ctx->d_gsz.reserve(np) || ctx->d_gpoff.reserve(np) || ctx->d_gnp.reserve(np) ||
+  if (ctx->d_gsz.reserve(np) || ctx->d_gpoff.reserve(np) || ctx->d_gnp.reserve(np) ||
       ctx->d_gwoff.reserve(np) || ctx->d_gprim.reserve(std::max<size_t>(prim.size(), 1)) ||
       ctx->d_gw.reserve(std::max<size_t>(w.size(), 1)) || ctx->d_glead.reserve(std::max<size_t>(ng, 1)) ||
       ctx->d_gQ.reserve(std::max<size_t>(ng, 1))) {
     ctx->err = "device allocation for sibling-group data failed";
     return CQG_ERR_OOM;
   }
-  CUCHK(cudaMemcpy(ctx->d_pair_Qc.p, ctx->pair_Qc.data(), np * sizeof(double), cudaMemcpyHostToDevice));
   CUCHK(cudaMemcpy(ctx->d_gsz.p, ctx->pair_gsz.data(), np * sizeof(int), cudaMemcpyHostToDevice));
   CUCHK(cudaMemcpy(ctx->d_gpoff.p, gpoff.data(), np * sizeof(int), cudaMemcpyHostToDevice));
   CUCHK(cudaMemcpy(ctx->d_gnp.p, gnp.data(), np * sizeof(int), cudaMemcpyHostToDevice));
@@ -269,7 +388,7 @@ static cqg_status upload_groups(cqg_ctx *ctx, const std::vector<int> &fam, doubl
     CUCHK(cudaMemcpy(ctx->d_glead.p, ctx->glead.data(), ng * sizeof(int), cudaMemcpyHostToDevice));
     CUCHK(cudaMemcpy(ctx->d_gQ.p, ctx->gQ.data(), ng * sizeof(double), cudaMemcpyHostToDevice));
   }
-  ctx->group_prim_pairs = (long long)prim.size();
+  ctx->groups_ready = true;
   return CQG_OK;
 }
 
@@ -329,20 +448,6 @@ static void return_side_streams(cqg_ctx *ctx) {
   }
   if (ctx->side) destroy_side_streams(ctx->side);
   ctx->side = nullptr;
-}
-
-// The class launches of the one-electron kernels over the context's pairs (sorted by class),
-// dealt to the side streams when the context holds or may lease them.
-static OneEShells make_one_e_shells(const cqg_ctx *ctx) {
-  OneEShells sh;
-  sh.L = ctx->d_shL.p;
-  sh.nprim = ctx->d_shnp.p;
-  sh.poff = ctx->d_shpoff.p;
-  sh.bf = ctx->d_bf.p;
-  sh.alpha = ctx->d_alpha.p;
-  sh.coef = ctx->d_coef.p;
-  sh.center = ctx->d_center.p;
-  return sh;
 }
 
 // The active block table: bra-group tasks for the sibling classes, or pair tasks for all.
@@ -600,7 +705,6 @@ cqg_status cqg_create(cqg_ctx **out, int device) {
   }
   ctx->boys = (const double *)boys;
   ctx->boys_rows = (const double *)rows;
-  for (int i = 0; i < 4 + 2 * CQG_NQC + 2; ++i) cudaEventCreate(&ctx->ev[i]);
   for (int k = 0; k < CQG_NQC; ++k) {
     ctx->sibling_min[k] = default_sibling_min(k);
     ctx->class_order[k] = k;
@@ -608,7 +712,6 @@ cqg_status cqg_create(cqg_ctx **out, int device) {
     qclass_split(k, i, j);
     ctx->shape_var[k] = is_tensor_first(kPairClass[i][0], kPairClass[i][1], kPairClass[j][0], kPairClass[j][1]);
   }
-  ctx->events = true;
   cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, device);
   *out = ctx;
   return CQG_OK;
@@ -617,6 +720,7 @@ cqg_status cqg_create(cqg_ctx **out, int device) {
 cqg_status cqg_destroy(cqg_ctx *ctx) {
   if (!ctx) return CQG_OK;
   cudaSetDevice(ctx->device);
+  cudaDeviceSynchronize();   // the buffers go back to the pool
   ctx->d_center.release(); ctx->d_bf.release(); ctx->d_sz.release();
   ctx->d_pair_sh.release(); ctx->d_pair_Q.release(); ctx->d_pair_poff.release(); ctx->d_pair_np.release();
   ctx->d_pair_kk.release(); ctx->d_blkacc.release();
@@ -624,7 +728,7 @@ cqg_status cqg_destroy(cqg_ctx *ctx) {
   ctx->d_coef.release(); ctx->d_oe.release(); ctx->d_charges.release();
   ctx->d_shmol.release(); ctx->d_mshoff.release(); ctx->d_mnsh.release(); ctx->d_mnbf.release();
   ctx->d_molbk.release(); ctx->d_mxoff.release(); ctx->d_mMoff.release(); ctx->d_active.release();
-  ctx->d_prim.release(); ctx->d_exp.release();
+  ctx->d_prim.release(); ctx->d_exp.release(); ctx->d_setup.release();
   ctx->d_M.release(); ctx->d_Mmax.release(); ctx->d_Mpair.release(); ctx->d_flags.release();
   ctx->d_cnt.release(); ctx->d_off.release(); ctx->d_range.release(); ctx->d_scan_tmp.release();
   ctx->d_qhead.release();
@@ -662,6 +766,11 @@ cqg_status cqg_set_list_budget(cqg_ctx *ctx, long long quartets) {
 
 cqg_status cqg_set_timing(cqg_ctx *ctx, int on) {
   if (!ctx) return CQG_ERR_BAD_ARG;
+  if (on && !ctx->events) {
+    CUCHK(cudaSetDevice(ctx->device));
+    for (int i = 0; i < 4 + 2 * CQG_NQC + 2; ++i) CUCHK(cudaEventCreate(&ctx->ev[i]));
+    ctx->events = true;
+  }
   ctx->timing = on ? 1 : 0;
   return CQG_OK;
 }
@@ -758,27 +867,27 @@ cqg_status cqg_set_basis_batch(cqg_ctx *ctx, int nmol, const int *nshell_per_mol
       ctx->d_mnbf.reserve(nmol) || ctx->d_mxoff.reserve(nmol) || ctx->d_mMoff.reserve(nmol) ||
       ctx->d_active.reserve(nmol))
     return CQG_ERR_OOM;
-  CUCHK(cudaMemcpy(ctx->d_center.p, c3.data(), nshell * sizeof(double3), cudaMemcpyHostToDevice));
-  CUCHK(cudaMemcpy(ctx->d_bf.p, ctx->hbf.data(), nshell * sizeof(int), cudaMemcpyHostToDevice));
-  CUCHK(cudaMemcpy(ctx->d_sz.p, ctx->hsz.data(), nshell * sizeof(int), cudaMemcpyHostToDevice));
-  CUCHK(cudaMemcpy(ctx->d_shmol.p, ctx->hshmol.data(), nshell * sizeof(int), cudaMemcpyHostToDevice));
-  CUCHK(cudaMemcpy(ctx->d_mshoff.p, ctx->m_shoff.data(), nmol * sizeof(int), cudaMemcpyHostToDevice));
-  CUCHK(cudaMemcpy(ctx->d_mnsh.p, ctx->m_nsh.data(), nmol * sizeof(int), cudaMemcpyHostToDevice));
-  CUCHK(cudaMemcpy(ctx->d_mnbf.p, ctx->m_nbf.data(), nmol * sizeof(int), cudaMemcpyHostToDevice));
-  CUCHK(cudaMemcpy(ctx->d_mxoff.p, ctx->m_xoff.data(), nmol * sizeof(long long), cudaMemcpyHostToDevice));
-  CUCHK(cudaMemcpy(ctx->d_mMoff.p, ctx->m_Moff.data(), nmol * sizeof(long long), cudaMemcpyHostToDevice));
+  CUCHK(cudaMemcpyAsync(ctx->d_center.p, c3.data(), nshell * sizeof(double3), cudaMemcpyHostToDevice, 0));
+  CUCHK(cudaMemcpyAsync(ctx->d_bf.p, ctx->hbf.data(), nshell * sizeof(int), cudaMemcpyHostToDevice, 0));
+  CUCHK(cudaMemcpyAsync(ctx->d_sz.p, ctx->hsz.data(), nshell * sizeof(int), cudaMemcpyHostToDevice, 0));
+  CUCHK(cudaMemcpyAsync(ctx->d_shmol.p, ctx->hshmol.data(), nshell * sizeof(int), cudaMemcpyHostToDevice, 0));
+  CUCHK(cudaMemcpyAsync(ctx->d_mshoff.p, ctx->m_shoff.data(), nmol * sizeof(int), cudaMemcpyHostToDevice, 0));
+  CUCHK(cudaMemcpyAsync(ctx->d_mnsh.p, ctx->m_nsh.data(), nmol * sizeof(int), cudaMemcpyHostToDevice, 0));
+  CUCHK(cudaMemcpyAsync(ctx->d_mnbf.p, ctx->m_nbf.data(), nmol * sizeof(int), cudaMemcpyHostToDevice, 0));
+  CUCHK(cudaMemcpyAsync(ctx->d_mxoff.p, ctx->m_xoff.data(), nmol * sizeof(long long), cudaMemcpyHostToDevice, 0));
+  CUCHK(cudaMemcpyAsync(ctx->d_mMoff.p, ctx->m_Moff.data(), nmol * sizeof(long long), cudaMemcpyHostToDevice, 0));
   ctx->h_active.assign(nmol, 1);
-  CUCHK(cudaMemcpy(ctx->d_active.p, ctx->h_active.data(), nmol, cudaMemcpyHostToDevice));
+  CUCHK(cudaMemcpyAsync(ctx->d_active.p, ctx->h_active.data(), nmol, cudaMemcpyHostToDevice, 0));
   // raw shells (one-electron integrals)
   {
     if (ctx->d_shL.reserve(nshell) || ctx->d_shnp.reserve(nshell) || ctx->d_shpoff.reserve(nshell) ||
         ctx->d_alpha.reserve(tot) || ctx->d_coef.reserve(tot))
       return CQG_ERR_OOM;
-    CUCHK(cudaMemcpy(ctx->d_shL.p, L, nshell * sizeof(int), cudaMemcpyHostToDevice));
-    CUCHK(cudaMemcpy(ctx->d_shnp.p, nprim, nshell * sizeof(int), cudaMemcpyHostToDevice));
-    CUCHK(cudaMemcpy(ctx->d_shpoff.p, ctx->hpoff.data(), nshell * sizeof(int), cudaMemcpyHostToDevice));
-    CUCHK(cudaMemcpy(ctx->d_alpha.p, alpha, tot * sizeof(double), cudaMemcpyHostToDevice));
-    CUCHK(cudaMemcpy(ctx->d_coef.p, coef, tot * sizeof(double), cudaMemcpyHostToDevice));
+    CUCHK(cudaMemcpyAsync(ctx->d_shL.p, L, nshell * sizeof(int), cudaMemcpyHostToDevice, 0));
+    CUCHK(cudaMemcpyAsync(ctx->d_shnp.p, nprim, nshell * sizeof(int), cudaMemcpyHostToDevice, 0));
+    CUCHK(cudaMemcpyAsync(ctx->d_shpoff.p, ctx->hpoff.data(), nshell * sizeof(int), cudaMemcpyHostToDevice, 0));
+    CUCHK(cudaMemcpyAsync(ctx->d_alpha.p, alpha, tot * sizeof(double), cudaMemcpyHostToDevice, 0));
+    CUCHK(cudaMemcpyAsync(ctx->d_coef.p, coef, tot * sizeof(double), cudaMemcpyHostToDevice, 0));
   }
   // pairs within each molecule, by class, internal orientation L_a >= L_b (a >= b when equal L)
   std::vector<std::vector<int2>> bycls(CQG_NPC);
@@ -796,48 +905,25 @@ cqg_status cqg_set_basis_batch(cqg_ctx *ctx, int nmol, const int *nshell_per_mol
   }
   ctx->pc_beg[CQG_NPC] = (int)ctx->pair_sh.size();
   ctx->pair_Q.assign(ctx->pair_sh.size(), 0.0);
-  cqg_status st = upload_pairs(ctx, 0.0);
+  const int npairs = (int)ctx->pair_sh.size();
+  std::vector<int> npr(npairs);
+  for (int i = 0; i < npairs; ++i) npr[i] = nprim[ctx->pair_sh[i].x] * nprim[ctx->pair_sh[i].y];
+  cqg_status st = upload_pairs(ctx, 0.0, npr);
   if (st != CQG_OK) return st;
   // Schwarz on the device with all primitive pairs (computeSchwartz uses precision 0)
   Pairs P = make_pairs(ctx);
   Shells S = make_shells(ctx);
-  double *dQ = ctx->d_pair_Q.p;
-  cudaError_t e = cudaSuccess;
-  e = e ? e : launch_schwarz<0, 0>(ctx, P, S, ctx->pc_beg[0], ctx->pc_beg[1], dQ);
-  e = e ? e : launch_schwarz<1, 0>(ctx, P, S, ctx->pc_beg[1], ctx->pc_beg[2], dQ);
-  e = e ? e : launch_schwarz<1, 1>(ctx, P, S, ctx->pc_beg[2], ctx->pc_beg[3], dQ);
-  e = e ? e : launch_schwarz<2, 0>(ctx, P, S, ctx->pc_beg[3], ctx->pc_beg[4], dQ);
-  e = e ? e : launch_schwarz<2, 1>(ctx, P, S, ctx->pc_beg[4], ctx->pc_beg[5], dQ);
-  e = e ? e : launch_schwarz<2, 2>(ctx, P, S, ctx->pc_beg[5], ctx->pc_beg[6], dQ);
-  e = e ? e : launch_schwarz<3, 0>(ctx, P, S, ctx->pc_beg[6], ctx->pc_beg[7], dQ);
-  e = e ? e : launch_schwarz<3, 1>(ctx, P, S, ctx->pc_beg[7], ctx->pc_beg[8], dQ);
-  e = e ? e : launch_schwarz<3, 2>(ctx, P, S, ctx->pc_beg[8], ctx->pc_beg[9], dQ);
-  e = e ? e : launch_schwarz<3, 3>(ctx, P, S, ctx->pc_beg[9], ctx->pc_beg[10], dQ);
-  if (e != cudaSuccess) {
-    ctx->err = std::string("schwarz kernels: ") + cudaGetErrorString(e);
-    return CQG_ERR_CUDA;
-  }
-  CUCHK(cudaDeviceSynchronize());
-  CUCHK(cudaMemcpy(ctx->pair_Q.data(), dQ, ctx->pair_Q.size() * sizeof(double), cudaMemcpyDeviceToHost));
-  if (nmol == 1) {
-    ctx->Qmat.assign((size_t)nshell * nshell, 0.0);
-    for (size_t i = 0; i < ctx->pair_sh.size(); ++i) {
-      int a = ctx->pair_sh[i].x, b = ctx->pair_sh[i].y;
-      ctx->Qmat[a + (size_t)b * nshell] = ctx->pair_Q[i];
-      ctx->Qmat[b + (size_t)a * nshell] = ctx->pair_Q[i];
-    }
-  } else {
-    ctx->Qmat.clear();
-  }
-  // Sibling groups per pair class (csrc/siblings.h), their largest Q and the size of the
-  // union of their members' screened primitive pairs.
-  const int npairs = (int)ctx->pair_sh.size();
-  const std::vector<int> fam = cqg_sib::shell_families(nshell, L, nprim, ctx->hpoff.data(), alpha, centers,
-                                                       ctx->hshmol.data());
-  std::vector<int> pgid(npairs), prank(npairs), gnp_of(npairs);   // gnp_of: by group id
-  std::vector<double> gq_of(npairs, 0.0);
+  CUCHK(each_pair_class(ctx, 0, true, [&](int c, const int2 *, long long, cudaStream_t s) -> cudaError_t {
+    CQG_PAIR_CLASS_SWITCH(c, launch_schwarz, ctx, P, S, ctx->pc_beg[c], ctx->pc_beg[c + 1], ctx->d_pair_Q.p, s)
+  }));
+  // meanwhile the sibling groups per pair class (csrc/siblings.h): the shells of each group's
+  // members, in the leader's order
+  ctx->fam = cqg_sib::shell_families(nshell, L, nprim, ctx->hpoff.data(), alpha, centers, ctx->hshmol.data());
+  ctx->groups_ready = false;
+  const std::vector<int> &fam = ctx->fam;
+  std::vector<int> pgid(npairs), prank(npairs);
+  int ngroups0 = 0;
   {
-    int gbase = 0;
     std::vector<int> pa, pb, gid, rank;
     for (int c = 0; c < CQG_NPC; ++c) {
       const int b0 = ctx->pc_beg[c], n = ctx->pc_beg[c + 1] - b0;
@@ -850,30 +936,54 @@ cqg_status cqg_set_basis_batch(cqg_ctx *ctx, int nmol, const int *nshell_per_mol
       const int cap = sibling_cap(kPairClass[c][0], kPairClass[c][1]);
       const int ng = cqg_sib::pair_groups(n, pa.data(), pb.data(), L, fam, cap, gid, rank);
       for (int k = 0; k < n; ++k) {
-        pgid[b0 + k] = gbase + gid[k];
+        pgid[b0 + k] = ngroups0 + gid[k];
         prank[b0 + k] = rank[k];
       }
-      gbase += ng;
+      ngroups0 += ng;
     }
-    std::vector<std::vector<int>> members(gbase);
-    for (int i = 0; i < npairs; ++i) members[pgid[i]].push_back(i);
-    std::vector<PrimPair> tmp;
-    std::vector<double> w;
-    for (int g = 0; g < gbase; ++g) {
-      double q = 0.0;
-      for (int i : members[g]) q = std::max(q, ctx->pair_Q[i]);
-      gq_of[g] = q;
-      tmp.clear();
-      w.clear();
-      group_prims(ctx, members[g].data(), (int)members[g].size(), 1, 1e-24, fam, tmp, w);
-      gnp_of[g] = (int)tmp.size();
+  }
+  // the primitive pairs that each pair and each group (the union of its members') keeps
+  std::vector<int> gnp_of(ngroups0), gstart(ngroups0 + 1, 0);
+  std::vector<double> gq_of(ngroups0, 0.0);
+  {
+    for (int i = 0; i < npairs; ++i) ++gstart[pgid[i] + 1];
+    for (int g = 0; g < ngroups0; ++g) gstart[g + 1] += gstart[g];
+    std::vector<int2> gsh(npairs);
+    for (int i = 0; i < npairs; ++i) gsh[gstart[pgid[i]] + prank[i]] = ctx->pair_sh[i];
+    for (int g = 0; g < ngroups0; ++g)
+      for (int k = gstart[g] + 1; k < gstart[g + 1]; ++k)
+        if (!cqg_sib::same_orientation(gsh[k].x, gsh[gstart[g]].x, fam)) std::swap(gsh[k].x, gsh[k].y);
+    if (ctx->d_setup.reserve(3 * (size_t)npairs + 2 * (size_t)ngroups0 + 2)) return CQG_ERR_OOM;
+    int2 *d_gsh = (int2 *)ctx->d_setup.p;
+    int *d_np = ctx->d_setup.p + 2 * (size_t)npairs, *d_gnp = d_np + npairs, *d_gstart = d_gnp + ngroups0;
+    CUCHK(cudaMemcpyAsync(d_gsh, gsh.data(), npairs * sizeof(int2), cudaMemcpyHostToDevice, 0));
+    CUCHK(cudaMemcpyAsync(d_gstart, gstart.data(), (ngroups0 + 1) * sizeof(int), cudaMemcpyHostToDevice, 0));
+    k_prims<<<(npairs + 127) / 128, 128>>>(make_one_e_shells(ctx), ctx->d_pair_sh.p, npairs, kPrimThresh, d_np, nullptr,
+                                           nullptr);
+    k_count_prims<<<(ngroups0 + 127) / 128, 128>>>(make_one_e_shells(ctx), d_gstart, d_gsh, ngroups0, kPrimThresh,
+                                                   d_gnp);
+    CUCHK(cudaGetLastError());
+    CUCHK(cudaMemcpy(npr.data(), d_np, npairs * sizeof(int), cudaMemcpyDeviceToHost));
+    CUCHK(cudaMemcpy(gnp_of.data(), d_gnp, ngroups0 * sizeof(int), cudaMemcpyDeviceToHost));
+    CUCHK(cudaMemcpy(ctx->pair_Q.data(), ctx->d_pair_Q.p, npairs * sizeof(double), cudaMemcpyDeviceToHost));
+  }
+  for (int i = 0; i < npairs; ++i) gq_of[pgid[i]] = std::max(gq_of[pgid[i]], ctx->pair_Q[i]);
+  if (nmol == 1) {
+    ctx->Qmat.assign((size_t)nshell * nshell, 0.0);
+    for (size_t i = 0; i < ctx->pair_sh.size(); ++i) {
+      int a = ctx->pair_sh[i].x, b = ctx->pair_sh[i].y;
+      ctx->Qmat[a + (size_t)b * nshell] = ctx->pair_Q[i];
+      ctx->Qmat[b + (size_t)a * nshell] = ctx->pair_Q[i];
     }
+  } else {
+    ctx->Qmat.clear();
   }
   // Sort each class by (molecule, primitive-count bucket of the group, group Q descending,
   // group, member), stable.  The members of a group become consecutive pairs led by the
   // first, and Qc (the group's Q) is non-increasing within each bucket.  Per (molecule,
   // class) bucket starts -> molbk (pair index) and molgbk (group index).
-  auto bucket_of = [&](int i) { return prim_bucket(gnp_of[pgid[i]]); };
+  std::vector<int> bucket(npairs);
+  for (int i = 0; i < npairs; ++i) bucket[i] = prim_bucket(gnp_of[pgid[i]]);
   const int NB1 = CQG_NBUCKET + 1;
   std::vector<int> molbk((size_t)nmol * CQG_NPC * NB1, 0), molgbk((size_t)nmol * CQG_NPC * NB1, 0);
   std::vector<int> new_gid(npairs);
@@ -882,10 +992,9 @@ cqg_status cqg_set_basis_batch(cqg_ctx *ctx, int nmol, const int *nshell_per_mol
     std::vector<int> idx(b1 - b0);
     std::iota(idx.begin(), idx.end(), b0);
     std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) {
-      int mx = ctx->hshmol[ctx->pair_sh[x].x], my = ctx->hshmol[ctx->pair_sh[y].x];
+      const int mx = ctx->hshmol[ctx->pair_sh[x].x], my = ctx->hshmol[ctx->pair_sh[y].x];
       if (mx != my) return mx < my;
-      int bx = bucket_of(x), by = bucket_of(y);
-      if (bx != by) return bx < by;
+      if (bucket[x] != bucket[y]) return bucket[x] < bucket[y];
       const double qx = gq_of[pgid[x]], qy = gq_of[pgid[y]];
       if (qx != qy) return qx > qy;
       if (pgid[x] != pgid[y]) return pgid[x] < pgid[y];
@@ -894,7 +1003,7 @@ cqg_status cqg_set_basis_batch(cqg_ctx *ctx, int nmol, const int *nshell_per_mol
     // bucket starts per molecule: first index of (m, bk); empty buckets start where the next begins
     std::vector<int> first((size_t)nmol * NB1, -1);
     for (int k = 0; k < (int)idx.size(); ++k) {
-      const int m = ctx->hshmol[ctx->pair_sh[idx[k]].x], bk = bucket_of(idx[k]);
+      const int m = ctx->hshmol[ctx->pair_sh[idx[k]].x], bk = bucket[idx[k]];
       if (first[(size_t)m * NB1 + bk] < 0) first[(size_t)m * NB1 + bk] = b0 + k;
     }
     int next = b1;
@@ -910,12 +1019,14 @@ cqg_status cqg_set_basis_batch(cqg_ctx *ctx, int nmol, const int *nshell_per_mol
     for (int bk = 0; bk <= CQG_NBUCKET; ++bk) ctx->bucket_beg[c][bk] = molbk[(size_t)c * NB1 + bk];
     std::vector<int2> sh2;
     std::vector<double> q2;
-    std::vector<int> g2;
+    std::vector<int> g2, n2;
     for (int i : idx) {
       sh2.push_back(ctx->pair_sh[i]);
       q2.push_back(ctx->pair_Q[i]);
       g2.push_back(pgid[i]);
+      n2.push_back(npr[i]);
     }
+    std::copy(n2.begin(), n2.end(), npr.begin() + b0);
     std::copy(sh2.begin(), sh2.end(), ctx->pair_sh.begin() + b0);
     std::copy(q2.begin(), q2.end(), ctx->pair_Q.begin() + b0);
     std::copy(g2.begin(), g2.end(), new_gid.begin() + b0);
@@ -943,13 +1054,17 @@ cqg_status cqg_set_basis_batch(cqg_ctx *ctx, int nmol, const int *nshell_per_mol
     }
     for (size_t k = 0; k < molbk.size(); ++k) molgbk[k] = molbk[k] < npairs ? pair_group[molbk[k]] : ngroups;
   }
-  if (ctx->d_molbk.reserve(molbk.size()) || ctx->d_molgbk.reserve(molgbk.size())) return CQG_ERR_OOM;
-  CUCHK(cudaMemcpy(ctx->d_molbk.p, molbk.data(), molbk.size() * sizeof(int), cudaMemcpyHostToDevice));
-  CUCHK(cudaMemcpy(ctx->d_molgbk.p, molgbk.data(), molgbk.size() * sizeof(int), cudaMemcpyHostToDevice));
-  st = upload_pairs(ctx, 1e-24);
+  if (ctx->d_molbk.reserve(molbk.size()) || ctx->d_molgbk.reserve(molgbk.size()) || ctx->d_pair_Qc.reserve(npairs))
+    return CQG_ERR_OOM;
+  CUCHK(cudaMemcpyAsync(ctx->d_molbk.p, molbk.data(), molbk.size() * sizeof(int), cudaMemcpyHostToDevice, 0));
+  CUCHK(cudaMemcpyAsync(ctx->d_molgbk.p, molgbk.data(), molgbk.size() * sizeof(int), cudaMemcpyHostToDevice, 0));
+  CUCHK(cudaMemcpyAsync(ctx->d_pair_Qc.p, ctx->pair_Qc.data(), npairs * sizeof(double), cudaMemcpyHostToDevice, 0));
+  st = upload_pairs(ctx, kPrimThresh, npr);
   if (st != CQG_OK) return st;
-  st = upload_groups(ctx, fam, 1e-24);
-  if (st != CQG_OK) return st;
+  if (ctx->siblings) {
+    st = upload_groups(ctx, kPrimThresh);
+    if (st != CQG_OK) return st;
+  }
   st = build_expansions(ctx);
   if (st != CQG_OK) return st;
   {
@@ -971,6 +1086,7 @@ cqg_status cqg_set_basis_batch(cqg_ctx *ctx, int nmol, const int *nshell_per_mol
       ctx->d_Mmax.reserve(1) || ctx->d_flags.reserve(4) || ctx->d_blkacc.reserve(kBlkAcc * CQG_NQC) ||
       ctx->d_Mpair.reserve(std::max<size_t>(ctx->pair_sh.size(), 1)))
     return CQG_ERR_OOM;
+  CUCHK(cudaDeviceSynchronize());   // written on the legacy stream, read on the callers' streams
   return CQG_OK;
 }
 
@@ -1894,6 +2010,11 @@ cqg_status cqg_set_fusion(cqg_ctx *ctx, int tier) {
 
 cqg_status cqg_set_siblings(cqg_ctx *ctx, int on) {
   if (!ctx) return CQG_ERR_BAD_ARG;
+  if (on && ctx->nshell > 0 && !ctx->groups_ready) {
+    CUCHK(cudaSetDevice(ctx->device));
+    const cqg_status st = upload_groups(ctx, kPrimThresh);
+    if (st != CQG_OK) return st;
+  }
   ctx->siblings = on ? 1 : 0;
   select_block_table(ctx);
   return CQG_OK;

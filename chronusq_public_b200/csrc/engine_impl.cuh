@@ -166,25 +166,31 @@ __device__ __forceinline__ void mol_view(const DigestGroups &dg, int g, int m, c
 }
 
 // ------------------------------------------------------------------ kernels ---
-// Schwarz: Q(ab) = sqrt(max_ij |(ij|ij)|) for pairs [beg, end) of one class.
+// Schwarz: Q(ab) = sqrt(max_ij |(ij|ij)|) for pairs [beg, end) of one class, 2^ls lanes per
+// pair, each with a share of the bra's primitive pairs.
 template <int LA, int LB>
 __global__ void __launch_bounds__(128) k_schwarz(Pairs P, Shells S, const double *__restrict__ boys_g,
-                                                 int beg, int end, double *__restrict__ Qout) {
+                                                 int beg, int end, int ls, double *__restrict__ Qout) {
   __shared__ __align__(16) double boys[BOYS_ROWS_SIZE];
   load_boys<2 * (LA + LB)>(boys_g, boys);
   __syncthreads();
-  int i = beg + blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= end) return;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, sub = t & ((1 << ls) - 1);
+  const int i = min(beg + (t >> ls), end - 1);
   constexpr int NA = nfun_c(LA), NB = nfun_c(LB), NAB = NA * NB;
   int2 s = P.sh[i];
   double3 A = S.center[s.x], B = S.center[s.y];
   double out[NAB * NAB];
   const PrimPair *pp = P.prim + P.poff[i];
-  EriClass<LA, LB, LA, LB>::template run<double>(pp, P.np[i], pp, P.np[i], A, B, A, B, boys, out);
+  const int np = P.np[i], b0 = (np * sub) >> ls, b1 = (np * (sub + 1)) >> ls;
+  EriClass<LA, LB, LA, LB>::template run<double>(pp + b0, b1 - b0, pp, np, A, B, A, B, boys, out);
   double mx = 0.0;
 #pragma unroll
-  for (int ij = 0; ij < NAB; ++ij) mx = fmax(mx, fabs(out[ij * NAB + ij]));
-  Qout[i] = sqrt(mx);
+  for (int ij = 0; ij < NAB; ++ij) {
+    double v = out[ij * NAB + ij];
+    for (int o = (1 << ls) >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    mx = fmax(mx, fabs(v));
+  }
+  if (sub == 0 && beg + (t >> ls) < end) Qout[i] = sqrt(mx);
 }
 
 // Block norms M(s1,s2) = max over matrices of max|X_i(block)|, and input checks.
@@ -1388,24 +1394,41 @@ __global__ void k_fma_probe(T *out, int iters, T seed) {
     }                                                                              \
   } while (0)
 
+// Device memory of the contexts, from a process-wide pool (engine.cu): *bytes is rounded up to
+// the block's size.  A block may be handed to another context, on any stream, as soon as it
+// is given back, so it is given back only when the device has finished with it.
+cudaError_t cqg_pool_alloc(void **p, size_t *bytes, int *device);
+void cqg_pool_free(void *p, size_t bytes, int device);
+
 template <typename T>
 struct DevBuf {
   T *p = nullptr;
-  size_t n = 0;
+  size_t n = 0, bytes = 0;
+  int device = 0;
+  // At least m elements; a larger buffer replaces the old one (contents are not kept) after
+  // the device has finished with it.
   cudaError_t reserve(size_t m) {
     if (m <= n) return cudaSuccess;
-    if (p) cudaFree(p);
-    p = nullptr;
-    n = 0;
-    size_t want = std::max<size_t>(m, 1);
-    cudaError_t e = cudaMalloc(&p, want * sizeof(T));
-    if (e == cudaSuccess) n = want;
-    return e;
+    if (p) {
+      const cudaError_t e = cudaDeviceSynchronize();
+      if (e != cudaSuccess) return e;
+      release();
+    }
+    const size_t want = std::max<size_t>(m, 1);
+    size_t b = want * sizeof(T);
+    void *q = nullptr;
+    const cudaError_t e = cqg_pool_alloc(&q, &b, &device);
+    if (e != cudaSuccess) return e;
+    p = (T *)q;
+    n = want;
+    bytes = b;
+    return cudaSuccess;
   }
+  // gives the buffer back; the device has finished with it
   void release() {
-    if (p) cudaFree(p);
+    if (p) cqg_pool_free(p, bytes, device);
     p = nullptr;
-    n = 0;
+    n = bytes = 0;
   }
 };
 
@@ -1478,9 +1501,9 @@ struct cqg_ctx {
   DevBuf<unsigned long long> d_blkacc;
   int launches = 0;
   DevBuf<PrimPair> d_prim;
+  DevBuf<int> d_setup;                 // cqg_set_basis: group members, primitive-pair counts
   const double *boys = nullptr;        // kBoysTable (boys_eval) and kBoysRows (load_boys) on the context's
   const double *boys_rows = nullptr;   // device: module constants, valid as long as its CUDA context
-  long long prim_pairs_total = 0;
   // Hermite expansion tables (k_expansions) of each pair class's primitive pairs: offset in
   // d_exp and index of the class's first primitive pair
   DevBuf<double> d_exp;
@@ -1507,7 +1530,8 @@ struct cqg_ctx {
   std::vector<int> pair_gsz, glead;
   std::vector<double> pair_Qc, gQ;
   int gc_beg[CQG_NPC + 1] = {0};      // first group of each pair class
-  long long group_prim_pairs = 0;
+  std::vector<int> fam;               // shell families (siblings.h)
+  bool groups_ready = false;          // the group arrays of the current basis are on the device
   DevBuf<int> d_molgbk, d_gsz, d_gpoff, d_gnp, d_gwoff, d_glead;
   DevBuf<double> d_pair_Qc, d_gQ, d_gw;
   DevBuf<PrimPair> d_gprim;
@@ -1521,7 +1545,7 @@ struct cqg_ctx {
   // classes, most work first, as the last uncaptured contraction counted it (a captured one
   // launches in this order)
   int class_order[CQG_NQC];
-  cudaEvent_t ev[4 + 2 * CQG_NQC + 2];
+  cudaEvent_t ev[4 + 2 * CQG_NQC + 2] = {};   // made when timing is first switched on
   bool events = false;
   cqg_stats stats;
   double *oe_table = nullptr;   // device address of the fixed charge table (cqg_one_e_noalloc)
@@ -1594,7 +1618,7 @@ static cudaError_t launch_tc(cqg_ctx *ctx, int blk, long long n, cudaStream_t st
 }
 
 template <int LA, int LB>
-static cudaError_t launch_schwarz(cqg_ctx *ctx, Pairs P, Shells S, int beg, int end, double *Q) {
+static cudaError_t launch_schwarz(cqg_ctx *ctx, Pairs P, Shells S, int beg, int end, double *Q, cudaStream_t st) {
   int n = end - beg;
   if (n <= 0) return cudaSuccess;
   if constexpr (is_warp_class(LA, LB, LA, LB)) {
@@ -1603,11 +1627,14 @@ static cudaError_t launch_schwarz(cqg_ctx *ctx, Pairs P, Shells S, int beg, int 
     constexpr int wpb = per_warp * 4 <= 200u * 1024u ? 4 : per_warp * 2 <= 200u * 1024u ? 2 : 1;
     cudaError_t e = allow_smem(&k_schwarz_warp<LA, LB>, per_warp * wpb, ctx->device, allowed);
     if (e != cudaSuccess) return e;
-    k_schwarz_warp<LA, LB><<<std::min((n + wpb - 1) / wpb, ctx->nsm * 16), 32 * wpb, per_warp * wpb>>>(
+    k_schwarz_warp<LA, LB><<<std::min((n + wpb - 1) / wpb, ctx->nsm * 16), 32 * wpb, per_warp * wpb, st>>>(
         P, S, ctx->boys, beg, end, Q);
     return cudaGetLastError();
   } else {
-    k_schwarz<LA, LB><<<(n + 127) / 128, 128>>>(P, S, ctx->boys_rows, beg, end, Q);
+    int ls = 0;   // up to a lane per primitive pair of the class's longest bra
+    while (ls < 5 && (2 << ls) <= ctx->pc_np_max[pair_class_c(LA, LB)]) ++ls;
+    k_schwarz<LA, LB><<<(unsigned)((((long long)n << ls) + 127) / 128), 128, 0, st>>>(P, S, ctx->boys_rows, beg, end, ls,
+                                                                                  Q);
     return cudaGetLastError();
   }
 }
