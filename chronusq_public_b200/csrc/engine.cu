@@ -177,9 +177,11 @@ static __global__ void k_count_prims(OneEShells S, const int *__restrict__ start
 }
 
 // Primitive pairs of shell pairs [0, n), a thread per pair: their number (out == null), or
-// the pairs themselves from out + poff[i].  thresh = 0 keeps all.
+// the pairs themselves from out + poff[i] and, with `cols`, in blocked columns from row
+// coff[i].  thresh = 0 keeps all.
 static __global__ void k_prims(OneEShells S, const int2 *__restrict__ sh, int n, double thresh, int *__restrict__ np,
-                               const int *__restrict__ poff, PrimPair *__restrict__ out) {
+                               const int *__restrict__ poff, PrimPair *__restrict__ out,
+                               const int *__restrict__ coff, double2 *__restrict__ cols) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int a = sh[i].x, b = sh[i].y;
@@ -197,6 +199,12 @@ static __global__ void k_prims(OneEShells S, const int2 *__restrict__ sh, int n,
       if (out) {
         pp.Kp *= c;
         out[poff[i] + k] = pp;
+        if (cols) {
+          double2 *r = cols + (size_t)(coff[i] + k) * kPrimRow + (i & 31);
+          r[0] = make_double2(pp.p, pp.Kp);
+          r[32] = make_double2(pp.Px, pp.Py);
+          r[64] = make_double2(pp.Pz, pp.ip);
+        }
       }
       ++k;
     }
@@ -237,8 +245,26 @@ static cqg_status upload_pairs(cqg_ctx *ctx, double thresh, const std::vector<in
   CUCHK(cudaMemcpyAsync(ctx->d_pair_poff.p, poff.data(), np * sizeof(int), cudaMemcpyHostToDevice, 0));
   CUCHK(cudaMemcpyAsync(ctx->d_pair_np.p, npr.data(), np * sizeof(int), cudaMemcpyHostToDevice, 0));
   CUCHK(cudaMemcpyAsync(ctx->d_pair_kk.p, kk.data(), np * sizeof(int), cudaMemcpyHostToDevice, 0));
+  if (thresh > 0.0) {   // the pairs' final order: blocked columns too
+    std::vector<int> coff(np);
+    size_t rows = 0;
+    for (size_t b = 0; b < np; b += 32) {
+      int most = 0;
+      for (size_t i = b; i < std::min(np, b + 32); ++i) {
+        coff[i] = (int)rows;
+        most = std::max(most, npr[i]);
+      }
+      rows += most;
+    }
+    if (ctx->d_pair_coff.reserve(np) || ctx->d_cols.reserve(std::max<size_t>(rows, 1) * kPrimRow)) {
+      ctx->err = "device allocation for pair data failed";
+      return CQG_ERR_OOM;
+    }
+    CUCHK(cudaMemcpyAsync(ctx->d_pair_coff.p, coff.data(), np * sizeof(int), cudaMemcpyHostToDevice, 0));
+  }
   k_prims<<<(unsigned)((np + 127) / 128), 128>>>(make_one_e_shells(ctx), ctx->d_pair_sh.p, (int)np, thresh, nullptr,
-                                                  ctx->d_pair_poff.p, ctx->d_prim.p);
+                                                  ctx->d_pair_poff.p, ctx->d_prim.p, ctx->d_pair_coff.p,
+                                                  thresh > 0.0 ? ctx->d_cols.p : nullptr);
   CUCHK(cudaGetLastError());
   return CQG_OK;
 }
@@ -729,6 +755,7 @@ cqg_status cqg_destroy(cqg_ctx *ctx) {
   ctx->d_shmol.release(); ctx->d_mshoff.release(); ctx->d_mnsh.release(); ctx->d_mnbf.release();
   ctx->d_molbk.release(); ctx->d_mxoff.release(); ctx->d_mMoff.release(); ctx->d_active.release();
   ctx->d_prim.release(); ctx->d_exp.release(); ctx->d_setup.release();
+  ctx->d_cols.release(); ctx->d_pair_coff.release();
   ctx->d_M.release(); ctx->d_Mmax.release(); ctx->d_Mpair.release(); ctx->d_flags.release();
   ctx->d_cnt.release(); ctx->d_off.release(); ctx->d_range.release(); ctx->d_scan_tmp.release();
   ctx->d_qhead.release();
@@ -959,7 +986,7 @@ cqg_status cqg_set_basis_batch(cqg_ctx *ctx, int nmol, const int *nshell_per_mol
     CUCHK(cudaMemcpyAsync(d_gsh, gsh.data(), npairs * sizeof(int2), cudaMemcpyHostToDevice, 0));
     CUCHK(cudaMemcpyAsync(d_gstart, gstart.data(), (ngroups0 + 1) * sizeof(int), cudaMemcpyHostToDevice, 0));
     k_prims<<<(npairs + 127) / 128, 128>>>(make_one_e_shells(ctx), ctx->d_pair_sh.p, npairs, kPrimThresh, d_np, nullptr,
-                                           nullptr);
+                                           nullptr, nullptr, nullptr);
     k_count_prims<<<(ngroups0 + 127) / 128, 128>>>(make_one_e_shells(ctx), d_gstart, d_gsh, ngroups0, kPrimThresh,
                                                    d_gnp);
     CUCHK(cudaGetLastError());

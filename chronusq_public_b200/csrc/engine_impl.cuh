@@ -114,6 +114,8 @@ struct Pairs {
   const int *np;        // number of primitive pairs (after primitive screening)
   const int *kk;        // nprim(a) * nprim(b) of the contracted shells (model count)
   const PrimPair *prim;
+  const double2 *cols;  // the same primitive pairs in blocked columns (PrimCols): pair i's are
+  const int *coff;      // column i % 32 of the rows from coff[i]
   // Sibling groups: pairs whose shells have the same centres, angular momenta and
   // exponents (segmented copies of one general contraction) and differ only in their
   // contraction coefficients.  The members of a group are consecutive pairs, led by the
@@ -171,7 +173,7 @@ __device__ __forceinline__ void mol_view(const DigestGroups &dg, int g, int m, c
 template <int LA, int LB>
 __global__ void __launch_bounds__(128) k_schwarz(Pairs P, Shells S, const double *__restrict__ boys_g,
                                                  int beg, int end, int ls, double *__restrict__ Qout) {
-  __shared__ __align__(16) double boys[BOYS_ROWS_SIZE];
+  __shared__ __align__(16) double boys[boys_rows_size(2 * (LA + LB))];
   load_boys<2 * (LA + LB)>(boys_g, boys);
   __syncthreads();
   const int t = blockIdx.x * blockDim.x + threadIdx.x, sub = t & ((1 << ls) - 1);
@@ -886,7 +888,7 @@ __device__ __forceinline__ void eri_jk_list(const uint2 *__restrict__ ql, const 
                                             const Pairs &P, const Shells &S, const double *__restrict__ boys_g,
                                             const DigestGroups &dg, unsigned long long *__restrict__ qhead,
                                             int chunk, LaneShare share) {
-  __shared__ __align__(16) double boys[BOYS_ROWS_SIZE];
+  __shared__ __align__(16) double boys[boys_rows_size(LA + LB + LC + LD)];
   load_boys<LA + LB + LC + LD>(boys_g, boys);
   __syncthreads();
   const long long beg = range[2 * blk], end = range[2 * blk + 1];
@@ -923,8 +925,9 @@ __global__ void __launch_bounds__(kEriThreads) k_eri_jk(const uint2 *__restrict_
 // Classes whose kernel is compiled for MB resident CTAs per SM (launch bounds with a
 // minimum block count; the other classes keep the compiler's own register choice).
 // Measured on (H2O)_32 cc-pVDZ against the kernels without the minimum: (ps|ps) 151 -> 128
-// registers 4.3 % faster, (pp|ss) 157 -> 128 2.9 %, (ds|ps) 199 -> 168 2.8 %; (ps|ss) at
-// five CTAs (95 registers) no faster, (ss|ss) at five (96, spilling) 17 % slower.
+// registers 4.3 % faster, (pp|ss) 157 -> 128 2.9 %, (ds|ps) 199 -> 168 2.8 %; (ss|ss) at
+// five (96, spilling) 17 % slower.  (ps|ss) and (dp|ss) are held at three CTAs (208 and 242
+// registers without).
 template <int LA, int LB, int LC, int LD>
 struct EriMinBlocks {
   static constexpr int v = 0;
@@ -942,7 +945,11 @@ struct EriMinBlocks<2, 0, 1, 0> {
   static constexpr int v = 3;
 };
 template <>
-struct EriMinBlocks<2, 1, 0, 0> {   // 168 registers, as without the lane sharing of eri_jk_plain (else 242)
+struct EriMinBlocks<1, 0, 0, 0> {
+  static constexpr int v = 3;
+};
+template <>
+struct EriMinBlocks<2, 1, 0, 0> {
   static constexpr int v = 3;
 };
 
@@ -968,7 +975,8 @@ __device__ __forceinline__ int eri_jk_plain(const uint2 e, const bool valid, con
   double v[NA * NB * NC * ND];
   if (valid) {
     const double3 A = S.center[ab.x], B = S.center[ab.y], C = S.center[cd.x], D = S.center[cd.y];
-    const PrimPair *bp = P.prim + P.poff[e.x], *kp = P.prim + P.poff[e.y];
+    PrimCols bp = {P.cols + (size_t)P.coff[e.x] * kPrimRow + (e.x & 31)},
+             kp = {P.cols + (size_t)P.coff[e.y] * kPrimRow + (e.y & 31)};
     int nb1 = nb, nk1 = nk;
     if (ls) {
       const int s = threadIdx.x & ((1 << ls) - 1);
@@ -978,8 +986,8 @@ __device__ __forceinline__ int eri_jk_plain(const uint2 e, const bool valid, con
       const int b0 = (nb * sb) >> lb, k0 = (nk * sk) >> lk;
       nb1 = ((nb * (sb + 1)) >> lb) - b0;
       nk1 = ((nk * (sk + 1)) >> lk) - k0;
-      bp += b0;
-      kp += k0;
+      bp = bp + b0;
+      kp = kp + k0;
     }
     if constexpr (sizeof(T) == sizeof(double)) {
       EriClass<LA, LB, LC, LD>::template run<double>(bp, nb1, kp, nk1, A, B, C, D, boys, v);
@@ -1071,7 +1079,7 @@ template <int LA, int LB, int LC, int LD, typename T, int NT>
 __global__ void __launch_bounds__(NT) k_eri_gc(const uint2 *__restrict__ ql, const long long *__restrict__ range,
                                                 int blk, Pairs P, Shells S, const double *__restrict__ boys_g,
                                                 DigestGroups dg, unsigned long long *__restrict__ qhead, int chunk) {
-  __shared__ __align__(16) double boys[BOYS_ROWS_SIZE];
+  __shared__ __align__(16) double boys[boys_rows_size(LA + LB + LC + LD)];
   load_boys<LA + LB + LC + LD>(boys_g, boys);
   __syncthreads();
   const long long beg = range[2 * blk], end = range[2 * blk + 1];
@@ -1501,6 +1509,8 @@ struct cqg_ctx {
   DevBuf<unsigned long long> d_blkacc;
   int launches = 0;
   DevBuf<PrimPair> d_prim;
+  DevBuf<double2> d_cols;
+  DevBuf<int> d_pair_coff;
   DevBuf<int> d_setup;                 // cqg_set_basis: group members, primitive-pair counts
   const double *boys = nullptr;        // kBoysTable (boys_eval) and kBoysRows (load_boys) on the context's
   const double *boys_rows = nullptr;   // device: module constants, valid as long as its CUDA context
@@ -1667,6 +1677,8 @@ static inline Pairs make_pairs(cqg_ctx *ctx) {
   P.np = ctx->d_pair_np.p;
   P.kk = ctx->d_pair_kk.p;
   P.prim = ctx->d_prim.p;
+  P.cols = ctx->d_cols.p;
+  P.coff = ctx->d_pair_coff.p;
   P.Qc = ctx->d_pair_Qc.p;
   P.glead = ctx->d_glead.p;
   P.gQ = ctx->d_gQ.p;

@@ -94,7 +94,7 @@ template <int TIER>
 __global__ void __launch_bounds__(kEriThreads, TIER == 1 ? 4 : 2)
     k_eri_fused(const uint2 *__restrict__ ql, const long long *__restrict__ range, Pairs P, Shells S,
                 const double *__restrict__ boys_g, DigestGroups dg, unsigned long long *__restrict__ head) {
-  __shared__ __align__(16) double boys[BOYS_ROWS_SIZE];
+  __shared__ __align__(16) double boys[boys_rows_size(TIER == 1 ? 1 : 5)]   /* the tier's longest rows */;
   __shared__ long long s_beg[kMaxSlots], s_end[kMaxSlots], s_start[kMaxSlots + 1];
   __shared__ unsigned long long s_claim;
   constexpr int NC = TIER == 1 ? kNT1 : kNT2;

@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(128) k_eri_tc(const uint2 *__restrict__ ql, co
   for (int n = 0; n < HT; ++n)
 #pragma unroll
     for (int i = 0; i < 2; ++i) odd |= (unsigned)(warpmd::herm_total(8 * n + 2 * t + i) & 1) << (2 * n + i);
-  const double *rows = rows_g + (size_t)L * BOYS_ROWS_SIZE;
+  const double *rows = rows_g + boys_rows_off(L);
   const long long beg = range[2 * blk], end = range[2 * blk + 1];
   if (take <= 0) {
     const long long warps = (long long)gridDim.x * (blockDim.x >> 5);

@@ -3,15 +3,15 @@
 For every shell-quartet class (la lb | lc ld) with la >= lb, lc >= ld and the bra pair
 class not below the ket pair class, this emits one fully unrolled device function
 
-    template <typename T>
-    __device__ void eri_<la><lb><lc><ld>(const PrimPair* bra, int nbra,
-                                         const PrimPair* ket, int nket,
+    template <typename T, typename Prims>     // Prims: const PrimPair* or PrimCols
+    __device__ void eri_<la><lb><lc><ld>(const Prims bra, int nbra,
+                                         const Prims ket, int nket,
                                          double3 A, double3 B, double3 C, double3 D,
                                          const double* boys_tab, T* out)
 
 that returns the contracted, normalised (ab|cd) over the reference's basis functions
 (spherical for pure shells) in row-major [a][b][c][d] order.  ``boys_tab`` is the
-shared-memory Boys table of ``stage_boys<L>`` (eri_common.cuh), L = la+lb+lc+ld.
+shared-memory Boys rows of ``load_boys<L>`` (eri_common.cuh), L = la+lb+lc+ld.
 
 Method (McMurchie & Davidson, J. Comput. Phys. 26, 218 (1978); notation of Helgaker,
 Jorgensen & Olsen ch. 9.5 and 9.9):
@@ -22,8 +22,8 @@ Jorgensen & Olsen ch. 9.5 and 9.9):
 The ket Hermite sum is accumulated over ket primitive pairs into W[tuv][cd] for one bra
 primitive pair, and the bra Hermite transform is applied once per bra primitive pair.
 E coefficients are built per primitive pair by the 1D recursion; R by the standard
-downward recursion on n from R^n_000 = (-2 rho)^n F_n(rho |PQ|^2).  Boys values come
-from :file:`boys.cuh` in FP64 regardless of ``T``; everything after them runs in ``T``.
+downward recursion on n from R^n_000 = (-2 rho)^n F_n(rho |PQ|^2) (class_arg, class_rows).  Boys values come
+from :file:`eri_common.cuh` in FP64 regardless of ``T``; everything after them runs in ``T``.
 
 Run:  python gen_eri.py <out.cuh> [maxl]
 """
@@ -205,7 +205,7 @@ def _emit_tile(g, nbt, la, lb, lc, ld, ca, cb, cc, cd, hp, hidx, ncd, members=No
                 needb[d].add((a[k], b[k]))
     for j in range(nbt):
         bt = "b%d" % j
-        g.w("const PrimPair pb%d = bra[ib + %d];" % (j, j))
+        g.w("const PrimPair pb%d = prim_at(bra, ib + %d);" % (j, j))
         g.w("const double p%d = pb%d.p;" % (j, j))
         g.w("const T %so2p = T(0.5 * pb%d.ip);" % (bt, j))
         for d in "xyz":
@@ -248,28 +248,40 @@ def _emit_tile(g, nbt, la, lb, lc, ld, ca, cb, cc, cd, hp, hidx, ncd, members=No
                 ci += 1
         return kterms
 
+    def boys(tags):
+        """Boys values G<j>k<ktag> of the primitive quartets (j, ktag, qname): the polynomial of
+        all of them when one is near in this lane, the far constants otherwise."""
+        for (j, ktag, qname) in tags:
+            v = "%d%s" % (j, ktag)
+            g.w("const double PQx%s = pb%d.Px - p%s.Px, PQy%s = pb%d.Py - p%s.Py, PQz%s = pb%d.Pz - p%s.Pz;"
+                % (v, j, ktag, v, j, ktag, v, j, ktag))
+            g.w("const double pm%s = p%d * %s;" % (v, j, qname))
+            g.w("const ClassArg arg%s = class_arg<%d>(p%d + %s, pm%s, PQx%s * PQx%s + PQy%s * PQy%s + PQz%s * PQz%s);"
+                % (v, L, j, qname, v, v, v, v, v, v, v))
+            g.w("double G%s[%d];" % (v, L + 1))
+        g.w("if (%s) {" % " && ".join("arg%d%s.far" % (j, ktag) for (j, ktag, _) in tags))
+        for (j, ktag, _) in tags:
+            g.w("  class_far<%d>(G%d%s);" % (L, j, ktag))
+        g.w("} else {")
+        for (j, ktag, _) in tags:
+            g.w("  class_rows<%d>(arg%d%s, boys_tab, G%d%s);" % (L, j, ktag, j, ktag))
+        g.w("}")
+
     def chain(j, ktag, qname, kterms, r):
-        """One primitive quartet (bra primitive j, ket primitive p<ktag>): Boys values, the R
-        recursion and the ket transform into W."""
+        """One primitive quartet (bra primitive j, ket primitive p<ktag>): the R recursion from
+        its Boys values and the ket transform into W."""
         g.w("{")
         g.ind += 1
-        g.w("const double pq = p%d + %s;" % (j, qname))
-        g.w("const double rpq = rsqrt(pq);")
-        g.w("const double rho = p%d * %s * (rpq * rpq);" % (j, qname))
-        g.w("const double PQx = pb%d.Px - p%s.Px, PQy = pb%d.Py - p%s.Py, PQz = pb%d.Pz - p%s.Pz;"
-            % (j, ktag, j, ktag, j, ktag))
-        g.w("const double Tb = rho * (PQx * PQx + PQy * PQy + PQz * PQz);")
-        g.w("double F[%d];" % (L + 1))
-        g.w("boys_eval_sm<%d>(Tb, boys_tab, F);" % L)
-        g.w("double fac = pb%d.Kp * p%s.Kp * rpq;" % (j, ktag))
+        v = "%d%s" % (j, ktag)
+        g.w("double fac = pb%d.Kp * p%s.Kp * arg%s.y;" % (j, ktag, v))
         if L > 0:
-            g.w("const double m2r = -2.0 * rho;")
+            g.w("const double m2r = -2.0 * pm%s * (arg%s.y * arg%s.y);" % (v, v, v))
         for n in range(L + 1):
-            g.w("const T %s%d_0_0_0 = T(fac * F[%d]);" % (r, n, n))
+            g.w("const T %s%d_0_0_0 = T(fac * G%s[%d]);" % (r, n, v, n))
             if n < L:
                 g.w("fac *= m2r;")
         if L > 0:
-            g.w("const T Xpq = T(PQx), Ypq = T(PQy), Zpq = T(PQz);")
+            g.w("const T Xpq = T(PQx%s), Ypq = T(PQy%s), Zpq = T(PQz%s);" % (v, v, v))
         for n in range(L - 1, -1, -1):
             for tot in range(1, L - n + 1):
                 for (t, u, v) in cart_list(tot):
@@ -312,30 +324,32 @@ def _emit_tile(g, nbt, la, lb, lc, ld, ca, cb, cc, cd, hp, hidx, ncd, members=No
         g.ind += 1
         tiles = []
         for m in range(nkt):
-            g.w("const PrimPair pk%d = ket[ik + %d];" % (m, m))
+            g.w("const PrimPair pk%d = prim_at(ket, ik + %d);" % (m, m))
         for m in range(nkt):
             tiles.append(ket_quantities("k%d" % m, "qk%d" % m, "kc%d_" % m))
+        boys([(j, "k%d" % m, "qk%d" % m) for j in range(nbt) for m in range(nkt)])
         for j in range(nbt):
             for m in range(nkt):
                 chain(j, "k%d" % m, "qk%d" % m, tiles[m], "r%dk%d_" % (j, m))
         g.ind -= 1
         g.w("}")
         g.w("PrimPair pk_next;")
-        g.w("if (ik < nket) pk_next = ket[ik];")
+        g.w("if (ik < nket) pk_next = prim_at(ket, ik);")
         g.w("for (; ik < nket; ++ik) {")
     elif prefetch:
         g.w("PrimPair pk_next;")
-        g.w("if (nket > 0) pk_next = ket[0];")
+        g.w("if (nket > 0) pk_next = prim_at(ket, 0);")
         g.w("for (int ik = 0; ik < nket; ++ik) {")
     else:
         g.w("for (int ik = 0; ik < nket; ++ik) {")
     g.ind += 1
     if prefetch or nkt > 1:
         g.w("const PrimPair pk = pk_next;")
-        g.w("if (ik + 1 < nket) pk_next = ket[ik + 1];")
+        g.w("if (ik + 1 < nket) pk_next = prim_at(ket, ik + 1);")
     else:
-        g.w("const PrimPair pk = ket[ik];")
+        g.w("const PrimPair pk = prim_at(ket, ik);")
     kterms = ket_quantities("k", "q", "kc_")
+    boys([(j, "k", "q") for j in range(nbt)])
     for j in range(nbt):
         chain(j, "k", "q", kterms, "r%d_" % j)
     g.ind -= 1
@@ -384,11 +398,11 @@ def gen_class(la, lb, lc, ld, pa, pb, pc, pd, nbt=1, members=None, nkt=1, prefet
     hidx = {h: k for k, h in enumerate(hp)}
     mb, mk = members if members else (1, 1)
     g = Gen()
-    g.lines.append("template <typename T>")
+    g.lines.append("template <typename T, typename Prims>" if not members else "template <typename T>")
     if not members:
         name = "eri_%d%d%d%d" % (la, lb, lc, ld)
-        g.lines.append("__device__ __forceinline__ void %s(const PrimPair* __restrict__ bra, int nbra,"
-                       " const PrimPair* __restrict__ ket, int nket, double3 A, double3 B, double3 C,"
+        g.lines.append("__device__ __forceinline__ void %s(const Prims bra, int nbra,"
+                       " const Prims ket, int nket, double3 A, double3 B, double3 C,"
                        " double3 D, const double* __restrict__ boys_tab, T* __restrict__ out) {" % name)
     else:
         name = "eri_gc_%d%d%d%d_%dx%d" % (la, lb, lc, ld, mb, mk)
@@ -542,36 +556,56 @@ def members_header(specs):
     return "\n".join(parts) + "\n"
 
 
-# The Boys function's table (eri_common.cuh): BOYS_NT points T_i = 0.1 i, orders 0..BOYS_NORD-1.
-BOYS_NT, BOYS_NORD, BOYS_NTAYLOR, BOYS_MAXL = 361, 32, 8, 12
+# The Boys function's table and rows (eri_common.cuh): BOYS_NT points T_i = 0.1 i, orders
+# 0..BOYS_NORD-1; rows of L on the points i / 8 up to BOYS_TMAX[L], then the far row.
+BOYS_NT, BOYS_NORD, BOYS_NTAYLOR, BOYS_MAXL = 521, 32, 8, 12
+BOYS_TMAX = [36, 40, 44, 47, 50, 52] + [36] * 7
+
+
+def boys_values(T, nmax):
+    """F_0..F_nmax at the points T (extended precision): the highest order from its ascending
+    series, the lower ones by F_m = (2 T F_{m+1} + e^-T) / (2 m + 1)."""
+    ld = np.longdouble
+    T = np.asarray(T, dtype=ld)
+    ex = np.exp(-T)
+    term = np.full(len(T), ld(1) / ld(2 * nmax + 1))
+    tot = term.copy()
+    for k in range(1, 500):
+        term = term * (ld(2) * T / ld(2 * nmax + 2 * k + 1))
+        tot += term
+    F = [None] * (nmax + 1)
+    F[nmax] = ex * tot
+    for m in range(nmax - 1, -1, -1):
+        F[m] = (ld(2) * T * F[m + 1] + ex) / ld(2 * m + 1)
+    return np.stack(F, 1), ex
+
+
+def boys_rows(L):
+    """Rows of total angular momentum L, (points + far row) x 10."""
+    ld = np.longdouble
+    n = 8 * BOYS_TMAX[L] + 1
+    base, nc = (0, 10) if L == 1 else (L, BOYS_NTAYLOR + 1)
+    F, ex = boys_values(np.arange(n, dtype=ld) / ld(8), base + nc)
+    fact = np.cumprod(np.array([1] + list(range(1, nc)), dtype=ld))
+    rows = np.zeros((n + 1, BOYS_NTAYLOR + 2), dtype=ld)
+    rows[:n, :nc] = F[:, base:base + nc] / fact
+    if L != 1:
+        rows[:n, nc] = ex
+    c = np.sqrt(ld("3.14159265358979323846264338327950288")) / 2
+    for k in range(base):
+        c = c * ld(2 * k + 1) / 2
+    rows[n, 0] = c
+    if L == 1:
+        rows[n, 1] = c / 2
+    return rows.astype(np.float64)
 
 
 def boys_header():
     """Header text with the Boys tables as constants of the module: kBoysTable (F_n(0.1 i),
-    then exp(-0.1 i)) and kBoysRows (per L = 0..BOYS_MAXL the rows of load_boys).  The highest
-    order comes from its ascending series in extended precision, the lower ones by downward
-    recursion F_m = (2 T F_{m+1} + e^-T) / (2 m + 1)."""
-    ld = np.longdouble
-    T = np.arange(BOYS_NT, dtype=ld) / ld(10)
-    nmax = BOYS_NORD - 1
-    ex = np.exp(-T)
-    term = np.full(BOYS_NT, ld(1) / ld(2 * nmax + 1))
-    tot = term.copy()
-    for k in range(1, 400):
-        term = term * (ld(2) * T / ld(2 * nmax + 2 * k + 1))
-        tot += term
-    F = [None] * BOYS_NORD
-    F[nmax] = ex * tot
-    for m in range(nmax - 1, -1, -1):
-        F[m] = (ld(2) * T * F[m + 1] + ex) / ld(2 * m + 1)
-    F = np.stack(F, 1)                      # [i][n]
+    then exp(-0.1 i)) and kBoysRows (the rows of L = 0..BOYS_MAXL, one after the other)."""
+    F, ex = boys_values(np.arange(BOYS_NT, dtype=np.longdouble) / np.longdouble(10), BOYS_NORD - 1)
     table = np.concatenate([F.reshape(-1), ex]).astype(np.float64)
-    inv_fact = [ld(1)]
-    for k in range(1, BOYS_NTAYLOR + 1):
-        inv_fact.append(inv_fact[-1] / ld(k))
-    rows = np.concatenate([
-        np.concatenate([F[:, L:L + BOYS_NTAYLOR + 1] * np.array(inv_fact), ex[:, None]], 1).reshape(-1)
-        for L in range(BOYS_MAXL + 1)]).astype(np.float64)
+    rows = np.concatenate([boys_rows(L).reshape(-1) for L in range(BOYS_MAXL + 1)])
 
     def array(name, v):
         body = ",\n".join(", ".join(repr(float(x)) for x in v[k:k + 8]) for k in range(0, len(v), 8))
@@ -580,6 +614,7 @@ def boys_header():
         "// GENERATED by gen_eri.py (Boys tables) -- do not edit.", "#pragma once",
         "static_assert(BOYS_NT == %d && BOYS_NORD == %d && BOYS_NTAYLOR == %d && BOYS_MAXL == %d, \"table layout\");"
         % (BOYS_NT, BOYS_NORD, BOYS_NTAYLOR, BOYS_MAXL),
+        "static_assert(boys_rows_off(BOYS_MAXL + 1) == %d, \"rows layout\");" % len(rows),
         array("kBoysTable", table), array("kBoysRows", rows), ""])
 
 
@@ -600,8 +635,8 @@ def main(path, maxl=2):
                             prefetch=(la, lb, lc, ld) not in NO_KET_PREFETCH)
         parts.append(code)
         parts.append("template <> struct EriClass<%d, %d, %d, %d> {" % (la, lb, lc, ld))
-        parts.append("  template <typename T> static __device__ __forceinline__ void run(const PrimPair* bra, int nbra,"
-                     " const PrimPair* ket, int nket, double3 A, double3 B, double3 C, double3 D,"
+        parts.append("  template <typename T, typename Prims> static __device__ __forceinline__ void run(const Prims bra, int nbra,"
+                     " const Prims ket, int nket, double3 A, double3 B, double3 C, double3 D,"
                      " const double* boys_tab, T* out) {")
         parts.append("    eri_%d%d%d%d<T>(bra, nbra, ket, nket, A, B, C, D, boys_tab, out);" % (la, lb, lc, ld))
         parts.append("  }")

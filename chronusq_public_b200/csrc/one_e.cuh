@@ -356,7 +356,7 @@ __global__ void OE_BOUNDS
                   const double *__restrict__ Zc, const double3 *__restrict__ Rc, const double *__restrict__ boys,
                   double *S0, double *T0, double *V0, int ld, OneEMols om) {
   constexpr int NC = oe_ncart(LA) * oe_ncart(LB);
-  __align__(16) OE_SHARED double rows[BOYS_ROWS_SIZE];
+  __align__(16) OE_SHARED double rows[boys_rows_size(LA + LB)];
   OE_SHARED double blocks[OE_WARPS][NC];
 #ifdef __CUDACC__
   load_boys<LA + LB>(boys, rows);
