@@ -579,6 +579,94 @@ static const eri_launcher *const kEriLaunch = kEriTables.t;      // FP64 class l
 static const eri_launcher *const kEriLaunch32 = kEriTables.t + CQG_NQC;
 static inline eri_launcher list_launcher(int vb) { return kEriTables.t[vb]; }
 
+// Scratch of one contraction, in doubles: per group the accumulators Gh, Gh in the internal
+// order and the Coulomb sums by pair (d_G, one memset), per distinct X its copy in the
+// internal order and per group its Coulomb blocks by pair (d_XP).
+struct CallScratch {
+  size_t matrix, pairs;
+  explicit CallScratch(const cqg_ctx *ctx) : pairs(0) {
+    matrix = ctx->nmol > 1 ? (size_t)ctx->packed : (size_t)ctx->nbf * ctx->nbf;
+    for (int c = 0; c < CQG_NPC; ++c)
+      pairs += (size_t)(ctx->pc_beg[c + 1] - ctx->pc_beg[c]) * nfun(kPairClass[c][0]) * nfun(kPairClass[c][1]);
+  }
+  size_t group() const { return 2 * matrix + pairs; }
+  size_t inputs(int nx, int ng) const { return nx * matrix + ng * pairs; }
+};
+
+static DigestGroups make_digest(const cqg_ctx *ctx, int ng, const double *const *Xg, const double *sJ, const double *sK,
+                                int nx, const double *const *Xall, int ldx) {
+  const CallScratch cs(ctx);
+  DigestGroups dg;
+  memset(&dg, 0, sizeof(dg));
+  dg.ng = ng;
+  dg.ldx = ldx;
+  dg.batch = ctx->nmol > 1;
+  dg.xoff = ctx->d_mxoff.p;
+  dg.nbf = ctx->d_mnbf.p;
+  for (int g = 0; g < ng; ++g) {
+    int u = 0;
+    while (u < nx && Xall[u] != Xg[g]) ++u;
+    dg.X[g] = Xg[g];
+    dg.G[g] = ctx->d_G.p + g * cs.group();
+    dg.GP[g] = dg.G[g] + cs.matrix;
+    dg.JP[g] = dg.GP[g] + cs.matrix;
+    dg.XP[g] = ctx->d_XP.p + u * cs.matrix;
+    dg.DP[g] = ctx->d_XP.p + nx * cs.matrix + g * cs.pairs;
+    dg.sJ[g] = sJ[g];
+    dg.sK[g] = sK[g];
+  }
+  long long off = 0;
+  for (int c = 0; c < CQG_NPC; ++c) {
+    dg.joff[c] = off;
+    dg.jbeg[c] = ctx->pc_beg[c];
+    dg.jn[c] = ctx->pc_beg[c + 1] - ctx->pc_beg[c];
+    off += (long long)dg.jn[c] * nfun(kPairClass[c][0]) * nfun(kPairClass[c][1]);
+  }
+  return dg;
+}
+
+// Block norms, input checks, internal copies of X: everything the screening and the digests
+// read of the input matrices.  Zeroes the accumulators and counters first.
+static cqg_status launch_norms(cqg_ctx *ctx, const DigestGroups &dg, int nx, const double *const *Xall, int ldx,
+                               const Mols &mols, cudaStream_t st) {
+  const CallScratch cs(ctx);
+  CUCHK(cudaMemsetAsync(ctx->d_flags.p, 0, 4 * sizeof(int), st));
+  CUCHK(cudaMemsetAsync(ctx->d_Mmax.p, 0, sizeof(double), st));
+  CUCHK(cudaMemsetAsync(ctx->d_blkacc.p, 0, kBlkAcc * CQG_NQC * sizeof(unsigned long long), st));
+  CUCHK(cudaMemsetAsync(ctx->d_mhead.p, 0, sizeof(unsigned long long), st));
+  CUCHK(cudaMemsetAsync(ctx->d_G.p, 0, dg.ng * cs.group() * sizeof(double), st));
+  XList xl;
+  xl.n = nx;
+  for (int i = 0; i < nx; ++i) {
+    xl.X[i] = Xall[i];
+    xl.P[i] = ctx->d_XP.p + i * cs.matrix;
+  }
+  dim3 g((ctx->max_nsh + 127) / 128, ctx->max_nsh, ctx->nmol);
+  k_blocknorm<<<g, 128, 0, st>>>(xl, ldx, mols, ctx->d_bf.p, ctx->d_sz.p, ctx->d_pf.p, ctx->d_M.p,
+                                 ctx->d_M.p + ctx->Mtotal, ctx->d_flags.p, 1e-12);
+  const long long nn = ctx->Mtotal;
+  k_maxreduce<<<(int)std::min<long long>((nn + 255) / 256, 1184), 256, 0, st>>>(ctx->d_M.p, nn, ctx->d_Mmax.p);
+  const int npairs = (int)ctx->pair_sh.size();
+  k_pairnorm<<<(npairs + 255) / 256, 256, 0, st>>>(ctx->d_pair_sh.p, npairs, mols, make_shells(ctx), ctx->d_shL.p,
+                                                   ctx->d_sz.p, ctx->d_M.p, ctx->d_Mpair.p, dg);
+  CUCHK(cudaGetLastError());
+  return CQG_OK;
+}
+
+// AX += 0.5 (Gh + Gh^T) of every group, once the class launches are done.
+static cqg_status launch_finalize(cqg_ctx *ctx, const DigestGroups &dg, double *const *AXg, int ldax, const Mols &mols,
+                                  cudaStream_t st) {
+  const int npairs = (int)ctx->pair_sh.size();
+  k_pair_add<<<(npairs + 255) / 256, 256, 0, st>>>(ctx->d_pair_sh.p, npairs, mols, make_shells(ctx), ctx->d_shL.p,
+                                                   ctx->d_sz.p, dg);
+  for (int g = 0; g < dg.ng; ++g) {
+    dim3 grid((ctx->max_nbf + 31) / 32, (ctx->max_nbf + 31) / 32, ctx->nmol), blk(32, 8);
+    k_finalize<<<grid, blk, 0, st>>>(dg.G[g], dg.GP[g], mols, AXg[g], ldax);
+  }
+  CUCHK(cudaGetLastError());
+  return CQG_OK;
+}
+
 // The class launches of one contraction, dealt in turn to the caller's stream and the side
 // streams: fork() makes the side streams wait for what the caller's stream holds so far,
 // next() gives the stream of the next launch, join() makes the caller's stream wait for the
@@ -755,7 +843,8 @@ cqg_status cqg_destroy(cqg_ctx *ctx) {
   ctx->d_shmol.release(); ctx->d_mshoff.release(); ctx->d_mnsh.release(); ctx->d_mnbf.release();
   ctx->d_molbk.release(); ctx->d_mxoff.release(); ctx->d_mMoff.release(); ctx->d_active.release();
   ctx->d_prim.release(); ctx->d_exp.release(); ctx->d_setup.release();
-  ctx->d_cols.release(); ctx->d_pair_coff.release();
+  ctx->d_cols.release(); ctx->d_pair_coff.release(); ctx->d_pf.release(); ctx->d_pos.release(); ctx->d_mfoff.release();
+  ctx->d_XP.release();
   ctx->d_M.release(); ctx->d_Mmax.release(); ctx->d_Mpair.release(); ctx->d_flags.release();
   ctx->d_cnt.release(); ctx->d_off.release(); ctx->d_range.release(); ctx->d_scan_tmp.release();
   ctx->d_qhead.release();
@@ -886,14 +975,32 @@ cqg_status cqg_set_basis_batch(cqg_ctx *ctx, int nmol, const int *nshell_per_mol
     ctx->Mtotal = mo;
   }
   ctx->nbf = ctx->m_nbf[0];
+  // internal order of each molecule's functions: by angular momentum, component, shell
+  std::vector<int2> pf(nshell);
+  std::vector<int> foff(nmol), pos;
+  for (int m = 0; m < nmol; ++m) {
+    const int s0 = ctx->m_shoff[m], s1 = s0 + ctx->m_nsh[m];
+    int first[CQG_MAXL + 2] = {0}, count[CQG_MAXL + 1] = {0}, rank[CQG_MAXL + 1] = {0};
+    for (int s = s0; s < s1; ++s) ++count[L[s]];
+    for (int l = 0; l <= CQG_MAXL; ++l) first[l + 1] = first[l] + count[l] * nfun(l);
+    foff[m] = (int)pos.size();
+    for (int s = s0; s < s1; ++s) {
+      pf[s] = make_int2(first[L[s]] + rank[L[s]]++, count[L[s]]);
+      for (int k = 0; k < ctx->hsz[s]; ++k) pos.push_back(pf[s].x + k * pf[s].y);
+    }
+  }
   // shells and molecule layout to device
   std::vector<double3> c3(nshell);
   for (int s = 0; s < nshell; ++s) c3[s] = make_double3(centers[3 * s], centers[3 * s + 1], centers[3 * s + 2]);
   if (ctx->d_center.reserve(nshell) || ctx->d_bf.reserve(nshell) || ctx->d_sz.reserve(nshell) ||
       ctx->d_shmol.reserve(nshell) || ctx->d_mshoff.reserve(nmol) || ctx->d_mnsh.reserve(nmol) ||
       ctx->d_mnbf.reserve(nmol) || ctx->d_mxoff.reserve(nmol) || ctx->d_mMoff.reserve(nmol) ||
-      ctx->d_active.reserve(nmol))
+      ctx->d_active.reserve(nmol) || ctx->d_pf.reserve(nshell) || ctx->d_pos.reserve(pos.size()) ||
+      ctx->d_mfoff.reserve(nmol))
     return CQG_ERR_OOM;
+  CUCHK(cudaMemcpyAsync(ctx->d_pf.p, pf.data(), nshell * sizeof(int2), cudaMemcpyHostToDevice, 0));
+  CUCHK(cudaMemcpyAsync(ctx->d_pos.p, pos.data(), pos.size() * sizeof(int), cudaMemcpyHostToDevice, 0));
+  CUCHK(cudaMemcpyAsync(ctx->d_mfoff.p, foff.data(), nmol * sizeof(int), cudaMemcpyHostToDevice, 0));
   CUCHK(cudaMemcpyAsync(ctx->d_center.p, c3.data(), nshell * sizeof(double3), cudaMemcpyHostToDevice, 0));
   CUCHK(cudaMemcpyAsync(ctx->d_bf.p, ctx->hbf.data(), nshell * sizeof(int), cudaMemcpyHostToDevice, 0));
   CUCHK(cudaMemcpyAsync(ctx->d_sz.p, ctx->hsz.data(), nshell * sizeof(int), cudaMemcpyHostToDevice, 0));
@@ -1129,7 +1236,6 @@ cqg_status cqg_get_schwarz(cqg_ctx *ctx, double *Q) {
   return CQG_OK;
 }
 
-// Whether quartet class k goes through the class-fused kernel of `tier` (0: none).
 // whether work list vb (part * CQG_NQC + class) goes through the class-fused kernel of
 // `tier` (the pair entries of the tier's classes; a class index k < CQG_NQC is its FP64 list)
 static bool class_fused(int tier, int vb) {
@@ -1145,11 +1251,13 @@ static bool class_fused(int tier, int vb) {
 // digest pointed at scratch accumulators, and keep the fastest.
 static cqg_status autotune_shapes(cqg_ctx *ctx, const long long *crange, cudaStream_t st, const DigestGroups &dg) {
   DigestGroups scratch = dg;
-  size_t per = 0;
-  for (int g = 0; g < dg.ng; ++g) per = std::max<size_t>(per, 1);
-  const size_t gsize = ctx->nmol > 1 ? (size_t)ctx->packed : (size_t)ctx->nbf * ctx->nbf;
-  if (ctx->d_Gscratch.reserve(gsize) != cudaSuccess) return CQG_ERR_OOM;
-  for (int g = 0; g < dg.ng; ++g) scratch.G[g] = ctx->d_Gscratch.p;
+  const CallScratch cs(ctx);
+  if (ctx->d_Gscratch.reserve(cs.group()) != cudaSuccess) return CQG_ERR_OOM;
+  for (int g = 0; g < dg.ng; ++g) {
+    scratch.G[g] = ctx->d_Gscratch.p;
+    scratch.GP[g] = scratch.G[g] + cs.matrix;
+    scratch.JP[g] = scratch.GP[g] + cs.matrix;
+  }
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -1282,29 +1390,17 @@ static cqg_status contract_graph(cqg_ctx *ctx, int ngroups, const double *const 
                                  const double *sJ, const double *sK, int nx_all, const double *const *Xall, int ldx,
                                  int ldax, cudaStream_t st) {
   const Mols mols = make_mols(ctx);
-  const size_t gsize = ctx->nmol > 1 ? (size_t)ctx->packed : (size_t)ctx->nbf * ctx->nbf;
-  if ((size_t)ngroups * gsize > ctx->d_G.n || (size_t)ctx->graph_capacity > ctx->d_qlist.n ||
-      (size_t)ctx->graph_capacity > ctx->d_qmask.n) {
+  const CallScratch scratch(ctx);
+  if ((size_t)ngroups * scratch.group() > ctx->d_G.n || scratch.inputs(nx_all, ngroups) > ctx->d_XP.n ||
+      (size_t)ctx->graph_capacity > ctx->d_qlist.n || (size_t)ctx->graph_capacity > ctx->d_qmask.n) {
     ctx->err = "graph mode: buffers were not reserved for this call (cqg_set_graph_mode)";
     return CQG_ERR_STATE;
   }
-  XList xl;
-  xl.n = nx_all;
-  for (int i = 0; i < nx_all; ++i) xl.X[i] = Xall[i];
   const double cut32 = ctx->policy == CQG_PREC_MIXED ? ctx->fp32_cutoff : 0.0;
-  CUCHK(cudaMemsetAsync(ctx->d_flags.p, 0, 4 * sizeof(int), st));
-  CUCHK(cudaMemsetAsync(ctx->d_Mmax.p, 0, sizeof(double), st));
-  CUCHK(cudaMemsetAsync(ctx->d_blkacc.p, 0, kBlkAcc * CQG_NQC * sizeof(unsigned long long), st));
-  CUCHK(cudaMemsetAsync(ctx->d_mhead.p, 0, sizeof(unsigned long long), st));
-  CUCHK(cudaMemsetAsync(ctx->d_G.p, 0, (size_t)ngroups * gsize * sizeof(double), st));
+  const DigestGroups dg = make_digest(ctx, ngroups, Xg, sJ, sK, nx_all, Xall, ldx);
   {
-    dim3 g((ctx->max_nsh + 127) / 128, ctx->max_nsh, ctx->nmol);
-    k_blocknorm<<<g, 128, 0, st>>>(xl, ldx, mols, ctx->d_bf.p, ctx->d_sz.p, ctx->d_M.p, ctx->d_M.p + ctx->Mtotal, ctx->d_flags.p, 1e-12);
-    const long long nn = ctx->Mtotal;
-    k_maxreduce<<<(int)std::min<long long>((nn + 255) / 256, 1184), 256, 0, st>>>(ctx->d_M.p, nn, ctx->d_Mmax.p);
-    const int npairs = (int)ctx->pair_sh.size();
-    k_pairnorm<<<(npairs + 255) / 256, 256, 0, st>>>(ctx->d_pair_sh.p, npairs, mols, ctx->d_shmol.p, ctx->d_M.p,
-                                                     ctx->d_Mpair.p);
+    const cqg_status ns = launch_norms(ctx, dg, nx_all, Xall, ldx, mols, st);
+    if (ns != CQG_OK) return ns;
   }
   Pairs P = make_pairs(ctx);
   const int nb = (ctx->ntask + 7) / 8;
@@ -1322,19 +1418,6 @@ static cqg_status contract_graph(cqg_ctx *ctx, int ngroups, const double *const 
                                         (long long)kListParts * ctx->ntask, 0, ctx->graph_capacity,
                                         make_mask_cache(ctx));
   CUCHK(cudaGetLastError());
-  DigestGroups dg;
-  memset(&dg, 0, sizeof(dg));
-  dg.ng = ngroups;
-  dg.ldx = ldx;
-  dg.batch = ctx->nmol > 1;
-  dg.xoff = ctx->d_mxoff.p;
-  dg.nbf = ctx->d_mnbf.p;
-  for (int g = 0; g < ngroups; ++g) {
-    dg.X[g] = Xg[g];
-    dg.G[g] = ctx->d_G.p + (size_t)g * gsize;
-    dg.sJ[g] = sJ[g];
-    dg.sK[g] = sK[g];
-  }
   CUCHK(cudaMemsetAsync(ctx->d_qhead.p, 0, CQG_NLIST * sizeof(unsigned long long), st));
   int launches = 7;   // block norms, max, pair norms, list count, scan, ranges, list fill
   if (ctx->fused_tier) {
@@ -1369,12 +1452,11 @@ static cqg_status contract_graph(cqg_ctx *ctx, int ngroups, const double *const 
     }
   }
   CUCHK(cs.join());
-  for (int g = 0; g < ngroups; ++g) {
-    dim3 grid((ctx->max_nbf + 31) / 32, (ctx->max_nbf + 31) / 32, ctx->nmol), blk(32, 8);
-    k_finalize<<<grid, blk, 0, st>>>(dg.G[g], mols, AXg[g], ldax);
-    ++launches;
+  {
+    const cqg_status fs = launch_finalize(ctx, dg, AXg, ldax, mols, st);
+    if (fs != CQG_OK) return fs;
   }
-  CUCHK(cudaGetLastError());
+  launches += 1 + ngroups;
   ctx->launches = launches;
   ctx->stats.launches = launches;
   return CQG_OK;
@@ -1383,10 +1465,14 @@ static cqg_status contract_graph(cqg_ctx *ctx, int ngroups, const double *const 
 static cqg_status contract_device(cqg_ctx *ctx, int ngroups, const double *const *Xg, double *const *AXg,
                                   const double *sJ, const double *sK, int nx_all, const double *const *Xall,
                                   int ldx, int ldax, cudaStream_t st) {
-  const int n = ctx->nbf;
   const Mols mols = make_mols(ctx);
-  // Gh of every molecule: n x n for one molecule, packed per molecule for a batch
-  const size_t gsize = ctx->nmol > 1 ? (size_t)ctx->packed : (size_t)n * n;
+  const CallScratch scratch(ctx);
+  if (ctx->d_G.reserve((size_t)ngroups * scratch.group()) != cudaSuccess ||
+      ctx->d_XP.reserve(scratch.inputs(nx_all, ngroups)) != cudaSuccess) {
+    ctx->err = "accumulator allocation failed";
+    return CQG_ERR_OOM;
+  }
+  const DigestGroups dg = make_digest(ctx, ngroups, Xg, sJ, sK, nx_all, Xall, ldx);
   // the survivor-mask cache: grow it to what the last count pass asked for (tasks that did
   // not fit tested their bounds twice), before this call's first launch; never in graph
   // mode, whose captured launches hold the buffer's address
@@ -1400,27 +1486,11 @@ static cqg_status contract_device(cqg_ctx *ctx, int ngroups, const double *const
   }
   if (ctx->timing) CUCHK(cudaEventRecord(ctx->ev[0], st));
   // 1. block norms + checks
-  XList xl;
-  xl.n = nx_all;
-  for (int i = 0; i < nx_all; ++i) xl.X[i] = Xall[i];
-  CUCHK(cudaMemsetAsync(ctx->d_flags.p, 0, 4 * sizeof(int), st));
-  CUCHK(cudaMemsetAsync(ctx->d_Mmax.p, 0, sizeof(double), st));
-  CUCHK(cudaMemsetAsync(ctx->d_blkacc.p, 0, kBlkAcc * CQG_NQC * sizeof(unsigned long long), st));
-  CUCHK(cudaMemsetAsync(ctx->d_mhead.p, 0, sizeof(unsigned long long), st));
   const double cut32 = ctx->policy == CQG_PREC_MIXED ? ctx->fp32_cutoff : 0.0;
-  ctx->launches = 0;
   {
-    dim3 g((ctx->max_nsh + 127) / 128, ctx->max_nsh, ctx->nmol);
-    k_blocknorm<<<g, 128, 0, st>>>(xl, ldx, mols, ctx->d_bf.p, ctx->d_sz.p, ctx->d_M.p, ctx->d_M.p + ctx->Mtotal, ctx->d_flags.p, 1e-12);
-    CUCHK(cudaGetLastError());
-    long long nn = ctx->Mtotal;
-    int nb = (int)std::min<long long>((nn + 255) / 256, 1184);
-    k_maxreduce<<<nb, 256, 0, st>>>(ctx->d_M.p, nn, ctx->d_Mmax.p);
-    const int npairs = (int)ctx->pair_sh.size();
-    k_pairnorm<<<(npairs + 255) / 256, 256, 0, st>>>(ctx->d_pair_sh.p, npairs, mols, ctx->d_shmol.p, ctx->d_M.p,
-                                                     ctx->d_Mpair.p);
-    CUCHK(cudaGetLastError());
-    ctx->launches += 3;
+    const cqg_status ns = launch_norms(ctx, dg, nx_all, Xall, ldx, mols, st);
+    if (ns != CQG_OK) return ns;
+    ctx->launches = 3;
   }
   // 2. quartet lists
   Pairs P = make_pairs(ctx);
@@ -1498,21 +1568,6 @@ static cqg_status contract_device(cqg_ctx *ctx, int ngroups, const double *const
     return CQG_ERR_OOM;
   }
   ctx->stats.chunks = (long long)chunk_vt.size() - 1;
-  if (ctx->d_G.reserve((size_t)ngroups * gsize) != cudaSuccess) return CQG_ERR_OOM;
-  CUCHK(cudaMemsetAsync(ctx->d_G.p, 0, (size_t)ngroups * gsize * sizeof(double), st));
-  DigestGroups dg;
-  memset(&dg, 0, sizeof(dg));
-  dg.ng = ngroups;
-  dg.ldx = ldx;
-  dg.batch = ctx->nmol > 1;
-  dg.xoff = ctx->d_mxoff.p;
-  dg.nbf = ctx->d_mnbf.p;
-  for (int g = 0; g < ngroups; ++g) {
-    dg.X[g] = Xg[g];
-    dg.G[g] = ctx->d_G.p + (size_t)g * gsize;
-    dg.sJ[g] = sJ[g];
-    dg.sK[g] = sK[g];
-  }
   memset(ctx->stats.class_quartets, 0, sizeof(ctx->stats.class_quartets));
   memset(ctx->stats.class_ms, 0, sizeof(ctx->stats.class_ms));
   ctx->stats.ms_fused = 0.0;
@@ -1649,11 +1704,10 @@ static cqg_status contract_device(cqg_ctx *ctx, int ngroups, const double *const
   }
   if (ctx->timing) CUCHK(cudaEventRecord(ctx->ev[2], st));
   // 4. AX += 0.5 (Gh + Gh^T)
-  for (int g = 0; g < ngroups; ++g) {
-    dim3 grid((ctx->max_nbf + 31) / 32, (ctx->max_nbf + 31) / 32, ctx->nmol), blk(32, 8);
-    k_finalize<<<grid, blk, 0, st>>>(dg.G[g], mols, AXg[g], ldax);
-    CUCHK(cudaGetLastError());
-    ctx->launches += 1;
+  {
+    const cqg_status fs = launch_finalize(ctx, dg, AXg, ldax, mols, st);
+    if (fs != CQG_OK) return fs;
+    ctx->launches += 1 + ngroups;
   }
   if (ctx->timing) CUCHK(cudaEventRecord(ctx->ev[3], st));
   ctx->stats.quartets = nquart;
@@ -1964,9 +2018,10 @@ cqg_status cqg_set_graph_mode(cqg_ctx *ctx, long long capacity, int max_groups) 
   CUCHK(cudaSetDevice(ctx->device));
   ctx->graph_capacity = capacity;
   if (capacity > 0) {
-    const size_t gsize = ctx->nmol > 1 ? (size_t)ctx->packed : (size_t)ctx->nbf * ctx->nbf;
+    const CallScratch cs(ctx);
+    const int ng = std::max(max_groups, 1);
     if (ctx->d_qlist.reserve((size_t)capacity) || ctx->d_qmask.reserve((size_t)capacity) ||
-        ctx->d_G.reserve((size_t)std::max(max_groups, 1) * gsize)) {
+        ctx->d_G.reserve(ng * cs.group()) || ctx->d_XP.reserve(cs.inputs(ng, ng))) {
       ctx->graph_capacity = 0;
       return CQG_ERR_OOM;
     }

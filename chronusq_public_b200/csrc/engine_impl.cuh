@@ -91,6 +91,12 @@ struct Shells {
   const double3 *center;
   const int *bf;     // first basis function of the shell within its molecule
   const int *mol;    // molecule of the shell
+  // the shell's functions in the internal order of the per-thread classes: component k is
+  // function pf.x + k pf.y of its molecule.  Shells of one angular momentum are together,
+  // component by component: the lanes of a warp hold kets of one class at one bra, and their
+  // exchange blocks X(c, a), Gh(c, a) then lie in a few lines of column a (for (H2O)_32 cc-pVDZ,
+  // 8 for a p component instead of up to 32 of the 48 of a column)
+  const int2 *pf;
 };
 
 // Per-molecule layout: a context holds nmol >= 1 molecules (a batch).  Matrices of
@@ -103,6 +109,8 @@ struct Mols {
   const long long *Moff;         // offset of molecule m's nsh_m x nsh_m block-norm matrix
   const long long *xoff;         // offset of molecule m's matrices in packed storage
   const int *nbf;                // basis functions of molecule m
+  const int *foff;               // basis functions of the molecules before m
+  const int *pos;                // [foff[m] + r]: internal position of function r (Shells.pf)
   const unsigned char *active;   // molecule m takes part in the call
   const int *molbk;              // [m][ket pair class][bucket + 1]: first pair of each bucket
   const int *molgbk;             // the same in group index space: first group of each bucket
@@ -149,6 +157,15 @@ struct DigestGroups {
   int batch;                      // matrices are packed per molecule (Mols.xoff / nbf)
   const long long *xoff;
   const int *nbf;
+  // for the per-thread classes: X and Gh in the internal order (leading dimension nbf), and the
+  // Coulomb blocks by shell pair, component k of pair i of class c at joff[c] + k jn[c] + i -
+  // jbeg[c]: the kets of a warp are nearly consecutive pairs
+  const double *XP[CQG_MAXG];
+  double *GP[CQG_MAXG];
+  const double *DP[CQG_MAXG];
+  double *JP[CQG_MAXG];
+  long long joff[CQG_NPC];
+  int jn[CQG_NPC], jbeg[CQG_NPC];
 };
 
 // base pointers and leading dimensions of molecule m's X and Gh
@@ -198,10 +215,11 @@ __global__ void __launch_bounds__(128) k_schwarz(Pairs P, Shells S, const double
 // Block norms M(s1,s2) = max over matrices of max|X_i(block)|, and input checks.
 struct XList {
   const double *X[8];
+  double *P[8];   // the same in the internal order (Shells.pf), written here
   int n;
 };
 static __global__ void k_blocknorm(XList xl, int ldx, Mols mols, const int *__restrict__ bf,
-                            const int *__restrict__ sz, double *__restrict__ M, double *__restrict__ MT,
+                            const int *__restrict__ sz, const int2 *__restrict__ pf, double *__restrict__ M, double *__restrict__ MT,
                             int *__restrict__ flags, double sym_tol) {
   const int mol = blockIdx.z;
   const int nsh = mols.nsh[mol];
@@ -219,10 +237,13 @@ static __global__ void k_blocknorm(XList xl, int ldx, Mols mols, const int *__re
   int r0 = bf[g1], c0 = bf[g2], nr = sz[g1], nc = sz[g2];
   if (mols.nmol > 1) ldx = mols.nbf[mol];
   const long long xo = mols.nmol > 1 ? mols.xoff[mol] : 0;
+  const int n = mols.nbf[mol];
+  const int2 p1 = pf[g1], p2 = pf[g2];
   double mx = 0.0;
   int bad = 0, asym = 0;
   for (int m = 0; m < xl.n; ++m) {
     const double *X = xl.X[m] + xo;
+    double *P = xl.P[m] + xo;
     for (int c = 0; c < nc; ++c)
       for (int r = 0; r < nr; ++r) {
         double v = X[(size_t)(r0 + r) + (size_t)(c0 + c) * ldx];
@@ -231,6 +252,7 @@ static __global__ void k_blocknorm(XList xl, int ldx, Mols mols, const int *__re
         double av = fabs(v);
         mx = fmax(mx, av);
         if (fabs(v - t) > sym_tol * fmax(1.0, av)) asym = 1;
+        P[(size_t)(p1.x + r * p1.y) + (size_t)(p2.x + c * p2.y) * n] = v;
       }
   }
   Mm[(size_t)s1 + (size_t)s2 * nsh] = mx;
@@ -305,15 +327,46 @@ __device__ __forceinline__ double quartet_bound(const double *__restrict__ col1,
   return m * qab * qcd;
 }
 
-// Mpair[i] = M(a, b) of shell pair i (its own block norm; molecule-local indices).
-static __global__ void k_pairnorm(const int2 *__restrict__ sh, int npairs, Mols mols, const int *__restrict__ shmol,
-                                  const double *__restrict__ M, double *__restrict__ Mpair) {
+// Mpair[i] = M(a, b) of shell pair i (its own block norm; molecule-local indices), and the
+// pair's block of each X with a Coulomb part to DP.
+static __global__ void k_pairnorm(const int2 *__restrict__ sh, int npairs, Mols mols, Shells S,
+                                  const int *__restrict__ shL, const int *__restrict__ sz, const double *__restrict__ M,
+                                  double *__restrict__ Mpair, DigestGroups dg) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= npairs) return;
   const int2 ab = sh[i];
-  const int mol = shmol[ab.x];
+  const int mol = S.mol[ab.x];
   const int nsh = mols.nsh[mol], shoff = mols.shoff[mol];
   Mpair[i] = M[mols.Moff[mol] + (ab.x - shoff) + (size_t)(ab.y - shoff) * nsh];
+  if (!mols.active[mol]) return;
+  const int c = pair_class_c(shL[ab.x], shL[ab.y]), na = sz[ab.x], nb = sz[ab.y], a0 = S.bf[ab.x], b0 = S.bf[ab.y];
+  for (int g = 0; g < dg.ng; ++g) {
+    if (dg.sJ[g] == 0.0) continue;
+    const double *X;
+    double *G, *D = const_cast<double *>(dg.DP[g]) + dg.joff[c] + (i - dg.jbeg[c]);
+    size_t ld, n;
+    mol_view(dg, g, mol, X, G, ld, n);
+    for (int k = 0; k < na * nb; ++k) D[(size_t)k * dg.jn[c]] = X[(size_t)(b0 + k % nb) + (size_t)(a0 + k / nb) * ld];
+  }
+}
+
+// The Coulomb sums of the shell pairs (JP) into Gh, after every class launch.
+static __global__ void k_pair_add(const int2 *__restrict__ sh, int npairs, Mols mols, Shells S,
+                                  const int *__restrict__ shL, const int *__restrict__ sz, DigestGroups dg) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= npairs) return;
+  const int2 ab = sh[i];
+  const int mol = S.mol[ab.x];
+  if (!mols.active[mol]) return;
+  const int c = pair_class_c(shL[ab.x], shL[ab.y]), na = sz[ab.x], nb = sz[ab.y], a0 = S.bf[ab.x], b0 = S.bf[ab.y];
+  for (int g = 0; g < dg.ng; ++g) {
+    if (dg.sJ[g] == 0.0) continue;
+    const double *X, *J = dg.JP[g] + dg.joff[c] + (i - dg.jbeg[c]);
+    double *G;
+    size_t ld, n;
+    mol_view(dg, g, mol, X, G, ld, n);
+    for (int k = 0; k < na * nb; ++k) G[(size_t)(a0 + k / nb) + (size_t)(b0 + k % nb) * n] += J[(size_t)k * dg.jn[c]];
+  }
 }
 
 // Per-block screening tallies in blkacc[kBlkAcc * blk + ...]: model primitive quartets
@@ -726,77 +779,83 @@ __device__ __forceinline__ double warp_sum(double x) {
 // k_finalize).  All lanes of the warp call this; `valid` lanes hold a quartet, and when
 // every lane shares the bra pair (`bra_uniform`) the Gh(a,b) sums are reduced across the
 // warp before one atomic per element.
-template <int NA, int NB, int NC, int ND>
-__device__ __forceinline__ void digest(const double *v, double deg, int a0, int b0, int c0, int d0,
-                                       const DigestGroups &dg, bool valid, bool bra_uniform, int mol) {
+// Exchange updates go to Gh(c, a), Gh(d, b), Gh(d, a), Gh(c, b) and X is read in the same
+// orientation (both are symmetric in the end, k_finalize adds (Gh + Gh^T) / 2), so the bra
+// index, the same across a bra-uniform warp, is the column.  What bounds this part is the
+// number of lines a warp's loads and atomics touch: hence the internal order of X and Gh and
+// the Coulomb blocks by pair: (ps|ps) 5.69 -> 4.69 ms, (pp|ps) 4.20 -> 3.83, (ds|ps) 3.44 -> 3.00
+// per (H2O)_32 cc-pVDZ build, before the stripes of eri_jk_list.
+template <int LA, int LB, int LC, int LD>
+__device__ __forceinline__ void digest(const double *v, double deg, int bra, int ket, const Pairs &P, const Shells &S,
+                                       const DigestGroups &dg, bool valid, bool bra_uniform) {
+  constexpr int NA = nfun_c(LA), NB = nfun_c(LB), NC = nfun_c(LC), ND = nfun_c(LD);
+  constexpr int CB = pair_class_c(LA, LB), CK = pair_class_c(LC, LD);
   const int lane = threadIdx.x & 31;
+  const int2 ab = P.sh[bra], cd = P.sh[ket];
+  const int2 pa = S.pf[ab.x], pb = S.pf[ab.y], pc = S.pf[cd.x], pd = S.pf[cd.y];
+  const int mol = dg.batch ? S.mol[ab.x] : 0;
+  const size_t n = (size_t)dg.nbf[mol];
+  const long long xo = dg.batch ? dg.xoff[mol] : 0;
   for (int g = 0; g < dg.ng; ++g) {
-    const double *Xv;
-    double *G;
-    size_t ld, n;
-    mol_view(dg, g, mol, Xv, G, ld, n);
-    const double *__restrict__ X = Xv;
     const double sJ = dg.sJ[g] * deg;
     const double sK = 0.5 * dg.sK[g] * deg;
     if (dg.sJ[g] != 0.0) {
+      const long long jb = dg.joff[CB] + (bra - dg.jbeg[CB]), jk = dg.joff[CK] + (ket - dg.jbeg[CK]);
+      const int nb = dg.jn[CB], nk = dg.jn[CK];
+      const double *__restrict__ D = dg.DP[g];
+      double *J = dg.JP[g];
       double xdc[NC * ND], xba[NA * NB];
 #pragma unroll
-      for (int c = 0; c < NC; ++c)
+      for (int k = 0; k < NC * ND; ++k) xdc[k] = valid ? __ldg(D + jk + (long long)k * nk) : 0.0;
 #pragma unroll
-        for (int d = 0; d < ND; ++d) xdc[c * ND + d] = valid ? __ldg(X + (d0 + d) + (c0 + c) * ld) : 0.0;
+      for (int k = 0; k < NA * NB; ++k) xba[k] = valid ? __ldg(D + jb + (long long)k * nb) : 0.0;
 #pragma unroll
-      for (int a = 0; a < NA; ++a)
+      for (int k = 0; k < NA * NB; ++k) {
+        double s = 0.0;
 #pragma unroll
-        for (int b = 0; b < NB; ++b) xba[a * NB + b] = valid ? __ldg(X + (b0 + b) + (a0 + a) * ld) : 0.0;
-#pragma unroll
-      for (int a = 0; a < NA; ++a)
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-          double s = 0.0;
-#pragma unroll
-          for (int cd = 0; cd < NC * ND; ++cd) s += xdc[cd] * v[(a * NB + b) * NC * ND + cd];
-          s *= sJ;
-          if (bra_uniform) {
-            s = warp_sum(s);
-            if (lane == 0) atomicAdd(G + (a0 + a) + (b0 + b) * n, s);
-          } else if (valid) {
-            atomicAdd(G + (a0 + a) + (b0 + b) * n, s);
-          }
+        for (int q = 0; q < NC * ND; ++q) s += xdc[q] * v[k * NC * ND + q];
+        s *= sJ;
+        if (bra_uniform) {
+          s = warp_sum(s);
+          if (lane == 0) atomicAdd(J + jb + (long long)k * nb, s);
+        } else if (valid) {
+          atomicAdd(J + jb + (long long)k * nb, s);
         }
+      }
       if (valid) {
 #pragma unroll
-        for (int cd = 0; cd < NC * ND; ++cd) {
+        for (int q = 0; q < NC * ND; ++q) {
           double s = 0.0;
 #pragma unroll
-          for (int ab = 0; ab < NA * NB; ++ab) s += xba[ab] * v[ab * NC * ND + cd];
-          atomicAdd(G + (c0 + cd / ND) + (d0 + cd % ND) * n, sJ * s);
+          for (int k = 0; k < NA * NB; ++k) s += xba[k] * v[k * NC * ND + q];
+          atomicAdd(J + jk + (long long)q * nk, sJ * s);
         }
       }
     }
-    // Exchange updates go to Gh(c, a), Gh(d, b), Gh(d, a), Gh(c, b): k_finalize adds
-    // (Gh + Gh^T) / 2, so either orientation gives the same result, and with the bra
-    // index (the same across a bra-uniform warp) as the column the lanes' atomics land in
-    // one column of Gh.
     if (dg.sK[g] != 0.0 && valid) {
-      // X is symmetric (checked on entry): its exchange blocks are read as X(d, b), X(c, a),
-      // X(c, b), X(d, a), with the bra index (the same across a bra-uniform warp) as the column
+      // columns a and b, rows c and d, of X and Gh in the internal order
+      const double *__restrict__ X = dg.XP[g] + xo;
+      double *G = dg.GP[g] + xo;
+      auto at = [&](int2 row, int r, int2 col, int c) {
+        return (size_t)(row.x + r * row.y) + (size_t)(col.x + c * col.y) * n;
+      };
       double xbd[NB * ND], xac[NA * NC], xbc[NB * NC], xad[NA * ND];
 #pragma unroll
       for (int b = 0; b < NB; ++b)
 #pragma unroll
-        for (int d = 0; d < ND; ++d) xbd[b * ND + d] = __ldg(X + (d0 + d) + (b0 + b) * ld);
+        for (int d = 0; d < ND; ++d) xbd[b * ND + d] = __ldg(X + at(pd, d, pb, b));
 #pragma unroll
       for (int a = 0; a < NA; ++a)
 #pragma unroll
-        for (int c = 0; c < NC; ++c) xac[a * NC + c] = __ldg(X + (c0 + c) + (a0 + a) * ld);
+        for (int c = 0; c < NC; ++c) xac[a * NC + c] = __ldg(X + at(pc, c, pa, a));
 #pragma unroll
       for (int b = 0; b < NB; ++b)
 #pragma unroll
-        for (int c = 0; c < NC; ++c) xbc[b * NC + c] = __ldg(X + (c0 + c) + (b0 + b) * ld);
+        for (int c = 0; c < NC; ++c) xbc[b * NC + c] = __ldg(X + at(pc, c, pb, b));
 #pragma unroll
       for (int a = 0; a < NA; ++a)
 #pragma unroll
-        for (int d = 0; d < ND; ++d) xad[a * ND + d] = __ldg(X + (d0 + d) + (a0 + a) * ld);
+        for (int d = 0; d < ND; ++d) xad[a * ND + d] = __ldg(X + at(pd, d, pa, a));
 #pragma unroll
       for (int a = 0; a < NA; ++a)
 #pragma unroll
@@ -806,7 +865,7 @@ __device__ __forceinline__ void digest(const double *v, double deg, int a0, int 
           for (int b = 0; b < NB; ++b)
 #pragma unroll
             for (int d = 0; d < ND; ++d) s += xbd[b * ND + d] * v[((a * NB + b) * NC + c) * ND + d];
-          atomicAdd(G + (c0 + c) + (a0 + a) * n, sK * s);
+          atomicAdd(G + at(pc, c, pa, a), sK * s);
         }
 #pragma unroll
       for (int b = 0; b < NB; ++b)
@@ -817,7 +876,7 @@ __device__ __forceinline__ void digest(const double *v, double deg, int a0, int 
           for (int a = 0; a < NA; ++a)
 #pragma unroll
             for (int c = 0; c < NC; ++c) s += xac[a * NC + c] * v[((a * NB + b) * NC + c) * ND + d];
-          atomicAdd(G + (d0 + d) + (b0 + b) * n, sK * s);
+          atomicAdd(G + at(pd, d, pb, b), sK * s);
         }
 #pragma unroll
       for (int a = 0; a < NA; ++a)
@@ -828,7 +887,7 @@ __device__ __forceinline__ void digest(const double *v, double deg, int a0, int 
           for (int b = 0; b < NB; ++b)
 #pragma unroll
             for (int c = 0; c < NC; ++c) s += xbc[b * NC + c] * v[((a * NB + b) * NC + c) * ND + d];
-          atomicAdd(G + (d0 + d) + (a0 + a) * n, sK * s);
+          atomicAdd(G + at(pd, d, pa, a), sK * s);
         }
 #pragma unroll
       for (int b = 0; b < NB; ++b)
@@ -839,7 +898,7 @@ __device__ __forceinline__ void digest(const double *v, double deg, int a0, int 
           for (int a = 0; a < NA; ++a)
 #pragma unroll
             for (int d = 0; d < ND; ++d) s += xad[a * ND + d] * v[((a * NB + b) * NC + c) * ND + d];
-          atomicAdd(G + (c0 + c) + (b0 + b) * n, sK * s);
+          atomicAdd(G + at(pc, c, pb, b), sK * s);
         }
     }
   }
@@ -883,6 +942,11 @@ struct LaneShare {
   int nk_max;   // primitive pairs of the class's heaviest ket
 };
 constexpr int kLaneWork = 256;
+// A long list is claimed in kStripes interleaved stripes: in plain order the whole GPU works on a
+// handful of bras at a time, and the atomics of all warps meet in their few columns of Gh, in a
+// few L2 slices.  (H2O)_32 cc-pVDZ build 47.6 -> 44.7 ms with 8 stripes, 45.0 with 32 or 128; the
+// heaviest bras still come first within the first stripe.
+constexpr unsigned kStripes = 8, kStripeMin = 1u << 13;
 template <int LA, int LB, int LC, int LD, typename T>
 __device__ __forceinline__ void eri_jk_list(const uint2 *__restrict__ ql, const long long *__restrict__ range, int blk,
                                             const Pairs &P, const Shells &S, const double *__restrict__ boys_g,
@@ -898,15 +962,27 @@ __device__ __forceinline__ void eri_jk_list(const uint2 *__restrict__ ql, const 
   while (ls0 < 5 && ((end - beg) << (ls0 + 3)) <= share.lanes) ++ls0;
   const int target = (int)min((long long)INT_MAX, kLaneWork * max(1ll, (end - beg) / share.lanes));
   int nb = P.np[ql[beg].x];
+  // stripes of `per` claims of `chunk` entries (claims of one list: fewer than 2^31)
+  const unsigned nch = (unsigned)((end - beg + chunk - 1) / chunk), per = (nch + kStripes - 1) / kStripes;
+  const bool striped = ls0 == 0 && nb * share.nk_max <= target && nch >= kStripeMin;
   for (;;) {
     int ls = ls0;
     while (ls < 5 && ((nb * share.nk_max) >> ls) > target) ++ls;
+    if (striped) ls = 0;
     const int step = 32 >> ls, take = ls ? step : chunk;
     unsigned long long c0 = 0;
-    if (lane == 0) c0 = atomicAdd(qhead + blk, (unsigned long long)take);
+    if (lane == 0) c0 = atomicAdd(qhead + blk, (unsigned long long)(striped ? 1 : take));
     c0 = __shfl_sync(0xffffffffu, c0, 0);
+    if (striped) {
+      const unsigned t = (unsigned)c0;
+      if (t >= per * kStripes) return;
+      c0 = (unsigned long long)(t % kStripes * per + t / kStripes) * chunk;
+    }
     const long long cfirst = beg + (long long)c0;
-    if (cfirst >= end) return;   // the whole list is claimed
+    if (cfirst >= end) {
+      if (striped) continue;   // past the end of the last stripe
+      return;                  // the whole list is claimed
+    }
     const long long cend = min(cfirst + (long long)take, end);
     for (long long wfirst = cfirst; wfirst < cend; wfirst += step)
       nb = eri_jk_one<LA, LB, LC, LD, T>(ql, wfirst + (lane >> ls), wfirst, cend, P, S, boys, dg, ls);
@@ -924,10 +1000,10 @@ __global__ void __launch_bounds__(kEriThreads) k_eri_jk(const uint2 *__restrict_
 
 // Classes whose kernel is compiled for MB resident CTAs per SM (launch bounds with a
 // minimum block count; the other classes keep the compiler's own register choice).
-// Measured on (H2O)_32 cc-pVDZ against the kernels without the minimum: (ps|ps) 151 -> 128
-// registers 4.3 % faster, (pp|ss) 157 -> 128 2.9 %, (ds|ps) 199 -> 168 2.8 %; (ss|ss) at
-// five (96, spilling) 17 % slower.  (ps|ss) and (dp|ss) are held at three CTAs (208 and 242
-// registers without).
+// Measured on (H2O)_32 cc-pVDZ: (ps|ps) at 4 against 3 CTAs 4.3 % faster, (pp|ss) 2.9 %, (ds|ps) at
+// 3 against 2 2.8 %; (ds|ss) 1.99 ms at 4, 2.28 at the compiler's 3; (ps|ss) 7.57 ms at 5, 7.75 at
+// 4; (ss|ss) 3.76 ms at 4, 4.00 at 3 (168 registers).  (dp|ss) is held at 3 (242 registers
+// without).
 template <int LA, int LB, int LC, int LD>
 struct EriMinBlocks {
   static constexpr int v = 0;
@@ -945,8 +1021,16 @@ struct EriMinBlocks<2, 0, 1, 0> {
   static constexpr int v = 3;
 };
 template <>
+struct EriMinBlocks<0, 0, 0, 0> {
+  static constexpr int v = 4;
+};
+template <>
+struct EriMinBlocks<2, 0, 0, 0> {
+  static constexpr int v = 4;
+};
+template <>
 struct EriMinBlocks<1, 0, 0, 0> {
-  static constexpr int v = 3;
+  static constexpr int v = 5;
 };
 template <>
 struct EriMinBlocks<2, 1, 0, 0> {
@@ -1008,8 +1092,8 @@ __device__ __forceinline__ int eri_jk_plain(const uint2 e, const bool valid, con
   const unsigned bra0 = __shfl_sync(0xffffffffu, e.x, 0);
   const bool uniform = __all_sync(0xffffffffu, e.x == bra0);
   const double deg = (ab.x == ab.y ? 1.0 : 2.0) * (cd.x == cd.y ? 1.0 : 2.0) * (e.x == e.y ? 1.0 : 2.0);
-  digest<NA, NB, NC, ND>(v, deg, S.bf[ab.x], S.bf[ab.y], S.bf[cd.x], S.bf[cd.y], dg,
-                         valid && (threadIdx.x & ((1 << ls) - 1)) == 0, uniform, S.mol[ab.x]);
+  digest<LA, LB, LC, LD>(v, deg, (int)e.x, (int)e.y, P, S, dg, valid && (threadIdx.x & ((1 << ls) - 1)) == 0,
+                         uniform);
   return nb;
 }
 
@@ -1057,8 +1141,7 @@ __device__ __forceinline__ void eri_jk_group(const uint2 e, const bool valid, co
       const int pc = j < mk ? (int)e.y + j : (int)e.y;
       const int2 ab = P.sh[pa], cd = P.sh[pc];
       const double deg = (ab.x == ab.y ? 1.0 : 2.0) * (cd.x == cd.y ? 1.0 : 2.0) * (pa == pc ? 1.0 : 2.0);
-      digest<NA, NB, NC, ND>(v + (i * MK + j) * NQ, deg, S.bf[ab.x], S.bf[ab.y], S.bf[cd.x], S.bf[cd.y], dg, mv,
-                             uniform, S.mol[ab.x]);
+      digest<LA, LB, LC, LD>(v + (i * MK + j) * NQ, deg, pa, pc, P, S, dg, mv, uniform);
     }
   }
 }
@@ -1346,33 +1429,34 @@ __global__ void __launch_bounds__(128) k_schwarz_warp(Pairs P, Shells S, const d
 
 #include "eri_tc.cuh"
 
-// AX += 0.5 (Gh + Gh^T), molecule blockIdx.z of the context
-static __global__ void k_finalize(const double *__restrict__ Gh0, Mols mols, double *__restrict__ AX0, int ldax) {
+// AX += 0.5 (Gh + Gh^T), molecule blockIdx.z of the context; Gh = G0 plus GP0, which is in the
+// internal order.
+static __global__ void k_finalize(const double *__restrict__ G0, const double *__restrict__ GP0, Mols mols,
+                                  double *__restrict__ AX0, int ldax) {
   __shared__ double tile[32][33];
   const int mol = blockIdx.z;
   const int n = mols.nbf[mol];
   if (!mols.active[mol] || (int)(blockIdx.x * 32) >= n || (int)(blockIdx.y * 32) >= n) return;
-  const double *Gh = Gh0;
+  const double *G = G0, *GP = GP0;
   double *AX = AX0;
   if (mols.nmol > 1) {
-    Gh += mols.xoff[mol];
+    G += mols.xoff[mol];
+    GP += mols.xoff[mol];
     AX += mols.xoff[mol];
     ldax = n;
   }
+  const int *pos = mols.pos + mols.foff[mol];
+  auto gh = [&](int r, int c) { return G[(size_t)r + (size_t)c * n] + GP[(size_t)pos[r] + (size_t)pos[c] * n]; };
   int bx = blockIdx.x * 32, by = blockIdx.y * 32;
   int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
   for (int k = ty; k < 32; k += 8) {
     int rr = by + tx, cc = bx + k;
-    tile[k][tx] = (rr < n && cc < n) ? Gh[(size_t)rr + (size_t)cc * n] : 0.0;  // tile[k][tx] = Gh(by+tx, bx+k)
+    tile[k][tx] = (rr < n && cc < n) ? gh(rr, cc) : 0.0;  // tile[k][tx] = Gh(by+tx, bx+k)
   }
   __syncthreads();
   for (int k = ty; k < 32; k += 8) {
     int r = bx + tx, c = by + k;
-    if (r < n && c < n) {
-      double g = Gh[(size_t)r + (size_t)c * n];
-      double gt = tile[tx][k];  // Gh(by+k, bx+tx) = Gh(c, r)
-      AX[(size_t)r + (size_t)c * ldax] += 0.5 * (g + gt);
-    }
+    if (r < n && c < n) AX[(size_t)r + (size_t)c * ldax] += 0.5 * (gh(r, c) + tile[tx][k]);  // Gh(c, r)
   }
 }
 
@@ -1510,6 +1594,9 @@ struct cqg_ctx {
   int launches = 0;
   DevBuf<PrimPair> d_prim;
   DevBuf<double2> d_cols;
+  DevBuf<int2> d_pf;                   // internal order of the basis functions (Shells.pf, Mols.pos)
+  DevBuf<int> d_pos, d_mfoff;
+  DevBuf<double> d_XP;                 // per call: X in the internal order, Coulomb blocks of X by pair
   DevBuf<int> d_pair_coff;
   DevBuf<int> d_setup;                 // cqg_set_basis: group members, primitive-pair counts
   const double *boys = nullptr;        // kBoysTable (boys_eval) and kBoysRows (load_boys) on the context's
@@ -1696,6 +1783,7 @@ static inline Shells make_shells(cqg_ctx *ctx) {
   S.center = ctx->d_center.p;
   S.bf = ctx->d_bf.p;
   S.mol = ctx->d_shmol.p;
+  S.pf = ctx->d_pf.p;
   return S;
 }
 static inline Mols make_mols(cqg_ctx *ctx) {
@@ -1706,6 +1794,8 @@ static inline Mols make_mols(cqg_ctx *ctx) {
   M.Moff = ctx->d_mMoff.p;
   M.xoff = ctx->d_mxoff.p;
   M.nbf = ctx->d_mnbf.p;
+  M.foff = ctx->d_mfoff.p;
+  M.pos = ctx->d_pos.p;
   M.active = ctx->d_active.p;
   M.molbk = ctx->d_molbk.p;
   M.molgbk = ctx->d_molgbk.p;

@@ -496,11 +496,12 @@ WARP_CLASSES = {q for q in quartet_classes(3)
 
 
 # classes whose bra primitive pairs are walked several at a time, so that each ket
-# primitive pair read serves several primitive quartets.  Measured on (H2O)_32 cc-pVDZ:
-# (ss|ss) 12.3 -> 8.1 ms with 4 at a time (8: 12 % slower); (ps|ss) 12.85 -> 10.05 ms with 3
-# (156 registers, three CTAs per SM; 2: 10.58, 4: 11.42 ms).  (ps|ps), (pp|ss), (ds|ss),
-# (dp|ss) get 6-29 % slower with 2 (register pressure), so they keep one.
-BRA_TILE = {(0, 0, 0, 0): 4, (1, 0, 0, 0): 3}
+# primitive pair read serves several primitive quartets and their Boys chains overlap.
+# Measured on (H2O)_32 cc-pVDZ: (ss|ss) 3.76 ms with 4 at a time, 3.87 with 3, 3.83 with 2;
+# (ps|ss) 7.86 with 2 at four CTAs per SM, 8.91 with 3 at three (7.57 with 2 at five and no
+# prefetch).  With 2, (ps|ps) takes 5.45 instead of 4.29 ms, (pp|ss) 2.50 instead of 2.35,
+# (ds|ss) 2.22 instead of 1.99 (register pressure), so they keep one.
+BRA_TILE = {(0, 0, 0, 0): 4, (1, 0, 0, 0): 2}
 # the same for the sibling forms (members_header), whose member accumulators leave less room:
 # (ps|ss) 2 x 4 with three bra primitives at a time reaches 255 registers and spills
 GC_BRA_TILE = {(0, 0, 0, 0): 4}
@@ -513,11 +514,11 @@ GC_BRA_TILE = {(0, 0, 0, 0): 4}
 KET_TILE = {}
 
 # classes whose ket loop loads each primitive pair where it is used instead of one step
-# ahead.  Measured on (H2O)_32 cc-pVDZ with every per-thread class both ways: the prefetch
-# is worth 0.2-0.45 ms per class on the s and p classes ((ps|ss) 13.04 against 13.48 ms even
-# though the variant without it fits five CTAs per SM instead of four), and costs 0.03-0.13
-# ms on these, the spilling classes among them.
-NO_KET_PREFETCH = {(1, 1, 1, 1), (2, 0, 0, 0), (2, 0, 1, 1), (2, 0, 2, 0), (2, 1, 2, 0), (2, 2, 1, 0)}
+# ahead.  Measured on (H2O)_32 cc-pVDZ: without the prefetch (ss|ss) takes 3.76 instead of 4.19 ms
+# and (ps|ss) 7.75 instead of 7.86 (more primitive quartets in flight hide the load), while
+# (ps|ps), (pp|ss), (pp|ps) and (dp|ss) get 2 to 4 % slower; the d classes and the spilling
+# ones were 0.03-0.13 ms faster without it.
+NO_KET_PREFETCH = {(0, 0, 0, 0), (1, 0, 0, 0), (1, 1, 1, 1), (2, 0, 0, 0), (2, 0, 1, 1), (2, 0, 2, 0), (2, 1, 2, 0), (2, 2, 1, 0)}
 
 
 # Sibling-group classes of the engine (la, lb, lc, ld, mb, mk): their lists hold entries of
