@@ -313,10 +313,11 @@ class AOIntegrals:
 
     @staticmethod
     def _like(x):
+        """An output of formPT, which zeroes it."""
         if _is_torch(x):
             import torch
-            return torch.zeros_like(x)
-        return np.zeros(x.shape, order="F")
+            return torch.empty_like(x)
+        return np.empty(x.shape, order="F")
 
     def close(self):
         if getattr(self, "_ctx", None):

@@ -111,6 +111,8 @@ static double md_v1_digest_flops(int la, int lb, int lc, int ld) {
   return 24.0 * nfun(la) * nfun(lb) * nfun(lc) * nfun(ld);
 }
 
+constexpr size_t kListInitial = 1u << 16;   // list entries a new context has room for
+
 // the context's shells as the one-electron and primitive-pair kernels take them
 static OneEShells make_one_e_shells(const cqg_ctx *ctx) {
   OneEShells sh;
@@ -427,6 +429,8 @@ static std::vector<SideStreams *> g_side_spare;
 
 static void destroy_side_streams(SideStreams *s) {
   if (s->fork) cudaEventDestroy(s->fork);
+  if (s->read) cudaEventDestroy(s->read);
+  if (s->host) cudaFreeHost(s->host);
   for (int i = 0; i < kSideStreams; ++i) {
     if (s->done[i]) cudaEventDestroy(s->done[i]);
     if (s->st[i]) cudaStreamDestroy(s->st[i]);
@@ -449,7 +453,9 @@ static bool lease_side_streams(cqg_ctx *ctx) {
   }
   SideStreams *s = new SideStreams();
   s->device = ctx->device;
-  bool ok = cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming) == cudaSuccess;
+  bool ok = cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming) == cudaSuccess &&
+            cudaEventCreateWithFlags(&s->read, cudaEventDisableTiming) == cudaSuccess &&
+            cudaHostAlloc((void **)&s->host, kStateRead * sizeof(unsigned long long), cudaHostAllocDefault) == cudaSuccess;
   for (int i = 0; ok && i < kSideStreams; ++i)
     ok = cudaStreamCreateWithFlags(&s->st[i], cudaStreamNonBlocking) == cudaSuccess &&
          cudaEventCreateWithFlags(&s->done[i], cudaEventDisableTiming) == cudaSuccess;
@@ -514,7 +520,7 @@ static cqg_status build_block_tables(cqg_ctx *ctx) {
   cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, (long long *)nullptr, (long long *)nullptr,
                                 std::max<int>(kListParts * (int)task, 1));
   if (ctx->d_cnt.reserve(kListParts * task + 1) || ctx->d_off.reserve(kListParts * task + 1) ||
-      ctx->d_scan_tmp.reserve(scan_bytes + 16) || ctx->d_mslot.reserve(task + 1) || ctx->d_mhead.reserve(1) ||
+      ctx->d_scan_tmp.reserve(scan_bytes + 16) || ctx->d_mslot.reserve(task + 1) ||
       ctx->d_masks.reserve(kMaskStepsInitial))
     return CQG_ERR_OOM;
   return CQG_OK;
@@ -625,15 +631,12 @@ static DigestGroups make_digest(const cqg_ctx *ctx, int ng, const double *const 
   return dg;
 }
 
-// Block norms, input checks, internal copies of X: everything the screening and the digests
-// read of the input matrices.  Zeroes the accumulators and counters first.
+// Zeroes the call's state and accumulators, then block norms, input checks and the copies of X
+// that the screening and the digests read.
 static cqg_status launch_norms(cqg_ctx *ctx, const DigestGroups &dg, int nx, const double *const *Xall, int ldx,
                                const Mols &mols, cudaStream_t st) {
   const CallScratch cs(ctx);
-  CUCHK(cudaMemsetAsync(ctx->d_flags.p, 0, 4 * sizeof(int), st));
-  CUCHK(cudaMemsetAsync(ctx->d_Mmax.p, 0, sizeof(double), st));
-  CUCHK(cudaMemsetAsync(ctx->d_blkacc.p, 0, kBlkAcc * CQG_NQC * sizeof(unsigned long long), st));
-  CUCHK(cudaMemsetAsync(ctx->d_mhead.p, 0, sizeof(unsigned long long), st));
+  CUCHK(cudaMemsetAsync(ctx->d_state.p, 0, kStateWords * sizeof(unsigned long long), st));
   CUCHK(cudaMemsetAsync(ctx->d_G.p, 0, dg.ng * cs.group() * sizeof(double), st));
   XList xl;
   xl.n = nx;
@@ -642,26 +645,50 @@ static cqg_status launch_norms(cqg_ctx *ctx, const DigestGroups &dg, int nx, con
     xl.P[i] = ctx->d_XP.p + i * cs.matrix;
   }
   dim3 g((ctx->max_nsh + 127) / 128, ctx->max_nsh, ctx->nmol);
-  k_blocknorm<<<g, 128, 0, st>>>(xl, ldx, mols, ctx->d_bf.p, ctx->d_sz.p, ctx->d_pf.p, ctx->d_M.p,
-                                 ctx->d_M.p + ctx->Mtotal, ctx->d_flags.p, 1e-12);
-  const long long nn = ctx->Mtotal;
-  k_maxreduce<<<(int)std::min<long long>((nn + 255) / 256, 1184), 256, 0, st>>>(ctx->d_M.p, nn, ctx->d_Mmax.p);
-  const int npairs = (int)ctx->pair_sh.size();
-  k_pairnorm<<<(npairs + 255) / 256, 256, 0, st>>>(ctx->d_pair_sh.p, npairs, mols, make_shells(ctx), ctx->d_shL.p,
-                                                   ctx->d_sz.p, ctx->d_M.p, ctx->d_Mpair.p, dg);
+  k_blocknorm<<<g, 128, 0, st>>>(xl, ldx, mols, make_shells(ctx), ctx->d_sz.p, ctx->d_shL.p, ctx->d_M.p,
+                                 ctx->d_M.p + ctx->Mtotal, ctx->d_Mpair.p, dg, ctx->p_flags, ctx->p_Mmax, 1e-12);
   CUCHK(cudaGetLastError());
   return CQG_OK;
+}
+
+// The count pass of the screening, the list offsets of its tasks and the work lists' ranges.
+// Returns the launches made, or -1.
+static int launch_counts(cqg_ctx *ctx, const Pairs &P, const Mols &mols, double cut32, long long cap, cudaStream_t st) {
+  const int nb = (ctx->ntask + 7) / 8;
+  k_quartets<false><<<nb, 256, 0, st>>>(ctx->bt, ctx->ntask, P, ctx->d_M.p, ctx->d_M.p + ctx->Mtotal, ctx->d_Mpair.p,
+                                         mols, ctx->d_shmol.p, ctx->p_Mmax, ctx->thresh, cut32, ctx->d_cnt.p, nullptr,
+                                         nullptr, nullptr, ctx->p_blkacc, 0, 0, 0, 0, make_mask_cache(ctx));
+  if ((long long)kListParts * ctx->ntask <= kScanMax) {
+    k_scan_ranges<<<1, kScanThreads, 0, st>>>(ctx->bt, ctx->ntask, ctx->d_cnt.p, ctx->d_off.p, ctx->p_range, cap,
+                                              ctx->p_flags);
+    return cudaGetLastError() == cudaSuccess ? 2 : -1;
+  }
+  size_t scan_bytes = ctx->d_scan_tmp.n;
+  if (cub::DeviceScan::ExclusiveSum(ctx->d_scan_tmp.p, scan_bytes, ctx->d_cnt.p, ctx->d_off.p, kListParts * ctx->ntask,
+                                    st) != cudaSuccess)
+    return -1;
+  k_block_ranges<<<1, kRangeThreads, 0, st>>>(ctx->bt, ctx->ntask, ctx->d_cnt.p, ctx->d_off.p, ctx->p_range, cap,
+                                              ctx->p_flags);
+  return cudaGetLastError() == cudaSuccess ? 3 : -1;
+}
+
+// The fill pass for virtual tasks [vt0, vt1), whose entries start at list offset obase.
+static cudaError_t launch_fill(cqg_ctx *ctx, const Pairs &P, const Mols &mols, double cut32, long long vt0,
+                               long long vt1, long long obase, long long cap, cudaStream_t st) {
+  const int nb = (ctx->ntask + 7) / 8;
+  k_quartets<true><<<nb, 256, 0, st>>>(ctx->bt, ctx->ntask, P, ctx->d_M.p, ctx->d_M.p + ctx->Mtotal, ctx->d_Mpair.p,
+                                        mols, ctx->d_shmol.p, ctx->p_Mmax, ctx->thresh, cut32, nullptr, ctx->d_off.p,
+                                        ctx->d_qlist.p, ctx->d_qmask.p, nullptr, vt0, vt1, obase, cap,
+                                        make_mask_cache(ctx));
+  return cudaGetLastError();
 }
 
 // AX += 0.5 (Gh + Gh^T) of every group, once the class launches are done.
 static cqg_status launch_finalize(cqg_ctx *ctx, const DigestGroups &dg, double *const *AXg, int ldax, const Mols &mols,
                                   cudaStream_t st) {
-  const int npairs = (int)ctx->pair_sh.size();
-  k_pair_add<<<(npairs + 255) / 256, 256, 0, st>>>(ctx->d_pair_sh.p, npairs, mols, make_shells(ctx), ctx->d_shL.p,
-                                                   ctx->d_sz.p, dg);
   for (int g = 0; g < dg.ng; ++g) {
     dim3 grid((ctx->max_nbf + 31) / 32, (ctx->max_nbf + 31) / 32, ctx->nmol), blk(32, 8);
-    k_finalize<<<grid, blk, 0, st>>>(dg.G[g], dg.GP[g], mols, AXg[g], ldax);
+    k_finalize<<<grid, blk, 0, st>>>(dg, g, mols, ctx->d_bf.p, ctx->d_sz.p, ctx->d_shL.p, AXg[g], ldax);
   }
   CUCHK(cudaGetLastError());
   return CQG_OK;
@@ -837,21 +864,21 @@ cqg_status cqg_destroy(cqg_ctx *ctx) {
   cudaDeviceSynchronize();   // the buffers go back to the pool
   ctx->d_center.release(); ctx->d_bf.release(); ctx->d_sz.release();
   ctx->d_pair_sh.release(); ctx->d_pair_Q.release(); ctx->d_pair_poff.release(); ctx->d_pair_np.release();
-  ctx->d_pair_kk.release(); ctx->d_blkacc.release();
+  ctx->d_pair_kk.release();
   ctx->d_shL.release(); ctx->d_shnp.release(); ctx->d_shpoff.release(); ctx->d_alpha.release();
   ctx->d_coef.release(); ctx->d_oe.release(); ctx->d_charges.release();
   ctx->d_shmol.release(); ctx->d_mshoff.release(); ctx->d_mnsh.release(); ctx->d_mnbf.release();
   ctx->d_molbk.release(); ctx->d_mxoff.release(); ctx->d_mMoff.release(); ctx->d_active.release();
   ctx->d_prim.release(); ctx->d_exp.release(); ctx->d_setup.release();
   ctx->d_cols.release(); ctx->d_pair_coff.release(); ctx->d_pf.release(); ctx->d_pos.release(); ctx->d_mfoff.release();
+  ctx->d_pidx.release(); ctx->d_fsh.release();
   ctx->d_XP.release();
-  ctx->d_M.release(); ctx->d_Mmax.release(); ctx->d_Mpair.release(); ctx->d_flags.release();
-  ctx->d_cnt.release(); ctx->d_off.release(); ctx->d_range.release(); ctx->d_scan_tmp.release();
-  ctx->d_qhead.release();
+  ctx->d_M.release(); ctx->d_Mpair.release(); ctx->d_state.release();
+  ctx->d_cnt.release(); ctx->d_off.release(); ctx->d_scan_tmp.release();
   ctx->d_qlist.release(); ctx->d_G.release(); ctx->d_X.release(); ctx->d_AX.release(); ctx->d_Gscratch.release();
   ctx->d_molgbk.release(); ctx->d_gsz.release(); ctx->d_gpoff.release(); ctx->d_gnp.release(); ctx->d_gwoff.release();
   ctx->d_glead.release(); ctx->d_pair_Qc.release(); ctx->d_gQ.release(); ctx->d_gw.release(); ctx->d_gprim.release();
-  ctx->d_qmask.release(); ctx->d_masks.release(); ctx->d_mhead.release(); ctx->d_mslot.release();
+  ctx->d_qmask.release(); ctx->d_masks.release(); ctx->d_mslot.release();
   return_side_streams(ctx);
   if (ctx->events)
     for (int i = 0; i < 4 + 2 * CQG_NQC + 2; ++i) cudaEventDestroy(ctx->ev[i]);
@@ -977,7 +1004,7 @@ cqg_status cqg_set_basis_batch(cqg_ctx *ctx, int nmol, const int *nshell_per_mol
   ctx->nbf = ctx->m_nbf[0];
   // internal order of each molecule's functions: by angular momentum, component, shell
   std::vector<int2> pf(nshell);
-  std::vector<int> foff(nmol), pos;
+  std::vector<int> foff(nmol), pos, fsh;
   for (int m = 0; m < nmol; ++m) {
     const int s0 = ctx->m_shoff[m], s1 = s0 + ctx->m_nsh[m];
     int first[CQG_MAXL + 2] = {0}, count[CQG_MAXL + 1] = {0}, rank[CQG_MAXL + 1] = {0};
@@ -986,7 +1013,10 @@ cqg_status cqg_set_basis_batch(cqg_ctx *ctx, int nmol, const int *nshell_per_mol
     foff[m] = (int)pos.size();
     for (int s = s0; s < s1; ++s) {
       pf[s] = make_int2(first[L[s]] + rank[L[s]]++, count[L[s]]);
-      for (int k = 0; k < ctx->hsz[s]; ++k) pos.push_back(pf[s].x + k * pf[s].y);
+      for (int k = 0; k < ctx->hsz[s]; ++k) {
+        pos.push_back(pf[s].x + k * pf[s].y);
+        fsh.push_back(s - s0);
+      }
     }
   }
   // shells and molecule layout to device
@@ -996,8 +1026,9 @@ cqg_status cqg_set_basis_batch(cqg_ctx *ctx, int nmol, const int *nshell_per_mol
       ctx->d_shmol.reserve(nshell) || ctx->d_mshoff.reserve(nmol) || ctx->d_mnsh.reserve(nmol) ||
       ctx->d_mnbf.reserve(nmol) || ctx->d_mxoff.reserve(nmol) || ctx->d_mMoff.reserve(nmol) ||
       ctx->d_active.reserve(nmol) || ctx->d_pf.reserve(nshell) || ctx->d_pos.reserve(pos.size()) ||
-      ctx->d_mfoff.reserve(nmol))
+      ctx->d_mfoff.reserve(nmol) || ctx->d_fsh.reserve(fsh.size()))
     return CQG_ERR_OOM;
+  CUCHK(cudaMemcpyAsync(ctx->d_fsh.p, fsh.data(), fsh.size() * sizeof(int), cudaMemcpyHostToDevice, 0));
   CUCHK(cudaMemcpyAsync(ctx->d_pf.p, pf.data(), nshell * sizeof(int2), cudaMemcpyHostToDevice, 0));
   CUCHK(cudaMemcpyAsync(ctx->d_pos.p, pos.data(), pos.size() * sizeof(int), cudaMemcpyHostToDevice, 0));
   CUCHK(cudaMemcpyAsync(ctx->d_mfoff.p, foff.data(), nmol * sizeof(int), cudaMemcpyHostToDevice, 0));
@@ -1188,8 +1219,15 @@ cqg_status cqg_set_basis_batch(cqg_ctx *ctx, int nmol, const int *nshell_per_mol
     }
     for (size_t k = 0; k < molbk.size(); ++k) molgbk[k] = molbk[k] < npairs ? pair_group[molbk[k]] : ngroups;
   }
-  if (ctx->d_molbk.reserve(molbk.size()) || ctx->d_molgbk.reserve(molgbk.size()) || ctx->d_pair_Qc.reserve(npairs))
+  std::vector<int> pidx(ctx->Mtotal, -1);
+  for (int i = 0; i < npairs; ++i) {
+    const int x = ctx->pair_sh[i].x, y = ctx->pair_sh[i].y, m = ctx->hshmol[x], s0 = ctx->m_shoff[m];
+    pidx[ctx->m_Moff[m] + (y - s0) + (long long)(x - s0) * ctx->m_nsh[m]] = i;
+  }
+  if (ctx->d_molbk.reserve(molbk.size()) || ctx->d_molgbk.reserve(molgbk.size()) || ctx->d_pair_Qc.reserve(npairs) ||
+      ctx->d_pidx.reserve(pidx.size()))
     return CQG_ERR_OOM;
+  CUCHK(cudaMemcpyAsync(ctx->d_pidx.p, pidx.data(), pidx.size() * sizeof(int), cudaMemcpyHostToDevice, 0));
   CUCHK(cudaMemcpyAsync(ctx->d_molbk.p, molbk.data(), molbk.size() * sizeof(int), cudaMemcpyHostToDevice, 0));
   CUCHK(cudaMemcpyAsync(ctx->d_molgbk.p, molgbk.data(), molgbk.size() * sizeof(int), cudaMemcpyHostToDevice, 0));
   CUCHK(cudaMemcpyAsync(ctx->d_pair_Qc.p, ctx->pair_Qc.data(), npairs * sizeof(double), cudaMemcpyHostToDevice, 0));
@@ -1215,11 +1253,19 @@ cqg_status cqg_set_basis_batch(cqg_ctx *ctx, int nmol, const int *nshell_per_mol
   cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, (long long *)nullptr, (long long *)nullptr,
                                 std::max(kListParts * task, 1));
   if (ctx->d_cnt.reserve(kListParts * (size_t)task + 1) || ctx->d_off.reserve(kListParts * (size_t)task + 1) ||
-      ctx->d_range.reserve(2 * CQG_NLIST) || ctx->d_qhead.reserve(CQG_NLIST + 1) ||
+      ctx->d_state.reserve(kStateWords) || ctx->d_qlist.reserve(kListInitial) || ctx->d_qmask.reserve(kListInitial) ||
       ctx->d_scan_tmp.reserve(scan_bytes + 16) || ctx->d_M.reserve(2 * (size_t)std::max(ctx->Mtotal, 1LL)) ||
-      ctx->d_Mmax.reserve(1) || ctx->d_flags.reserve(4) || ctx->d_blkacc.reserve(kBlkAcc * CQG_NQC) ||
       ctx->d_Mpair.reserve(std::max<size_t>(ctx->pair_sh.size(), 1)))
     return CQG_ERR_OOM;
+  {
+    unsigned long long *w = ctx->d_state.p;
+    ctx->p_flags = (int *)w;
+    ctx->p_Mmax = (double *)(w + 2);
+    ctx->p_mhead = w + 3;
+    ctx->p_blkacc = w + 4;
+    ctx->p_range = (long long *)(w + 4 + kBlkAcc * CQG_NQC);
+    ctx->p_qhead = w + kStateRead;
+  }
   CUCHK(cudaDeviceSynchronize());   // written on the legacy stream, read on the callers' streams
   return CQG_OK;
 }
@@ -1297,7 +1343,7 @@ static cqg_status autotune_shapes(cqg_ctx *ctx, const long long *crange, cudaStr
     const int reps = m < n ? 1 : 2;
     if (m < n) {
       const long long sub[2] = {crange[2 * vb], crange[2 * vb] + m};
-      CUCHK(cudaMemcpyAsync(ctx->d_range.p + 2 * vb, sub, sizeof(sub), cudaMemcpyHostToDevice, st));
+      CUCHK(cudaMemcpyAsync(ctx->p_range + 2 * vb, sub, sizeof(sub), cudaMemcpyHostToDevice, st));
     }
     float best = 1e30f;
     Shape pick = cand[0];
@@ -1309,7 +1355,7 @@ static cqg_status autotune_shapes(cqg_ctx *ctx, const long long *crange, cudaStr
       ctx->shape_var[vb] = cw.var;
       float tbest = 1e30f;
       for (int rep = 0; rep < (ci < 0 ? 1 : reps); ++rep) {
-        CUCHK(cudaMemsetAsync(ctx->d_qhead.p + vb, 0, sizeof(unsigned long long), st));
+        CUCHK(cudaMemsetAsync(ctx->p_qhead + vb, 0, sizeof(unsigned long long), st));
         cudaEventRecord(e0, st);
         cudaError_t e = list_launcher(vb)(ctx, vb, m, st, scratch);
         cudaEventRecord(e1, st);
@@ -1329,7 +1375,7 @@ static cqg_status autotune_shapes(cqg_ctx *ctx, const long long *crange, cudaStr
         pick = cw;
       }
     }
-    if (m < n) CUCHK(cudaMemcpyAsync(ctx->d_range.p + 2 * vb, crange + 2 * vb, 2 * sizeof(long long),
+    if (m < n) CUCHK(cudaMemcpyAsync(ctx->p_range + 2 * vb, crange + 2 * vb, 2 * sizeof(long long),
                                      cudaMemcpyHostToDevice, st));
     ctx->shape_cta[vb] = pick.cta;
     ctx->shape_wpb[vb] = pick.wpb;
@@ -1349,7 +1395,7 @@ static cqg_status autotune_shapes(cqg_ctx *ctx, const long long *crange, cudaStr
     for (int tier = 0; tier <= 2; ++tier) {
       float t = 1e30f;
       for (int rep = 0; rep < 2; ++rep) {
-        CUCHK(cudaMemsetAsync(ctx->d_qhead.p, 0, CQG_NLIST * sizeof(unsigned long long), st));
+        CUCHK(cudaMemsetAsync(ctx->p_qhead, 0, CQG_NLIST * sizeof(unsigned long long), st));
         cudaEventRecord(e0, st);
         cudaError_t e = tier ? cqg_launch_fused(ctx, tier, st, scratch) : cudaSuccess;
         for (int vb = 0; vb < CQG_NLIST && e == cudaSuccess; ++vb) {
@@ -1402,24 +1448,14 @@ static cqg_status contract_graph(cqg_ctx *ctx, int ngroups, const double *const 
     const cqg_status ns = launch_norms(ctx, dg, nx_all, Xall, ldx, mols, st);
     if (ns != CQG_OK) return ns;
   }
-  Pairs P = make_pairs(ctx);
-  const int nb = (ctx->ntask + 7) / 8;
-  k_quartets<false><<<nb, 256, 0, st>>>(ctx->bt, ctx->ntask, P, ctx->d_M.p, ctx->d_M.p + ctx->Mtotal, ctx->d_Mpair.p, mols, ctx->d_shmol.p, ctx->d_Mmax.p,
-                                         ctx->thresh, cut32, ctx->d_cnt.p, nullptr, nullptr, nullptr, ctx->d_blkacc.p,
-                                         0, 0, 0, 0, make_mask_cache(ctx));
-  size_t scan_bytes = ctx->d_scan_tmp.n;
-  CUCHK(cub::DeviceScan::ExclusiveSum(ctx->d_scan_tmp.p, scan_bytes, ctx->d_cnt.p, ctx->d_off.p,
-                                      kListParts * ctx->ntask, st));
-  k_block_ranges<<<1, kRangeThreads, 0, st>>>(ctx->bt, ctx->ntask, ctx->d_cnt.p, ctx->d_off.p, ctx->d_range.p,
-                                    ctx->graph_capacity, ctx->d_flags.p);
-  k_quartets<true><<<nb, 256, 0, st>>>(ctx->bt, ctx->ntask, P, ctx->d_M.p, ctx->d_M.p + ctx->Mtotal, ctx->d_Mpair.p, mols, ctx->d_shmol.p, ctx->d_Mmax.p,
-                                        ctx->thresh, cut32, nullptr, ctx->d_off.p, ctx->d_qlist.p, ctx->d_qmask.p,
-                                        nullptr, 0,
-                                        (long long)kListParts * ctx->ntask, 0, ctx->graph_capacity,
-                                        make_mask_cache(ctx));
-  CUCHK(cudaGetLastError());
-  CUCHK(cudaMemsetAsync(ctx->d_qhead.p, 0, CQG_NLIST * sizeof(unsigned long long), st));
-  int launches = 7;   // block norms, max, pair norms, list count, scan, ranges, list fill
+  const Pairs P = make_pairs(ctx);
+  const int counted = launch_counts(ctx, P, mols, cut32, ctx->graph_capacity, st);
+  if (counted < 0) {
+    ctx->err = "screening launch failed";
+    return CQG_ERR_CUDA;
+  }
+  CUCHK(launch_fill(ctx, P, mols, cut32, 0, (long long)kListParts * ctx->ntask, 0, ctx->graph_capacity, st));
+  int launches = 2 + counted;   // block norms, list count and offsets, list fill
   if (ctx->fused_tier) {
     cudaError_t e = cqg_launch_fused(ctx, ctx->fused_tier, st, dg);
     ++launches;
@@ -1456,7 +1492,7 @@ static cqg_status contract_graph(cqg_ctx *ctx, int ngroups, const double *const 
     const cqg_status fs = launch_finalize(ctx, dg, AXg, ldax, mols, st);
     if (fs != CQG_OK) return fs;
   }
-  launches += 1 + ngroups;
+  launches += ngroups;
   ctx->launches = launches;
   ctx->stats.launches = launches;
   return CQG_OK;
@@ -1490,36 +1526,41 @@ static cqg_status contract_device(cqg_ctx *ctx, int ngroups, const double *const
   {
     const cqg_status ns = launch_norms(ctx, dg, nx_all, Xall, ldx, mols, st);
     if (ns != CQG_OK) return ns;
-    ctx->launches = 3;
+    ctx->launches = 1;
   }
-  // 2. quartet lists
-  Pairs P = make_pairs(ctx);
+  // 2. quartet lists: count, read the ranges back, and meanwhile fill the list as it is -- the
+  // host reads while the fill runs, and only a list that has outgrown its buffer is filled
+  // again
+  const Pairs P = make_pairs(ctx);
+  const long long nvt = (long long)kListParts * ctx->ntask;
   {
-    int nthr = 256, wpb = nthr / 32;
-    int nb = (ctx->ntask + wpb - 1) / wpb;
-    k_quartets<false><<<nb, nthr, 0, st>>>(ctx->bt, ctx->ntask, P, ctx->d_M.p, ctx->d_M.p + ctx->Mtotal, ctx->d_Mpair.p, mols, ctx->d_shmol.p, ctx->d_Mmax.p,
-                                            ctx->thresh,
-                                            cut32, ctx->d_cnt.p, nullptr, nullptr, nullptr, ctx->d_blkacc.p, 0, 0, 0,
-                                            0, make_mask_cache(ctx));
-    CUCHK(cudaGetLastError());
-    size_t scan_bytes = ctx->d_scan_tmp.n;
-    CUCHK(cub::DeviceScan::ExclusiveSum(ctx->d_scan_tmp.p, scan_bytes, ctx->d_cnt.p, ctx->d_off.p,
-                                      kListParts * ctx->ntask, st));
-    k_block_ranges<<<1, kRangeThreads, 0, st>>>(ctx->bt, ctx->ntask, ctx->d_cnt.p, ctx->d_off.p, ctx->d_range.p, LLONG_MAX,
-                                      ctx->d_flags.p);
-    CUCHK(cudaGetLastError());
-    ctx->launches += 2;
+    const int counted = launch_counts(ctx, P, mols, cut32, LLONG_MAX, st);
+    if (counted < 0) {
+      ctx->err = "screening launch failed";
+      return CQG_ERR_CUDA;
+    }
+    ctx->launches += counted;
   }
+  std::vector<unsigned long long> pageable;
+  unsigned long long *host = lease_side_streams(ctx) ? ctx->side->host : nullptr;
+  if (!host) {
+    pageable.resize(kStateRead);
+    host = pageable.data();
+  }
+  CUCHK(cudaMemcpyAsync(host, ctx->d_state.p, kStateRead * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+  if (ctx->side) CUCHK(cudaEventRecord(ctx->side->read, st));
+  const long long filled = (long long)std::min(ctx->d_qlist.n, ctx->d_qmask.n);
+  CUCHK(launch_fill(ctx, P, mols, cut32, 0, nvt, 0, filled, st));
+  ctx->launches += 1;
+  if (ctx->side) CUCHK(cudaEventSynchronize(ctx->side->read));
+  else CUCHK(cudaStreamSynchronize(st));
+  int hflags[4];
   long long hr[2 * CQG_NLIST];
   unsigned long long hacc[kBlkAcc * CQG_NQC];
-  int hflags[4];
-  CUCHK(cudaMemcpyAsync(hr, ctx->d_range.p, sizeof(hr), cudaMemcpyDeviceToHost, st));
-  CUCHK(cudaMemcpyAsync(hacc, ctx->d_blkacc.p, sizeof(hacc), cudaMemcpyDeviceToHost, st));
-  CUCHK(cudaMemcpyAsync(hflags, ctx->d_flags.p, sizeof(hflags), cudaMemcpyDeviceToHost, st));
-  unsigned long long hsteps = 0;
-  CUCHK(cudaMemcpyAsync(&hsteps, ctx->d_mhead.p, sizeof(hsteps), cudaMemcpyDeviceToHost, st));
-  CUCHK(cudaStreamSynchronize(st));
-  ctx->mask_steps_used = (long long)hsteps;
+  memcpy(hflags, host, sizeof(hflags));
+  ctx->mask_steps_used = (long long)host[3];
+  memcpy(hacc, host + 4, sizeof(hacc));
+  memcpy(hr, host + 4 + kBlkAcc * CQG_NQC, sizeof(hr));
   if (hflags[0]) {
     ctx->err = "input density contains NaN or Inf";
     return CQG_ERR_NONFINITE;
@@ -1535,7 +1576,6 @@ static cqg_status contract_device(cqg_ctx *ctx, int ngroups, const double *const
   const long long budget = std::max<long long>(ctx->list_budget, 1);
   std::vector<long long> chunk_vt;   // chunk boundaries in virtual tasks
   std::vector<long long> hoff, hcnt;
-  const long long nvt = (long long)kListParts * ctx->ntask;
   if (total <= budget) {
     chunk_vt = {0, nvt};
   } else {
@@ -1616,30 +1656,25 @@ static cqg_status contract_device(cqg_ctx *ctx, int ngroups, const double *const
           crange[2 * vb] = crange[2 * vb + 1] = 0;
         }
       }
-      CUCHK(cudaMemcpyAsync(ctx->d_range.p, crange, sizeof(crange), cudaMemcpyHostToDevice, st));
+      CUCHK(cudaMemcpyAsync(ctx->p_range, crange, sizeof(crange), cudaMemcpyHostToDevice, st));
     } else {
       for (int q = 0; q < 2 * CQG_NLIST; ++q) crange[q] = hr[q];
     }
-    {
-      int nthr = 256, wpb = nthr / 32;
-      int nb = (ctx->ntask + wpb - 1) / wpb;
-      k_quartets<true><<<nb, nthr, 0, st>>>(ctx->bt, ctx->ntask, P, ctx->d_M.p, ctx->d_M.p + ctx->Mtotal, ctx->d_Mpair.p, mols, ctx->d_shmol.p, ctx->d_Mmax.p,
-                                             ctx->thresh,
-                                             cut32, nullptr, ctx->d_off.p, ctx->d_qlist.p, ctx->d_qmask.p, nullptr,
-                                             vt0, vt1, obase,
-                                             (long long)std::min(ctx->d_qlist.n, ctx->d_qmask.n),
-                                             make_mask_cache(ctx));
-      CUCHK(cudaGetLastError());
+    if (chunk_vt.size() > 2 || total > filled) {
+      CUCHK(launch_fill(ctx, P, mols, cut32, vt0, vt1, obase, (long long)std::min(ctx->d_qlist.n, ctx->d_qmask.n), st));
       ctx->launches += 1;
     }
     if (ctx->timing && first_chunk) CUCHK(cudaEventRecord(ctx->ev[1], st));
+    bool tuned = false;
     if (ctx->autotune_pending && chunk_vt.size() == 2) {
+      tuned = true;
       cqg_status ts = autotune_shapes(ctx, crange, st, dg);
       if (ts != CQG_OK) return ts;
       ctx->autotune_pending = 0;
     }
-    // 3. ERI + digest per class, each list consumed through its work-queue head counter
-    CUCHK(cudaMemsetAsync(ctx->d_qhead.p, 0, CQG_NLIST * sizeof(unsigned long long), st));
+    // 3. ERI + digest per class, each list consumed through its work-queue head counter (zeroed
+    // with the call's state; again when the tuner or a chunk before has used them)
+    if (tuned || !first_chunk) CUCHK(cudaMemsetAsync(ctx->p_qhead, 0, CQG_NLIST * sizeof(unsigned long long), st));
     if (ctx->fused_tier) {   // the fused tier's lists in one launch (its time: ms_fused)
       if (ctx->timing) CUCHK(cudaEventRecord(ctx->ev[4 + 2 * CQG_NQC], st));
       cudaError_t e = cqg_launch_fused(ctx, ctx->fused_tier, st, dg);
@@ -1707,7 +1742,7 @@ static cqg_status contract_device(cqg_ctx *ctx, int ngroups, const double *const
   {
     const cqg_status fs = launch_finalize(ctx, dg, AXg, ldax, mols, st);
     if (fs != CQG_OK) return fs;
-    ctx->launches += 1 + ngroups;
+    ctx->launches += ngroups;
   }
   if (ctx->timing) CUCHK(cudaEventRecord(ctx->ev[3], st));
   ctx->stats.quartets = nquart;
@@ -2036,8 +2071,8 @@ cqg_status cqg_graph_status(cqg_ctx *ctx, long long *quartets, int *overflow, in
   CUCHK(cudaDeviceSynchronize());
   long long hr[2 * CQG_NLIST];
   int fl[4];
-  CUCHK(cudaMemcpy(fl, ctx->d_flags.p, sizeof(fl), cudaMemcpyDeviceToHost));
-  CUCHK(cudaMemcpy(hr, ctx->d_range.p, sizeof(hr), cudaMemcpyDeviceToHost));
+  CUCHK(cudaMemcpy(fl, ctx->p_flags, sizeof(fl), cudaMemcpyDeviceToHost));
+  CUCHK(cudaMemcpy(hr, ctx->p_range, sizeof(hr), cudaMemcpyDeviceToHost));
   if (quartets) *quartets = hr[2 * CQG_NLIST - 1];
   if (overflow) *overflow = fl[2];
   if (nonfinite) *nonfinite = fl[0];

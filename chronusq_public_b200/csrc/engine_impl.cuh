@@ -111,6 +111,10 @@ struct Mols {
   const int *nbf;                // basis functions of molecule m
   const int *foff;               // basis functions of the molecules before m
   const int *pos;                // [foff[m] + r]: internal position of function r (Shells.pf)
+  const int *fsh;                // [foff[m] + r]: shell of function r within the molecule
+  // [Moff[m] + y + x nsh]: pair index of shells (x, y) of molecule m in their internal
+  // orientation, -1 for the other order
+  const int *pidx;
   const unsigned char *active;   // molecule m takes part in the call
   const int *molbk;              // [m][ket pair class][bucket + 1]: first pair of each bucket
   const int *molgbk;             // the same in group index space: first group of each bucket
@@ -218,65 +222,65 @@ struct XList {
   double *P[8];   // the same in the internal order (Shells.pf), written here
   int n;
 };
-static __global__ void k_blocknorm(XList xl, int ldx, Mols mols, const int *__restrict__ bf,
-                            const int *__restrict__ sz, const int2 *__restrict__ pf, double *__restrict__ M, double *__restrict__ MT,
-                            int *__restrict__ flags, double sym_tol) {
+// Thread (s1, s2) of molecule blockIdx.z: the block of rows s1, columns s2.  Besides the norm
+// and the checks it writes everything a call reads of the block later: the matrices in the
+// internal order, and where (s2, s1) is a shell pair, the pair's norm and Coulomb blocks.
+static __global__ void k_blocknorm(XList xl, int ldx, Mols mols, Shells S, const int *__restrict__ sz,
+                                   const int *__restrict__ shL, double *__restrict__ M, double *__restrict__ MT,
+                                   double *__restrict__ Mpair, DigestGroups dg, int *__restrict__ flags,
+                                   double *__restrict__ Mmax, double sym_tol) {
   const int mol = blockIdx.z;
   const int nsh = mols.nsh[mol];
-  int s1 = blockIdx.x * blockDim.x + threadIdx.x;
-  int s2 = blockIdx.y;
-  if (s1 >= nsh || s2 >= nsh) return;
-  double *Mm = M + mols.Moff[mol];
-  double *MTm = MT + mols.Moff[mol];
-  if (!mols.active[mol]) {
-    Mm[(size_t)s1 + (size_t)s2 * nsh] = 0.0;
-    MTm[(size_t)s2 + (size_t)s1 * nsh] = 0.0;
-    return;
-  }
-  const int g1 = mols.shoff[mol] + s1, g2 = mols.shoff[mol] + s2;
-  int r0 = bf[g1], c0 = bf[g2], nr = sz[g1], nc = sz[g2];
-  if (mols.nmol > 1) ldx = mols.nbf[mol];
-  const long long xo = mols.nmol > 1 ? mols.xoff[mol] : 0;
-  const int n = mols.nbf[mol];
-  const int2 p1 = pf[g1], p2 = pf[g2];
+  const int s1 = blockIdx.x * blockDim.x + threadIdx.x;
+  const int s2 = blockIdx.y;
+  if (s2 >= nsh) return;   // whole blocks
   double mx = 0.0;
-  int bad = 0, asym = 0;
-  for (int m = 0; m < xl.n; ++m) {
-    const double *X = xl.X[m] + xo;
-    double *P = xl.P[m] + xo;
-    for (int c = 0; c < nc; ++c)
-      for (int r = 0; r < nr; ++r) {
-        double v = X[(size_t)(r0 + r) + (size_t)(c0 + c) * ldx];
-        double t = X[(size_t)(c0 + c) + (size_t)(r0 + r) * ldx];
-        if (!isfinite(v)) bad = 1;
-        double av = fabs(v);
-        mx = fmax(mx, av);
-        if (fabs(v - t) > sym_tol * fmax(1.0, av)) asym = 1;
-        P[(size_t)(p1.x + r * p1.y) + (size_t)(p2.x + c * p2.y) * n] = v;
+  if (s1 < nsh) {
+    double *Mm = M + mols.Moff[mol], *MTm = MT + mols.Moff[mol];
+    const int pair = mols.pidx[mols.Moff[mol] + s1 + (size_t)s2 * nsh];
+    if (mols.active[mol]) {
+      const int g1 = mols.shoff[mol] + s1, g2 = mols.shoff[mol] + s2;
+      const int r0 = S.bf[g1], c0 = S.bf[g2], nr = sz[g1], nc = sz[g2], n = mols.nbf[mol];
+      if (mols.nmol > 1) ldx = n;
+      const long long xo = mols.nmol > 1 ? mols.xoff[mol] : 0;
+      const int2 p1 = S.pf[g1], p2 = S.pf[g2];
+      int bad = 0, asym = 0;
+      for (int m = 0; m < xl.n; ++m) {
+        const double *X = xl.X[m] + xo;
+        double *P = xl.P[m] + xo;
+        for (int c = 0; c < nc; ++c)
+          for (int r = 0; r < nr; ++r) {
+            double v = X[(size_t)(r0 + r) + (size_t)(c0 + c) * ldx];
+            double t = X[(size_t)(c0 + c) + (size_t)(r0 + r) * ldx];
+            if (!isfinite(v)) bad = 1;
+            double av = fabs(v);
+            mx = fmax(mx, av);
+            if (fabs(v - t) > sym_tol * fmax(1.0, av)) asym = 1;
+            P[(size_t)(p1.x + r * p1.y) + (size_t)(p2.x + c * p2.y) * n] = v;
+          }
       }
-  }
-  Mm[(size_t)s1 + (size_t)s2 * nsh] = mx;
-  MTm[(size_t)s2 + (size_t)s1 * nsh] = mx;   // transposed copy: M(s1, .) as a contiguous column
-  if (bad) atomicOr(flags + 0, 1);
-  if (asym) atomicOr(flags + 1, 1);
-}
-
-static __global__ void k_maxreduce(const double *__restrict__ M, long long n, double *__restrict__ out) {
-  __shared__ double sm[32];
-  double mx = 0.0;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    mx = fmax(mx, M[i]);
-  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = mx;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    mx = threadIdx.x < (blockDim.x >> 5) ? sm[threadIdx.x] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (threadIdx.x == 0) {
-      // non-negative doubles order like their bit patterns
-      atomicMax((unsigned long long *)out, (unsigned long long)__double_as_longlong(mx));
+      if (bad) atomicOr(flags + 0, 1);
+      if (asym) atomicOr(flags + 1, 1);
+      if (pair >= 0) {   // a = s2 (columns), b = s1 (rows)
+        const int cls = pair_class_c(shL[g2], shL[g1]);
+        for (int g = 0; g < dg.ng; ++g) {
+          if (dg.sJ[g] == 0.0) continue;
+          const double *X = dg.X[g] + xo;
+          double *D = const_cast<double *>(dg.DP[g]) + dg.joff[cls] + (pair - dg.jbeg[cls]);
+          for (int c = 0; c < nc; ++c)
+            for (int r = 0; r < nr; ++r)
+              D[(size_t)(c * nr + r) * dg.jn[cls]] = X[(size_t)(r0 + r) + (size_t)(c0 + c) * ldx];
+        }
+      }
     }
+    Mm[(size_t)s1 + (size_t)s2 * nsh] = mx;
+    MTm[(size_t)s2 + (size_t)s1 * nsh] = mx;   // transposed copy: M(s1, .) as a contiguous column
+    if (pair >= 0) Mpair[pair] = mx;
   }
+  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  // non-negative doubles order like their bit patterns
+  if ((threadIdx.x & 31) == 0 && mx > 0.0)
+    atomicMax((unsigned long long *)Mmax, (unsigned long long)__double_as_longlong(mx));
 }
 
 // One screening task = (class block, bra pair).  Blocks are listed in task order.
@@ -325,48 +329,6 @@ __device__ __forceinline__ double quartet_bound(const double *__restrict__ col1,
   m = fmax(m, col1[s3]);
   m = fmax(m, col2[s3]);
   return m * qab * qcd;
-}
-
-// Mpair[i] = M(a, b) of shell pair i (its own block norm; molecule-local indices), and the
-// pair's block of each X with a Coulomb part to DP.
-static __global__ void k_pairnorm(const int2 *__restrict__ sh, int npairs, Mols mols, Shells S,
-                                  const int *__restrict__ shL, const int *__restrict__ sz, const double *__restrict__ M,
-                                  double *__restrict__ Mpair, DigestGroups dg) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= npairs) return;
-  const int2 ab = sh[i];
-  const int mol = S.mol[ab.x];
-  const int nsh = mols.nsh[mol], shoff = mols.shoff[mol];
-  Mpair[i] = M[mols.Moff[mol] + (ab.x - shoff) + (size_t)(ab.y - shoff) * nsh];
-  if (!mols.active[mol]) return;
-  const int c = pair_class_c(shL[ab.x], shL[ab.y]), na = sz[ab.x], nb = sz[ab.y], a0 = S.bf[ab.x], b0 = S.bf[ab.y];
-  for (int g = 0; g < dg.ng; ++g) {
-    if (dg.sJ[g] == 0.0) continue;
-    const double *X;
-    double *G, *D = const_cast<double *>(dg.DP[g]) + dg.joff[c] + (i - dg.jbeg[c]);
-    size_t ld, n;
-    mol_view(dg, g, mol, X, G, ld, n);
-    for (int k = 0; k < na * nb; ++k) D[(size_t)k * dg.jn[c]] = X[(size_t)(b0 + k % nb) + (size_t)(a0 + k / nb) * ld];
-  }
-}
-
-// The Coulomb sums of the shell pairs (JP) into Gh, after every class launch.
-static __global__ void k_pair_add(const int2 *__restrict__ sh, int npairs, Mols mols, Shells S,
-                                  const int *__restrict__ shL, const int *__restrict__ sz, DigestGroups dg) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= npairs) return;
-  const int2 ab = sh[i];
-  const int mol = S.mol[ab.x];
-  if (!mols.active[mol]) return;
-  const int c = pair_class_c(shL[ab.x], shL[ab.y]), na = sz[ab.x], nb = sz[ab.y], a0 = S.bf[ab.x], b0 = S.bf[ab.y];
-  for (int g = 0; g < dg.ng; ++g) {
-    if (dg.sJ[g] == 0.0) continue;
-    const double *X, *J = dg.JP[g] + dg.joff[c] + (i - dg.jbeg[c]);
-    double *G;
-    size_t ld, n;
-    mol_view(dg, g, mol, X, G, ld, n);
-    for (int k = 0; k < na * nb; ++k) G[(size_t)(a0 + k / nb) + (size_t)(b0 + k % nb) * n] += J[(size_t)k * dg.jn[c]];
-  }
 }
 
 // Per-block screening tallies in blkacc[kBlkAcc * blk + ...]: model primitive quartets
@@ -754,6 +716,49 @@ static __global__ void k_block_ranges(BlockTable bt, int ntask, const long long 
   if (vb >= kListParts * bt.nblk) return;
   const int part = vb / bt.nblk, b = vb % bt.nblk;
   const long long t0 = (long long)part * ntask + bt.task_beg[b], t1 = (long long)part * ntask + bt.task_beg[b + 1];
+  long long beg = 0, end = 0;
+  if (t1 > t0) {
+    beg = off[t0];
+    end = off[t1 - 1] + cnt[t1 - 1];
+  } else if (t0 > 0) {
+    beg = end = off[t0 - 1] + cnt[t0 - 1];
+  }
+  range[2 * vb] = min(beg, cap);
+  range[2 * vb + 1] = min(end, cap);
+}
+
+// The scan of the counts and the ranges by one block, for lists of few tasks (one launch
+// instead of the three of the device-wide scan).
+constexpr int kScanThreads = 1024, kScanMax = 32 * kScanThreads;
+static __global__ void __launch_bounds__(kScanThreads) k_scan_ranges(BlockTable bt, int ntask,
+                                                                     const long long *__restrict__ cnt,
+                                                                     long long *off, long long *__restrict__ range,
+                                                                     long long cap, int *__restrict__ flags) {
+  __shared__ long long part[32];
+  const int nv = kListParts * ntask, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int per = (nv + kScanThreads - 1) / kScanThreads, v0 = min(nv, (int)threadIdx.x * per), v1 = min(nv, v0 + per);
+  long long sum = 0;
+  for (int v = v0; v < v1; ++v) sum += cnt[v];
+  long long inc = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const long long y = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += y;
+  }
+  if (lane == 31) part[warp] = inc;
+  __syncthreads();
+  long long before = inc - sum;
+  for (int w = 0; w < warp; ++w) before += part[w];
+  for (int v = v0; v < v1; ++v) {
+    off[v] = before;
+    before += cnt[v];
+  }
+  __syncthreads();   // block-wide: the offsets written above are read below
+  const int vb = threadIdx.x;
+  if (vb == 0 && ntask > 0 && off[nv - 1] + cnt[nv - 1] > cap) flags[2] = 1;   // list overflow
+  if (vb >= kListParts * bt.nblk) return;
+  const int p = vb / bt.nblk, b = vb % bt.nblk;
+  const int t0 = p * ntask + bt.task_beg[b], t1 = p * ntask + bt.task_beg[b + 1];
   long long beg = 0, end = 0;
   if (t1 > t0) {
     beg = off[t0];
@@ -1429,15 +1434,16 @@ __global__ void __launch_bounds__(128) k_schwarz_warp(Pairs P, Shells S, const d
 
 #include "eri_tc.cuh"
 
-// AX += 0.5 (Gh + Gh^T), molecule blockIdx.z of the context; Gh = G0 plus GP0, which is in the
-// internal order.
-static __global__ void k_finalize(const double *__restrict__ G0, const double *__restrict__ GP0, Mols mols,
-                                  double *__restrict__ AX0, int ldax) {
+// AX += 0.5 (Gh + Gh^T) of group g, molecule blockIdx.z of the context; Gh = G plus GP, which is
+// in the internal order, plus the Coulomb sums of the shell pairs, JP.
+static __global__ void k_finalize(DigestGroups dg, int g, Mols mols, const int *__restrict__ bf,
+                                  const int *__restrict__ sz, const int *__restrict__ shL, double *__restrict__ AX0,
+                                  int ldax) {
   __shared__ double tile[32][33];
   const int mol = blockIdx.z;
   const int n = mols.nbf[mol];
   if (!mols.active[mol] || (int)(blockIdx.x * 32) >= n || (int)(blockIdx.y * 32) >= n) return;
-  const double *G = G0, *GP = GP0;
+  const double *G = dg.G[g], *GP = dg.GP[g];
   double *AX = AX0;
   if (mols.nmol > 1) {
     G += mols.xoff[mol];
@@ -1445,8 +1451,22 @@ static __global__ void k_finalize(const double *__restrict__ G0, const double *_
     AX += mols.xoff[mol];
     ldax = n;
   }
-  const int *pos = mols.pos + mols.foff[mol];
-  auto gh = [&](int r, int c) { return G[(size_t)r + (size_t)c * n] + GP[(size_t)pos[r] + (size_t)pos[c] * n]; };
+  const int *pos = mols.pos + mols.foff[mol], *fsh = mols.fsh + mols.foff[mol];
+  const int nsh = mols.nsh[mol], shoff = mols.shoff[mol];
+  const int *pidx = mols.pidx + mols.Moff[mol];
+  const bool coulomb = dg.sJ[g] != 0.0;
+  auto gh = [&](int r, int c) {
+    double v = G[(size_t)r + (size_t)c * n] + GP[(size_t)pos[r] + (size_t)pos[c] * n];
+    if (coulomb) {
+      const int y = fsh[r], x = fsh[c], pair = pidx[y + (size_t)x * nsh];
+      if (pair >= 0) {
+        const int gx = shoff + x, gy = shoff + y, cls = pair_class_c(shL[gx], shL[gy]);
+        const int k = (c - bf[gx]) * sz[gy] + (r - bf[gy]);
+        v += dg.JP[g][dg.joff[cls] + (size_t)k * dg.jn[cls] + (pair - dg.jbeg[cls])];
+      }
+    }
+    return v;
+  };
   int bx = blockIdx.x * 32, by = blockIdx.y * 32;
   int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
   for (int k = ty; k < 32; k += 8) {
@@ -1532,9 +1552,14 @@ struct DevBuf {
 constexpr int kSideStreams = 7;
 struct SideStreams {
   int device = 0;
+  unsigned long long *host = nullptr;   // pinned: the call state as read back (kStateRead words)
+  cudaEvent_t read = nullptr;
   cudaStream_t st[kSideStreams] = {};
   cudaEvent_t done[kSideStreams] = {}, fork = nullptr;
 };
+
+// words of the call state: flags, Mmax, mask-cache head, tallies, ranges | work-queue heads
+constexpr int kStateRead = 4 + kBlkAcc * CQG_NQC + 2 * CQG_NLIST, kStateWords = kStateRead + CQG_NLIST + 1;
 
 struct cqg_ctx {
   int device = 0;
@@ -1558,7 +1583,14 @@ struct cqg_ctx {
   // class-fused persistent kernel (eri_fused.cu); set by the autotuner or cqg_set_fusion
   int fused_tier = 0;
   double fusion_ms[3] = {0.0, 0.0, 0.0};   // autotuner's times of the three forms (ms)
-  DevBuf<unsigned long long> d_qhead;  // work-queue head counter of every work list, then the fused one
+  // Per-call state, one buffer: zeroed by one memset, and read back by one copy up to `range`.
+  DevBuf<unsigned long long> d_state;
+  int *p_flags = nullptr;                  // non-finite, asymmetric, list overflow
+  double *p_Mmax = nullptr;
+  unsigned long long *p_mhead = nullptr;   // MaskCache::head
+  unsigned long long *p_blkacc = nullptr;  // screening tallies, kBlkAcc per class
+  long long *p_range = nullptr;            // [begin, end) of every work list
+  unsigned long long *p_qhead = nullptr;   // work-queue head of every work list, then the fused one
   int autotune_pending = 0;
   long long graph_capacity = 0;        // > 0: sync-free contraction for CUDA-graph capture
   bool class_possible[CQG_NQC] = {false};
@@ -1590,12 +1622,11 @@ struct cqg_ctx {
   DevBuf<double> d_alpha, d_coef;
   DevBuf<double> d_oe;       // host-mode staging of S, T, V
   DevBuf<double> d_charges;  // Z then R (3 per charge)
-  DevBuf<unsigned long long> d_blkacc;
   int launches = 0;
   DevBuf<PrimPair> d_prim;
   DevBuf<double2> d_cols;
   DevBuf<int2> d_pf;                   // internal order of the basis functions (Shells.pf, Mols.pos)
-  DevBuf<int> d_pos, d_mfoff;
+  DevBuf<int> d_pos, d_mfoff, d_pidx, d_fsh;
   DevBuf<double> d_XP;                 // per call: X in the internal order, Coulomb blocks of X by pair
   DevBuf<int> d_pair_coff;
   DevBuf<int> d_setup;                 // cqg_set_basis: group members, primitive-pair counts
@@ -1609,9 +1640,8 @@ struct cqg_ctx {
   int pc_prim[CQG_NPC + 1] = {0};   // first primitive pair of each pair class
   int pc_np_max[CQG_NPC] = {0};   // most primitive pairs of a pair, per class
   // per-call scratch
-  DevBuf<double> d_M, d_Mmax, d_Mpair;
-  DevBuf<int> d_flags;
-  DevBuf<long long> d_cnt, d_off, d_range;
+  DevBuf<double> d_M, d_Mpair;
+  DevBuf<long long> d_cnt, d_off;
   DevBuf<unsigned char> d_scan_tmp;
   DevBuf<uint2> d_qlist;
   DevBuf<double> d_G, d_X, d_AX, d_Gscratch;
@@ -1635,7 +1665,6 @@ struct cqg_ctx {
   DevBuf<unsigned short> d_qmask;     // member masks, parallel to d_qlist
   // survivor-mask cache of the screening passes (MaskCache): steps, head, per-task slots
   DevBuf<uint2> d_masks;
-  DevBuf<unsigned long long> d_mhead;
   DevBuf<long long> d_mslot;
   long long mask_steps_used = 0;      // steps the last count pass asked for
   SideStreams *side = nullptr;   // leased on first use (ClassStreams in engine.cu)
@@ -1708,9 +1737,9 @@ static cudaError_t launch_tc(cqg_ctx *ctx, int blk, long long n, cudaStream_t st
   const Expansions X = {ctx->d_exp.p + ctx->exp_off[bc], ctx->d_exp.p + ctx->exp_off[kc], ctx->exp_prim0[bc],
                         ctx->exp_prim0[kc]};
   const int take = std::min(32, ctx->shape_qpw[blk]);
-  k_eri_tc<LA, LB, LC, LD><<<blocks, 32 * wpb, per_warp * wpb, st>>>(ctx->d_qlist.p, ctx->d_range.p, blk,
+  k_eri_tc<LA, LB, LC, LD><<<blocks, 32 * wpb, per_warp * wpb, st>>>(ctx->d_qlist.p, ctx->p_range, blk,
                                                                     make_pairs(ctx), make_shells(ctx), X,
-                                                                    ctx->boys_rows, dg, ctx->d_qhead.p, take);
+                                                                    ctx->boys_rows, dg, ctx->p_qhead, take);
   return cudaGetLastError();
 }
 
@@ -1750,7 +1779,7 @@ static cudaError_t launch_expansions(cqg_ctx *ctx) {
 static inline MaskCache make_mask_cache(cqg_ctx *ctx) {
   MaskCache mc;
   mc.masks = ctx->d_masks.p;
-  mc.head = ctx->d_mhead.p;
+  mc.head = ctx->p_mhead;
   mc.slot = ctx->d_mslot.p;
   mc.cap = (long long)ctx->d_masks.n;
   return mc;
@@ -1796,6 +1825,8 @@ static inline Mols make_mols(cqg_ctx *ctx) {
   M.nbf = ctx->d_mnbf.p;
   M.foff = ctx->d_mfoff.p;
   M.pos = ctx->d_pos.p;
+  M.fsh = ctx->d_fsh.p;
+  M.pidx = ctx->d_pidx.p;
   M.active = ctx->d_active.p;
   M.molbk = ctx->d_molbk.p;
   M.molgbk = ctx->d_molgbk.p;
@@ -1831,12 +1862,12 @@ static cudaError_t launch_gc(cqg_ctx *ctx, int blk, long long n, cudaStream_t st
   const long long nb = n > 0 ? std::min<long long>((n + nt - 1) / nt, cap) : cap;
   const int chunk = 32 * (ctx->shape_qpw[blk] > 0 ? ctx->shape_qpw[blk] : 1);
   if (nt == 64)
-    k_eri_gc<LA, LB, LC, LD, T, 64><<<(unsigned)nb, 64, 0, st>>>(ctx->d_qlist.p, ctx->d_range.p, blk,
+    k_eri_gc<LA, LB, LC, LD, T, 64><<<(unsigned)nb, 64, 0, st>>>(ctx->d_qlist.p, ctx->p_range, blk,
                                                                 make_pairs(ctx), make_shells(ctx), ctx->boys_rows,
-                                                                dg, ctx->d_qhead.p, chunk);
+                                                                dg, ctx->p_qhead, chunk);
   else
     k_eri_gc<LA, LB, LC, LD, T, kEriThreads><<<(unsigned)nb, kEriThreads, 0, st>>>(
-        ctx->d_qlist.p, ctx->d_range.p, blk, make_pairs(ctx), make_shells(ctx), ctx->boys_rows, dg, ctx->d_qhead.p,
+        ctx->d_qlist.p, ctx->p_range, blk, make_pairs(ctx), make_shells(ctx), ctx->boys_rows, dg, ctx->p_qhead,
         chunk);
   return cudaGetLastError();
 }
@@ -1869,8 +1900,8 @@ static cudaError_t launch_eri(cqg_ctx *ctx, int blk, long long n, cudaStream_t s
     // up to 32 lanes per quartet (eri_jk_list)
     const long long nb = n > 0 ? std::min<long long>((32 * n + kEriThreads - 1) / kEriThreads, cap) : cap;
     const int chunk = 32 * (ctx->shape_qpw[blk] > 0 ? ctx->shape_qpw[blk] : 1);
-    kernel<<<(unsigned)nb, kEriThreads, 0, st>>>(ctx->d_qlist.p, ctx->d_range.p, blk, make_pairs(ctx), make_shells(ctx),
-                                                 ctx->boys_rows, dg, ctx->d_qhead.p, chunk, share);
+    kernel<<<(unsigned)nb, kEriThreads, 0, st>>>(ctx->d_qlist.p, ctx->p_range, blk, make_pairs(ctx), make_shells(ctx),
+                                                 ctx->boys_rows, dg, ctx->p_qhead, chunk, share);
     return cudaGetLastError();
   }
 }

@@ -162,18 +162,18 @@ bool cqg_fused_member(int tier, int la, int lb, int lc, int ld) {
   return tier == 2 && !is_warp_class(la, lb, lc, ld) && la <= 2 && lb <= 2 && lc <= 2 && ld <= 2;
 }
 
-// One launch of the fused kernel of `tier` over the current list ranges (d_range); the
-// head counter d_qhead[CQG_NLIST] is zeroed on the stream first.
+// One launch of the fused kernel of `tier` over the current list ranges (p_range); the
+// head counter p_qhead[CQG_NLIST] is zeroed on the stream first.
 cudaError_t cqg_launch_fused(cqg_ctx *ctx, int tier, cudaStream_t st, const DigestGroups &dg) {
-  cudaError_t e = cudaMemsetAsync(ctx->d_qhead.p + CQG_NLIST, 0, sizeof(unsigned long long), st);
+  cudaError_t e = cudaMemsetAsync(ctx->p_qhead + CQG_NLIST, 0, sizeof(unsigned long long), st);
   if (e != cudaSuccess) return e;
   const int per_sm = tier == 1 ? 4 : 2;
   const unsigned blocks = (unsigned)(ctx->nsm * per_sm);
   if (tier == 1)
-    k_eri_fused<1><<<blocks, kEriThreads, 0, st>>>(ctx->d_qlist.p, ctx->d_range.p, make_pairs(ctx), make_shells(ctx),
-                                                   ctx->boys_rows, dg, ctx->d_qhead.p + CQG_NLIST);
+    k_eri_fused<1><<<blocks, kEriThreads, 0, st>>>(ctx->d_qlist.p, ctx->p_range, make_pairs(ctx), make_shells(ctx),
+                                                   ctx->boys_rows, dg, ctx->p_qhead + CQG_NLIST);
   else
-    k_eri_fused<2><<<blocks, kEriThreads, 0, st>>>(ctx->d_qlist.p, ctx->d_range.p, make_pairs(ctx), make_shells(ctx),
-                                                   ctx->boys_rows, dg, ctx->d_qhead.p + CQG_NLIST);
+    k_eri_fused<2><<<blocks, kEriThreads, 0, st>>>(ctx->d_qlist.p, ctx->p_range, make_pairs(ctx), make_shells(ctx),
+                                                   ctx->boys_rows, dg, ctx->p_qhead + CQG_NLIST);
   return cudaGetLastError();
 }
