@@ -35,7 +35,8 @@ EXPORTED = [
     "cqg_mlp_gemm_bf16", "cqg_mlp_silu_bwd", "cqg_mlp_to_bf16", "cqg_mlp_colsum", "cqg_mlp_mse", "cqg_mlp_adam",
     "cqg_one_e_noalloc", "cqg_dipole", "cqg_get_schedule", "cqg_set_schedule",
     "cqg_set_fusion", "cqg_get_fusion", "cqg_mlp_adam_dev", "cqg_set_siblings", "cqg_get_siblings",
-    "cqg_schedule_lists", "cqg_list_class", "cqg_set_sibling_min",
+    "cqg_schedule_lists", "cqg_list_class", "cqg_set_sibling_min", "cqg_mlp_forward", "cqg_mlp_backward",
+    "cqg_mlp_adam_tensors",
 ]
 
 
@@ -115,6 +116,11 @@ def load(path: str = LIB_PATH):
     L.cqg_mlp_mse.argtypes = [vp, vp, vp, ll, f, vp, vp, vp]
     L.cqg_mlp_adam.argtypes = [vp, vp, vp, vp, ll, f, f, f, f, ctypes.c_int, f, vp, vp]
     L.cqg_mlp_adam_dev.argtypes = [vp, vp, vp, vp, ll, vp, f, f, f, f, vp, vp]
+    pv = ctypes.POINTER(vp)
+    L.cqg_mlp_forward.argtypes = [ctypes.c_int, i, ctypes.c_int, vp, pv, pv, pv, pv, vp]
+    L.cqg_mlp_backward.argtypes = [ctypes.c_int, i, ctypes.c_int, vp, pv, pv, pv, vp, vp, vp, vp]
+    L.cqg_mlp_adam_tensors.argtypes = [ctypes.c_int, pv, pv, pv, pv, ctypes.POINTER(ll), ctypes.POINTER(f), pv, vp, f,
+                                       f, f, f, ctypes.c_int, vp]
     L.cqg_class_name.argtypes = [ctypes.c_int]
     L.cqg_class_name.restype = ctypes.c_char_p
     L.cqg_probe_fma_peak.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_double, d]
@@ -130,7 +136,7 @@ def load(path: str = LIB_PATH):
                  "cqg_mlp_gemm_bf16", "cqg_mlp_silu_bwd", "cqg_mlp_to_bf16", "cqg_mlp_colsum", "cqg_mlp_mse",
                  "cqg_mlp_adam", "cqg_one_e_noalloc", "cqg_dipole", "cqg_get_schedule", "cqg_set_schedule", "cqg_set_fusion", "cqg_get_fusion", "cqg_mlp_adam_dev",
                  "cqg_set_siblings", "cqg_get_siblings", "cqg_schedule_lists", "cqg_list_class",
-                 "cqg_set_sibling_min"]:
+                 "cqg_set_sibling_min", "cqg_mlp_forward", "cqg_mlp_backward", "cqg_mlp_adam_tensors"]:
         getattr(L, name).restype = ctypes.c_int
     _lib = L
     return L

@@ -3,25 +3,27 @@
 //
 //   k_gemm_bf16 : C[m][n] (+)= sum_k A(m,k) B(n,k), A and B BF16 with arbitrary strides
 //                 (transposes are strides), on the tensor cores: mma.sync m16n8k16 BF16 x
-//                 BF16 -> FP32 over 128 x 128 x 32 block tiles staged in shared memory
-//                 (8 warps, 32 x 64 each); optional fused epilogue Z = C + bias (FP32) and
-//                 Y = SiLU(Z) (BF16).
-//   k_silu_bwd  : dZ = dY * SiLU'(Z)  (BF16 out, the next GEMM's operand)
-//   k_colsum    : db[n] = sum_m dZ[m][n]
+//                 BF16 -> FP32 over block tiles that come through a ring of asynchronous
+//                 copies; optional fused epilogue Z = C + bias (FP32) and Y = SiLU(Z) (BF16).
+//                 or, backward, dZ = C * SiLU'(Z) (BF16, the next GEMMs' operand) and its column sums
+//   k_dz_colsum : the output layer's dZ in BF16 and db[n] = sum_m dZ[m][n]
 //   k_mse       : masked squared error, its gradient, and the loss sum
-//   k_adam      : Adam step on FP32 master weights, BF16 copy for the next pass
-//   k_cast_bf16 : FP32 -> BF16
+//   k_adam      : Adam step on FP32 master weights, BF16 copy for the next pass, all tensors of
+//                 the network in one launch
+//   k_silu_bwd, k_to_bf16 : the elementwise parts alone (cqg_mlp_silu_bwd, cqg_mlp_to_bf16)
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <algorithm>
+#include <atomic>
+#include <utility>
 
 #include "../../include/cqgpu.h"
 
 namespace {
 
-constexpr int GM = 128, GN = 128, GK = 32, GKP = GK + 8;   // large block tile; padded smem rows
+constexpr int GM = 128, GN = 128, GK = 32;   // large block tile, k per tile
 
 __device__ __forceinline__ float silu(float z) { return z / (1.0f + __expf(-z)); }
 __device__ __forceinline__ float silu_grad(float z) {
@@ -42,125 +44,322 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4],
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// Stage rows [r0, r0 + 128) x k [k0, k0 + 32) of X(r, k) = X[r * sr + k * sk] into S[row][k]
-// (zero outside nrows x K).  Rows or k contiguous and 16-byte aligned: 8-element vector
-// loads; anything else element by element.
-template <int ROWS>
-__device__ __forceinline__ void stage_tile(const __nv_bfloat16 *__restrict__ X, long long sr, long long sk, int r0,
-                                           int nrows, int k0, int K, bool vec_k, bool vec_r,
-                                           __nv_bfloat16 (*S)[GKP]) {
-  const int tid = threadIdx.x, nth = blockDim.x;
-  const __nv_bfloat16 zero = __float2bfloat16(0.f);
-  if (vec_k) {                 // sk == 1, sr % 8 == 0, K % 8 == 0, X 16-byte aligned
-    for (int e = tid; e < ROWS * (GK / 8); e += nth) {
-      const int rr = e / (GK / 8), kv = (e % (GK / 8)) * 8;
-      const int r = r0 + rr, k = k0 + kv;
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (r < nrows && k < K) v = *reinterpret_cast<const uint4 *>(X + (long long)r * sr + k);
-      *reinterpret_cast<uint4 *>(&S[rr][kv]) = v;
-    }
-  } else if (vec_r) {          // sr == 1, sk % 8 == 0, nrows % 8 == 0, X 16-byte aligned
-    for (int e = tid; e < GK * (ROWS / 8); e += nth) {
-      const int kk = e / (ROWS / 8), rv = (e % (ROWS / 8)) * 8;
-      const int r = r0 + rv, k = k0 + kk;
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (r < nrows && k < K) v = *reinterpret_cast<const uint4 *>(X + r + (long long)k * sk);
-      const __nv_bfloat16 *h = reinterpret_cast<const __nv_bfloat16 *>(&v);
+// How an operand tile lies in shared memory: as [row][k] (k contiguous in memory, or any
+// strides, staged element by element) or as [k][row] (rows contiguous); ldmatrix, transposing
+// for the second, gives the same fragments from either.
+enum { TILE_K = 0, TILE_R = 1, TILE_ANY = 2 };
+constexpr int GP = GK + 8;   // padded row of a [row][k] tile: 80 bytes, no ldmatrix bank conflicts
+
+__device__ __forceinline__ void cp_async16(unsigned dst, const void *src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], unsigned addr, bool trans) {
+  if (trans)
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+  else
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+
+// A thread's 16-byte copies of one operand's tiles, ROWS rows from r0 x GK of k, of
+// X(r, k) = X[r * sr + k * sk] (zero outside nrows x K).  Addresses and row bounds are worked
+// out once: the products of a training step are short, and five tiles' worth of index
+// arithmetic before the first copy was a third of their time.
+template <int ROWS, int NT>
+struct TileCopy {
+  static constexpr int NC = ROWS * (GK / 8) / NT;
+  const __nv_bfloat16 *src[NC];
+  long long step;    // elements from one tile to the next
+  unsigned dst[NC];  // offset in the tile
+  int most[NC], k[NC], mul;
+  __device__ __forceinline__ TileCopy(const __nv_bfloat16 *X, long long sr, long long sk, int r0, int nrows, int kb,
+                                      int mode) {
+    const bool kin = mode == TILE_K;
+    step = kin ? GK : GK * sk;
+    mul = kin ? 2 : 16;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) S[rv + i][kk] = h[i];
+    for (int c = 0; c < NC; ++c) {
+      const int e = c * NT + threadIdx.x;
+      const int r = r0 + (kin ? e / (GK / 8) : e % (ROWS / 8) * 8);
+      k[c] = kin ? e % (GK / 8) * 8 : e / (ROWS / 8);
+      dst[c] = 2 * (kin ? (r - r0) * GP + k[c] : k[c] * (ROWS + 8) + r - r0);
+      most[c] = max(0, min(16, (nrows - r) * (kin ? 16 : 2)));
+      src[c] = most[c] ? X + r * sr + (kb + k[c]) * sk : X;
     }
-  } else if (sk <= sr) {       // k varies fastest across threads
-    for (int e = tid; e < ROWS * GK; e += nth) {
-      const int rr = e / GK, kk = e % GK;
-      const int r = r0 + rr, k = k0 + kk;
-      S[rr][kk] = (r < nrows && k < K) ? X[(long long)r * sr + (long long)k * sk] : zero;
+  }
+  // tile kt of k [kb + kt * GK, ...), `left` = K - that
+  __device__ __forceinline__ void start(unsigned tile, int kt, int left) const {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const int bytes = min(most[c], max(0, (left - k[c]) * mul));
+      cp_async16(tile + dst[c], bytes ? src[c] + kt * step : src[c], bytes);
     }
-  } else {                     // rows vary fastest across threads
-    for (int e = tid; e < ROWS * GK; e += nth) {
-      const int kk = e / ROWS, rr = e % ROWS;
-      const int r = r0 + rr, k = k0 + kk;
-      S[rr][kk] = (r < nrows && k < K) ? X[(long long)r * sr + (long long)k * sk] : zero;
+  }
+};
+
+// The same tile, [row][k], for operands that 16-byte copies cannot take; complete on return.
+template <int ROWS, int NT>
+__device__ __forceinline__ void stage_any(const __nv_bfloat16 *__restrict__ X, long long sr, long long sk, int r0,
+                                          int nrows, int k0, int K, __nv_bfloat16 *S) {
+  const __nv_bfloat16 zero = __float2bfloat16(0.f);
+  const bool k_fast = sk <= sr;   // the smaller stride across threads
+  constexpr int U = 8;            // loads in flight
+#pragma unroll 1
+  for (int e0 = threadIdx.x; e0 < ROWS * GK; e0 += NT * U) {
+    __nv_bfloat16 v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int e = e0 + u * NT;
+      const int r = r0 + (k_fast ? e / GK : e % ROWS), k = k0 + (k_fast ? e % GK : e / ROWS);
+      v[u] = (r < nrows && k < K) ? X[(long long)r * sr + (long long)k * sk] : zero;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int e = e0 + u * NT;
+      S[(k_fast ? e / GK : e % ROWS) * GP + (k_fast ? e % GK : e / ROWS)] = v[u];
     }
   }
 }
 
+// One product of a launch.  split: the block reduces k in [z kchunk, (z + 1) kchunk) and adds
+// its partial tile to C with atomics (C zeroed by the caller), no epilogue.  fold: the block
+// reduces all of K, in partial sums over kchunk each.  dact: the epilogue is the backward
+// step through the layer below, Y = bf16(value * SiLU'(dact)) and its column sums added to
+// db; C is not written.
+struct Gemm {
+  const __nv_bfloat16 *A, *B;
+  long long sam, sak, sbn, sbk, ldc, ldy;
+  float *C;
+  const float *bias, *dact;
+  float *db;
+  __nv_bfloat16 *Y;
+  int M, N, K, kchunk, nbn, nbm, nbz;
+  unsigned char amode, bmode, act, accumulate, split, fold, pairs;   // pairs: C, Y and dact take 2-wide accesses
+  __host__ int blocks() const { return nbn * nbm * nbz; }
+};
+
 // Block tile BM x BN (BM, BN multiples of 32), warps of 32 x WN output each (WN = 64 or 32):
 // (BM / 32) x (BN / WN) warps; per 16-wide k step a warp issues 2 x (WN / 8) tensor-core
 // tiles.  128 x 128 with 8 warps of 32 x 64 for large problems, 64 x 64 with 4 warps of
-// 32 x 32 when the large tiles would leave most of the 148 SMs idle.
-template <int BM, int BN, int WN>
-__global__ void __launch_bounds__((BM / 32) * (BN / WN) * 32)
-    k_gemm_bf16(const __nv_bfloat16 *__restrict__ A, long long sam, long long sak, const __nv_bfloat16 *__restrict__ B,
-                long long sbn, long long sbk, float *__restrict__ C, long long ldc, int M, int N, int K,
-                const float *__restrict__ bias, __nv_bfloat16 *__restrict__ Y, long long ldy, int act, int accumulate,
-                int kchunk) {
-  constexpr int NWM = BM / 32, NJ = WN / 8;
-  __shared__ __align__(16) __nv_bfloat16 As[BM][GKP];
-  __shared__ __align__(16) __nv_bfloat16 Bs[BN][GKP];
+// 32 x 32 when the large tiles would leave most of the 148 SMs idle.  A training step's
+// products (2048 x 256 x 256) are chains of load latencies, not arithmetic: tiles of 32 k come
+// through a ring of STAGES asynchronous copies, and two products of one layer (its weight
+// gradient and the gradient of its input) share a launch, the first `blocks0` blocks for g0.
+// Measured, 2048 rows, width 256: a layer forward 17 us cold (9.1 us back to back) from one
+// synchronous tile at a time before; the backward pass 70 us for six launches.
+template <int BM, int BN, int WN, int STAGES>
+__global__ void __launch_bounds__((BM / 32) * (BN / WN) * 32, BM == 64 ? 3 : 2)
+    k_gemm_bf16(const __grid_constant__ Gemm g0, const __grid_constant__ Gemm g1, int blocks0) {
+  constexpr int NWM = BM / 32, NJ = WN / 8, NT = NWM * (BN / WN) * 32;
+  constexpr int ASZ = BM * GP, BSZ = BN * GP;   // [k][row] tiles, GK x (rows + 8), fit as well
+  constexpr bool CAN_FOLD = BM == 64;           // the registers of a second accumulator
+  static_assert(GK * (BM + 8) <= ASZ && GK * (BN + 8) <= BSZ, "tile buffers");
+  extern __shared__ __align__(16) __nv_bfloat16 tiles[];
+  const bool first = (int)blockIdx.x < blocks0;
+  const Gemm p = first ? g0 : g1;
+  const int blk = first ? blockIdx.x : blockIdx.x - blocks0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wm = (warp % NWM) * 32, wn = (warp / NWM) * WN;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  const int M = p.M, N = p.N, K = p.K;
+  const int n0 = blk % p.nbn * BN, m0 = blk / p.nbn % p.nbm * BM, z = blk / (p.nbn * p.nbm);
   const int g = lane >> 2, t = lane & 3;
-  const bool a16 = (reinterpret_cast<uintptr_t>(A) & 15) == 0, b16 = (reinterpret_cast<uintptr_t>(B) & 15) == 0;
-  const bool avk = a16 && sak == 1 && sam % 8 == 0 && K % 8 == 0;
-  const bool avr = a16 && !avk && sam == 1 && sak % 8 == 0 && M % 8 == 0;
-  const bool bvk = b16 && sbk == 1 && sbn % 8 == 0 && K % 8 == 0;
-  const bool bvr = b16 && !bvk && sbn == 1 && sbk % 8 == 0 && N % 8 == 0;
-  float acc[2][NJ][4];
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < NJ; ++j)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.f;
-  // split K (kchunk > 0): this block reduces k in [kb, ke) and adds its partial tile to C
-  // with atomics (C zeroed by the caller); no epilogue then
-  const int kb = kchunk > 0 ? blockIdx.z * kchunk : 0, ke = kchunk > 0 ? min(K, kb + kchunk) : K;
-  for (int k0 = kb; k0 < ke; k0 += GK) {
-    stage_tile<BM>(A, sam, sak, m0, M, k0, ke, avk, avr, As);
-    stage_tile<BN>(B, sbn, sbk, n0, N, k0, ke, bvk, bvr, Bs);
-    __syncthreads();
-#pragma unroll
-    for (int ks = 0; ks < GK; ks += 16) {
-      uint32_t af[2][4], bf[NJ][2];
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int r = wm + i * 16 + g;
-        af[i][0] = *reinterpret_cast<const uint32_t *>(&As[r][ks + 2 * t]);
-        af[i][1] = *reinterpret_cast<const uint32_t *>(&As[r + 8][ks + 2 * t]);
-        af[i][2] = *reinterpret_cast<const uint32_t *>(&As[r][ks + 2 * t + 8]);
-        af[i][3] = *reinterpret_cast<const uint32_t *>(&As[r + 8][ks + 2 * t + 8]);
-      }
-#pragma unroll
-      for (int j = 0; j < NJ; ++j) {
-        const int c = wn + j * 8 + g;
-        bf[j][0] = *reinterpret_cast<const uint32_t *>(&Bs[c][ks + 2 * t]);
-        bf[j][1] = *reinterpret_cast<const uint32_t *>(&Bs[c][ks + 2 * t + 8]);
-      }
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < NJ; ++j) mma_16816(acc[i][j], af[i], bf[j]);
-    }
-    __syncthreads();
-  }
+  float acc[2][NJ][4], tot[CAN_FOLD ? 2 : 1][CAN_FOLD ? NJ : 1][4];
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < NJ; ++j)
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const int m = m0 + wm + i * 16 + g + (q >> 1) * 8, n = n0 + wn + j * 8 + 2 * t + (q & 1);
-        if (m >= M || n >= N) continue;
-        if (kchunk > 0) {
-          atomicAdd(C + m * ldc + n, acc[i][j][q]);
-          continue;
-        }
-        float z = acc[i][j][q] + (bias ? bias[n] : 0.f);
-        if (accumulate) z += C[m * ldc + n];
-        C[m * ldc + n] = z;
-        if (Y) Y[m * ldy + n] = __float2bfloat16(act ? silu(z) : z);
+        acc[i][j][q] = 0.f;
+        if constexpr (CAN_FOLD) tot[i][j][q] = 0.f;
       }
+  const int kb = p.split ? z * p.kchunk : 0, ke = p.split ? min(K, kb + p.kchunk) : K;
+  const int nkt = (ke - kb + GK - 1) / GK;
+  const __nv_bfloat16 *A = p.A, *B = p.B;
+  const long long sam = p.sam, sak = p.sak, sbn = p.sbn, sbk = p.sbk;
+  const int amode = p.amode, bmode = p.bmode;
+  // partial sums over `fold` tiles; a shorter one (the last part of K) goes first, as it
+  // would finish first if the parts were blocks of their own
+  const int fold = CAN_FOLD && p.fold ? p.kchunk / GK : 0, lead = fold ? nkt % fold : 0;
+  const TileCopy<BM, NT> ca(A, sam, sak, m0, M, kb, amode);
+  const TileCopy<BN, NT> cb(B, sbn, sbk, n0, N, kb, bmode);
+  auto issue = [&](int it) {
+    if (it < nkt) {
+      __nv_bfloat16 *As = tiles + (it % STAGES) * (ASZ + BSZ), *Bs = As + ASZ;
+      const int kt = it < lead ? nkt - lead + it : it - lead, k0 = kb + kt * GK;
+      if (amode != TILE_ANY)
+        ca.start((unsigned)__cvta_generic_to_shared(As), kt, ke - k0);
+      else
+        stage_any<BM, NT>(A, sam, sak, m0, M, k0, ke, As);
+      if (bmode != TILE_ANY)
+        cb.start((unsigned)__cvta_generic_to_shared(Bs), kt, ke - k0);
+      else
+        stage_any<BN, NT>(B, sbn, sbk, n0, N, k0, ke, Bs);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+#pragma unroll 1
+  for (int it = 0; it < STAGES - 1; ++it) issue(it);
+  // the lane's ldmatrix row and column within a 16 x 16 block of either kind of tile
+  const int j8 = lane >> 3, l8 = lane & 7;
+  const bool at = amode == TILE_R, bt = bmode == TILE_R;
+#pragma unroll 1
+  for (int kt = 0; kt < nkt; ++kt) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2) : "memory");
+    __syncthreads();   // tile kt is here, and tile kt - 1 has been used by every warp
+    issue(kt + STAGES - 1);
+    const __nv_bfloat16 *As = tiles + (kt % STAGES) * (ASZ + BSZ), *Bs = As + ASZ;
+#pragma unroll
+    for (int ks = 0; ks < GK; ks += 16) {
+      uint32_t af[2][4], bf[NJ][2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const __nv_bfloat16 *q = at ? As + (ks + l8 + (j8 >> 1) * 8) * (BM + 8) + wm + i * 16 + (j8 & 1) * 8
+                                    : As + (wm + i * 16 + l8 + (j8 & 1) * 8) * GP + ks + (j8 >> 1) * 8;
+        ldmatrix_x4(af[i], (unsigned)__cvta_generic_to_shared(q), at);
+      }
+#pragma unroll
+      for (int j = 0; j < NJ; j += 2) {
+        const __nv_bfloat16 *q = bt ? Bs + (ks + l8 + (j8 & 1) * 8) * (BN + 8) + wn + j * 8 + (j8 >> 1) * 8
+                                    : Bs + (wn + j * 8 + l8 + (j8 >> 1) * 8) * GP + ks + (j8 & 1) * 8;
+        uint32_t r[4];
+        ldmatrix_x4(r, (unsigned)__cvta_generic_to_shared(q), bt);
+        bf[j][0] = r[0];
+        bf[j][1] = r[1];
+        bf[j + 1][0] = r[2];
+        bf[j + 1][1] = r[3];
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) mma_16816(acc[i][j], af[i], bf[j]);
+    }
+    if constexpr (CAN_FOLD) {
+      if (fold && (kt + 1 - lead) % fold == 0) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int j = 0; j < NJ; ++j)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              tot[i][j][q] += acc[i][j][q];
+              acc[i][j][q] = 0.f;
+            }
+      }
+    }
+  }
+  if constexpr (CAN_FOLD) {
+    if (fold) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) acc[i][j][q] = tot[i][j][q];
+    }
+  }
+  float *C = p.C;
+  __nv_bfloat16 *Y = p.Y;
+  const long long ldc = p.ldc, ldy = p.ldy;
+  const bool pairs = p.pairs;
+  if (p.split) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int m = m0 + wm + i * 16 + g + h * 8, n = n0 + wn + j * 8 + 2 * t;
+          if (m >= M || n >= N) continue;
+          float *c = C + m * ldc + n;
+          if (pairs && n + 1 < N) {
+            atomicAdd(reinterpret_cast<float2 *>(c), make_float2(acc[i][j][2 * h], acc[i][j][2 * h + 1]));
+          } else {
+            atomicAdd(c, acc[i][j][2 * h]);
+            if (n + 1 < N) atomicAdd(c + 1, acc[i][j][2 * h + 1]);
+          }
+        }
+    return;
+  }
+  // the other epilogues from shared memory, four rows of two neighbouring columns a thread at
+  // a time: short code (unrolled over the accumulators, instruction misses were 2 us of a
+  // launch) with its loads in flight
+  constexpr int SP = BN + 8, CG = BN / 2, RSTEP = NT / CG, U = 4;
+  static_assert(BM * SP * 4 <= STAGES * (ASZ + BSZ) * 2 && BM % (RSTEP * U) == 0, "epilogue tile");
+  float *S = reinterpret_cast<float *>(tiles);
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        *reinterpret_cast<float2 *>(S + (wm + i * 16 + g + h * 8) * SP + wn + j * 8 + 2 * t) =
+            make_float2(acc[i][j][2 * h], acc[i][j][2 * h + 1]);
+  __syncthreads();
+  const int c2 = threadIdx.x % CG * 2, n = n0 + c2;
+  if (n >= N) return;
+  const bool two = n + 1 < N, both = pairs && two;
+  const float *bias = p.bias, *dact = p.dact;
+  const bool act = p.act;
+  const float *src = dact ? dact : p.accumulate ? C : nullptr;   // the activation's argument, or what C holds
+  const long long lds = dact ? ldy : ldc;
+  const float b0 = bias ? bias[n] : 0.f, b1 = bias && two ? bias[n + 1] : 0.f;
+  float s0 = 0.f, s1 = 0.f;
+#pragma unroll 1
+  for (int r0 = threadIdx.x / CG; r0 < min(BM, M - m0); r0 += RSTEP * U) {
+    float2 d[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int r = r0 + u * RSTEP;
+      d[u] = make_float2(0.f, 0.f);
+      if (src && m0 + r < M) {
+        const float *q = src + (m0 + r) * lds + n;
+        if (both)
+          d[u] = *reinterpret_cast<const float2 *>(q);
+        else
+          d[u] = make_float2(q[0], two ? q[1] : 0.f);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int r = r0 + u * RSTEP;
+      if (m0 + r >= M) break;
+      const float2 v = *reinterpret_cast<const float2 *>(S + r * SP + c2);
+      const float z0 = v.x + b0 + (dact ? 0.f : d[u].x), z1 = v.y + b1 + (dact ? 0.f : d[u].y);
+      __nv_bfloat16 y0, y1;
+      if (dact) {
+        y0 = __float2bfloat16(z0 * silu_grad(d[u].x));
+        y1 = __float2bfloat16(z1 * silu_grad(d[u].y));
+        s0 += __bfloat162float(y0);
+        s1 += __bfloat162float(y1);
+      } else {
+        float *c = C + (m0 + r) * ldc + n;
+        if (both) {
+          *reinterpret_cast<float2 *>(c) = make_float2(z0, z1);
+        } else {
+          c[0] = z0;
+          if (two) c[1] = z1;
+        }
+        if (!Y) continue;
+        y0 = __float2bfloat16(act ? silu(z0) : z0);
+        y1 = __float2bfloat16(act ? silu(z1) : z1);
+      }
+      __nv_bfloat16 *y = Y + (m0 + r) * ldy + n;
+      if (both) {
+        *reinterpret_cast<__nv_bfloat162 *>(y) = __halves2bfloat162(y0, y1);
+      } else {
+        y[0] = y0;
+        if (two) y[1] = y1;
+      }
+    }
+  }
+  if (dact) {
+    atomicAdd(p.db + n, s0);
+    if (two) atomicAdd(p.db + n + 1, s1);
+  }
 }
 
 __global__ void k_silu_bwd(const float *__restrict__ dY, const float *__restrict__ Z, __nv_bfloat16 *__restrict__ dZ,
@@ -174,18 +373,35 @@ __global__ void k_to_bf16(const float *__restrict__ x, __nv_bfloat16 *__restrict
   if (i < n) y[i] = __float2bfloat16(x[i]);
 }
 
-// db[n] += sum over rows [blockIdx.y * 256, +256) of dZ[m][n]: 32 columns x 8 row groups
-// per block (a warp reads 32 consecutive columns of one row), partial sums reduced in shared
-// memory, one atomic per column and block (db zeroed by the caller).
-__global__ void __launch_bounds__(256) k_colsum(const __nv_bfloat16 *__restrict__ dZ, int M, int N,
-                                                float *__restrict__ db) {
+// The backward step's first pass: dZ = dY in BF16 (dY null: `in` holds it already) and its
+// column sums, db[n] += sum_m dZ[m][n] (db zeroed by the caller).  A block takes 32 columns x
+// kColRows rows, a warp one row at a time (coalesced); one atomic per column and block.
+// (The layers below get both from the epilogue of k_gemm_bf16: as kernels of their own, SiLU'
+// and the sums took 4 + 17 us per layer of 2048 x 256.)
+constexpr int kColRows = 64;
+__global__ void __launch_bounds__(256) k_dz_colsum(const float *__restrict__ dY,
+                                                   const __nv_bfloat16 *__restrict__ in,
+                                                   __nv_bfloat16 *__restrict__ out, int M, int N,
+                                                   float *__restrict__ db) {
   __shared__ float part[8][33];
   const int c = threadIdx.x & 31, rg = threadIdx.x >> 5;
   const int n = blockIdx.x * 32 + c;
-  const int m0 = blockIdx.y * 256, m1 = min(M, m0 + 256);
+  const int m0 = blockIdx.y * kColRows, m1 = min(M, m0 + kColRows);
   float s = 0.f;
-  if (n < N)
-    for (int m = m0 + rg; m < m1; m += 8) s += __bfloat162float(dZ[(long long)m * N + n]);
+  if (n < N) {
+#pragma unroll 4
+    for (int m = m0 + rg; m < m1; m += 8) {
+      const long long e = (long long)m * N + n;
+      __nv_bfloat16 v;
+      if (in) {
+        v = in[e];
+      } else {
+        v = __float2bfloat16(dY[e]);
+        out[e] = v;
+      }
+      s += __bfloat162float(v);
+    }
+  }
   part[rg][c] = s;
   __syncthreads();
   if (rg == 0 && n < N) {
@@ -217,37 +433,124 @@ __global__ void k_mse(const float *__restrict__ pred, const float *__restrict__ 
   if (threadIdx.x == 0) atomicAdd(loss, red[0]);
 }
 
-__global__ void k_adam(float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m1,
-                       float *__restrict__ m2, long long n, float lr, float b1, float b2, float eps, float bc1,
-                       float bc2, float wd, __nv_bfloat16 *__restrict__ wbf) {
+// One Adam step of up to kAdamTensors tensors (blockIdx.y), bias-corrected, decoupled weight
+// decay folded into the gradient, with an optional BF16 copy.  The learning rate and the two
+// bias corrections 1 - b^step come from device memory when `hyper` is given (a captured step
+// is then replayed with a schedule that changes from step to step).
+constexpr int kAdamTensors = 16;
+struct AdamTensors {
+  float *w[kAdamTensors], *m1[kAdamTensors], *m2[kAdamTensors];
+  const float *g[kAdamTensors];
+  __nv_bfloat16 *wbf[kAdamTensors];
+  long long n[kAdamTensors];
+  float wd[kAdamTensors];
+};
+__global__ void __launch_bounds__(256) k_adam(AdamTensors ts, const float *__restrict__ hyper, float lr, float bc1,
+                                              float bc2, float b1, float b2, float eps) {
+  const int k = blockIdx.y;
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float gi = g[i] + wd * w[i];
+  if (i >= ts.n[k]) return;
+  if (hyper) {
+    lr = hyper[0];
+    bc1 = hyper[1];
+    bc2 = hyper[2];
+  }
+  float *w = ts.w[k], *m1 = ts.m1[k], *m2 = ts.m2[k];
+  const float w0 = w[i], gi = ts.g[k][i] + ts.wd[k] * w0;
   const float a = b1 * m1[i] + (1.f - b1) * gi;
   const float b = b2 * m2[i] + (1.f - b2) * gi * gi;
   m1[i] = a;
   m2[i] = b;
-  const float upd = lr * (a / bc1) / (sqrtf(b / bc2) + eps);
-  w[i] -= upd;
-  if (wbf) wbf[i] = __float2bfloat16(w[i]);
+  const float w1 = w0 - lr * (a / bc1) / (sqrtf(b / bc2) + eps);
+  w[i] = w1;
+  if (ts.wbf[k]) ts.wbf[k][i] = __float2bfloat16(w1);
 }
 
-// The same step with the learning rate and the two bias corrections read from device memory
-// (hyper = {lr, 1 - b1^step, 1 - b2^step}), so that a captured training step can be replayed
-// with a schedule that changes from step to step.
-__global__ void k_adam_dev(float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m1,
-                           float *__restrict__ m2, long long n, const float *__restrict__ hyper, float b1, float b2,
-                           float eps, float wd, __nv_bfloat16 *__restrict__ wbf) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float lr = hyper[0], bc1 = hyper[1], bc2 = hyper[2];
-  const float gi = g[i] + wd * w[i];
-  const float a = b1 * m1[i] + (1.f - b1) * gi;
-  const float b = b2 * m2[i] + (1.f - b2) * gi * gi;
-  m1[i] = a;
-  m2[i] = b;
-  w[i] -= lr * (a / bc1) / (sqrtf(b / bc2) + eps);
-  if (wbf) wbf[i] = __float2bfloat16(w[i]);
+// Shared memory above the default 48 KB, asked for once per kernel and device.
+template <typename K>
+cudaError_t allow_tiles(K kernel, int bytes, std::atomic<bool> (&done)[64]) {
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  const int slot = device < 64 ? device : 0;
+  if (device < 64 && done[slot].load(std::memory_order_relaxed)) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) done[slot].store(true, std::memory_order_relaxed);
+  return e;
+}
+
+constexpr int kBigStages = 4, kSmallStages = 6;
+constexpr int kBigSmem = kBigStages * (GM + GN) * GP * 2, kSmallSmem = kSmallStages * (64 + 64) * GP * 2;
+
+Gemm gemm_of(const void *A, long long sam, long long sak, const void *B, long long sbn, long long sbk, float *C,
+             long long ldc, int M, int N, int K) {
+  // 16-byte copies need 16-byte aligned rows (of k or of rows)
+  auto mode = [](const void *p, long long sr, long long sk) {
+    if ((reinterpret_cast<uintptr_t>(p) & 15) != 0) return TILE_ANY;
+    return sk == 1 && sr % 8 == 0 ? TILE_K : sr == 1 && sk % 8 == 0 ? TILE_R : TILE_ANY;
+  };
+  Gemm g = {};
+  g.A = (const __nv_bfloat16 *)A;
+  g.B = (const __nv_bfloat16 *)B;
+  g.sam = sam;
+  g.sak = sak;
+  g.sbn = sbn;
+  g.sbk = sbk;
+  g.amode = mode(A, sam, sak);
+  g.bmode = mode(B, sbn, sbk);
+  g.C = C;
+  g.ldc = ldc;
+  g.M = M;
+  g.N = N;
+  g.K = K;
+  return g;
+}
+
+// Two waves of 148 SMs or more of large tiles.
+bool big_tiles(int M, int N) { return (long long)((N + GN - 1) / GN) * ((M + GM - 1) / GM) >= 296; }
+
+void set_pairs(Gemm &g) {
+  auto aligned = [](const void *p, int bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; };
+  g.pairs = (!g.C || (g.ldc % 2 == 0 && aligned(g.C, 8))) && (!g.Y || (g.ldy % 2 == 0 && aligned(g.Y, 4))) &&
+            (!g.dact || (g.ldy % 2 == 0 && aligned(g.dact, 8)));
+}
+
+void tile_by(Gemm &g, int bm, int bn) {
+  g.nbn = (g.N + bn - 1) / bn;
+  g.nbm = (g.M + bm - 1) / bm;
+  g.nbz = 1;
+}
+
+// Few 64 x 64 output tiles and a long reduction (weight gradients: K = batch rows): K split so
+// that about two waves of blocks run; 0 for one part.
+int k_parts(const Gemm &g) {
+  const long long tiles = (long long)((g.N + 63) / 64) * ((g.M + 63) / 64);
+  if (tiles >= 148 || g.K < 128) return 0;
+  const int splits = (int)std::min<long long>(std::min<long long>((296 + tiles - 1) / tiles, g.K / GK), 64);
+  return splits > 1 ? ((g.K + splits - 1) / splits + GK - 1) / GK * GK : 0;
+}
+
+void split_k(Gemm &g) {
+  g.kchunk = k_parts(g);
+  if (g.kchunk > 0) {
+    g.split = 1;
+    g.nbz = (g.K + g.kchunk - 1) / g.kchunk;
+  }
+}
+
+cqg_status launch_big(const Gemm &g, cudaStream_t st) {
+  static std::atomic<bool> allowed[64];
+  if (allow_tiles(&k_gemm_bf16<GM, GN, 64, kBigStages>, kBigSmem, allowed) != cudaSuccess) return CQG_ERR_CUDA;
+  k_gemm_bf16<GM, GN, 64, kBigStages><<<g.blocks(), 256, kBigSmem, st>>>(g, g, g.blocks());
+  return CQG_OK;
+}
+
+cqg_status launch_small(const Gemm &g, const Gemm *second, cudaStream_t st) {
+  static std::atomic<bool> allowed[64];
+  if (allow_tiles(&k_gemm_bf16<64, 64, 32, kSmallStages>, kSmallSmem, allowed) != cudaSuccess) return CQG_ERR_CUDA;
+  const int n = g.blocks() + (second ? second->blocks() : 0);
+  k_gemm_bf16<64, 64, 32, kSmallStages><<<n, 128, kSmallSmem, st>>>(g, second ? *second : g, g.blocks());
+  return CQG_OK;
 }
 
 inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -261,35 +564,29 @@ cqg_status cqg_mlp_gemm_bf16(const void *A, long long sam, long long sak, const 
                              int act, int accumulate, void *stream) {
   if (!A || !B || !C || M < 0 || N < 0 || K < 0) return CQG_ERR_BAD_ARG;
   if (M == 0 || N == 0) return CQG_OK;
-  const long long big_blocks = (long long)((N + GN - 1) / GN) * ((M + GM - 1) / GM);
   cudaStream_t st = (cudaStream_t)stream;
-  const __nv_bfloat16 *a = (const __nv_bfloat16 *)A, *b = (const __nv_bfloat16 *)B;
-  if (big_blocks >= 296) {   // two waves of 148 SMs or more: large tiles
-    if ((M + GM - 1) / GM > 65535) return CQG_ERR_BAD_ARG;   // grid.y limit
-    dim3 grid((N + GN - 1) / GN, (M + GM - 1) / GM);
-    k_gemm_bf16<GM, GN, 64><<<grid, 256, 0, st>>>(a, sam, sak, b, sbn, sbk, C, ldc, M, N, K, bias,
-                                                  (__nv_bfloat16 *)Y, ldy, act, accumulate, 0);
+  Gemm g = gemm_of(A, sam, sak, B, sbn, sbk, C, ldc, M, N, K);
+  g.bias = bias;
+  g.Y = (__nv_bfloat16 *)Y;
+  g.ldy = ldy;
+  g.act = act != 0;
+  g.accumulate = accumulate != 0;
+  set_pairs(g);
+  const bool big = big_tiles(M, N);
+  if ((M + (big ? GM : 64) - 1) / (big ? GM : 64) > 65535) return CQG_ERR_BAD_ARG;
+  cqg_status s;
+  if (big) {
+    tile_by(g, GM, GN);
+    s = launch_big(g, st);
   } else {
-    if ((M + 63) / 64 > 65535) return CQG_ERR_BAD_ARG;
-    const long long tiles = (long long)((N + 63) / 64) * ((M + 63) / 64);
-    // few output tiles and a long reduction (weight gradients: K = batch rows): split K over
-    // blockIdx.z so that about two waves of CTAs run, partial tiles added with atomics
-    int splits = 1;
-    if (!bias && !Y && tiles < 148 && K >= 4 * GK) {
-      splits = (int)std::min<long long>((296 + tiles - 1) / tiles, K / (2 * GK));
-      splits = std::max(1, std::min(splits, 64));
-    }
-    const int kchunk = splits > 1 ? ((K + splits - 1) / splits + GK - 1) / GK * GK : 0;
-    if (kchunk > 0) {
-      splits = (K + kchunk - 1) / kchunk;
-      if (!accumulate) {
-        if (cudaMemset2DAsync(C, ldc * sizeof(float), 0, N * sizeof(float), M, st) != cudaSuccess) return CQG_ERR_CUDA;
-      }
-    }
-    dim3 grid((N + 63) / 64, (M + 63) / 64, splits);
-    k_gemm_bf16<64, 64, 32><<<grid, 128, 0, st>>>(a, sam, sak, b, sbn, sbk, C, ldc, M, N, K, bias,
-                                                  (__nv_bfloat16 *)Y, ldy, act, accumulate, kchunk);
+    tile_by(g, 64, 64);
+    if (!bias && !Y) split_k(g);
+    if (g.split && !accumulate &&
+        cudaMemset2DAsync(C, ldc * sizeof(float), 0, N * sizeof(float), M, st) != cudaSuccess)
+      return CQG_ERR_CUDA;
+    s = launch_small(g, nullptr, st);
   }
+  if (s != CQG_OK) return s;
   return cudaGetLastError() == cudaSuccess ? CQG_OK : CQG_ERR_CUDA;
 }
 
@@ -309,9 +606,9 @@ cqg_status cqg_mlp_colsum(const void *dZ, int M, int N, float *db, void *stream)
   if (N <= 0) return CQG_OK;
   if (cudaMemsetAsync(db, 0, (size_t)N * sizeof(float), (cudaStream_t)stream) != cudaSuccess) return CQG_ERR_CUDA;
   if (M <= 0) return CQG_OK;
-  if ((M + 255) / 256 > 65535) return CQG_ERR_BAD_ARG;
-  dim3 grid((N + 31) / 32, (M + 255) / 256);
-  k_colsum<<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16 *)dZ, M, N, db);
+  if ((M + kColRows - 1) / kColRows > 65535) return CQG_ERR_BAD_ARG;
+  dim3 grid((N + 31) / 32, (M + kColRows - 1) / kColRows);
+  k_dz_colsum<<<grid, 256, 0, (cudaStream_t)stream>>>(nullptr, (const __nv_bfloat16 *)dZ, nullptr, M, N, db);
   return cudaGetLastError() == cudaSuccess ? CQG_OK : CQG_ERR_CUDA;
 }
 
@@ -322,20 +619,115 @@ cqg_status cqg_mlp_mse(const float *pred, const float *target, const float *mask
   return cudaGetLastError() == cudaSuccess ? CQG_OK : CQG_ERR_CUDA;
 }
 
+cqg_status cqg_mlp_adam_tensors(int nt, float *const *w, const float *const *g, float *const *m1, float *const *m2,
+                                const long long *n, const float *weight_decay, void *const *wbf, const float *hyper,
+                                float lr, float b1, float b2, float eps, int step, void *stream) {
+  if (nt <= 0 || nt > kAdamTensors || !w || !g || !m1 || !m2 || !n || !weight_decay || !wbf || (!hyper && step < 1))
+    return CQG_ERR_BAD_ARG;
+  AdamTensors ts = {};
+  long long most = 0;
+  for (int k = 0; k < nt; ++k) {
+    if (n[k] <= 0) return CQG_ERR_BAD_ARG;
+    ts.w[k] = w[k];
+    ts.g[k] = g[k];
+    ts.m1[k] = m1[k];
+    ts.m2[k] = m2[k];
+    ts.wbf[k] = (__nv_bfloat16 *)wbf[k];
+    ts.n[k] = n[k];
+    ts.wd[k] = weight_decay[k];
+    most = std::max(most, n[k]);
+  }
+  const float bc1 = hyper ? 1.f : 1.f - powf(b1, (float)step), bc2 = hyper ? 1.f : 1.f - powf(b2, (float)step);
+  k_adam<<<dim3(nblk(most, 256), nt), 256, 0, (cudaStream_t)stream>>>(ts, hyper, lr, bc1, bc2, b1, b2, eps);
+  return cudaGetLastError() == cudaSuccess ? CQG_OK : CQG_ERR_CUDA;
+}
+
 cqg_status cqg_mlp_adam(float *w, const float *g, float *m1, float *m2, long long n, float lr, float b1, float b2,
                         float eps, int step, float weight_decay, void *wbf, void *stream) {
-  if (n <= 0 || step < 1) return CQG_ERR_BAD_ARG;
-  const float bc1 = 1.f - powf(b1, (float)step), bc2 = 1.f - powf(b2, (float)step);
-  k_adam<<<nblk(n, 256), 256, 0, (cudaStream_t)stream>>>(w, g, m1, m2, n, lr, b1, b2, eps, bc1, bc2, weight_decay,
-                                                         (__nv_bfloat16 *)wbf);
-  return cudaGetLastError() == cudaSuccess ? CQG_OK : CQG_ERR_CUDA;
+  if (step < 1) return CQG_ERR_BAD_ARG;
+  return cqg_mlp_adam_tensors(1, &w, &g, &m1, &m2, &n, &weight_decay, &wbf, nullptr, lr, b1, b2, eps, step, stream);
 }
 
 cqg_status cqg_mlp_adam_dev(float *w, const float *g, float *m1, float *m2, long long n, const float *hyper,
                             float b1, float b2, float eps, float weight_decay, void *wbf, void *stream) {
-  if (n <= 0 || !hyper) return CQG_ERR_BAD_ARG;
-  k_adam_dev<<<nblk(n, 256), 256, 0, (cudaStream_t)stream>>>(w, g, m1, m2, n, hyper, b1, b2, eps, weight_decay,
-                                                             (__nv_bfloat16 *)wbf);
+  if (!hyper) return CQG_ERR_BAD_ARG;
+  return cqg_mlp_adam_tensors(1, &w, &g, &m1, &m2, &n, &weight_decay, &wbf, hyper, 0.f, b1, b2, eps, 0, stream);
+}
+
+cqg_status cqg_mlp_forward(int nl, const int *dims, int M, const void *X, const void *const *W, const float *const *b,
+                           float *const *Z, void *const *Y, void *stream) {
+  if (nl <= 0 || !dims || M < 0 || !X || !W || !b || !Z || !Y) return CQG_ERR_BAD_ARG;
+  const void *h = X;
+  for (int i = 0; i < nl; ++i) {
+    const int K = dims[i], N = dims[i + 1];
+    const bool last = i == nl - 1;
+    const cqg_status st = cqg_mlp_gemm_bf16(h, K, 1, W[i], K, 1, Z[i], N, M, N, K, b[i], last ? nullptr : Y[i], N,
+                                            last ? 0 : 1, 0, stream);
+    if (st != CQG_OK) return st;
+    h = Y[i];
+  }
+  return CQG_OK;
+}
+
+cqg_status cqg_mlp_backward(int nl, const int *dims, int M, const float *dout, const void *const *H,
+                            const float *const *Z, const void *const *W, void *dZ0, void *dZ1, float *grads,
+                            void *stream) {
+  if (nl <= 0 || !dims || M < 0 || !dout || !H || !Z || !W || !dZ0 || !dZ1 || !grads) return CQG_ERR_BAD_ARG;
+  if ((M + 63) / 64 > 65535) return CQG_ERR_BAD_ARG;
+  cudaStream_t st = (cudaStream_t)stream;
+  long long nw = 0, nb = 0;
+  for (int i = 0; i < nl; ++i) {
+    if (dims[i] <= 0 || dims[i + 1] <= 0) return CQG_ERR_BAD_ARG;
+    nw += (long long)dims[i] * dims[i + 1];
+    nb += dims[i + 1];
+  }
+  // weight gradients of the layers, then bias gradients: all are added into zeros
+  if (cudaMemsetAsync(grads, 0, (size_t)(nw + nb) * sizeof(float), st) != cudaSuccess) return CQG_ERR_CUDA;
+  if (M == 0) return CQG_OK;
+  float *gw = grads + nw, *gb = grads + nw + nb;
+  __nv_bfloat16 *dZ = (__nv_bfloat16 *)dZ0, *next = (__nv_bfloat16 *)dZ1;
+  const int nout = dims[nl];
+  gb -= nout;
+  k_dz_colsum<<<dim3((nout + 31) / 32, (M + kColRows - 1) / kColRows), 256, 0, st>>>(dout, nullptr, dZ, M, nout, gb);
+  for (int i = nl - 1; i >= 0; --i) {
+    const int K = dims[i], N = dims[i + 1];
+    gw -= (long long)K * N;
+    // dW[n][k] = sum_m dZ[m][n] h[m][k]
+    Gemm w = gemm_of(dZ, 1, N, H[i], 1, K, gw, K, N, K, M);
+    w.accumulate = 1;
+    set_pairs(w);
+    const bool wbig = big_tiles(N, K);
+    tile_by(w, wbig ? GM : 64, wbig ? GN : 64);
+    if (!wbig) split_k(w);
+    cqg_status s = CQG_OK;
+    if (i > 0) {
+      // dh[m][k] = sum_n dZ[m][n] W[n][k], through the SiLU of the layer below: the next dZ.
+      // In partial sums as k_parts() would split them: the order in which split products add up
+      Gemm x = gemm_of(dZ, N, 1, W[i], 1, K, nullptr, K, M, K, N);
+      gb -= K;
+      x.dact = Z[i - 1];
+      x.Y = next;
+      x.ldy = K;
+      x.db = gb;
+      set_pairs(x);
+      const bool xbig = big_tiles(M, K);
+      tile_by(x, xbig ? GM : 64, xbig ? GN : 64);
+      if (!xbig) {
+        x.kchunk = k_parts(x);
+        x.fold = x.kchunk > 0;
+      }
+      if (!xbig && !wbig) {
+        s = launch_small(x, &w, st);
+      } else {
+        s = xbig ? launch_big(x, st) : launch_small(x, nullptr, st);
+        if (s == CQG_OK) s = wbig ? launch_big(w, st) : launch_small(w, nullptr, st);
+      }
+    } else {
+      s = wbig ? launch_big(w, st) : launch_small(w, nullptr, st);
+    }
+    if (s != CQG_OK) return s;
+    std::swap(dZ, next);
+  }
   return cudaGetLastError() == cudaSuccess ? CQG_OK : CQG_ERR_CUDA;
 }
 
