@@ -1005,10 +1005,12 @@ __global__ void __launch_bounds__(kEriThreads) k_eri_jk(const uint2 *__restrict_
 
 // Classes whose kernel is compiled for MB resident CTAs per SM (launch bounds with a
 // minimum block count; the other classes keep the compiler's own register choice).
-// Measured on (H2O)_32 cc-pVDZ: (ps|ps) at 4 against 3 CTAs 4.3 % faster, (pp|ss) 2.9 %, (ds|ps) at
-// 3 against 2 2.8 %; (ds|ss) 1.99 ms at 4, 2.28 at the compiler's 3; (ps|ss) 7.57 ms at 5, 7.75 at
-// 4; (ss|ss) 3.76 ms at 4, 4.00 at 3 (168 registers).  (dp|ss) is held at 3 (242 registers
-// without).
+// Measured on (H2O)_32 cc-pVDZ: (ps|ps) at 4 against 3 CTAs 4.3 % faster, at 5 4.26 -> 5.79 ms;
+// (ds|ps) at 3 against 2 2.8 %, at 4 2.67 -> 3.00 ms; (pp|ss) 2.23 ms at 5, 2.35 at 4; (ds|ss) 1.97
+// ms at 4, 2.28 at the compiler's 3 (1.92 at 5, but 0.37 instead of 0.33 ms on (H2O)_11); (ps|ss)
+// 7.53 ms at 5, 7.75 at 4, 8.18 at 6; (ss|ss) 3.75 ms at 4, 4.00 at 3 (168 registers), 4.01 at 5;
+// (dp|ss) 1.06 ms at 4, 1.13 at 3; (pp|ps) 3.32 ms at the compiler's 2, 3.36 at 3.  They are bound
+// by the latency of their chains and loads, up to the registers that spill.
 template <int LA, int LB, int LC, int LD>
 struct EriMinBlocks {
   static constexpr int v = 0;
@@ -1019,7 +1021,7 @@ struct EriMinBlocks<1, 0, 1, 0> {
 };
 template <>
 struct EriMinBlocks<1, 1, 0, 0> {
-  static constexpr int v = 4;
+  static constexpr int v = 5;
 };
 template <>
 struct EriMinBlocks<2, 0, 1, 0> {
@@ -1039,7 +1041,7 @@ struct EriMinBlocks<1, 0, 0, 0> {
 };
 template <>
 struct EriMinBlocks<2, 1, 0, 0> {
-  static constexpr int v = 3;
+  static constexpr int v = 4;
 };
 
 template <int LA, int LB, int LC, int LD, typename T, int MB>
