@@ -14,6 +14,7 @@
 //                      the scales are folded into the digest).
 #include "engine_impl.cuh"
 
+#include <list>
 #include <map>
 #include <mutex>
 
@@ -26,13 +27,20 @@
 // time (each free waits for the device; together 4 to 20 ms for ten waters).  Freed blocks are
 // kept for the next request of their size class: powers of two up to 1 MiB, eighths of one
 // above.  (With the primitive pairs formed on the device as well, setting up (H2O)_10 cc-pVDZ
-// takes 2.1 ms instead of 13.4.)  Blocks above kPoolLargest are not kept, and at most kPoolKeep bytes are per process
-// and device; a request that the device cannot meet gives the kept blocks back first.
+// takes 2.1 ms instead of 13.4.)  Blocks above kPoolLargest are not kept, and at most kPoolKeep
+// bytes are per process and device: a freed block takes the place of those that have lain there
+// longest (with new blocks turned away instead, a pool filled by earlier, larger contexts made
+// the same set-up 4.5 ms).  A request that the device cannot meet gives all of them back first.
 namespace {
 constexpr size_t kPoolLargest = 64u << 20, kPoolKeep = 256u << 20;
 struct DevicePool {
+  struct Block {
+    size_t bytes;
+    void *p;
+  };
   std::mutex mutex;
-  std::multimap<size_t, void *> blocks;
+  std::list<Block> blocks;   // in the order in which they were freed
+  std::multimap<size_t, std::list<Block>::iterator> by_size;
   size_t kept = 0;
 };
 DevicePool &device_pool(int device) {
@@ -55,12 +63,13 @@ cudaError_t cqg_pool_alloc(void **p, size_t *bytes, int *device) {
   DevicePool &pool = device_pool(*device);
   if (*device < 64 && size <= kPoolLargest) {
     std::lock_guard<std::mutex> lock(pool.mutex);
-    auto it = pool.blocks.find(size);
-    if (it != pool.blocks.end()) {
-      *p = it->second;
+    auto it = pool.by_size.find(size);
+    if (it != pool.by_size.end()) {
+      *p = it->second->p;
       *bytes = size;
       pool.kept -= size;
-      pool.blocks.erase(it);
+      pool.blocks.erase(it->second);
+      pool.by_size.erase(it);
       return cudaSuccess;
     }
   }
@@ -69,8 +78,9 @@ cudaError_t cqg_pool_alloc(void **p, size_t *bytes, int *device) {
     cudaGetLastError();
     {
       std::lock_guard<std::mutex> lock(pool.mutex);
-      for (auto &b : pool.blocks) cudaFree(b.second);
+      for (auto &b : pool.blocks) cudaFree(b.p);
       pool.blocks.clear();
+      pool.by_size.clear();
       pool.kept = 0;
     }
     e = cudaMalloc(p, size);
@@ -84,16 +94,27 @@ cudaError_t cqg_pool_alloc(void **p, size_t *bytes, int *device) {
 }
 
 void cqg_pool_free(void *p, size_t bytes, int device) {
-  if (device < 64 && bytes <= kPoolLargest) {
-    DevicePool &pool = device_pool(device);
+  if (device >= 64 || bytes > kPoolLargest) {
+    cudaFree(p);
+    return;
+  }
+  DevicePool &pool = device_pool(device);
+  std::list<DevicePool::Block> out;
+  {
     std::lock_guard<std::mutex> lock(pool.mutex);
-    if (pool.kept + bytes <= kPoolKeep) {
-      pool.blocks.emplace(bytes, p);
-      pool.kept += bytes;
-      return;
+    pool.blocks.push_back({bytes, p});
+    pool.by_size.emplace(bytes, std::prev(pool.blocks.end()));
+    pool.kept += bytes;
+    while (pool.kept > kPoolKeep) {
+      const auto old = pool.blocks.begin();
+      auto it = pool.by_size.find(old->bytes);
+      while (it->second != old) ++it;
+      pool.by_size.erase(it);
+      pool.kept -= old->bytes;
+      out.splice(out.end(), pool.blocks, old);
     }
   }
-  cudaFree(p);
+  for (auto &b : out) cudaFree(b.p);
 }
 
 static const char *kLetters = "spdfg";
