@@ -385,8 +385,8 @@ __global__ void __launch_bounds__(256) k_dz_colsum(const float *__restrict__ dY,
                                                    float *__restrict__ db) {
   __shared__ float part[8][33];
   const int c = threadIdx.x & 31, rg = threadIdx.x >> 5;
-  const int n = blockIdx.x * 32 + c;
-  const int m0 = blockIdx.y * kColRows, m1 = min(M, m0 + kColRows);
+  const int n = blockIdx.y * 32 + c;
+  const int m0 = blockIdx.x * kColRows, m1 = (int)min((long long)M, (long long)m0 + kColRows);
   float s = 0.f;
   if (n < N) {
 #pragma unroll 4
@@ -606,8 +606,8 @@ cqg_status cqg_mlp_colsum(const void *dZ, int M, int N, float *db, void *stream)
   if (N <= 0) return CQG_OK;
   if (cudaMemsetAsync(db, 0, (size_t)N * sizeof(float), (cudaStream_t)stream) != cudaSuccess) return CQG_ERR_CUDA;
   if (M <= 0) return CQG_OK;
-  if ((M + kColRows - 1) / kColRows > 65535) return CQG_ERR_BAD_ARG;
-  dim3 grid((N + 31) / 32, (M + kColRows - 1) / kColRows);
+  if ((M + 255) / 256 > 65535 || (N + 31) / 32 > 65535) return CQG_ERR_BAD_ARG;
+  dim3 grid((M + kColRows - 1) / kColRows, (N + 31) / 32);
   k_dz_colsum<<<grid, 256, 0, (cudaStream_t)stream>>>(nullptr, (const __nv_bfloat16 *)dZ, nullptr, M, N, db);
   return cudaGetLastError() == cudaSuccess ? CQG_OK : CQG_ERR_CUDA;
 }
@@ -622,23 +622,27 @@ cqg_status cqg_mlp_mse(const float *pred, const float *target, const float *mask
 cqg_status cqg_mlp_adam_tensors(int nt, float *const *w, const float *const *g, float *const *m1, float *const *m2,
                                 const long long *n, const float *weight_decay, void *const *wbf, const float *hyper,
                                 float lr, float b1, float b2, float eps, int step, void *stream) {
-  if (nt <= 0 || nt > kAdamTensors || !w || !g || !m1 || !m2 || !n || !weight_decay || !wbf || (!hyper && step < 1))
+  if (nt <= 0 || !w || !g || !m1 || !m2 || !n || !weight_decay || !wbf || (!hyper && step < 1))
     return CQG_ERR_BAD_ARG;
-  AdamTensors ts = {};
-  long long most = 0;
-  for (int k = 0; k < nt; ++k) {
+  for (int k = 0; k < nt; ++k)
     if (n[k] <= 0) return CQG_ERR_BAD_ARG;
-    ts.w[k] = w[k];
-    ts.g[k] = g[k];
-    ts.m1[k] = m1[k];
-    ts.m2[k] = m2[k];
-    ts.wbf[k] = (__nv_bfloat16 *)wbf[k];
-    ts.n[k] = n[k];
-    ts.wd[k] = weight_decay[k];
-    most = std::max(most, n[k]);
-  }
   const float bc1 = hyper ? 1.f : 1.f - powf(b1, (float)step), bc2 = hyper ? 1.f : 1.f - powf(b2, (float)step);
-  k_adam<<<dim3(nblk(most, 256), nt), 256, 0, (cudaStream_t)stream>>>(ts, hyper, lr, bc1, bc2, b1, b2, eps);
+  for (int k0 = 0; k0 < nt; k0 += kAdamTensors) {
+    AdamTensors ts = {};
+    const int m = std::min(kAdamTensors, nt - k0);
+    long long most = 0;
+    for (int k = 0; k < m; ++k) {
+      ts.w[k] = w[k0 + k];
+      ts.g[k] = g[k0 + k];
+      ts.m1[k] = m1[k0 + k];
+      ts.m2[k] = m2[k0 + k];
+      ts.wbf[k] = (__nv_bfloat16 *)wbf[k0 + k];
+      ts.n[k] = n[k0 + k];
+      ts.wd[k] = weight_decay[k0 + k];
+      most = std::max(most, ts.n[k]);
+    }
+    k_adam<<<dim3(nblk(most, 256), m), 256, 0, (cudaStream_t)stream>>>(ts, hyper, lr, bc1, bc2, b1, b2, eps);
+  }
   return cudaGetLastError() == cudaSuccess ? CQG_OK : CQG_ERR_CUDA;
 }
 
@@ -673,7 +677,7 @@ cqg_status cqg_mlp_backward(int nl, const int *dims, int M, const float *dout, c
                             const float *const *Z, const void *const *W, void *dZ0, void *dZ1, float *grads,
                             void *stream) {
   if (nl <= 0 || !dims || M < 0 || !dout || !H || !Z || !W || !dZ0 || !dZ1 || !grads) return CQG_ERR_BAD_ARG;
-  if ((M + 63) / 64 > 65535) return CQG_ERR_BAD_ARG;
+  if ((M + GM - 1) / GM > 65535) return CQG_ERR_BAD_ARG;   // as cqg_mlp_gemm_bf16
   cudaStream_t st = (cudaStream_t)stream;
   long long nw = 0, nb = 0;
   for (int i = 0; i < nl; ++i) {
@@ -688,7 +692,8 @@ cqg_status cqg_mlp_backward(int nl, const int *dims, int M, const float *dout, c
   __nv_bfloat16 *dZ = (__nv_bfloat16 *)dZ0, *next = (__nv_bfloat16 *)dZ1;
   const int nout = dims[nl];
   gb -= nout;
-  k_dz_colsum<<<dim3((nout + 31) / 32, (M + kColRows - 1) / kColRows), 256, 0, st>>>(dout, nullptr, dZ, M, nout, gb);
+  if ((nout + 31) / 32 > 65535) return CQG_ERR_BAD_ARG;
+  k_dz_colsum<<<dim3((M + kColRows - 1) / kColRows, (nout + 31) / 32), 256, 0, st>>>(dout, nullptr, dZ, M, nout, gb);
   for (int i = nl - 1; i >= 0; --i) {
     const int K = dims[i], N = dims[i + 1];
     gw -= (long long)K * N;

@@ -299,7 +299,7 @@ cqg_status cqg_mlp_adam_dev(float *w, const float *g, float *m1, float *m2, long
  * gradients, packed in `grads`: dW[0], ..., dW[nl-1], db[0], ..., db[nl-1].  dZ0 and dZ1
  * are scratch of M x max(dims[1..nl]) BF16 elements each.
  * cqg_mlp_adam_tensors: the step of cqg_mlp_adam (hyper null) or cqg_mlp_adam_dev (hyper given)
- * for nt <= 16 tensors; w, g, m1, m2, n, weight_decay, wbf (entries may be null) have nt entries. */
+ * for nt tensors, 16 per launch; w, g, m1, m2, n, weight_decay, wbf (entries may be null) have nt entries. */
 cqg_status cqg_mlp_forward(int nl, const int *dims, int M, const void *X, const void *const *W,
                            const float *const *b, float *const *Z, void *const *Y, void *stream);
 cqg_status cqg_mlp_backward(int nl, const int *dims, int M, const float *dout, const void *const *H,

@@ -61,10 +61,11 @@ def test_backward_pass(batch, width):
         assert bool(((got.double() - ref).abs() <= tol + 1e-30).all())
 
 
-def test_adam_of_all_tensors():
+@pytest.mark.parametrize("layers", [2, 9])   # fewer tensors than a launch takes, and more
+def test_adam_of_all_tensors(layers):
     _gpu()
     from chronusq_public_b200.guess_model import PairMLP
-    m = PairMLP(width=40, layers=2, seed=5, maxf=14)
+    m = PairMLP(width=40, layers=layers, seed=5, maxf=14)
     rng = np.random.default_rng(7)
     gW, gb = ([torch.tensor(rng.standard_normal(x.shape), dtype=torch.float32, device="cuda") for x in xs]
               for xs in (m.W, m.b))
