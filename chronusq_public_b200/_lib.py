@@ -12,6 +12,8 @@ import os
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libcqgpu.so")
 
+MLP_DX_MAX = 148 * 64 * 64   # CQG_MLP_DX_MAX
+
 _lib = None
 
 
@@ -118,7 +120,7 @@ def load(path: str = LIB_PATH):
     L.cqg_mlp_adam_dev.argtypes = [vp, vp, vp, vp, ll, vp, f, f, f, f, vp, vp]
     pv = ctypes.POINTER(vp)
     L.cqg_mlp_forward.argtypes = [ctypes.c_int, i, ctypes.c_int, vp, pv, pv, pv, pv, vp]
-    L.cqg_mlp_backward.argtypes = [ctypes.c_int, i, ctypes.c_int, vp, pv, pv, pv, vp, vp, vp, vp]
+    L.cqg_mlp_backward.argtypes = [ctypes.c_int, i, ctypes.c_int, vp, pv, pv, pv, vp, vp, vp, vp, vp]
     L.cqg_mlp_adam_tensors.argtypes = [ctypes.c_int, pv, pv, pv, pv, ctypes.POINTER(ll), ctypes.POINTER(f), pv, vp, f,
                                        f, f, f, ctypes.c_int, vp]
     L.cqg_class_name.argtypes = [ctypes.c_int]

@@ -6,7 +6,9 @@
 //                 BF16 -> FP32 over block tiles that come through a ring of asynchronous
 //                 copies; optional fused epilogue Z = C + bias (FP32) and Y = SiLU(Z) (BF16).
 //                 or, backward, dZ = C * SiLU'(Z) (BF16, the next GEMMs' operand) and its column sums
-//   k_dz_colsum : the output layer's dZ in BF16 and db[n] = sum_m dZ[m][n]
+//   k_gemm_parts: C[m][n] += sum_k A(m,k) B(n,k), the parts of a split K added with atomics (the
+//                 gradient of a layer's input)
+//   k_dz_colsum : a layer's dZ in BF16, through SiLU' for the hidden ones, and db[n] = sum_m dZ[m][n]
 //   k_mse       : masked squared error, its gradient, and the loss sum
 //   k_adam      : Adam step on FP32 master weights, BF16 copy for the next pass, all tensors of
 //                 the network in one launch
@@ -123,10 +125,9 @@ __device__ __forceinline__ void stage_any(const __nv_bfloat16 *__restrict__ X, l
 }
 
 // One product of a launch.  split: the block reduces k in [z kchunk, (z + 1) kchunk) and adds
-// its partial tile to C with atomics (C zeroed by the caller), no epilogue.  fold: the block
-// reduces all of K, in partial sums over kchunk each.  dact: the epilogue is the backward
-// step through the layer below, Y = bf16(value * SiLU'(dact)) and its column sums added to
-// db; C is not written.
+// its partial tile to C with atomics (C zeroed by the caller), no epilogue.  dact: the
+// epilogue is the backward step through the layer below, Y = bf16(value * SiLU'(dact)) and its
+// column sums added to db; C is not written.
 struct Gemm {
   const __nv_bfloat16 *A, *B;
   long long sam, sak, sbn, sbk, ldc, ldy;
@@ -135,7 +136,7 @@ struct Gemm {
   float *db;
   __nv_bfloat16 *Y;
   int M, N, K, kchunk, nbn, nbm, nbz;
-  unsigned char amode, bmode, act, accumulate, split, fold, pairs;   // pairs: C, Y and dact take 2-wide accesses
+  unsigned char amode, bmode, act, accumulate, split, pairs;   // pairs: C, Y and dact take 2-wide accesses
   __host__ int blocks() const { return nbn * nbm * nbz; }
 };
 
@@ -144,16 +145,16 @@ struct Gemm {
 // tiles.  128 x 128 with 8 warps of 32 x 64 for large problems, 64 x 64 with 4 warps of
 // 32 x 32 when the large tiles would leave most of the 148 SMs idle.  A training step's
 // products (2048 x 256 x 256) are chains of load latencies, not arithmetic: tiles of 32 k come
-// through a ring of STAGES asynchronous copies, and two products of one layer (its weight
-// gradient and the gradient of its input) share a launch, the first `blocks0` blocks for g0.
+// through a ring of STAGES asynchronous copies, and two products (the weight gradients of two
+// layers, or one with the gradient of its layer's input) share a launch, the first `blocks0`
+// blocks for g0.
 // Measured, 2048 rows, width 256: a layer forward 17 us cold (9.1 us back to back) from one
-// synchronous tile at a time before; the backward pass 70 us for six launches.
+// synchronous tile at a time before.
 template <int BM, int BN, int WN, int STAGES>
 __global__ void __launch_bounds__((BM / 32) * (BN / WN) * 32, BM == 64 ? 3 : 2)
     k_gemm_bf16(const __grid_constant__ Gemm g0, const __grid_constant__ Gemm g1, int blocks0) {
   constexpr int NWM = BM / 32, NJ = WN / 8, NT = NWM * (BN / WN) * 32;
   constexpr int ASZ = BM * GP, BSZ = BN * GP;   // [k][row] tiles, GK x (rows + 8), fit as well
-  constexpr bool CAN_FOLD = BM == 64;           // the registers of a second accumulator
   static_assert(GK * (BM + 8) <= ASZ && GK * (BN + 8) <= BSZ, "tile buffers");
   extern __shared__ __align__(16) __nv_bfloat16 tiles[];
   const bool first = (int)blockIdx.x < blocks0;
@@ -164,30 +165,24 @@ __global__ void __launch_bounds__((BM / 32) * (BN / WN) * 32, BM == 64 ? 3 : 2)
   const int M = p.M, N = p.N, K = p.K;
   const int n0 = blk % p.nbn * BN, m0 = blk / p.nbn % p.nbm * BM, z = blk / (p.nbn * p.nbm);
   const int g = lane >> 2, t = lane & 3;
-  float acc[2][NJ][4], tot[CAN_FOLD ? 2 : 1][CAN_FOLD ? NJ : 1][4];
+  float acc[2][NJ][4];
 #pragma unroll
   for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < NJ; ++j)
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        acc[i][j][q] = 0.f;
-        if constexpr (CAN_FOLD) tot[i][j][q] = 0.f;
-      }
+      for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.f;
   const int kb = p.split ? z * p.kchunk : 0, ke = p.split ? min(K, kb + p.kchunk) : K;
   const int nkt = (ke - kb + GK - 1) / GK;
   const __nv_bfloat16 *A = p.A, *B = p.B;
   const long long sam = p.sam, sak = p.sak, sbn = p.sbn, sbk = p.sbk;
   const int amode = p.amode, bmode = p.bmode;
-  // partial sums over `fold` tiles; a shorter one (the last part of K) goes first, as it
-  // would finish first if the parts were blocks of their own
-  const int fold = CAN_FOLD && p.fold ? p.kchunk / GK : 0, lead = fold ? nkt % fold : 0;
   const TileCopy<BM, NT> ca(A, sam, sak, m0, M, kb, amode);
   const TileCopy<BN, NT> cb(B, sbn, sbk, n0, N, kb, bmode);
-  auto issue = [&](int it) {
-    if (it < nkt) {
-      __nv_bfloat16 *As = tiles + (it % STAGES) * (ASZ + BSZ), *Bs = As + ASZ;
-      const int kt = it < lead ? nkt - lead + it : it - lead, k0 = kb + kt * GK;
+  auto issue = [&](int kt) {
+    if (kt < nkt) {
+      __nv_bfloat16 *As = tiles + (kt % STAGES) * (ASZ + BSZ), *Bs = As + ASZ;
+      const int k0 = kb + kt * GK;
       if (amode != TILE_ANY)
         ca.start((unsigned)__cvta_generic_to_shared(As), kt, ke - k0);
       else
@@ -200,7 +195,7 @@ __global__ void __launch_bounds__((BM / 32) * (BN / WN) * 32, BM == 64 ? 3 : 2)
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
 #pragma unroll 1
-  for (int it = 0; it < STAGES - 1; ++it) issue(it);
+  for (int kt = 0; kt < STAGES - 1; ++kt) issue(kt);
   // the lane's ldmatrix row and column within a 16 x 16 block of either kind of tile
   const int j8 = lane >> 3, l8 = lane & 7;
   const bool at = amode == TILE_R, bt = bmode == TILE_R;
@@ -234,29 +229,6 @@ __global__ void __launch_bounds__((BM / 32) * (BN / WN) * 32, BM == 64 ? 3 : 2)
       for (int i = 0; i < 2; ++i)
 #pragma unroll
         for (int j = 0; j < NJ; ++j) mma_16816(acc[i][j], af[i], bf[j]);
-    }
-    if constexpr (CAN_FOLD) {
-      if (fold && (kt + 1 - lead) % fold == 0) {
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-          for (int j = 0; j < NJ; ++j)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              tot[i][j][q] += acc[i][j][q];
-              acc[i][j][q] = 0.f;
-            }
-      }
-    }
-  }
-  if constexpr (CAN_FOLD) {
-    if (fold) {
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < NJ; ++j)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) acc[i][j][q] = tot[i][j][q];
     }
   }
   float *C = p.C;
@@ -362,6 +334,123 @@ __global__ void __launch_bounds__((BM / 32) * (BN / WN) * 32, BM == 64 ? 3 : 2)
   }
 }
 
+// Rows [r0, r0 + 64) x k [k0, k0 + 32) of X(r, k) = X[r * sr + k * sk] into S[row][k] (zero outside
+// nrows x K).  Rows or k contiguous and 16-byte aligned: 8-element loads; anything else element
+// by element.
+constexpr int kPartTile = 64;
+static_assert(148 * kPartTile * kPartTile == CQG_MLP_DX_MAX, "fewer than 148 tiles (k_parts) are split");
+__device__ __forceinline__ void stage_part(const __nv_bfloat16 *__restrict__ X, long long sr, long long sk, int r0,
+                                           int nrows, int k0, int K, bool vec_k, bool vec_r,
+                                           __nv_bfloat16 (*S)[GP]) {
+  const int tid = threadIdx.x, nth = blockDim.x;
+  const __nv_bfloat16 zero = __float2bfloat16(0.f);
+  if (vec_k) {                 // sk == 1, sr % 8 == 0, K % 8 == 0, X 16-byte aligned
+    for (int e = tid; e < kPartTile * (GK / 8); e += nth) {
+      const int rr = e / (GK / 8), kv = (e % (GK / 8)) * 8;
+      const int r = r0 + rr, k = k0 + kv;
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (r < nrows && k < K) v = *reinterpret_cast<const uint4 *>(X + (long long)r * sr + k);
+      *reinterpret_cast<uint4 *>(&S[rr][kv]) = v;
+    }
+  } else if (vec_r) {          // sr == 1, sk % 8 == 0, nrows % 8 == 0, X 16-byte aligned
+    for (int e = tid; e < GK * (kPartTile / 8); e += nth) {
+      const int kk = e / (kPartTile / 8), rv = (e % (kPartTile / 8)) * 8;
+      const int r = r0 + rv, k = k0 + kk;
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (r < nrows && k < K) v = *reinterpret_cast<const uint4 *>(X + r + (long long)k * sk);
+      const __nv_bfloat16 *h = reinterpret_cast<const __nv_bfloat16 *>(&v);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) S[rv + i][kk] = h[i];
+    }
+  } else if (sk <= sr) {       // k varies fastest across threads
+    for (int e = tid; e < kPartTile * GK; e += nth) {
+      const int rr = e / GK, kk = e % GK;
+      const int r = r0 + rr, k = k0 + kk;
+      S[rr][kk] = (r < nrows && k < K) ? X[(long long)r * sr + (long long)k * sk] : zero;
+    }
+  } else {                     // rows vary fastest across threads
+    for (int e = tid; e < kPartTile * GK; e += nth) {
+      const int kk = e / kPartTile, rr = e % kPartTile;
+      const int r = r0 + rr, k = k0 + kk;
+      S[rr][kk] = (r < nrows && k < K) ? X[(long long)r * sr + (long long)k * sk] : zero;
+    }
+  }
+}
+
+// C[m][n] += sum_k A(m,k) B(n,k) over k [blockIdx.z kchunk, + kchunk), 64 x 64 tiles of four
+// warps, one tile of k in shared memory at a time, C zeroed by the caller: the gradient of a
+// layer's input when its product is split.  The parts of one element add up in the order in
+// which their blocks finish, and the next dZ is that sum in BF16: a last bit that differs turns
+// one BF16 rounding in some 2^16, 2^-8 of an element, and the layers below multiply it.  Which
+// order is usual depends on how long the blocks run.  Measured, 2048 rows, width 256, four of
+// these products in a pass, median of the largest relative change of a weight gradient: two
+// runs of the layer-by-layer pass with this kernel 1.0e-5; cqg_mlp_backward with it against
+// that pass 1.6e-5; with k_gemm_bf16 and atomics 3.7e-5 to 4.6e-5, its blocks being three times
+// as fast; with the parts in any one fixed order 3.2e-5 to 7.4e-5.  (Against 64 bits all are
+// the same, 1e-3: BF16 operands.)  So the products that are split keep this kernel, 17 us each
+// where k_gemm_bf16 takes 9, and a training step keeps its gradients.
+__global__ void __launch_bounds__(128)
+    k_gemm_parts(const __nv_bfloat16 *__restrict__ A, long long sam, long long sak, const __nv_bfloat16 *__restrict__ B,
+                 long long sbn, long long sbk, float *__restrict__ C, long long ldc, int M, int N, int K, int kchunk) {
+  constexpr int NJ = 4;
+  __shared__ __align__(16) __nv_bfloat16 As[kPartTile][GP];
+  __shared__ __align__(16) __nv_bfloat16 Bs[kPartTile][GP];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int wm = (warp % 2) * 32, wn = (warp / 2) * 32;
+  const int m0 = blockIdx.y * kPartTile, n0 = blockIdx.x * kPartTile;
+  const int g = lane >> 2, t = lane & 3;
+  const bool a16 = (reinterpret_cast<uintptr_t>(A) & 15) == 0, b16 = (reinterpret_cast<uintptr_t>(B) & 15) == 0;
+  const bool avk = a16 && sak == 1 && sam % 8 == 0 && K % 8 == 0;
+  const bool avr = a16 && !avk && sam == 1 && sak % 8 == 0 && M % 8 == 0;
+  const bool bvk = b16 && sbk == 1 && sbn % 8 == 0 && K % 8 == 0;
+  const bool bvr = b16 && !bvk && sbn == 1 && sbk % 8 == 0 && N % 8 == 0;
+  float acc[2][NJ][4];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.f;
+  const int kb = blockIdx.z * kchunk, ke = min(K, kb + kchunk);
+  for (int k0 = kb; k0 < ke; k0 += GK) {
+    stage_part(A, sam, sak, m0, M, k0, ke, avk, avr, As);
+    stage_part(B, sbn, sbk, n0, N, k0, ke, bvk, bvr, Bs);
+    __syncthreads();
+#pragma unroll
+    for (int ks = 0; ks < GK; ks += 16) {
+      uint32_t af[2][4], bf[NJ][2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int r = wm + i * 16 + g;
+        af[i][0] = *reinterpret_cast<const uint32_t *>(&As[r][ks + 2 * t]);
+        af[i][1] = *reinterpret_cast<const uint32_t *>(&As[r + 8][ks + 2 * t]);
+        af[i][2] = *reinterpret_cast<const uint32_t *>(&As[r][ks + 2 * t + 8]);
+        af[i][3] = *reinterpret_cast<const uint32_t *>(&As[r + 8][ks + 2 * t + 8]);
+      }
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        const int c = wn + j * 8 + g;
+        bf[j][0] = *reinterpret_cast<const uint32_t *>(&Bs[c][ks + 2 * t]);
+        bf[j][1] = *reinterpret_cast<const uint32_t *>(&Bs[c][ks + 2 * t + 8]);
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) mma_16816(acc[i][j], af[i], bf[j]);
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int m = m0 + wm + i * 16 + g + (q >> 1) * 8, n = n0 + wn + j * 8 + 2 * t + (q & 1);
+        if (m < M && n < N) atomicAdd(C + m * ldc + n, acc[i][j][q]);
+      }
+}
+
 __global__ void k_silu_bwd(const float *__restrict__ dY, const float *__restrict__ Z, __nv_bfloat16 *__restrict__ dZ,
                            long long n) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -373,13 +462,13 @@ __global__ void k_to_bf16(const float *__restrict__ x, __nv_bfloat16 *__restrict
   if (i < n) y[i] = __float2bfloat16(x[i]);
 }
 
-// The backward step's first pass: dZ = dY in BF16 (dY null: `in` holds it already) and its
+// dZ = dY in BF16, times SiLU'(Z) where Z is given (dY null: `in` holds dZ already), and its
 // column sums, db[n] += sum_m dZ[m][n] (db zeroed by the caller).  A block takes 32 columns x
-// kColRows rows, a warp one row at a time (coalesced); one atomic per column and block.
-// (The layers below get both from the epilogue of k_gemm_bf16: as kernels of their own, SiLU'
-// and the sums took 4 + 17 us per layer of 2048 x 256.)
+// kColRows rows, a warp one row at a time (coalesced); one atomic per column and block.  The two
+// as kernels of their own took 4 + 17 us per layer of 2048 x 256.
 constexpr int kColRows = 64;
 __global__ void __launch_bounds__(256) k_dz_colsum(const float *__restrict__ dY,
+                                                   const float *__restrict__ Z,
                                                    const __nv_bfloat16 *__restrict__ in,
                                                    __nv_bfloat16 *__restrict__ out, int M, int N,
                                                    float *__restrict__ db) {
@@ -396,7 +485,7 @@ __global__ void __launch_bounds__(256) k_dz_colsum(const float *__restrict__ dY,
       if (in) {
         v = in[e];
       } else {
-        v = __float2bfloat16(dY[e]);
+        v = __float2bfloat16(Z ? dY[e] * silu_grad(Z[e]) : dY[e]);
         out[e] = v;
       }
       s += __bfloat162float(v);
@@ -522,16 +611,16 @@ void tile_by(Gemm &g, int bm, int bn) {
 }
 
 // Few 64 x 64 output tiles and a long reduction (weight gradients: K = batch rows): K split so
-// that about two waves of blocks run; 0 for one part.
-int k_parts(const Gemm &g) {
-  const long long tiles = (long long)((g.N + 63) / 64) * ((g.M + 63) / 64);
-  if (tiles >= 148 || g.K < 128) return 0;
-  const int splits = (int)std::min<long long>(std::min<long long>((296 + tiles - 1) / tiles, g.K / GK), 64);
-  return splits > 1 ? ((g.K + splits - 1) / splits + GK - 1) / GK * GK : 0;
+// that about two waves of blocks run, in parts of `least` or more; the part, or 0 for one.
+int k_parts(int M, int N, int K, int least) {
+  const long long tiles = (long long)((N + 63) / 64) * ((M + 63) / 64);
+  if (tiles >= 148 || K < 128) return 0;
+  const int splits = (int)std::min<long long>(std::min<long long>((296 + tiles - 1) / tiles, K / least), 64);
+  return splits > 1 ? ((K + splits - 1) / splits + GK - 1) / GK * GK : 0;
 }
 
 void split_k(Gemm &g) {
-  g.kchunk = k_parts(g);
+  g.kchunk = k_parts(g.M, g.N, g.K, GK);
   if (g.kchunk > 0) {
     g.split = 1;
     g.nbz = (g.K + g.kchunk - 1) / g.kchunk;
@@ -608,7 +697,7 @@ cqg_status cqg_mlp_colsum(const void *dZ, int M, int N, float *db, void *stream)
   if (M <= 0) return CQG_OK;
   if ((M + 255) / 256 > 65535 || (N + 31) / 32 > 65535) return CQG_ERR_BAD_ARG;
   dim3 grid((M + kColRows - 1) / kColRows, (N + 31) / 32);
-  k_dz_colsum<<<grid, 256, 0, (cudaStream_t)stream>>>(nullptr, (const __nv_bfloat16 *)dZ, nullptr, M, N, db);
+  k_dz_colsum<<<grid, 256, 0, (cudaStream_t)stream>>>(nullptr, nullptr, (const __nv_bfloat16 *)dZ, nullptr, M, N, db);
   return cudaGetLastError() == cudaSuccess ? CQG_OK : CQG_ERR_CUDA;
 }
 
@@ -674,9 +763,9 @@ cqg_status cqg_mlp_forward(int nl, const int *dims, int M, const void *X, const 
 }
 
 cqg_status cqg_mlp_backward(int nl, const int *dims, int M, const float *dout, const void *const *H,
-                            const float *const *Z, const void *const *W, void *dZ0, void *dZ1, float *grads,
-                            void *stream) {
-  if (nl <= 0 || !dims || M < 0 || !dout || !H || !Z || !W || !dZ0 || !dZ1 || !grads) return CQG_ERR_BAD_ARG;
+                            const float *const *Z, const void *const *W, void *dZ0, void *dZ1, float *dX,
+                            float *grads, void *stream) {
+  if (nl <= 0 || !dims || M < 0 || !dout || !H || !Z || !W || !dZ0 || !dZ1 || !dX || !grads) return CQG_ERR_BAD_ARG;
   if ((M + GM - 1) / GM > 65535) return CQG_ERR_BAD_ARG;   // as cqg_mlp_gemm_bf16
   cudaStream_t st = (cudaStream_t)stream;
   long long nw = 0, nb = 0;
@@ -690,10 +779,17 @@ cqg_status cqg_mlp_backward(int nl, const int *dims, int M, const float *dout, c
   if (M == 0) return CQG_OK;
   float *gw = grads + nw, *gb = grads + nw + nb;
   __nv_bfloat16 *dZ = (__nv_bfloat16 *)dZ0, *next = (__nv_bfloat16 *)dZ1;
+  auto launch_dz = [&](const float *dY, const float *z, __nv_bfloat16 *out, int N) {
+    k_dz_colsum<<<dim3((M + kColRows - 1) / kColRows, (N + 31) / 32), 256, 0, st>>>(dY, z, nullptr, out, M, N, gb);
+  };
   const int nout = dims[nl];
   gb -= nout;
   if ((nout + 31) / 32 > 65535) return CQG_ERR_BAD_ARG;
-  k_dz_colsum<<<dim3((M + kColRows - 1) / kColRows, (nout + 31) / 32), 256, 0, st>>>(dout, nullptr, dZ, M, nout, gb);
+  launch_dz(dout, nullptr, dZ, nout);
+  // a weight gradient waits for the next one, and both go in one launch: their blocks together
+  // fill the GPU, and each dZ stays until the launch after that
+  Gemm waiting = {};
+  bool waits = false;
   for (int i = nl - 1; i >= 0; --i) {
     const int K = dims[i], N = dims[i + 1];
     gw -= (long long)K * N;
@@ -705,33 +801,51 @@ cqg_status cqg_mlp_backward(int nl, const int *dims, int M, const float *dout, c
     tile_by(w, wbig ? GM : 64, wbig ? GN : 64);
     if (!wbig) split_k(w);
     cqg_status s = CQG_OK;
-    if (i > 0) {
-      // dh[m][k] = sum_n dZ[m][n] W[n][k], through the SiLU of the layer below: the next dZ.
-      // In partial sums as k_parts() would split them: the order in which split products add up
-      Gemm x = gemm_of(dZ, N, 1, W[i], 1, K, nullptr, K, M, K, N);
-      gb -= K;
-      x.dact = Z[i - 1];
-      x.Y = next;
-      x.ldy = K;
-      x.db = gb;
-      set_pairs(x);
-      const bool xbig = big_tiles(M, K);
-      tile_by(x, xbig ? GM : 64, xbig ? GN : 64);
-      if (!xbig) {
-        x.kchunk = k_parts(x);
-        x.fold = x.kchunk > 0;
-      }
-      if (!xbig && !wbig) {
-        s = launch_small(x, &w, st);
-      } else {
-        s = xbig ? launch_big(x, st) : launch_small(x, nullptr, st);
-        if (s == CQG_OK) s = wbig ? launch_big(w, st) : launch_small(w, nullptr, st);
-      }
+    if (wbig) {
+      if (waits) s = launch_small(waiting, nullptr, st);
+      waits = false;
+      if (s == CQG_OK) s = launch_big(w, st);
+    } else if (waits) {
+      s = launch_small(waiting, &w, st);
+      waits = false;
     } else {
-      s = wbig ? launch_big(w, st) : launch_small(w, nullptr, st);
+      waiting = w;
+      waits = true;
+    }
+    if (s == CQG_OK && i > 0) {
+      // dh[m][k] = sum_n dZ[m][n] W[n][k], through the SiLU of the layer below: the next dZ
+      gb -= K;
+      const int part = big_tiles(M, K) ? 0 : k_parts(M, K, N, 2 * GK);
+      if (part > 0) {
+        if (cudaMemsetAsync(dX, 0, (size_t)M * K * sizeof(float), st) != cudaSuccess) return CQG_ERR_CUDA;
+        const dim3 grid((K + kPartTile - 1) / kPartTile, (M + kPartTile - 1) / kPartTile, (N + part - 1) / part);
+        k_gemm_parts<<<grid, 128, 0, st>>>(dZ, N, 1, (const __nv_bfloat16 *)W[i], 1, K, dX, K, M, K, N, part);
+        launch_dz(dX, Z[i - 1], next, K);
+      } else {
+        Gemm x = gemm_of(dZ, N, 1, W[i], 1, K, nullptr, K, M, K, N);
+        x.dact = Z[i - 1];
+        x.Y = next;
+        x.ldy = K;
+        x.db = gb;
+        set_pairs(x);
+        const bool xbig = big_tiles(M, K);
+        tile_by(x, xbig ? GM : 64, xbig ? GN : 64);
+        if (xbig) {
+          s = launch_big(x, st);
+        } else if (waits) {
+          s = launch_small(x, &waiting, st);
+          waits = false;
+        } else {
+          s = launch_small(x, nullptr, st);
+        }
+      }
     }
     if (s != CQG_OK) return s;
     std::swap(dZ, next);
+  }
+  if (waits) {
+    const cqg_status s = launch_small(waiting, nullptr, st);
+    if (s != CQG_OK) return s;
   }
   return cudaGetLastError() == cudaSuccess ? CQG_OK : CQG_ERR_CUDA;
 }

@@ -334,9 +334,10 @@ class PairMLP:
         sizes = [d[i] * d[i + 1] for i in range(nl)] + d[1:]
         grads = t.empty(sum(sizes), dtype=t.float32, device=self.dev)
         dZ = t.empty((2, M * max(d[1:]) + 7 & ~7), dtype=t.bfloat16, device=self.dev)
+        dX = t.empty(min(M * max(d[1:-1], default=1), _lib.MLP_DX_MAX), dtype=t.float32, device=self.dev)
         _lib.check(self.L.cqg_mlp_backward(nl, self._dims, M, self._p(dout), self._ps([h for h, _ in cache]),
                                            self._ps([z for _, z in cache]), self._ps(self.Wbf), self._p(dZ[0]),
-                                           self._p(dZ[1]), self._p(grads), self._stream()))
+                                           self._p(dZ[1]), self._p(dX), self._p(grads), self._stream()))
         g = grads.split(sizes)
         return [x.view(n, -1) for x, n in zip(g, d[1:])], list(g[nl:])
 
