@@ -292,25 +292,34 @@ static cqg_status upload_pairs(cqg_ctx *ctx, double thresh, const std::vector<in
   return CQG_OK;
 }
 
-// Expansion tables of the current primitive pairs, for the tensor-core classes.  They need a
-// d or f shell: without one no class uses them and none are built.
+// Expansion tables of the current primitive pairs, of every pair class that some quartet class
+// of the basis takes to the tensor-core kernel: those of d and f shells, and without any the
+// p-p pairs, for the tensor form of (pp|pp).  launch_tc refuses a class without its tables.
 static cqg_status build_expansions(cqg_ctx *ctx) {
-  if (ctx->maxl < 2) return CQG_OK;
   static const int size[CQG_NPC] = {
       warpmd::ExpansionDims<0, 0>::SIZE, warpmd::ExpansionDims<1, 0>::SIZE, warpmd::ExpansionDims<1, 1>::SIZE,
       warpmd::ExpansionDims<2, 0>::SIZE, warpmd::ExpansionDims<2, 1>::SIZE, warpmd::ExpansionDims<2, 2>::SIZE,
       warpmd::ExpansionDims<3, 0>::SIZE, warpmd::ExpansionDims<3, 1>::SIZE, warpmd::ExpansionDims<3, 2>::SIZE,
       warpmd::ExpansionDims<3, 3>::SIZE};
+  bool wanted[CQG_NPC] = {false};
+  for (int k = 0; k < CQG_NQC; ++k) {
+    int i, j;
+    qclass_split(k, i, j);
+    const int la = kPairClass[i][0], lb = kPairClass[i][1], lc = kPairClass[j][0], ld = kPairClass[j][1];
+    if (ctx->pc_beg[i + 1] == ctx->pc_beg[i] || ctx->pc_beg[j + 1] == ctx->pc_beg[j]) continue;
+    if (is_warp_class(la, lb, lc, ld) || is_variant_class(la, lb, lc, ld)) wanted[i] = wanted[j] = true;
+  }
   size_t total = 0;
   for (int c = 0; c < CQG_NPC; ++c) {
     ctx->exp_off[c] = total;
-    total += (size_t)(ctx->pc_prim[c + 1] - ctx->pc_prim[c]) * size[c];
+    if (wanted[c]) total += (size_t)(ctx->pc_prim[c + 1] - ctx->pc_prim[c]) * size[c];
     ctx->exp_prim0[c] = ctx->pc_prim[c];
   }
   if (ctx->d_exp.reserve(std::max<size_t>(total, 1)) != cudaSuccess) {
     ctx->err = "device allocation for the expansion tables failed";
     return CQG_ERR_OOM;
   }
+  std::copy(wanted, wanted + CQG_NPC, ctx->exp_have);
   CUCHK((launch_expansions<0, 0>(ctx)));
   CUCHK((launch_expansions<1, 0>(ctx)));
   CUCHK((launch_expansions<1, 1>(ctx)));
@@ -980,6 +989,7 @@ cqg_status cqg_set_basis_batch(cqg_ctx *ctx, int nmol, const int *nshell_per_mol
   ctx->nmol = nmol;
   ctx->nshell = nshell;
   ctx->maxl = maxl;
+  std::fill(ctx->exp_have, ctx->exp_have + CQG_NPC, false);   // the tables are the old basis's
   ctx->hL.assign(L, L + nshell);
   ctx->hnprim.assign(nprim, nprim + nshell);
   ctx->halpha.assign(alpha, alpha + tot);

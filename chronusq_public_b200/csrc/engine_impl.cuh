@@ -1639,6 +1639,7 @@ struct cqg_ctx {
   DevBuf<double> d_exp;
   size_t exp_off[CQG_NPC] = {0};
   int exp_prim0[CQG_NPC] = {0};
+  bool exp_have[CQG_NPC] = {false};   // the class's tables are those of the current basis
   int pc_prim[CQG_NPC + 1] = {0};   // first primitive pair of each pair class
   int pc_np_max[CQG_NPC] = {0};   // most primitive pairs of a pair, per class
   // per-call scratch
@@ -1736,6 +1737,7 @@ static cudaError_t launch_tc(cqg_ctx *ctx, int blk, long long n, cudaStream_t st
   const long long cap = (long long)ctx->nsm * cta;
   const int blocks = (int)(n > 0 ? std::min<long long>((n + wpb - 1) / wpb, cap) : cap);
   const int bc = pair_class_c(LA, LB), kc = pair_class_c(LC, LD);
+  if (!ctx->exp_have[bc] || !ctx->exp_have[kc]) return cudaErrorInvalidValue;   // no tables to read
   const Expansions X = {ctx->d_exp.p + ctx->exp_off[bc], ctx->d_exp.p + ctx->exp_off[kc], ctx->exp_prim0[bc],
                         ctx->exp_prim0[kc]};
   const int take = std::min(32, ctx->shape_qpw[blk]);
@@ -1772,7 +1774,7 @@ template <int LA, int LB>
 static cudaError_t launch_expansions(cqg_ctx *ctx) {
   constexpr int c = pair_class_c(LA, LB);
   const int beg = ctx->pc_beg[c], n = ctx->pc_beg[c + 1] - beg;
-  if (n <= 0) return cudaSuccess;
+  if (n <= 0 || !ctx->exp_have[c]) return cudaSuccess;
   k_expansions<LA, LB><<<std::min((n + 3) / 4, ctx->nsm * 16), 128>>>(
       make_pairs(ctx), make_shells(ctx), beg, beg + n, ctx->exp_prim0[c], ctx->d_exp.p + ctx->exp_off[c]);
   return cudaGetLastError();
