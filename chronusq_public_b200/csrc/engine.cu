@@ -1324,8 +1324,11 @@ static bool class_fused(int tier, int vb) {
 }
 
 // Launch-shape autotuner: for every (precision, class) list with work, time each candidate
-// shape (persistent CTAs per SM; warps per CTA for the warp-cooperative classes) with the
-// digest pointed at scratch accumulators, and keep the fastest.
+// shape (persistent CTAs per SM; warps per CTA for the tensor-core classes; entries claimed at
+// a time; kernel form) with the digest pointed at scratch accumulators, and keep the fastest.  The
+// defaults come first, the resident grid and the claim that follows the list's length, and stay
+// unless another is kKeep faster: two runs of one shape differ by that much.
+constexpr float kKeep = 0.98f;
 static cqg_status autotune_shapes(cqg_ctx *ctx, const long long *crange, cudaStream_t st, const DigestGroups &dg) {
   DigestGroups scratch = dg;
   const CallScratch cs(ctx);
@@ -1351,24 +1354,30 @@ static cqg_status autotune_shapes(cqg_ctx *ctx, const long long *crange, cudaStr
     struct Shape {
       int cta, wpb, qpw, var;
     };
-    // (CTAs per SM, warps per CTA, quartets claimed per warp, kernel form)
-    std::vector<Shape> cand;
+    // (CTAs per SM, warps per CTA, quartets claimed per warp, kernel form); 0: the default
+    const int form = both && is_tensor_first(la, lb, lc, ld) && vb < CQG_NQC ? 1 : 0;
+    std::vector<Shape> cand = {{0, 0, 0, form}};
     if (sibling) {   // sibling lists: also CTAs of 64 threads (2 warps)
       for (int w : {2, 4})
         for (int c : {4, 8, 16})
           for (int q : {1, 4}) cand.push_back({c, w, q, 0});
     } else if (!warp) {
+      if (form) cand.push_back({0, 0, 0, 0});
+      cand.push_back({0, 0, 4, 0});
       for (int c : {4, 8, 12, 16, 24})
         for (int q : {1, 4}) cand.push_back({c, 0, q, 0});
     }
     if (warp || both) {
+      const int v = warp ? 0 : 1;
+      if (both && !form) cand.push_back({0, 0, 0, 1});
+      for (int q : {1, 2, 4, 8}) cand.push_back({0, 0, q, v});
       for (int w : {1, 2, 4})
         for (int c : {8, 16, 32})
-          for (int q : {1, 4}) cand.push_back({c, w, q, warp ? 0 : 1});
+          for (int q : {1, 4}) cand.push_back({c, w, q, v});
     }
     // Long lists are timed on their first quarter (at least 2^20 quartets), after one
     // untimed run, one run per candidate; short lists in full, best of two runs.  The
-    // kernels read their range from d_range, so the sample range is written there and the
+    // kernels read their range from p_range, so the sample range is written there and the
     // full range put back afterwards.
     const long long m = n > (1ll << 20) ? std::max<long long>(1ll << 20, n / 4) : n;
     const int reps = m < n ? 1 : 2;
@@ -1376,7 +1385,7 @@ static cqg_status autotune_shapes(cqg_ctx *ctx, const long long *crange, cudaStr
       const long long sub[2] = {crange[2 * vb], crange[2 * vb] + m};
       CUCHK(cudaMemcpyAsync(ctx->p_range + 2 * vb, sub, sizeof(sub), cudaMemcpyHostToDevice, st));
     }
-    float best = 1e30f;
+    float best = 1e30f, tdefault = 1e30f;
     Shape pick = cand[0];
     for (int ci = (m < n ? -1 : 0); ci < (int)cand.size(); ++ci) {
       const Shape cw = cand[ci < 0 ? 0 : ci];
@@ -1385,7 +1394,9 @@ static cqg_status autotune_shapes(cqg_ctx *ctx, const long long *crange, cudaStr
       ctx->shape_qpw[vb] = cw.qpw;
       ctx->shape_var[vb] = cw.var;
       float tbest = 1e30f;
-      for (int rep = 0; rep < (ci < 0 ? 1 : reps); ++rep) {
+      // one more run, untimed, where a kernel's first launch would be the only one timed
+      const int lead = m < n && ci > 0 && cw.var != cand[ci - 1].var ? 1 : 0;
+      for (int rep = -lead; rep < (ci < 0 ? 1 : reps); ++rep) {
         CUCHK(cudaMemsetAsync(ctx->p_qhead + vb, 0, sizeof(unsigned long long), st));
         cudaEventRecord(e0, st);
         cudaError_t e = list_launcher(vb)(ctx, vb, m, st, scratch);
@@ -1399,11 +1410,13 @@ static cqg_status autotune_shapes(cqg_ctx *ctx, const long long *crange, cudaStr
         cudaEventSynchronize(e1);
         float ms = 0.f;
         cudaEventElapsedTime(&ms, e0, e1);
-        tbest = std::min(tbest, ms);
+        if (rep >= 0) tbest = std::min(tbest, ms);
       }
-      if (ci >= 0 && tbest < best) {
+      if (ci == 0 || (ci > 0 && tbest < best && tbest < kKeep * tdefault)) {
+        if (ci == 0) tdefault = tbest;
         best = tbest;
         pick = cw;
+        if (pick.cta == 0) pick.cta = ctx->used_cta;   // the grid that was timed
       }
     }
     if (m < n) CUCHK(cudaMemcpyAsync(ctx->p_range + 2 * vb, crange + 2 * vb, 2 * sizeof(long long),
@@ -1413,9 +1426,9 @@ static cqg_status autotune_shapes(cqg_ctx *ctx, const long long *crange, cudaStr
     ctx->shape_qpw[vb] = pick.qpw;
     ctx->shape_var[vb] = pick.var;
   }
-  // Class fusion: the lists of the tier-2 classes (every per-thread class up to (dd|dd)) as
-  // one launch per list with the shapes just tuned, as the tier-1 fused kernel plus per-list
-  // launches of the rest, and as the tier-2 fused kernel; full lists, each timed after one
+  // Class fusion: all lists as a build launches them (side streams, most work first), one launch
+  // per list with the shapes just tuned, with the tier-1 fused kernel in place of its lists, and
+  // with the tier-2 one (every per-thread class up to (dd|dd)); full lists, each timed after one
   // untimed run; the fastest is kept.
   bool any = false;
   for (int vb = 0; vb < CQG_NLIST; ++vb)
@@ -1424,16 +1437,23 @@ static cqg_status autotune_shapes(cqg_ctx *ctx, const long long *crange, cudaStr
     float best = 1e30f;
     int pick = 0;
     for (int tier = 0; tier <= 2; ++tier) {
+      std::vector<int> lists;
+      for (int o = 0; o < CQG_NQC; ++o)
+        for (int part = 0; part < kListParts; ++part) {
+          const int vb = part * CQG_NQC + ctx->class_order[o];
+          if (crange[2 * vb + 1] > crange[2 * vb] && !class_fused(tier, vb) && list_launcher(vb)) lists.push_back(vb);
+        }
       float t = 1e30f;
       for (int rep = 0; rep < 2; ++rep) {
         CUCHK(cudaMemsetAsync(ctx->p_qhead, 0, CQG_NLIST * sizeof(unsigned long long), st));
         cudaEventRecord(e0, st);
         cudaError_t e = tier ? cqg_launch_fused(ctx, tier, st, scratch) : cudaSuccess;
-        for (int vb = 0; vb < CQG_NLIST && e == cudaSuccess; ++vb) {
-          const long long n = crange[2 * vb + 1] - crange[2 * vb];
-          if (n <= 0 || !class_fused(2, vb) || class_fused(tier, vb)) continue;
-          e = list_launcher(vb)(ctx, vb, n, st, scratch);
-        }
+        ClassStreams side(ctx, st, (int)lists.size(), true);
+        if (e == cudaSuccess) e = side.fork();
+        for (size_t q = 0; q < lists.size() && e == cudaSuccess; ++q)
+          e = list_launcher(lists[q])(ctx, lists[q], crange[2 * lists[q] + 1] - crange[2 * lists[q]], side.next(), scratch);
+        const cudaError_t j = side.join();
+        if (e == cudaSuccess) e = j;
         cudaEventRecord(e1, st);
         if (e != cudaSuccess) {
           cudaEventDestroy(e0);

@@ -1584,6 +1584,7 @@ struct cqg_ctx {
   // 0: one launch per class list; 1 or 2: the lists of that tier's classes go through one
   // class-fused persistent kernel (eri_fused.cu); set by the autotuner or cqg_set_fusion
   int fused_tier = 0;
+  int used_cta = 0;   // CTAs per SM of the last class launch (the autotuner's record of a default)
   double fusion_ms[3] = {0.0, 0.0, 0.0};   // autotuner's times of the three forms (ms)
   // Per-call state, one buffer: zeroed by one memset, and read back by one copy up to `range`.
   DevBuf<unsigned long long> d_state;
@@ -1734,6 +1735,7 @@ static cudaError_t launch_tc(cqg_ctx *ctx, int blk, long long n, cudaStream_t st
   const int wpb = ctx->shape_wpb[blk] > 0 ? std::min(wpb_max, ctx->shape_wpb[blk]) : wpb_max;
   const int cta = ctx->shape_cta[blk] > 0 ? ctx->shape_cta[blk]
                                           : std::max(1, (int)(220u * 1024u / (per_warp * wpb + 1024)));
+  ctx->used_cta = cta;
   const long long cap = (long long)ctx->nsm * cta;
   const int blocks = (int)(n > 0 ? std::min<long long>((n + wpb - 1) / wpb, cap) : cap);
   const int bc = pair_class_c(LA, LB), kc = pair_class_c(LC, LD);
@@ -1862,6 +1864,7 @@ static cudaError_t launch_gc(cqg_ctx *ctx, int blk, long long n, cudaStream_t st
   if (n == 0) return cudaSuccess;   // n < 0: count unknown on the host (graph mode)
   const int nt = ctx->shape_wpb[blk] == 2 ? 64 : kEriThreads;
   const int cta = ctx->shape_cta[blk] > 0 ? ctx->shape_cta[blk] : 4;
+  ctx->used_cta = cta;
   const long long cap = (long long)ctx->nsm * cta;
   const long long nb = n > 0 ? std::min<long long>((n + nt - 1) / nt, cap) : cap;
   const int chunk = 32 * (ctx->shape_qpw[blk] > 0 ? ctx->shape_qpw[blk] : 1);
@@ -1900,6 +1903,7 @@ static cudaError_t launch_eri(cqg_ctx *ctx, int blk, long long n, cudaStream_t s
     const int resident = resident_ctas(kernel, kEriThreads, ctx->device, known);
     const LaneShare share = {ctx->nsm * resident * kEriThreads, ctx->pc_np_max[pair_class_c(LC, LD)]};
     const int cta = ctx->shape_cta[blk] > 0 ? ctx->shape_cta[blk] : resident;
+    ctx->used_cta = cta;
     const long long cap = (long long)ctx->nsm * cta;
     // up to 32 lanes per quartet (eri_jk_list)
     const long long nb = n > 0 ? std::min<long long>((32 * n + kEriThreads - 1) / kEriThreads, cap) : cap;
