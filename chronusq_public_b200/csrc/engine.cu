@@ -117,6 +117,23 @@ void cqg_pool_free(void *p, size_t bytes, int device) {
   for (auto &b : out) cudaFree(b.p);
 }
 
+// b.reserve(m) that keeps an outgrown buffer while graph mode is on (cqg_ctx::retired)
+template <typename T>
+static cudaError_t grow(cqg_ctx *ctx, DevBuf<T> &b, size_t m) {
+  if (m > b.n && b.p && ctx->graph_capacity > 0) {
+    ctx->retired.push_back({b.p, b.bytes, b.device});
+    b.p = nullptr;
+    b.n = b.bytes = 0;
+  }
+  return b.reserve(m);
+}
+static void release_retired(cqg_ctx *ctx) {
+  if (ctx->retired.empty()) return;
+  cudaDeviceSynchronize();
+  for (auto &r : ctx->retired) cqg_pool_free(r.p, r.bytes, r.device);
+  ctx->retired.clear();
+}
+
 static const char *kLetters = "spdfg";
 static char g_class_names[55][16];
 static bool g_names_init = false;
@@ -892,6 +909,7 @@ cqg_status cqg_destroy(cqg_ctx *ctx) {
   if (!ctx) return CQG_OK;
   cudaSetDevice(ctx->device);
   cudaDeviceSynchronize();   // the buffers go back to the pool
+  release_retired(ctx);
   ctx->d_center.release(); ctx->d_bf.release(); ctx->d_sz.release();
   ctx->d_pair_sh.release(); ctx->d_pair_Q.release(); ctx->d_pair_poff.release(); ctx->d_pair_np.release();
   ctx->d_pair_kk.release();
@@ -986,6 +1004,7 @@ cqg_status cqg_set_basis_batch(cqg_ctx *ctx, int nmol, const int *nshell_per_mol
     tot += nprim[s];
     maxl = std::max(maxl, L[s]);
   }
+  release_retired(ctx);
   ctx->nmol = nmol;
   ctx->nshell = nshell;
   ctx->maxl = maxl;
@@ -1554,8 +1573,8 @@ static cqg_status contract_device(cqg_ctx *ctx, int ngroups, const double *const
                                   int ldx, int ldax, cudaStream_t st) {
   const Mols mols = make_mols(ctx);
   const CallScratch scratch(ctx);
-  if (ctx->d_G.reserve((size_t)ngroups * scratch.group()) != cudaSuccess ||
-      ctx->d_XP.reserve(scratch.inputs(nx_all, ngroups)) != cudaSuccess) {
+  if (grow(ctx, ctx->d_G, (size_t)ngroups * scratch.group()) != cudaSuccess ||
+      grow(ctx, ctx->d_XP, scratch.inputs(nx_all, ngroups)) != cudaSuccess) {
     ctx->err = "accumulator allocation failed";
     return CQG_ERR_OOM;
   }
@@ -1653,8 +1672,8 @@ static cqg_status contract_device(cqg_ctx *ctx, int ngroups, const double *const
       cap = std::max(cap, hoff[v1 - 1] + hcnt[v1 - 1] - hoff[v0]);
     }
   }
-  if (ctx->d_qlist.reserve((size_t)std::max<long long>(cap, 1)) != cudaSuccess ||
-      ctx->d_qmask.reserve((size_t)std::max<long long>(cap, 1)) != cudaSuccess) {
+  if (grow(ctx, ctx->d_qlist, (size_t)std::max<long long>(cap, 1)) != cudaSuccess ||
+      grow(ctx, ctx->d_qmask, (size_t)std::max<long long>(cap, 1)) != cudaSuccess) {
     ctx->err = "quartet list allocation failed";
     return CQG_ERR_OOM;
   }
@@ -2112,6 +2131,8 @@ cqg_status cqg_set_graph_mode(cqg_ctx *ctx, long long capacity, int max_groups) 
       return CQG_ERR_OOM;
     }
     lease_side_streams(ctx);   // ahead of any capture
+  } else {
+    release_retired(ctx);
   }
   return CQG_OK;
 }

@@ -1671,6 +1671,14 @@ struct cqg_ctx {
   DevBuf<uint2> d_masks;
   DevBuf<long long> d_mslot;
   long long mask_steps_used = 0;      // steps the last count pass asked for
+  // buffers that a contraction outgrew while graph mode was on: captured launches hold their
+  // addresses, so they stay the context's own until graph mode or the basis ends
+  struct Retired {
+    void *p;
+    size_t bytes;
+    int device;
+  };
+  std::vector<Retired> retired;
   SideStreams *side = nullptr;   // leased on first use (ClassStreams in engine.cu)
   // classes, most work first, as the last uncaptured contraction counted it (a captured one
   // launches in this order)

@@ -186,7 +186,10 @@ cqg_status cqg_one_e_batch(cqg_ctx *ctx, const int *ncharge_per_mol, const doubl
  * quartets and up to `max_groups` distinct (X, AX) pairs are allowed per call; after a
  * replay, cqg_graph_status reports the screened quartet count and whether the capacity
  * overflowed (the result is then incomplete and must be recomputed with a larger
- * capacity) or the input was non-finite / asymmetric.  capacity = 0 restores the default.
+ * capacity) or the input was non-finite / asymmetric.  capacity = 0 restores the default and
+ * ends the captured graphs: later calls may replace the buffers whose addresses they hold (as
+ * may a larger capacity or a new basis).  While graph mode is on, host-pointer contractions
+ * keep the buffers that they outgrow, so graphs captured before stay valid.
  * Per-class statistics are not collected in graph mode. */
 cqg_status cqg_set_graph_mode(cqg_ctx *ctx, long long capacity, int max_groups);
 cqg_status cqg_graph_status(cqg_ctx *ctx, long long *quartets, int *overflow, int *nonfinite,
