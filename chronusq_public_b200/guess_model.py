@@ -318,9 +318,13 @@ class PairMLP:
         layer, its BF16 input and FP32 pre-activation for the backward pass."""
         t = self.torch
         M, nl = Xbf.shape[0], len(self.W)
-        # the hidden layers, all of one width, in one allocation per type
-        Z = list(t.empty((nl - 1, M, self.dims[1]), dtype=t.float32, device=self.dev).unbind())
-        Y = list(t.empty((nl - 1, M, self.dims[1]), dtype=t.bfloat16, device=self.dev).unbind())
+        # the hidden layers, all of one width, in one allocation per type; without a backward
+        # pass one Z, which nothing reads, and two Y in turn serve them all
+        nh = nl - 1
+        nz, ny = (nh, nh) if keep else (min(nh, 1), min(nh, 2))
+        Z = t.empty((nz, M, self.dims[1]), dtype=t.float32, device=self.dev).unbind()
+        Y = t.empty((ny, M, self.dims[1]), dtype=t.bfloat16, device=self.dev).unbind()
+        Z, Y = [Z[i % nz] for i in range(nh)], [Y[i % ny] for i in range(nh)]
         Z.append(t.empty((M, self.dims[-1]), dtype=t.float32, device=self.dev))
         _lib.check(self.L.cqg_mlp_forward(nl, self._dims, M, self._p(Xbf), self._ps(self.Wbf), self._ps(self.b),
                                           self._ps(Z), self._ps(Y + [None]), self._stream()))
