@@ -1896,7 +1896,7 @@ cudaError_t cqg_launch_fused(cqg_ctx *ctx, int tier, cudaStream_t st, const Dige
 template <int LA, int LB, int LC, int LD, typename T>
 static cudaError_t launch_eri(cqg_ctx *ctx, int blk, long long n, cudaStream_t st, const DigestGroups &dg) {
   if (n == 0) return cudaSuccess;   // n < 0: count unknown on the host (graph mode)
-  if constexpr (is_warp_class(LA, LB, LC, LD)) {
+  if constexpr (is_warp_class(LA, LB, LC, LD)) {   // FP32 lists too: the tensor form is FP64 throughout
     return launch_tc<LA, LB, LC, LD>(ctx, blk, n, st, dg);
   } else {
     if constexpr (is_variant_class(LA, LB, LC, LD)) {

@@ -43,8 +43,9 @@ enum { CQG_COULOMB = 0, CQG_EXCHANGE = 1 };
 enum {
   CQG_PREC_FP64 = 0,         /* every quartet in FP64 (the reference's arithmetic) */
   CQG_PREC_MIXED = 1         /* quartets whose density-weighted Schwarz bound (the screen's
-                                max block norm * Q_ab * Q_cd) is below the FP32 cutoff are
-                                evaluated in FP32, accumulated in FP64 */
+                                max block norm * Q_ab * Q_cd) is below the FP32 cutoff go to
+                                FP32 lists: the per-thread classes evaluate those in FP32 and
+                                accumulate in FP64, the tensor-core classes stay in FP64 */
 };
 
 typedef struct cqg_ctx cqg_ctx;
@@ -52,10 +53,10 @@ typedef struct cqg_ctx cqg_ctx;
 /* statistics of the last contraction on a context */
 typedef struct {
   long long quartets;              /* screened unique shell quartets (the unit of work) */
-  long long quartets_fp32;         /* of which evaluated in FP32 (mixed policy) */
+  long long quartets_fp32;         /* of which in FP32 lists (mixed policy) */
   long long prim_quartets;         /* primitive quartets evaluated */
   double model_flops;              /* MD-v1 model FLOPs of the screened quartets */
-  double model_flops_fp32;         /* of which in FP32 quartets */
+  double model_flops_fp32;         /* of which in FP32 lists */
   double ms_screen;                /* device time of screening + list build (ms) */
   double ms_eri;                   /* device time of ERI + digest kernels (ms) */
   double ms_total;                 /* device time of the whole call (ms) */
