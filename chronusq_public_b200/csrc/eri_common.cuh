@@ -245,7 +245,7 @@ template <int L>
 __device__ __forceinline__ ClassArg class_arg(double s, double m, double R2) {
   ClassArg c;
   const double z = m * R2;
-  c.far = z >= boys_tmax(L) * s;
+  c.far = !(z < boys_tmax(L) * s);   // also where z or s is not a number: its row is in the table
   c.y = class_rsqrt(c.far ? z : s);
   c.T = c.far ? boys_tfar(L) : z * (c.y * c.y);
   return c;
