@@ -747,15 +747,20 @@ static cqg_status launch_finalize(cqg_ctx *ctx, const DigestGroups &dg, double *
 // side streams.  Everything a launch reads was written on the caller's stream before the
 // fork, and later work on that stream comes after the join, so the buffers' lifetimes are
 // those of a single-stream call; under capture the fork and join become graph edges.
-// With one launch, or per-class timing on, the caller's stream takes them all.
+// With one launch, or per-class timing on, the caller's stream takes them all; so it does in a
+// capture on a context without a set, since one cannot be made there.
 struct ClassStreams {
   cqg_ctx *ctx;
   cudaStream_t st;
   int n;          // side streams in use
   int at = 0;
   ClassStreams(cqg_ctx *c, cudaStream_t s, int launches, bool may_lease) : ctx(c), st(s), n(0) {
-    if (launches > 1 && !c->timing && (c->side || (may_lease && lease_side_streams(c))))
+    if (launches > 1 && !c->timing && (c->side || (may_lease && !capturing(s) && lease_side_streams(c))))
       n = std::min(launches - 1, kSideStreams);
+  }
+  static bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(s, &status) == cudaSuccess && status != cudaStreamCaptureStatusNone;
   }
   cudaError_t fork() {
     if (n == 0) return cudaSuccess;
