@@ -38,7 +38,7 @@ EXPORTED = [
     "cqg_one_e_noalloc", "cqg_dipole", "cqg_get_schedule", "cqg_set_schedule",
     "cqg_set_fusion", "cqg_get_fusion", "cqg_mlp_adam_dev", "cqg_set_siblings", "cqg_get_siblings",
     "cqg_schedule_lists", "cqg_list_class", "cqg_set_sibling_min", "cqg_mlp_forward", "cqg_mlp_backward",
-    "cqg_mlp_adam_tensors",
+    "cqg_mlp_adam_tensors", "cqg_release_memory",
 ]
 
 
@@ -123,6 +123,7 @@ def load(path: str = LIB_PATH):
     L.cqg_mlp_backward.argtypes = [ctypes.c_int, i, ctypes.c_int, vp, pv, pv, pv, vp, vp, vp, vp, vp]
     L.cqg_mlp_adam_tensors.argtypes = [ctypes.c_int, pv, pv, pv, pv, ctypes.POINTER(ll), ctypes.POINTER(f), pv, vp, f,
                                        f, f, f, ctypes.c_int, vp]
+    L.cqg_release_memory.argtypes = [ctypes.c_int, ctypes.POINTER(ll)]
     L.cqg_class_name.argtypes = [ctypes.c_int]
     L.cqg_class_name.restype = ctypes.c_char_p
     L.cqg_probe_fma_peak.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_double, d]
@@ -138,7 +139,7 @@ def load(path: str = LIB_PATH):
                  "cqg_mlp_gemm_bf16", "cqg_mlp_silu_bwd", "cqg_mlp_to_bf16", "cqg_mlp_colsum", "cqg_mlp_mse",
                  "cqg_mlp_adam", "cqg_one_e_noalloc", "cqg_dipole", "cqg_get_schedule", "cqg_set_schedule", "cqg_set_fusion", "cqg_get_fusion", "cqg_mlp_adam_dev",
                  "cqg_set_siblings", "cqg_get_siblings", "cqg_schedule_lists", "cqg_list_class",
-                 "cqg_set_sibling_min", "cqg_mlp_forward", "cqg_mlp_backward", "cqg_mlp_adam_tensors"]:
+                 "cqg_set_sibling_min", "cqg_mlp_forward", "cqg_mlp_backward", "cqg_mlp_adam_tensors", "cqg_release_memory"]:
         getattr(L, name).restype = ctypes.c_int
     _lib = L
     return L
@@ -168,6 +169,14 @@ def schedule_lists():
         k = int(L.cqg_list_class(b))
         out.append(names[k] + (" siblings" if b >= n // 2 else ""))
     return out
+
+
+def release_memory(device: int = 0) -> int:
+    """Give the device memory that closed contexts left for later ones back to the driver
+    (at most 256 MiB are kept); returns the bytes."""
+    n = ctypes.c_longlong()
+    check(lib().cqg_release_memory(int(device), ctypes.byref(n)))
+    return int(n.value)
 
 
 def class_names():

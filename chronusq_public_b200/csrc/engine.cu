@@ -30,7 +30,8 @@
 // takes 2.1 ms instead of 13.4.)  Blocks above kPoolLargest are not kept, and at most kPoolKeep
 // bytes are per process and device: a freed block takes the place of those that have lain there
 // longest (with new blocks turned away instead, a pool filled by earlier, larger contexts made
-// the same set-up 4.5 ms).  A request that the device cannot meet gives all of them back first.
+// the same set-up 4.5 ms).  A request that the device cannot meet gives all of them back first,
+// and cqg_release_memory gives them back at any time.
 namespace {
 constexpr size_t kPoolLargest = 64u << 20, kPoolKeep = 256u << 20;
 struct DevicePool {
@@ -54,6 +55,19 @@ size_t pool_size(size_t bytes) {
   const size_t step = p / 16;   // an eighth of the power of two below
   return (bytes + step - 1) / step * step;
 }
+// Bytes given back.
+size_t empty_pool(DevicePool &pool) {
+  std::list<DevicePool::Block> out;
+  size_t bytes = 0;
+  {
+    std::lock_guard<std::mutex> lock(pool.mutex);
+    out.swap(pool.blocks);
+    pool.by_size.clear();
+    std::swap(bytes, pool.kept);
+  }
+  for (auto &b : out) cudaFree(b.p);
+  return bytes;
+}
 }  // namespace
 
 cudaError_t cqg_pool_alloc(void **p, size_t *bytes, int *device) {
@@ -76,13 +90,7 @@ cudaError_t cqg_pool_alloc(void **p, size_t *bytes, int *device) {
   e = cudaMalloc(p, size);
   if (e == cudaErrorMemoryAllocation) {   // give the kept blocks back and try once more
     cudaGetLastError();
-    {
-      std::lock_guard<std::mutex> lock(pool.mutex);
-      for (auto &b : pool.blocks) cudaFree(b.p);
-      pool.blocks.clear();
-      pool.by_size.clear();
-      pool.kept = 0;
-    }
+    empty_pool(pool);
     e = cudaMalloc(p, size);
   }
   if (e != cudaSuccess) {
@@ -908,6 +916,16 @@ cqg_status cqg_create(cqg_ctx **out, int device) {
   cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, device);
   *out = ctx;
   return CQG_OK;
+}
+
+cqg_status cqg_release_memory(int device, long long *bytes) {
+  int n = 0, old = 0;
+  if (cudaGetDeviceCount(&n) != cudaSuccess || cudaGetDevice(&old) != cudaSuccess) return CQG_ERR_CUDA;
+  if (device < 0 || device >= n) return CQG_ERR_BAD_ARG;
+  if (cudaSetDevice(device) != cudaSuccess) return CQG_ERR_CUDA;
+  const size_t freed = device < 64 ? empty_pool(device_pool(device)) : 0;
+  if (bytes) *bytes = (long long)freed;
+  return cudaSetDevice(old) == cudaSuccess ? CQG_OK : CQG_ERR_CUDA;
 }
 
 cqg_status cqg_destroy(cqg_ctx *ctx) {

@@ -76,6 +76,10 @@ const char *cqg_version(void);
 const char *cqg_status_string(cqg_status s);
 cqg_status cqg_create(cqg_ctx **ctx, int device);
 cqg_status cqg_destroy(cqg_ctx *ctx);
+/* Device buffers of destroyed contexts are kept for the next ones of the process (blocks up to
+ * 64 MiB, at most 256 MiB per device).  This gives the kept ones of `device` back to the
+ * driver; *bytes (may be NULL) receives how much.  Contexts in use are not touched. */
+cqg_status cqg_release_memory(int device, long long *bytes);
 const char *cqg_last_error(const cqg_ctx *ctx);
 
 /* Basis upload (replaces BasisSet::shells_ + mapSh2Bf, include/basisset.h;
