@@ -267,7 +267,7 @@ WARP_TO_DD = {"(dp|pp)", "(dp|dp)", "(dd|pp)", "(dd|ds)", "(dd|dp)", "(dd|dd)"} 
 
 def schedule_summary(ints, st):
     """The autotuned schedule of the lists that had work: per class, the kernel form (one
-    quartet per thread, warp-cooperative, or inside the class-fused kernel), CTAs per SM,
+    quartet per thread, a warp on a quartet (tensor cores), or inside the class-fused kernel), CTAs per SM,
     warps per CTA, quartets claimed per warp and the class kernel's time; plus the fusion
     tier in use, the fused kernel's time and the autotuner's times of the three tiers."""
     sch = ints.schedule()

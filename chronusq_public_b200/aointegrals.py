@@ -132,7 +132,7 @@ class AOIntegrals:
         """Per work list (lists named by ``_lib.schedule_lists()``: FP64 lists then FP32
         lists, each the quartet classes then the sibling-group lists): CTAs per SM, warps per
         CTA and quartets claimed per warp (0 = default), and the kernel form (1 =
-        warp-cooperative, 0 = one quartet per thread)."""
+        tensor-core, a warp on a quartet, 0 = one quartet per thread)."""
         n = int(self._L.cqg_schedule_lists())
         out = [(ctypes.c_int * n)() for _ in range(4)]
         _lib.check(self._L.cqg_get_schedule(self._ctx, *out), self._ctx)

@@ -1191,7 +1191,7 @@ __global__ void __launch_bounds__(NT) k_eri_gc(const uint2 *__restrict__ ql, con
   }
 }
 
-// ------------------------------------------------------------- warp-mode classes ---
+// ---------------------------------------------- a warp on a quartet or a pair ---
 // J/K digest of one quartet by a warp: V [a][b][c][d] in shared memory, lanes spread over the
 // elements of Gh (the same updates as digest()).  Xs: shared memory for the density blocks.
 template <int LA, int LB, int LC, int LD>
@@ -1573,13 +1573,14 @@ struct cqg_ctx {
   long long list_budget = 1LL << 32;   // quartets held in the list at once (8 B each: 32 GiB)
   int nsm = 148;                       // multiprocessors of the device
   // launch shapes per (precision, class) work list: persistent CTAs per SM and, for the
-  // warp-cooperative classes, warps per CTA (0 = default); set by the autotuner
+  // tensor-core classes, warps per CTA (0 = default); set by the autotuner
   int shape_cta[CQG_NLIST] = {0};
   int shape_wpb[CQG_NLIST] = {0};
-  // quartets a warp claims from the list's work queue at a time, in units of 32 for the
-  // per-thread classes (0 = default)
+  // entries a warp claims from the list's work queue at a time, in units of 32 for the
+  // per-thread classes and at most 32 for the tensor-core ones (0 = default: 32, and a number
+  // that follows the list's length)
   int shape_qpw[CQG_NLIST] = {0};
-  // kernel form of a list whose class has both: 0 = per-thread (default), 1 = warp-cooperative
+  // kernel form of a list whose class has both: 0 = per-thread, 1 = tensor-core
   int shape_var[CQG_NLIST] = {0};
   // 0: one launch per class list; 1 or 2: the lists of that tier's classes go through one
   // class-fused persistent kernel (eri_fused.cu); set by the autotuner or cqg_set_fusion
@@ -1692,14 +1693,14 @@ struct cqg_ctx {
 static inline Pairs make_pairs(cqg_ctx *ctx);
 static inline Shells make_shells(cqg_ctx *ctx);
 
-// classes evaluated by the warp-cooperative kernel (same rule as gen_eri.WARP_CLASSES)
+// classes that have the tensor-core kernel only (same rule as gen_eri.WARP_CLASSES)
 __host__ __device__ constexpr bool is_warp_class(int la, int lb, int lc, int ld) {
   return ncart_c(la) * ncart_c(lb) * ncart_c(lc) * ncart_c(ld) > 150 || la + lb + lc + ld >= 6;
 }
 
 // Per-thread classes whose live state overflows one thread's 255 registers (their
-// generated code spills to local memory): they also get the warp-cooperative kernel, and
-// the autotuner times both forms on the class's list and keeps the faster one.
+// generated code spills to local memory): they also get the tensor-core kernel, and the
+// autotuner times both forms on the class's list and keeps the faster one.
 __host__ __device__ constexpr bool is_variant_class(int la, int lb, int lc, int ld) {
   const int k = ((la * 4 + lb) * 4 + lc) * 4 + ld;
   return !is_warp_class(la, lb, lc, ld) &&

@@ -1,5 +1,5 @@
 // One share of the quartet-class kernels: the launchers -- and with them the per-thread,
-// warp-cooperative and sibling-group kernel instantiations -- of the classes k with
+// tensor-core and sibling-group kernel instantiations -- of the classes k with
 // k % CQG_NPART == CQG_PART.
 // The build compiles this file CQG_NPART times, once per share, in parallel; engine.cu
 // merges the shares' tables into one launcher table per precision.

@@ -484,8 +484,8 @@ def quartet_classes(maxl):
     return out
 
 
-# classes evaluated by the warp-cooperative kernel (eri_warp.cuh): their Cartesian output
-# ncart(a)ncart(b)ncart(c)ncart(d) exceeds 150 values or whose R_tuv set (L >= 6, 84+ values)
+# classes that have the tensor-core kernel only (eri_tc.cuh): their Cartesian output
+# ncart(a)ncart(b)ncart(c)ncart(d) exceeds 150 values, or their R_tuv set (L >= 6, 84+ values)
 # is too large for one thread's registers
 def _nc(l):
     return (l + 1) * (l + 2) // 2

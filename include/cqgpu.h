@@ -201,8 +201,8 @@ cqg_status cqg_graph_status(cqg_ctx *ctx, long long *quartets, int *overflow, in
                             int *asymmetric);
 /* Autotuner: the next (non-graph, single-chunk) contraction times every candidate launch
  * shape of each class work list (persistent CTAs per SM; warps per CTA for the
- * warp-cooperative classes; quartets claimed per warp from the list's work queue) and keeps
- * the fastest for later calls.  The shapes are read
+ * tensor-core classes; list entries claimed per warp from the list's work queue), the default
+ * first, and keeps the fastest for later calls.  The shapes are read
  * back with cqg_get_launch_shapes (cqg_schedule_lists() entries: FP64 lists then FP32 lists;
  * 0 = default). */
 cqg_status cqg_autotune_next(cqg_ctx *ctx);
@@ -211,9 +211,9 @@ cqg_status cqg_autotune_next(cqg_ctx *ctx);
 cqg_status cqg_set_active(cqg_ctx *ctx, const unsigned char *active);
 cqg_status cqg_get_launch_shapes(cqg_ctx *ctx, int *cta_per_sm, int *warps_per_cta);
 /* The same plus, per list, the work-queue chunk (the quartets one warp claims at a time:
- * per-thread kernels in units of 32, one per lane; warp-cooperative kernels one after the
- * other) and the kernel form (1 = warp-cooperative, 0 = one quartet per thread; classes
- * that have both forms get theirs from the autotuner).  For the sibling-entry lists, warps
+ * per-thread kernels in units of 32, one per lane; tensor-core kernels one after the other,
+ * at most 32) and the kernel form (1 = tensor-core, a warp on a quartet, 0 = one quartet
+ * per thread; classes that have both forms get theirs from the autotuner).  For the sibling-entry lists, warps
  * per CTA 2 selects CTAs of 64 threads (otherwise 128).  Any output may be NULL; 0 in the
  * first three = default. */
 cqg_status cqg_get_schedule(cqg_ctx *ctx, int *cta_per_sm, int *warps_per_cta, int *quartets_per_warp,
