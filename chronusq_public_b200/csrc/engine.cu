@@ -101,8 +101,16 @@ cudaError_t cqg_pool_alloc(void **p, size_t *bytes, int *device) {
   return cudaSuccess;
 }
 
+// Set while a thread frees buffers that the device may still be using (the wait for it failed,
+// as it does inside a stream capture): they go to the driver, which waits for them.
+static thread_local bool t_in_use = false;
+static void end_in_use() {
+  if (t_in_use) cudaGetLastError();   // of the wait and the frees: no later call's error
+  t_in_use = false;
+}
+
 void cqg_pool_free(void *p, size_t bytes, int device) {
-  if (device >= 64 || bytes > kPoolLargest) {
+  if (device >= 64 || bytes > kPoolLargest || t_in_use) {
     cudaFree(p);
     return;
   }
@@ -137,9 +145,10 @@ static cudaError_t grow(cqg_ctx *ctx, DevBuf<T> &b, size_t m) {
 }
 static void release_retired(cqg_ctx *ctx) {
   if (ctx->retired.empty()) return;
-  cudaDeviceSynchronize();
+  t_in_use = cudaDeviceSynchronize() != cudaSuccess;
   for (auto &r : ctx->retired) cqg_pool_free(r.p, r.bytes, r.device);
   ctx->retired.clear();
+  end_in_use();
 }
 
 static const char *kLetters = "spdfg";
@@ -931,8 +940,8 @@ cqg_status cqg_release_memory(int device, long long *bytes) {
 cqg_status cqg_destroy(cqg_ctx *ctx) {
   if (!ctx) return CQG_OK;
   cudaSetDevice(ctx->device);
-  cudaDeviceSynchronize();   // the buffers go back to the pool
   release_retired(ctx);
+  t_in_use = cudaDeviceSynchronize() != cudaSuccess;   // the buffers go back to the pool
   ctx->d_center.release(); ctx->d_bf.release(); ctx->d_sz.release();
   ctx->d_pair_sh.release(); ctx->d_pair_Q.release(); ctx->d_pair_poff.release(); ctx->d_pair_np.release();
   ctx->d_pair_kk.release();
@@ -950,6 +959,7 @@ cqg_status cqg_destroy(cqg_ctx *ctx) {
   ctx->d_molgbk.release(); ctx->d_gsz.release(); ctx->d_gpoff.release(); ctx->d_gnp.release(); ctx->d_gwoff.release();
   ctx->d_glead.release(); ctx->d_pair_Qc.release(); ctx->d_gQ.release(); ctx->d_gw.release(); ctx->d_gprim.release();
   ctx->d_qmask.release(); ctx->d_masks.release(); ctx->d_mslot.release();
+  end_in_use();
   return_side_streams(ctx);
   if (ctx->events)
     for (int i = 0; i < 4 + 2 * CQG_NQC + 2; ++i) cudaEventDestroy(ctx->ev[i]);
