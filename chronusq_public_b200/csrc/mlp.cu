@@ -4,22 +4,19 @@
 //   k_gemm_bf16 : C[m][n] (+)= sum_k A(m,k) B(n,k), A and B BF16 with arbitrary strides
 //                 (transposes are strides), on the tensor cores: mma.sync m16n8k16 BF16 x
 //                 BF16 -> FP32 over block tiles that come through a ring of asynchronous
-//                 copies; optional fused epilogue Z = C + bias (FP32) and Y = SiLU(Z) (BF16).
-//                 or, backward, dZ = C * SiLU'(Z) (BF16, the next GEMMs' operand) and its column sums
-//   k_gemm_parts: C[m][n] += sum_k A(m,k) B(n,k), the parts of a split K added with atomics (the
-//                 gradient of a layer's input)
-//   k_dz_colsum : a layer's dZ in BF16, through SiLU' for the hidden ones, and db[n] = sum_m dZ[m][n]
+//                 copies; optional fused epilogue Z = C + bias (FP32) and Y = SiLU(Z) (BF16)
+//   k_gemm_parts: the same product with K split over blocks, their parts added with atomics
+//   k_silu_bwd  : dZ = dY * SiLU'(Z)  (BF16 out, the next GEMM's operand)
+//   k_colsum    : db[n] = sum_m dZ[m][n]
 //   k_mse       : masked squared error, its gradient, and the loss sum
-//   k_adam      : Adam step on FP32 master weights, BF16 copy for the next pass, all tensors of
-//                 the network in one launch
-//   k_silu_bwd, k_to_bf16 : the elementwise parts alone (cqg_mlp_silu_bwd, cqg_mlp_to_bf16)
+//   k_adam      : Adam step on FP32 master weights, BF16 copy for the next pass
+//   k_to_bf16   : FP32 -> BF16
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <algorithm>
 #include <atomic>
-#include <utility>
 
 #include "../../include/cqgpu.h"
 
@@ -75,8 +72,7 @@ struct TileCopy {
   long long step;    // elements from one tile to the next
   unsigned dst[NC];  // offset in the tile
   int most[NC], k[NC], mul;
-  __device__ __forceinline__ TileCopy(const __nv_bfloat16 *X, long long sr, long long sk, int r0, int nrows, int kb,
-                                      int mode) {
+  __device__ __forceinline__ TileCopy(const __nv_bfloat16 *X, long long sr, long long sk, int r0, int nrows, int mode) {
     const bool kin = mode == TILE_K;
     step = kin ? GK : GK * sk;
     mul = kin ? 2 : 16;
@@ -87,10 +83,10 @@ struct TileCopy {
       k[c] = kin ? e % (GK / 8) * 8 : e / (ROWS / 8);
       dst[c] = 2 * (kin ? (r - r0) * GP + k[c] : k[c] * (ROWS + 8) + r - r0);
       most[c] = max(0, min(16, (nrows - r) * (kin ? 16 : 2)));
-      src[c] = most[c] ? X + r * sr + (kb + k[c]) * sk : X;
+      src[c] = most[c] ? X + r * sr + k[c] * sk : X;
     }
   }
-  // tile kt of k [kb + kt * GK, ...), `left` = K - that
+  // tile kt, of k from kt * GK; `left` = K - that
   __device__ __forceinline__ void start(unsigned tile, int kt, int left) const {
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
@@ -124,20 +120,14 @@ __device__ __forceinline__ void stage_any(const __nv_bfloat16 *__restrict__ X, l
   }
 }
 
-// One product of a launch.  split: the block reduces k in [z kchunk, (z + 1) kchunk) and adds
-// its partial tile to C with atomics (C zeroed by the caller), no epilogue.  dact: the
-// epilogue is the backward step through the layer below, Y = bf16(value * SiLU'(dact)) and its
-// column sums added to db; C is not written.
 struct Gemm {
   const __nv_bfloat16 *A, *B;
   long long sam, sak, sbn, sbk, ldc, ldy;
   float *C;
-  const float *bias, *dact;
-  float *db;
+  const float *bias;
   __nv_bfloat16 *Y;
-  int M, N, K, kchunk, nbn, nbm, nbz;
-  unsigned char amode, bmode, act, accumulate, split, pairs;   // pairs: C, Y and dact take 2-wide accesses
-  __host__ int blocks() const { return nbn * nbm * nbz; }
+  int M, N, K, nbn;
+  unsigned char amode, bmode, act, accumulate, pairs;   // pairs: C and Y take 2-wide accesses
 };
 
 // Block tile BM x BN (BM, BN multiples of 32), warps of 32 x WN output each (WN = 64 or 32):
@@ -145,25 +135,19 @@ struct Gemm {
 // tiles.  128 x 128 with 8 warps of 32 x 64 for large problems, 64 x 64 with 4 warps of
 // 32 x 32 when the large tiles would leave most of the 148 SMs idle.  A training step's
 // products (2048 x 256 x 256) are chains of load latencies, not arithmetic: tiles of 32 k come
-// through a ring of STAGES asynchronous copies, and two products (the weight gradients of two
-// layers, or one with the gradient of its layer's input) share a launch, the first `blocks0`
-// blocks for g0.
-// Measured, 2048 rows, width 256: a layer forward 17 us cold (9.1 us back to back) from one
-// synchronous tile at a time before.
+// through a ring of STAGES asynchronous copies.  Measured, 2048 rows, width 256: a layer forward
+// 9.1 us, 17 us with one synchronous tile at a time.
 template <int BM, int BN, int WN, int STAGES>
 __global__ void __launch_bounds__((BM / 32) * (BN / WN) * 32, BM == 64 ? 3 : 2)
-    k_gemm_bf16(const __grid_constant__ Gemm g0, const __grid_constant__ Gemm g1, int blocks0) {
+    k_gemm_bf16(const __grid_constant__ Gemm p) {
   constexpr int NWM = BM / 32, NJ = WN / 8, NT = NWM * (BN / WN) * 32;
   constexpr int ASZ = BM * GP, BSZ = BN * GP;   // [k][row] tiles, GK x (rows + 8), fit as well
   static_assert(GK * (BM + 8) <= ASZ && GK * (BN + 8) <= BSZ, "tile buffers");
   extern __shared__ __align__(16) __nv_bfloat16 tiles[];
-  const bool first = (int)blockIdx.x < blocks0;
-  const Gemm p = first ? g0 : g1;
-  const int blk = first ? blockIdx.x : blockIdx.x - blocks0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int wm = (warp % NWM) * 32, wn = (warp / NWM) * WN;
   const int M = p.M, N = p.N, K = p.K;
-  const int n0 = blk % p.nbn * BN, m0 = blk / p.nbn % p.nbm * BM, z = blk / (p.nbn * p.nbm);
+  const int n0 = (int)blockIdx.x % p.nbn * BN, m0 = (int)blockIdx.x / p.nbn * BM;
   const int g = lane >> 2, t = lane & 3;
   float acc[2][NJ][4];
 #pragma unroll
@@ -172,25 +156,24 @@ __global__ void __launch_bounds__((BM / 32) * (BN / WN) * 32, BM == 64 ? 3 : 2)
     for (int j = 0; j < NJ; ++j)
 #pragma unroll
       for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.f;
-  const int kb = p.split ? z * p.kchunk : 0, ke = p.split ? min(K, kb + p.kchunk) : K;
-  const int nkt = (ke - kb + GK - 1) / GK;
+  const int nkt = (K + GK - 1) / GK;
   const __nv_bfloat16 *A = p.A, *B = p.B;
   const long long sam = p.sam, sak = p.sak, sbn = p.sbn, sbk = p.sbk;
   const int amode = p.amode, bmode = p.bmode;
-  const TileCopy<BM, NT> ca(A, sam, sak, m0, M, kb, amode);
-  const TileCopy<BN, NT> cb(B, sbn, sbk, n0, N, kb, bmode);
+  const TileCopy<BM, NT> ca(A, sam, sak, m0, M, amode);
+  const TileCopy<BN, NT> cb(B, sbn, sbk, n0, N, bmode);
   auto issue = [&](int kt) {
     if (kt < nkt) {
       __nv_bfloat16 *As = tiles + (kt % STAGES) * (ASZ + BSZ), *Bs = As + ASZ;
-      const int k0 = kb + kt * GK;
+      const int k0 = kt * GK;
       if (amode != TILE_ANY)
-        ca.start((unsigned)__cvta_generic_to_shared(As), kt, ke - k0);
+        ca.start((unsigned)__cvta_generic_to_shared(As), kt, K - k0);
       else
-        stage_any<BM, NT>(A, sam, sak, m0, M, k0, ke, As);
+        stage_any<BM, NT>(A, sam, sak, m0, M, k0, K, As);
       if (bmode != TILE_ANY)
-        cb.start((unsigned)__cvta_generic_to_shared(Bs), kt, ke - k0);
+        cb.start((unsigned)__cvta_generic_to_shared(Bs), kt, K - k0);
       else
-        stage_any<BN, NT>(B, sbn, sbk, n0, N, k0, ke, Bs);
+        stage_any<BN, NT>(B, sbn, sbk, n0, N, k0, K, Bs);
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
@@ -235,26 +218,7 @@ __global__ void __launch_bounds__((BM / 32) * (BN / WN) * 32, BM == 64 ? 3 : 2)
   __nv_bfloat16 *Y = p.Y;
   const long long ldc = p.ldc, ldy = p.ldy;
   const bool pairs = p.pairs;
-  if (p.split) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < NJ; ++j)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int m = m0 + wm + i * 16 + g + h * 8, n = n0 + wn + j * 8 + 2 * t;
-          if (m >= M || n >= N) continue;
-          float *c = C + m * ldc + n;
-          if (pairs && n + 1 < N) {
-            atomicAdd(reinterpret_cast<float2 *>(c), make_float2(acc[i][j][2 * h], acc[i][j][2 * h + 1]));
-          } else {
-            atomicAdd(c, acc[i][j][2 * h]);
-            if (n + 1 < N) atomicAdd(c + 1, acc[i][j][2 * h + 1]);
-          }
-        }
-    return;
-  }
-  // the other epilogues from shared memory, four rows of two neighbouring columns a thread at
+  // the epilogue from shared memory, four rows of two neighbouring columns a thread at
   // a time: short code (unrolled over the accumulators, instruction misses were 2 us of a
   // launch) with its loads in flight
   constexpr int SP = BN + 8, CG = BN / 2, RSTEP = NT / CG, U = 4;
@@ -274,12 +238,9 @@ __global__ void __launch_bounds__((BM / 32) * (BN / WN) * 32, BM == 64 ? 3 : 2)
   const int c2 = threadIdx.x % CG * 2, n = n0 + c2;
   if (n >= N) return;
   const bool two = n + 1 < N, both = pairs && two;
-  const float *bias = p.bias, *dact = p.dact;
-  const bool act = p.act;
-  const float *src = dact ? dact : p.accumulate ? C : nullptr;   // the activation's argument, or what C holds
-  const long long lds = dact ? ldy : ldc;
+  const float *bias = p.bias;
+  const bool act = p.act, accumulate = p.accumulate;
   const float b0 = bias ? bias[n] : 0.f, b1 = bias && two ? bias[n + 1] : 0.f;
-  float s0 = 0.f, s1 = 0.f;
 #pragma unroll 1
   for (int r0 = threadIdx.x / CG; r0 < min(BM, M - m0); r0 += RSTEP * U) {
     float2 d[U];
@@ -287,8 +248,8 @@ __global__ void __launch_bounds__((BM / 32) * (BN / WN) * 32, BM == 64 ? 3 : 2)
     for (int u = 0; u < U; ++u) {
       const int r = r0 + u * RSTEP;
       d[u] = make_float2(0.f, 0.f);
-      if (src && m0 + r < M) {
-        const float *q = src + (m0 + r) * lds + n;
+      if (accumulate && m0 + r < M) {
+        const float *q = C + (m0 + r) * ldc + n;
         if (both)
           d[u] = *reinterpret_cast<const float2 *>(q);
         else
@@ -300,25 +261,16 @@ __global__ void __launch_bounds__((BM / 32) * (BN / WN) * 32, BM == 64 ? 3 : 2)
       const int r = r0 + u * RSTEP;
       if (m0 + r >= M) break;
       const float2 v = *reinterpret_cast<const float2 *>(S + r * SP + c2);
-      const float z0 = v.x + b0 + (dact ? 0.f : d[u].x), z1 = v.y + b1 + (dact ? 0.f : d[u].y);
-      __nv_bfloat16 y0, y1;
-      if (dact) {
-        y0 = __float2bfloat16(z0 * silu_grad(d[u].x));
-        y1 = __float2bfloat16(z1 * silu_grad(d[u].y));
-        s0 += __bfloat162float(y0);
-        s1 += __bfloat162float(y1);
+      const float z0 = v.x + b0 + d[u].x, z1 = v.y + b1 + d[u].y;
+      float *c = C + (m0 + r) * ldc + n;
+      if (both) {
+        *reinterpret_cast<float2 *>(c) = make_float2(z0, z1);
       } else {
-        float *c = C + (m0 + r) * ldc + n;
-        if (both) {
-          *reinterpret_cast<float2 *>(c) = make_float2(z0, z1);
-        } else {
-          c[0] = z0;
-          if (two) c[1] = z1;
-        }
-        if (!Y) continue;
-        y0 = __float2bfloat16(act ? silu(z0) : z0);
-        y1 = __float2bfloat16(act ? silu(z1) : z1);
+        c[0] = z0;
+        if (two) c[1] = z1;
       }
+      if (!Y) continue;
+      const __nv_bfloat16 y0 = __float2bfloat16(act ? silu(z0) : z0), y1 = __float2bfloat16(act ? silu(z1) : z1);
       __nv_bfloat16 *y = Y + (m0 + r) * ldy + n;
       if (both) {
         *reinterpret_cast<__nv_bfloat162 *>(y) = __halves2bfloat162(y0, y1);
@@ -328,17 +280,12 @@ __global__ void __launch_bounds__((BM / 32) * (BN / WN) * 32, BM == 64 ? 3 : 2)
       }
     }
   }
-  if (dact) {
-    atomicAdd(p.db + n, s0);
-    if (two) atomicAdd(p.db + n + 1, s1);
-  }
 }
 
 // Rows [r0, r0 + 64) x k [k0, k0 + 32) of X(r, k) = X[r * sr + k * sk] into S[row][k] (zero outside
 // nrows x K).  Rows or k contiguous and 16-byte aligned: 8-element loads; anything else element
 // by element.
 constexpr int kPartTile = 64;
-static_assert(148 * kPartTile * kPartTile == CQG_MLP_DX_MAX, "fewer than 148 tiles (k_parts) are split");
 __device__ __forceinline__ void stage_part(const __nv_bfloat16 *__restrict__ X, long long sr, long long sk, int r0,
                                            int nrows, int k0, int K, bool vec_k, bool vec_r,
                                            __nv_bfloat16 (*S)[GP]) {
@@ -378,17 +325,18 @@ __device__ __forceinline__ void stage_part(const __nv_bfloat16 *__restrict__ X, 
 }
 
 // C[m][n] += sum_k A(m,k) B(n,k) over k [blockIdx.z kchunk, + kchunk), 64 x 64 tiles of four
-// warps, one tile of k in shared memory at a time, C zeroed by the caller: the gradient of a
-// layer's input when its product is split.  The parts of one element add up in the order in
-// which their blocks finish, and the next dZ is that sum in BF16: a last bit that differs turns
-// one BF16 rounding in some 2^16, 2^-8 of an element, and the layers below multiply it.  Which
-// order is usual depends on how long the blocks run.  Measured, 2048 rows, width 256, four of
-// these products in a pass, median of the largest relative change of a weight gradient: two
-// runs of the layer-by-layer pass with this kernel 1.0e-5; cqg_mlp_backward with it against
-// that pass 1.6e-5; with k_gemm_bf16 and atomics 3.7e-5 to 4.6e-5, its blocks being three times
-// as fast; with the parts in any one fixed order 3.2e-5 to 7.4e-5.  (Against 64 bits all are
-// the same, 1e-3: BF16 operands.)  So the products that are split keep this kernel, 17 us each
-// where k_gemm_bf16 takes 9, and a training step keeps its gradients.
+// warps, one tile of k in shared memory at a time, C zeroed by the caller: the backward pass's
+// products that are split.  The parts of one element add up in the order in which their
+// blocks finish.  For the gradient of a layer's input that order is seen: the next dZ is the sum
+// in BF16, a last bit that differs turns one BF16 rounding in some 2^16, 2^-8 of an element, and
+// the layers below multiply it.  Which order is usual depends on how long the blocks run, on
+// the launches around them and on where the buffers lie.  Measured, 2048 rows, width 256, four
+// of these products in a pass, median of the largest relative change of a weight gradient
+// between two processes on the same inputs: 1e-6 to 1.3e-5 for this kernel in the layer-by-layer
+// pass; 1.4e-5 to 2e-5 with the whole pass in one call, the weight gradients of two layers in a
+// launch and SiLU' with the column sums in another; 2.5e-5 and more with the sum in one fixed
+// order or in blocks of k_gemm_bf16.  So the backward pass keeps this kernel (17 us a product
+// where k_gemm_bf16 takes 9) and its launches, and training runs keep their gradients.
 __global__ void __launch_bounds__(128)
     k_gemm_parts(const __nv_bfloat16 *__restrict__ A, long long sam, long long sak, const __nv_bfloat16 *__restrict__ B,
                  long long sbn, long long sbk, float *__restrict__ C, long long ldc, int M, int N, int K, int kchunk) {
@@ -462,35 +410,18 @@ __global__ void k_to_bf16(const float *__restrict__ x, __nv_bfloat16 *__restrict
   if (i < n) y[i] = __float2bfloat16(x[i]);
 }
 
-// dZ = dY in BF16, times SiLU'(Z) where Z is given (dY null: `in` holds dZ already), and its
-// column sums, db[n] += sum_m dZ[m][n] (db zeroed by the caller).  A block takes 32 columns x
-// kColRows rows, a warp one row at a time (coalesced); one atomic per column and block.  The two
-// as kernels of their own took 4 + 17 us per layer of 2048 x 256.
-constexpr int kColRows = 64;
-__global__ void __launch_bounds__(256) k_dz_colsum(const float *__restrict__ dY,
-                                                   const float *__restrict__ Z,
-                                                   const __nv_bfloat16 *__restrict__ in,
-                                                   __nv_bfloat16 *__restrict__ out, int M, int N,
-                                                   float *__restrict__ db) {
+// db[n] += sum over rows [blockIdx.y * 256, +256) of dZ[m][n]: 32 columns x 8 row groups
+// per block (a warp reads 32 consecutive columns of one row), partial sums reduced in shared
+// memory, one atomic per column and block (db zeroed by the caller).
+__global__ void __launch_bounds__(256) k_colsum(const __nv_bfloat16 *__restrict__ dZ, int M, int N,
+                                                float *__restrict__ db) {
   __shared__ float part[8][33];
   const int c = threadIdx.x & 31, rg = threadIdx.x >> 5;
-  const int n = blockIdx.y * 32 + c;
-  const int m0 = blockIdx.x * kColRows, m1 = (int)min((long long)M, (long long)m0 + kColRows);
+  const int n = blockIdx.x * 32 + c;
+  const int m0 = blockIdx.y * 256, m1 = min(M, m0 + 256);
   float s = 0.f;
-  if (n < N) {
-#pragma unroll 4
-    for (int m = m0 + rg; m < m1; m += 8) {
-      const long long e = (long long)m * N + n;
-      __nv_bfloat16 v;
-      if (in) {
-        v = in[e];
-      } else {
-        v = __float2bfloat16(Z ? dY[e] * silu_grad(Z[e]) : dY[e]);
-        out[e] = v;
-      }
-      s += __bfloat162float(v);
-    }
-  }
+  if (n < N)
+    for (int m = m0 + rg; m < m1; m += 8) s += __bfloat162float(dZ[(long long)m * N + n]);
   part[rg][c] = s;
   __syncthreads();
   if (rg == 0 && n < N) {
@@ -522,37 +453,37 @@ __global__ void k_mse(const float *__restrict__ pred, const float *__restrict__ 
   if (threadIdx.x == 0) atomicAdd(loss, red[0]);
 }
 
-// One Adam step of up to kAdamTensors tensors (blockIdx.y), bias-corrected, decoupled weight
-// decay folded into the gradient, with an optional BF16 copy.  The learning rate and the two
-// bias corrections 1 - b^step come from device memory when `hyper` is given (a captured step
-// is then replayed with a schedule that changes from step to step).
-constexpr int kAdamTensors = 16;
-struct AdamTensors {
-  float *w[kAdamTensors], *m1[kAdamTensors], *m2[kAdamTensors];
-  const float *g[kAdamTensors];
-  __nv_bfloat16 *wbf[kAdamTensors];
-  long long n[kAdamTensors];
-  float wd[kAdamTensors];
-};
-__global__ void __launch_bounds__(256) k_adam(AdamTensors ts, const float *__restrict__ hyper, float lr, float bc1,
-                                              float bc2, float b1, float b2, float eps) {
-  const int k = blockIdx.y;
+__global__ void k_adam(float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m1,
+                       float *__restrict__ m2, long long n, float lr, float b1, float b2, float eps, float bc1,
+                       float bc2, float wd, __nv_bfloat16 *__restrict__ wbf) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= ts.n[k]) return;
-  if (hyper) {
-    lr = hyper[0];
-    bc1 = hyper[1];
-    bc2 = hyper[2];
-  }
-  float *w = ts.w[k], *m1 = ts.m1[k], *m2 = ts.m2[k];
-  const float w0 = w[i], gi = ts.g[k][i] + ts.wd[k] * w0;
+  if (i >= n) return;
+  const float gi = g[i] + wd * w[i];
   const float a = b1 * m1[i] + (1.f - b1) * gi;
   const float b = b2 * m2[i] + (1.f - b2) * gi * gi;
   m1[i] = a;
   m2[i] = b;
-  const float w1 = w0 - lr * (a / bc1) / (sqrtf(b / bc2) + eps);
-  w[i] = w1;
-  if (ts.wbf[k]) ts.wbf[k][i] = __float2bfloat16(w1);
+  const float upd = lr * (a / bc1) / (sqrtf(b / bc2) + eps);
+  w[i] -= upd;
+  if (wbf) wbf[i] = __float2bfloat16(w[i]);
+}
+
+// The same step with the learning rate and the two bias corrections read from device memory
+// (hyper = {lr, 1 - b1^step, 1 - b2^step}), so that a captured training step can be replayed
+// with a schedule that changes from step to step.
+__global__ void k_adam_dev(float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m1,
+                           float *__restrict__ m2, long long n, const float *__restrict__ hyper, float b1, float b2,
+                           float eps, float wd, __nv_bfloat16 *__restrict__ wbf) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float lr = hyper[0], bc1 = hyper[1], bc2 = hyper[2];
+  const float gi = g[i] + wd * w[i];
+  const float a = b1 * m1[i] + (1.f - b1) * gi;
+  const float b = b2 * m2[i] + (1.f - b2) * gi * gi;
+  m1[i] = a;
+  m2[i] = b;
+  w[i] -= lr * (a / bc1) / (sqrtf(b / bc2) + eps);
+  if (wbf) wbf[i] = __float2bfloat16(w[i]);
 }
 
 // Shared memory above the default 48 KB, asked for once per kernel and device.
@@ -567,9 +498,6 @@ cudaError_t allow_tiles(K kernel, int bytes, std::atomic<bool> (&done)[64]) {
   if (e == cudaSuccess) done[slot].store(true, std::memory_order_relaxed);
   return e;
 }
-
-constexpr int kBigStages = 4, kSmallStages = 6;
-constexpr int kBigSmem = kBigStages * (GM + GN) * GP * 2, kSmallSmem = kSmallStages * (64 + 64) * GP * 2;
 
 Gemm gemm_of(const void *A, long long sam, long long sak, const void *B, long long sbn, long long sbk, float *C,
              long long ldc, int M, int N, int K) {
@@ -600,45 +528,25 @@ bool big_tiles(int M, int N) { return (long long)((N + GN - 1) / GN) * ((M + GM 
 
 void set_pairs(Gemm &g) {
   auto aligned = [](const void *p, int bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; };
-  g.pairs = (!g.C || (g.ldc % 2 == 0 && aligned(g.C, 8))) && (!g.Y || (g.ldy % 2 == 0 && aligned(g.Y, 4))) &&
-            (!g.dact || (g.ldy % 2 == 0 && aligned(g.dact, 8)));
-}
-
-void tile_by(Gemm &g, int bm, int bn) {
-  g.nbn = (g.N + bn - 1) / bn;
-  g.nbm = (g.M + bm - 1) / bm;
-  g.nbz = 1;
+  g.pairs = g.ldc % 2 == 0 && aligned(g.C, 8) && (!g.Y || (g.ldy % 2 == 0 && aligned(g.Y, 4)));
 }
 
 // Few 64 x 64 output tiles and a long reduction (weight gradients: K = batch rows): K split so
-// that about two waves of blocks run, in parts of `least` or more; the part, or 0 for one.
-int k_parts(int M, int N, int K, int least) {
+// that about two waves of blocks run, in parts of 64 or more; the part, or 0 for one.
+int k_parts(int M, int N, int K) {
   const long long tiles = (long long)((N + 63) / 64) * ((M + 63) / 64);
-  if (tiles >= 148 || K < 128) return 0;
-  const int splits = (int)std::min<long long>(std::min<long long>((296 + tiles - 1) / tiles, K / least), 64);
+  if (tiles >= 148 || K < 4 * GK) return 0;
+  const int splits = (int)std::min<long long>(std::min<long long>((296 + tiles - 1) / tiles, K / (2 * GK)), 64);
   return splits > 1 ? ((K + splits - 1) / splits + GK - 1) / GK * GK : 0;
 }
 
-void split_k(Gemm &g) {
-  g.kchunk = k_parts(g.M, g.N, g.K, GK);
-  if (g.kchunk > 0) {
-    g.split = 1;
-    g.nbz = (g.K + g.kchunk - 1) / g.kchunk;
-  }
-}
-
-cqg_status launch_big(const Gemm &g, cudaStream_t st) {
+template <int BM, int BN, int WN, int STAGES>
+cqg_status launch_gemm(Gemm &g, cudaStream_t st) {
   static std::atomic<bool> allowed[64];
-  if (allow_tiles(&k_gemm_bf16<GM, GN, 64, kBigStages>, kBigSmem, allowed) != cudaSuccess) return CQG_ERR_CUDA;
-  k_gemm_bf16<GM, GN, 64, kBigStages><<<g.blocks(), 256, kBigSmem, st>>>(g, g, g.blocks());
-  return CQG_OK;
-}
-
-cqg_status launch_small(const Gemm &g, const Gemm *second, cudaStream_t st) {
-  static std::atomic<bool> allowed[64];
-  if (allow_tiles(&k_gemm_bf16<64, 64, 32, kSmallStages>, kSmallSmem, allowed) != cudaSuccess) return CQG_ERR_CUDA;
-  const int n = g.blocks() + (second ? second->blocks() : 0);
-  k_gemm_bf16<64, 64, 32, kSmallStages><<<n, 128, kSmallSmem, st>>>(g, second ? *second : g, g.blocks());
+  constexpr int smem = STAGES * (BM + BN) * GP * 2;
+  if (allow_tiles(&k_gemm_bf16<BM, BN, WN, STAGES>, smem, allowed) != cudaSuccess) return CQG_ERR_CUDA;
+  g.nbn = (g.N + BN - 1) / BN;
+  k_gemm_bf16<BM, BN, WN, STAGES><<<g.nbn * ((g.M + BM - 1) / BM), (BM / 32) * (BN / WN) * 32, smem, st>>>(g);
   return CQG_OK;
 }
 
@@ -654,28 +562,26 @@ cqg_status cqg_mlp_gemm_bf16(const void *A, long long sam, long long sak, const 
   if (!A || !B || !C || M < 0 || N < 0 || K < 0) return CQG_ERR_BAD_ARG;
   if (M == 0 || N == 0) return CQG_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  Gemm g = gemm_of(A, sam, sak, B, sbn, sbk, C, ldc, M, N, K);
-  g.bias = bias;
-  g.Y = (__nv_bfloat16 *)Y;
-  g.ldy = ldy;
-  g.act = act != 0;
-  g.accumulate = accumulate != 0;
-  set_pairs(g);
   const bool big = big_tiles(M, N);
   if ((M + (big ? GM : 64) - 1) / (big ? GM : 64) > 65535) return CQG_ERR_BAD_ARG;
-  cqg_status s;
-  if (big) {
-    tile_by(g, GM, GN);
-    s = launch_big(g, st);
-  } else {
-    tile_by(g, 64, 64);
-    if (!bias && !Y) split_k(g);
-    if (g.split && !accumulate &&
-        cudaMemset2DAsync(C, ldc * sizeof(float), 0, N * sizeof(float), M, st) != cudaSuccess)
+  const int part = big || bias || Y ? 0 : k_parts(M, N, K);
+  if (part > 0) {
+    if (!accumulate && cudaMemset2DAsync(C, ldc * sizeof(float), 0, N * sizeof(float), M, st) != cudaSuccess)
       return CQG_ERR_CUDA;
-    s = launch_small(g, nullptr, st);
+    const dim3 grid((N + kPartTile - 1) / kPartTile, (M + kPartTile - 1) / kPartTile, (K + part - 1) / part);
+    k_gemm_parts<<<grid, 128, 0, st>>>((const __nv_bfloat16 *)A, sam, sak, (const __nv_bfloat16 *)B, sbn, sbk, C, ldc, M,
+                                       N, K, part);
+  } else {
+    Gemm g = gemm_of(A, sam, sak, B, sbn, sbk, C, ldc, M, N, K);
+    g.bias = bias;
+    g.Y = (__nv_bfloat16 *)Y;
+    g.ldy = ldy;
+    g.act = act != 0;
+    g.accumulate = accumulate != 0;
+    set_pairs(g);
+    const cqg_status s = big ? launch_gemm<GM, GN, 64, 4>(g, st) : launch_gemm<64, 64, 32, 6>(g, st);
+    if (s != CQG_OK) return s;
   }
-  if (s != CQG_OK) return s;
   return cudaGetLastError() == cudaSuccess ? CQG_OK : CQG_ERR_CUDA;
 }
 
@@ -695,9 +601,9 @@ cqg_status cqg_mlp_colsum(const void *dZ, int M, int N, float *db, void *stream)
   if (N <= 0) return CQG_OK;
   if (cudaMemsetAsync(db, 0, (size_t)N * sizeof(float), (cudaStream_t)stream) != cudaSuccess) return CQG_ERR_CUDA;
   if (M <= 0) return CQG_OK;
-  if ((M + 255) / 256 > 65535 || (N + 31) / 32 > 65535) return CQG_ERR_BAD_ARG;
-  dim3 grid((M + kColRows - 1) / kColRows, (N + 31) / 32);
-  k_dz_colsum<<<grid, 256, 0, (cudaStream_t)stream>>>(nullptr, nullptr, (const __nv_bfloat16 *)dZ, nullptr, M, N, db);
+  if ((M + 255) / 256 > 65535) return CQG_ERR_BAD_ARG;
+  dim3 grid((N + 31) / 32, (M + 255) / 256);
+  k_colsum<<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16 *)dZ, M, N, db);
   return cudaGetLastError() == cudaSuccess ? CQG_OK : CQG_ERR_CUDA;
 }
 
@@ -708,43 +614,21 @@ cqg_status cqg_mlp_mse(const float *pred, const float *target, const float *mask
   return cudaGetLastError() == cudaSuccess ? CQG_OK : CQG_ERR_CUDA;
 }
 
-cqg_status cqg_mlp_adam_tensors(int nt, float *const *w, const float *const *g, float *const *m1, float *const *m2,
-                                const long long *n, const float *weight_decay, void *const *wbf, const float *hyper,
-                                float lr, float b1, float b2, float eps, int step, void *stream) {
-  if (nt <= 0 || !w || !g || !m1 || !m2 || !n || !weight_decay || !wbf || (!hyper && step < 1))
-    return CQG_ERR_BAD_ARG;
-  for (int k = 0; k < nt; ++k)
-    if (n[k] <= 0) return CQG_ERR_BAD_ARG;
-  const float bc1 = hyper ? 1.f : 1.f - powf(b1, (float)step), bc2 = hyper ? 1.f : 1.f - powf(b2, (float)step);
-  for (int k0 = 0; k0 < nt; k0 += kAdamTensors) {
-    AdamTensors ts = {};
-    const int m = std::min(kAdamTensors, nt - k0);
-    long long most = 0;
-    for (int k = 0; k < m; ++k) {
-      ts.w[k] = w[k0 + k];
-      ts.g[k] = g[k0 + k];
-      ts.m1[k] = m1[k0 + k];
-      ts.m2[k] = m2[k0 + k];
-      ts.wbf[k] = (__nv_bfloat16 *)wbf[k0 + k];
-      ts.n[k] = n[k0 + k];
-      ts.wd[k] = weight_decay[k0 + k];
-      most = std::max(most, ts.n[k]);
-    }
-    k_adam<<<dim3(nblk(most, 256), m), 256, 0, (cudaStream_t)stream>>>(ts, hyper, lr, bc1, bc2, b1, b2, eps);
-  }
-  return cudaGetLastError() == cudaSuccess ? CQG_OK : CQG_ERR_CUDA;
-}
-
 cqg_status cqg_mlp_adam(float *w, const float *g, float *m1, float *m2, long long n, float lr, float b1, float b2,
                         float eps, int step, float weight_decay, void *wbf, void *stream) {
-  if (step < 1) return CQG_ERR_BAD_ARG;
-  return cqg_mlp_adam_tensors(1, &w, &g, &m1, &m2, &n, &weight_decay, &wbf, nullptr, lr, b1, b2, eps, step, stream);
+  if (n <= 0 || step < 1) return CQG_ERR_BAD_ARG;
+  const float bc1 = 1.f - powf(b1, (float)step), bc2 = 1.f - powf(b2, (float)step);
+  k_adam<<<nblk(n, 256), 256, 0, (cudaStream_t)stream>>>(w, g, m1, m2, n, lr, b1, b2, eps, bc1, bc2, weight_decay,
+                                                         (__nv_bfloat16 *)wbf);
+  return cudaGetLastError() == cudaSuccess ? CQG_OK : CQG_ERR_CUDA;
 }
 
 cqg_status cqg_mlp_adam_dev(float *w, const float *g, float *m1, float *m2, long long n, const float *hyper,
                             float b1, float b2, float eps, float weight_decay, void *wbf, void *stream) {
-  if (!hyper) return CQG_ERR_BAD_ARG;
-  return cqg_mlp_adam_tensors(1, &w, &g, &m1, &m2, &n, &weight_decay, &wbf, hyper, 0.f, b1, b2, eps, 0, stream);
+  if (n <= 0 || !hyper) return CQG_ERR_BAD_ARG;
+  k_adam_dev<<<nblk(n, 256), 256, 0, (cudaStream_t)stream>>>(w, g, m1, m2, n, hyper, b1, b2, eps, weight_decay,
+                                                             (__nv_bfloat16 *)wbf);
+  return cudaGetLastError() == cudaSuccess ? CQG_OK : CQG_ERR_CUDA;
 }
 
 cqg_status cqg_mlp_forward(int nl, const int *dims, int M, const void *X, const void *const *W, const float *const *b,
@@ -760,94 +644,6 @@ cqg_status cqg_mlp_forward(int nl, const int *dims, int M, const void *X, const 
     h = Y[i];
   }
   return CQG_OK;
-}
-
-cqg_status cqg_mlp_backward(int nl, const int *dims, int M, const float *dout, const void *const *H,
-                            const float *const *Z, const void *const *W, void *dZ0, void *dZ1, float *dX,
-                            float *grads, void *stream) {
-  if (nl <= 0 || !dims || M < 0 || !dout || !H || !Z || !W || !dZ0 || !dZ1 || !dX || !grads) return CQG_ERR_BAD_ARG;
-  if ((M + GM - 1) / GM > 65535) return CQG_ERR_BAD_ARG;   // as cqg_mlp_gemm_bf16
-  cudaStream_t st = (cudaStream_t)stream;
-  long long nw = 0, nb = 0;
-  for (int i = 0; i < nl; ++i) {
-    if (dims[i] <= 0 || dims[i + 1] <= 0) return CQG_ERR_BAD_ARG;
-    nw += (long long)dims[i] * dims[i + 1];
-    nb += dims[i + 1];
-  }
-  // weight gradients of the layers, then bias gradients: all are added into zeros
-  if (cudaMemsetAsync(grads, 0, (size_t)(nw + nb) * sizeof(float), st) != cudaSuccess) return CQG_ERR_CUDA;
-  if (M == 0) return CQG_OK;
-  float *gw = grads + nw, *gb = grads + nw + nb;
-  __nv_bfloat16 *dZ = (__nv_bfloat16 *)dZ0, *next = (__nv_bfloat16 *)dZ1;
-  auto launch_dz = [&](const float *dY, const float *z, __nv_bfloat16 *out, int N) {
-    k_dz_colsum<<<dim3((M + kColRows - 1) / kColRows, (N + 31) / 32), 256, 0, st>>>(dY, z, nullptr, out, M, N, gb);
-  };
-  const int nout = dims[nl];
-  gb -= nout;
-  if ((nout + 31) / 32 > 65535) return CQG_ERR_BAD_ARG;
-  launch_dz(dout, nullptr, dZ, nout);
-  // a weight gradient waits for the next one, and both go in one launch: their blocks together
-  // fill the GPU, and each dZ stays until the launch after that
-  Gemm waiting = {};
-  bool waits = false;
-  for (int i = nl - 1; i >= 0; --i) {
-    const int K = dims[i], N = dims[i + 1];
-    gw -= (long long)K * N;
-    // dW[n][k] = sum_m dZ[m][n] h[m][k]
-    Gemm w = gemm_of(dZ, 1, N, H[i], 1, K, gw, K, N, K, M);
-    w.accumulate = 1;
-    set_pairs(w);
-    const bool wbig = big_tiles(N, K);
-    tile_by(w, wbig ? GM : 64, wbig ? GN : 64);
-    if (!wbig) split_k(w);
-    cqg_status s = CQG_OK;
-    if (wbig) {
-      if (waits) s = launch_small(waiting, nullptr, st);
-      waits = false;
-      if (s == CQG_OK) s = launch_big(w, st);
-    } else if (waits) {
-      s = launch_small(waiting, &w, st);
-      waits = false;
-    } else {
-      waiting = w;
-      waits = true;
-    }
-    if (s == CQG_OK && i > 0) {
-      // dh[m][k] = sum_n dZ[m][n] W[n][k], through the SiLU of the layer below: the next dZ
-      gb -= K;
-      const int part = big_tiles(M, K) ? 0 : k_parts(M, K, N, 2 * GK);
-      if (part > 0) {
-        if (cudaMemsetAsync(dX, 0, (size_t)M * K * sizeof(float), st) != cudaSuccess) return CQG_ERR_CUDA;
-        const dim3 grid((K + kPartTile - 1) / kPartTile, (M + kPartTile - 1) / kPartTile, (N + part - 1) / part);
-        k_gemm_parts<<<grid, 128, 0, st>>>(dZ, N, 1, (const __nv_bfloat16 *)W[i], 1, K, dX, K, M, K, N, part);
-        launch_dz(dX, Z[i - 1], next, K);
-      } else {
-        Gemm x = gemm_of(dZ, N, 1, W[i], 1, K, nullptr, K, M, K, N);
-        x.dact = Z[i - 1];
-        x.Y = next;
-        x.ldy = K;
-        x.db = gb;
-        set_pairs(x);
-        const bool xbig = big_tiles(M, K);
-        tile_by(x, xbig ? GM : 64, xbig ? GN : 64);
-        if (xbig) {
-          s = launch_big(x, st);
-        } else if (waits) {
-          s = launch_small(x, &waiting, st);
-          waits = false;
-        } else {
-          s = launch_small(x, nullptr, st);
-        }
-      }
-    }
-    if (s != CQG_OK) return s;
-    std::swap(dZ, next);
-  }
-  if (waits) {
-    const cqg_status s = launch_small(waiting, nullptr, st);
-    if (s != CQG_OK) return s;
-  }
-  return cudaGetLastError() == cudaSuccess ? CQG_OK : CQG_ERR_CUDA;
 }
 
 }  // extern "C"

@@ -318,32 +318,44 @@ class PairMLP:
         layer, its BF16 input and FP32 pre-activation for the backward pass."""
         t = self.torch
         M, nl = Xbf.shape[0], len(self.W)
-        # the hidden layers, all of one width, in one allocation per type; without a backward
-        # pass one Z, which nothing reads, and two Y in turn serve them all
-        nh = nl - 1
-        nz, ny = (nh, nh) if keep else (min(nh, 1), min(nh, 2))
-        Z = t.empty((nz, M, self.dims[1]), dtype=t.float32, device=self.dev).unbind()
-        Y = t.empty((ny, M, self.dims[1]), dtype=t.bfloat16, device=self.dev).unbind()
-        Z, Y = [Z[i % nz] for i in range(nh)], [Y[i % ny] for i in range(nh)]
-        Z.append(t.empty((M, self.dims[-1]), dtype=t.float32, device=self.dev))
+        # without a backward pass one Z, which nothing reads, and two Y in turn serve the hidden
+        # layers, all of one width
+        Z, Y = [], []
+        for i, n in enumerate(self.dims[1:]):
+            last = i == nl - 1
+            Z.append(Z[0] if not keep and 0 < i and not last
+                     else t.empty((M, n), dtype=t.float32, device=self.dev))
+            Y.append(None if last else Y[i - 2] if not keep and i > 1
+                     else t.empty((M, n), dtype=t.bfloat16, device=self.dev))
         _lib.check(self.L.cqg_mlp_forward(nl, self._dims, M, self._p(Xbf), self._ps(self.Wbf), self._ps(self.b),
-                                          self._ps(Z), self._ps(Y + [None]), self._stream()))
-        return Z[-1], list(zip([Xbf] + Y, Z)) if keep else []
+                                          self._ps(Z), self._ps(Y), self._stream()))
+        return Z[-1], list(zip([Xbf] + Y[:-1], Z)) if keep else []
 
     def backward(self, dout, cache):
         """dout (M, maxf*maxf) FP32 = dLoss/dOutput -> FP32 weight and bias gradients."""
         t = self.torch
-        nl, M = len(self.W), cache[0][0].shape[0]
-        d = self.dims
-        sizes = [d[i] * d[i + 1] for i in range(nl)] + d[1:]
-        grads = t.empty(sum(sizes), dtype=t.float32, device=self.dev)
-        dZ = t.empty((2, M * max(d[1:]) + 7 & ~7), dtype=t.bfloat16, device=self.dev)
-        dX = t.empty(min(M * max(d[1:-1], default=1), _lib.MLP_DX_MAX), dtype=t.float32, device=self.dev)
-        _lib.check(self.L.cqg_mlp_backward(nl, self._dims, M, self._p(dout), self._ps([h for h, _ in cache]),
-                                           self._ps([z for _, z in cache]), self._ps(self.Wbf), self._p(dZ[0]),
-                                           self._p(dZ[1]), self._p(dX), self._p(grads), self._stream()))
-        g = grads.split(sizes)
-        return [x.view(n, -1) for x, n in zip(g, d[1:])], list(g[nl:])
+        nl = len(self.W)
+        gW, gb = [None] * nl, [None] * nl
+        dY = dout
+        for i in range(nl - 1, -1, -1):
+            h, Z = cache[i]
+            M, N, K = h.shape[0], self.dims[i + 1], self.dims[i]
+            dZ = t.empty((M, N), dtype=t.bfloat16, device=self.dev)
+            if i == nl - 1:
+                _lib.check(self.L.cqg_mlp_to_bf16(self._p(dY), self._p(dZ), M * N, self._stream()))
+            else:
+                _lib.check(self.L.cqg_mlp_silu_bwd(self._p(dY), self._p(Z), self._p(dZ), M * N, self._stream()))
+            gW[i] = t.empty((N, K), dtype=t.float32, device=self.dev)          # dW[n][k] = sum_m dZ[m][n] h[m][k]
+            _lib.check(self.L.cqg_mlp_gemm_bf16(self._p(dZ), 1, N, self._p(h), 1, K, self._p(gW[i]), K, N, K, M,
+                                                None, None, 0, 0, 0, self._stream()))
+            gb[i] = t.empty(N, dtype=t.float32, device=self.dev)
+            _lib.check(self.L.cqg_mlp_colsum(self._p(dZ), M, N, self._p(gb[i]), self._stream()))
+            if i > 0:                                                           # dX[m][k] = sum_n dZ[m][n] W[n][k]
+                dX = t.empty((M, K), dtype=t.float32, device=self.dev)
+                _lib.check(self.L.cqg_mlp_gemm_bf16(self._p(dZ), N, 1, self._p(self.Wbf[i]), 1, K, self._p(dX), K,
+                                                    M, K, N, None, None, 0, 0, 0, self._stream()))
+                dY = dX
+        return gW, gb
 
     def loss_grad(self, out, target, mask, inv_count: float):
         """Masked squared error sum * inv_count and its gradient."""
@@ -356,17 +368,13 @@ class PairMLP:
 
     def adam(self, gW, gb, lr: float, wd: float = 0.0):
         self.step += 1
-        self._adam(gW, gb, None, lr, wd)
-
-    def _adam(self, gW, gb, hyper, lr, wd):
-        """One launch for all weights and biases (the biases without weight decay)."""
-        nl = len(self.W)
-        n = (ctypes.c_longlong * (2 * nl))(*[x.numel() for x in self.W], *[x.numel() for x in self.b])
-        decay = (ctypes.c_float * (2 * nl))(*[wd] * nl)
-        _lib.check(self.L.cqg_mlp_adam_tensors(2 * nl, self._ps(self.W + self.b), self._ps(list(gW) + list(gb)),
-                                               self._ps(self.mW + self.mb), self._ps(self.vW + self.vb), n, decay,
-                                               self._ps(self.Wbf + [None] * nl), self._p(hyper), lr, 0.9, 0.999, 1e-8,
-                                               self.step, self._stream()))
+        for i in range(len(self.W)):
+            _lib.check(self.L.cqg_mlp_adam(self._p(self.W[i]), self._p(gW[i]), self._p(self.mW[i]),
+                                           self._p(self.vW[i]), self.W[i].numel(), lr, 0.9, 0.999, 1e-8, self.step,
+                                           wd, self._p(self.Wbf[i]), self._stream()))
+            _lib.check(self.L.cqg_mlp_adam(self._p(self.b[i]), self._p(gb[i]), self._p(self.mb[i]),
+                                           self._p(self.vb[i]), self.b[i].numel(), lr, 0.9, 0.999, 1e-8, self.step,
+                                           0.0, None, self._stream()))
 
     # ------------------------------------------------------------------ training ---
     def normalise_inputs(self, X: np.ndarray):
@@ -378,7 +386,13 @@ class PairMLP:
         """Adam step with {lr, 1 - b1^step, 1 - b2^step} read from the device tensor `hyper`
         (capturable in a CUDA graph); the host step counter advances as in :meth:`adam`."""
         self.step += 1
-        self._adam(gW, gb, hyper, 0.0, wd)
+        for i in range(len(self.W)):
+            _lib.check(self.L.cqg_mlp_adam_dev(self._p(self.W[i]), self._p(gW[i]), self._p(self.mW[i]),
+                                               self._p(self.vW[i]), self.W[i].numel(), self._p(hyper), 0.9, 0.999,
+                                               1e-8, wd, self._p(self.Wbf[i]), self._stream()))
+            _lib.check(self.L.cqg_mlp_adam_dev(self._p(self.b[i]), self._p(gb[i]), self._p(self.mb[i]),
+                                               self._p(self.vb[i]), self.b[i].numel(), self._p(hyper), 0.9, 0.999,
+                                               1e-8, 0.0, None, self._stream()))
 
     def fit(self, X, T, M, epochs: int = 40, batch: int = 2048, lr: float = 2e-3, seed: int = 0, log=None,
             graph: bool = True):

@@ -300,25 +300,12 @@ cqg_status cqg_mlp_adam_dev(float *w, const float *g, float *m1, float *m2, long
                             const float *hyper, float b1, float b2, float eps, float weight_decay,
                             void *wbf, void *stream);
 
-/* A whole pass per call.  dims: nl + 1 layer sizes; W[i] BF16 dims[i+1] x dims[i] (row-major).
- * cqg_mlp_forward: Z[i] = h_i W[i]^T + b[i] (FP32, M x dims[i+1]), h_{i+1} = Y[i] = SiLU(Z[i]) in BF16
- * for all but the last layer (Y[nl-1] is not used), h_0 = X (BF16, M x dims[0]).
- * cqg_mlp_backward: from dout = dLoss/dZ[nl-1] and the layers' inputs H[i] = h_i, the FP32
- * gradients, packed in `grads`: dW[0], ..., dW[nl-1], db[0], ..., db[nl-1].  dZ0 and dZ1
- * are scratch of M x max(dims[1..nl]) BF16 elements each, dX of min(M x max(dims[1..nl-1]),
- * CQG_MLP_DX_MAX) FP32 elements (one at least).
- * cqg_mlp_adam_tensors: the step of cqg_mlp_adam (hyper null) or cqg_mlp_adam_dev (hyper given)
- * for nt tensors, 16 per launch; w, g, m1, m2, n, weight_decay, wbf (entries may be null) have nt entries. */
-#define CQG_MLP_DX_MAX (148 * 64 * 64)
+/* The forward pass in one call.  dims: nl + 1 layer sizes; W[i] BF16 dims[i+1] x dims[i]
+ * (row-major).  Z[i] = h_i W[i]^T + b[i] (FP32, M x dims[i+1]), h_{i+1} = Y[i] = SiLU(Z[i]) in BF16
+ * for all but the last layer (Y[nl-1] is not used), h_0 = X (BF16, M x dims[0]).  Layers may
+ * share Z and, two apart, Y. */
 cqg_status cqg_mlp_forward(int nl, const int *dims, int M, const void *X, const void *const *W,
                            const float *const *b, float *const *Z, void *const *Y, void *stream);
-cqg_status cqg_mlp_backward(int nl, const int *dims, int M, const float *dout, const void *const *H,
-                            const float *const *Z, const void *const *W, void *dZ0, void *dZ1,
-                            float *dX, float *grads, void *stream);
-cqg_status cqg_mlp_adam_tensors(int nt, float *const *w, const float *const *g, float *const *m1,
-                                float *const *m2, const long long *n, const float *weight_decay,
-                                void *const *wbf, const float *hyper, float lr, float b1, float b2,
-                                float eps, int step, void *stream);
 
 /* FP64 / FP32 FMA throughput probe used to report roofline fractions: runs a dependent
  * FMA chain kernel for `ms_target` ms and returns achieved TFLOP/s in *tflops. */
